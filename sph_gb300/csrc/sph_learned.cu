@@ -10,9 +10,10 @@
 //   (k_relax_learned then applies the network's displacement and lists the
 //    particles that take the plain relaxation for k_relax_fallback)
 //
-// Training: a generic tcgen05 GEMM (strided BF16 operands staged in shared
-// memory, FP32 accumulation), bias/activation kernels, Adam on FP32 master
-// weights; sample collection and the calibration of the error output.
+// Training: k_train, the forward and backward pass of a batch on the tensor
+// cores (a tile of 128 samples at a time, weight gradients accumulated in
+// tensor memory), k_adam on FP32 master weights; sample collection and the
+// calibration of the error output.
 #include <algorithm>
 #include <cstddef>
 #include <cmath>
@@ -473,7 +474,7 @@ k_mlp(int n, const __nv_bfloat16 *__restrict__ feat, const __nv_bfloat16 *__rest
 }
 
 // ---------------------------------------------------------------------------
-// generic tcgen05 GEMM for training
+// generic tcgen05 GEMM (sph_learned_gemm_check)
 // ---------------------------------------------------------------------------
 
 // C[m][n] (ldc) = sum_k A(m, k) B(n, k), A(m, k) = A[m * sam + k * sak],
@@ -561,111 +562,342 @@ k_gemm(int M, int N, int K, const __nv_bfloat16 *__restrict__ A, long long sam, 
 }
 
 // ---------------------------------------------------------------------------
-// elementwise training kernels
+// training: one batch is two kernels
 // ---------------------------------------------------------------------------
 
-// Z (rows x cols, FP32 pre-activation without bias) -> Zb = Z + bf16(b)
-// (kept), H = act(Zb) = 2 GELU(Zb) in BF16, computed as the inference kernel
-// computes it (which adds the bias in BF16 through the tensor cores).  One
-// thread per pair of columns (cols even).
-__global__ void k_bias_act(int rows, int cols, float *__restrict__ Z, const float *__restrict__ b,
-                           __nv_bfloat16 *__restrict__ H)
+// Forward and backward pass of one batch, 128 samples at a time: a CTA
+// gathers a tile of samples, runs the three layers, the loss gradient and
+// the backward products with everything that passes between them in shared
+// memory, tensor memory or registers, and adds the tile's weight gradients
+// to accumulators that stay in tensor memory; at its end it writes its
+// partial gradients, which k_adam sums over the CTAs in their order.
+//
+// Why one kernel: a batch of 4,096 is 2.4e8 multiply-adds, about 1 us of one
+// SM's tensor core per tile, but as separate products its operands make
+// eight round trips through memory, and the weight gradients -- 4,096 deep
+// and at most 128 x 128 wide -- leave all but one SM idle.  What bounds a
+// tile here is the chain of its seven dependent products and their
+// epilogues.  A whole training step of 4,096 samples: 2.66 ms as separate
+// GEMMs and elementwise kernels, 20 us here (GB300).
+//
+// The transposed operands of the backward products (W2, W3 by rows; the
+// activations, gradients and features as M x K with K over the samples) are
+// MN-major views of the very tiles the forward pass staged.  The same
+// arithmetic as the inference kernel in the same K order: the activations
+// are bit for bit its own.
+constexpr int kTrainThreads = 512;
+constexpr uint32_t kTrainTmem = 512;
+// tensor memory columns
+constexpr uint32_t kColAcc = 0;     // the running product
+constexpr uint32_t kColW2 = 128;    // dW2 [h2][h1]
+constexpr uint32_t kColW1 = 256;    // dW1 [h1][in]
+constexpr uint32_t kColW3 = 288;    // dW3^T [h2][out]
+constexpr uint32_t kColB2 = 304;    // db2 [h2] in the first of 16 columns
+
+struct alignas(128) TrainSmem {
+    unsigned char w1[HID * IN * 2];
+    unsigned char w2[HID * HID * 2];
+    unsigned char w3[OUT * HID * 2];
+    unsigned char x[128 * IN * 2];
+    unsigned char h1[128 * HID * 2];   // activations, then dZ1
+    unsigned char h2[128 * HID * 2];   // activations, then dZ2
+    unsigned char dy[128 * OUT * 2];
+    unsigned char ones[128 * 16 * 2];  // column 0 = 1: column sums as a product
+    float b1[HID], b2[HID], b3[OUT];   // biases as the forward pass adds them
+    double loss[4];
+    float db3[4][4];
+    uint64_t mbar;
+    uint32_t taddr;
+};
+
+// A row-major BF16 matrix of `cols` columns into a K-major tile.
+__device__ __forceinline__ void stage_matrix(unsigned char *tile, const __nv_bfloat16 *__restrict__ w,
+                                             int rows, int cols)
 {
-    const long long e = 2 * ((long long)blockIdx.x * blockDim.x + threadIdx.x);
-    if (e >= (long long)rows * cols) return;
-    const int c = (int)(e % cols);
-    const float z0 = Z[e] + __bfloat162float(__float2bfloat16(b[c]));
-    const float z1 = Z[e + 1] + __bfloat162float(__float2bfloat16(b[c + 1]));
-    Z[e] = z0;
-    Z[e + 1] = z1;
-    *reinterpret_cast<uint32_t *>(H + e) = tc::act_bf16x2(z0, z1);
+    const int chunks = cols >> 3;
+    const uint4 *src = reinterpret_cast<const uint4 *>(w);
+    for (int e = threadIdx.x; e < rows * chunks; e += blockDim.x) {
+        const int r = e / chunks, k = e % chunks;
+        *reinterpret_cast<uint4 *>(tile + tc::kmajor_offset(r, 8 * k, cols)) = __ldcg(src + e);
+    }
 }
 
-// Y += b3; dY = mask * 2 (Y - T) / rows (BF16); the squared error is added to *loss.
-__global__ void k_out_grad(int rows, float *__restrict__ Y, const float *__restrict__ b3,
-                           const float4 *__restrict__ T, int cmask, __nv_bfloat16 *__restrict__ dY,
-                           double *__restrict__ loss)
+// Makes the CTA's shared-memory writes visible to the tensor core and joins
+// the CTA; false once any thread's wait has given up.
+__device__ __forceinline__ bool join_for_mma(bool ok)
 {
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    double l = 0.0;
-    if (r < rows) {
-        const float4 tt = T[r];
-        const float tv[4] = {tt.x, tt.y, tt.z, tt.w};
-        for (int c = 0; c < OUT; ++c) {
-            const float y = Y[r * OUT + c] + b3[c];
-            Y[r * OUT + c] = y;
-            float g = 0.0f;
-            if (c < 3 && ((cmask >> c) & 1)) {
-                const float d = y - tv[c];
-                l += (double)d * d;
-                g = 2.0f * d / (float)rows;
+    tc::fence_async_smem();
+    tc::fence_before_sync();
+    const bool all = __syncthreads_and(ok) != 0;
+    tc::fence_after_sync();
+    return all;
+}
+
+// cmask: outputs in the loss (bit 0, 1 displacement, bit 2 error); trunk =
+// false: the output layer's gradients alone.  part: gridDim.x x NPARAM
+// gradients, ploss: gridDim.x squared-error sums.
+__global__ void __launch_bounds__(kTrainThreads, 1)
+k_train(int tiles, const int *__restrict__ order, const __nv_bfloat16 *__restrict__ X,
+        const float4 *__restrict__ T, const __nv_bfloat16 *__restrict__ wbf,
+        const float *__restrict__ wf, int cmask, bool trunk, float *__restrict__ part,
+        double *__restrict__ ploss, unsigned *__restrict__ err)
+{
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    TrainSmem &s = *reinterpret_cast<TrainSmem *>(smem_raw);
+    const int t = threadIdx.x, w = t >> 5, lane = t & 31;
+    // a thread's share of an accumulator: one row, 32 columns
+    const int row = 32 * (w & 3) + lane, c0 = 32 * (w >> 2);
+    if (w == 0) {
+        tc::tmem_alloc(&s.taddr, kTrainTmem);
+        tc::tmem_relinquish();
+    }
+    if (t == 0) {
+        tc::mbar_init(&s.mbar, 1);
+        tc::mbar_fence_init();
+    }
+    for (int e = t; e < 128 * 16; e += kTrainThreads)
+        *reinterpret_cast<__nv_bfloat16 *>(s.ones + tc::kmajor_offset(e >> 4, e & 15, 16)) =
+            __float2bfloat16((e & 15) == 0 ? 1.0f : 0.0f);
+    // samples do not depend on the previous step; the weights do
+    const int first = blockIdx.x;
+    const int xr = t >> 2, xk = t & 3;  // the thread's 16-byte piece of a feature row
+    uint4 xv = make_uint4(0, 0, 0, 0);
+    float4 tv = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    auto load_tile = [&](int tile) {
+        xv = __ldg(reinterpret_cast<const uint4 *>(X + (size_t)__ldg(order + tile * 128 + xr) * IN) + xk);
+        if (w < 4) tv = __ldg(T + __ldg(order + tile * 128 + row));
+    };
+    load_tile(first);
+    pdl_enter();
+    stage_matrix(s.w1, wbf + OFF_W1, HID, IN);
+    stage_matrix(s.w2, wbf + OFF_W2, HID, HID);
+    stage_matrix(s.w3, wbf + OFF_W3, OUT, HID);
+    if (t < HID) {
+        s.b1[t] = __bfloat162float(__float2bfloat16(__ldcg(wf + OFF_B1 + t)));
+        s.b2[t] = __bfloat162float(__float2bfloat16(__ldcg(wf + OFF_B2 + t)));
+    }
+    if (t < OUT) s.b3[t] = __ldcg(wf + OFF_B3 + t);
+
+    const float rows_f = (float)(tiles * 128);
+    const uint32_t lane_base = (uint32_t)(32 * (w & 3)) << 16;
+    uint32_t tm = 0, phase = 0;
+    bool ok = true, any = false;
+    double loss = 0.0;
+    float db3[3] = {0.0f, 0.0f, 0.0f};
+    auto wait = [&]() {
+        const bool done = tc::mbar_wait(&s.mbar, phase);
+        phase ^= 1u;
+        tc::fence_after_sync();
+        return done;
+    };
+    // z = product + bias; the activations go to tile h, act'(z) to g
+    float g1[32], g2[32];
+    auto hidden = [&](unsigned char *h, const float *b, float (&g)[32]) {
+        float v[32];
+        tc::tmem_ld32(tm + kColAcc + lane_base + (uint32_t)c0, v);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            uint32_t o[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const int c = 8 * q + 2 * e;
+                const float z0 = v[c] + b[c0 + c], z1 = v[c + 1] + b[c0 + c + 1];
+                o[e] = tc::act_bf16x2(z0, z1);
+                g[c] = act_grad(z0);
+                g[c + 1] = act_grad(z1);
             }
-            dY[r * OUT + c] = __float2bfloat16(g);
+            *reinterpret_cast<uint4 *>(h + tc::kmajor_offset(row, c0 + 8 * q, HID)) =
+                make_uint4(o[0], o[1], o[2], o[3]);
         }
+    };
+    // dZ = dH act'(z) into tile h
+    auto back = [&](unsigned char *h, const float (&g)[32]) {
+        float v[32];
+        tc::tmem_ld32(tm + kColAcc + lane_base + (uint32_t)c0, v);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            uint32_t o[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const int c = 8 * q + 2 * e;
+                asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(o[e]) : "f"(v[c + 1] * g[c + 1]), "f"(v[c] * g[c]));
+            }
+            *reinterpret_cast<uint4 *>(h + tc::kmajor_offset(row, c0 + 8 * q, HID)) =
+                make_uint4(o[0], o[1], o[2], o[3]);
+        }
+    };
+    const uint32_t aw1 = tc::smem_u32(s.w1), aw2 = tc::smem_u32(s.w2), aw3 = tc::smem_u32(s.w3),
+                   ax = tc::smem_u32(s.x), ah1 = tc::smem_u32(s.h1), ah2 = tc::smem_u32(s.h2),
+                   ady = tc::smem_u32(s.dy), aones = tc::smem_u32(s.ones);
+    for (int tile = first; tile < tiles; tile += gridDim.x) {
+        *reinterpret_cast<uint4 *>(s.x + tc::kmajor_offset(xr, 8 * xk, IN)) = xv;
+        const float4 target = tv;
+        if (!join_for_mma(ok)) { ok = false; break; }
+        tm = s.taddr;
+        // layer 1
+        if (t == 0) {
+            tc::mma_operands(tm + kColAcc, tc::k_major(ax, IN), tc::k_major(aw1, IN), HID, IN, false);
+            tc::mma_commit(&s.mbar);
+        }
+        if (tile + (int)gridDim.x < tiles) load_tile(tile + gridDim.x);
+        ok = wait();
+        hidden(s.h1, s.b1, g1);
+        if (!join_for_mma(ok)) { ok = false; break; }
+        // layer 2
+        if (t == 0) {
+            tc::mma_operands(tm + kColAcc, tc::k_major(ah1, HID), tc::k_major(aw2, HID), HID, HID, false);
+            tc::mma_commit(&s.mbar);
+        }
+        ok = wait();
+        hidden(s.h2, s.b2, g2);
+        if (!join_for_mma(ok)) { ok = false; break; }
+        // layer 3
+        if (t == 0) {
+            tc::mma_operands(tm + kColAcc, tc::k_major(ah2, HID), tc::k_major(aw3, HID), OUT, HID, false);
+            tc::mma_commit(&s.mbar);
+        }
+        ok = wait();
+        if (w < 4) {
+            // dY = mask * 2 (Y - T) / rows
+            float y[16];
+            tc::tmem_ld16(tm + kColAcc + lane_base, y);
+            const float tt[3] = {target.x, target.y, target.z};
+            uint32_t d16[3];
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                float g = 0.0f;
+                if ((cmask >> c) & 1) {
+                    const float d = (y[c] + s.b3[c]) - tt[c];
+                    loss += (double)d * d;
+                    g = 2.0f * d / rows_f;
+                }
+                const __nv_bfloat16 gb = __float2bfloat16(g);
+                db3[c] += __bfloat162float(gb);
+                d16[c] = (uint32_t)__bfloat16_as_ushort(gb);
+            }
+            *reinterpret_cast<uint4 *>(s.dy + tc::kmajor_offset(row, 0, OUT)) =
+                make_uint4(d16[0] | (d16[1] << 16), d16[2], 0u, 0u);
+            *reinterpret_cast<uint4 *>(s.dy + tc::kmajor_offset(row, 8, OUT)) = make_uint4(0u, 0u, 0u, 0u);
+        }
+        if (!join_for_mma(ok)) { ok = false; break; }
+        // dW3^T = H2^T dY, dH2 = dY W3
+        if (t == 0) {
+            tc::mma_operands(tm + kColW3, tc::mn_major(ah2, HID), tc::mn_major(ady, OUT), OUT, 128, any);
+            if (trunk)
+                tc::mma_operands(tm + kColAcc, tc::k_major(ady, OUT), tc::mn_major(aw3, HID), HID, OUT, false);
+            tc::mma_commit(&s.mbar);
+        }
+        ok = wait();
+        if (trunk) {
+            back(s.h2, g2);
+            if (!join_for_mma(ok)) { ok = false; break; }
+            // dH1 = dZ2 W2, dW2 = dZ2^T H1, db2 = dZ2^T 1
+            if (t == 0) {
+                tc::mma_operands(tm + kColAcc, tc::k_major(ah2, HID), tc::mn_major(aw2, HID), HID, HID, false);
+                tc::mma_operands(tm + kColW2, tc::mn_major(ah2, HID), tc::mn_major(ah1, HID), HID, 128, any);
+                tc::mma_operands(tm + kColB2, tc::mn_major(ah2, HID), tc::mn_major(aones, 16), 16, 128, any);
+                tc::mma_commit(&s.mbar);
+            }
+            ok = wait();
+            back(s.h1, g1);
+            if (!join_for_mma(ok)) { ok = false; break; }
+            // dW1 = dZ1^T X
+            if (t == 0) {
+                tc::mma_operands(tm + kColW1, tc::mn_major(ah1, HID), tc::mn_major(ax, IN), IN, 128, any);
+                tc::mma_commit(&s.mbar);
+            }
+            ok = wait();
+        }
+        any = true;
+        // the tile's buffers are free again once every thread is past its
+        // wait: the next tile's join follows its feature store, so the store
+        // itself must wait here
+        if (!join_for_mma(ok)) { ok = false; break; }
     }
-    // block reduction of the loss
-    __shared__ double sh[32];
-    for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
-    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = l;
+    if (ok) {
+        float *p = part + (size_t)blockIdx.x * NPARAM;
+        if (trunk) {
+            float v[32];
+            tc::tmem_ld32(tm + kColW2 + lane_base + (uint32_t)c0, v);
+            float4 *d = reinterpret_cast<float4 *>(p + OFF_W2 + row * HID + c0);
+#pragma unroll
+            for (int q = 0; q < 8; ++q) d[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+            if (w < 4) {
+                tc::tmem_ld32(tm + kColW1 + lane_base, v);
+                float4 *d1 = reinterpret_cast<float4 *>(p + OFF_W1 + row * IN);
+#pragma unroll
+                for (int q = 0; q < 8; ++q)
+                    d1[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+            } else if (w < 8) {
+                float u[16];
+                tc::tmem_ld16(tm + kColB2 + lane_base, u);
+                p[OFF_B2 + row] = u[0];
+            }
+        }
+        if (w >= 8 && w < 12) {
+            float u[16];
+            tc::tmem_ld16(tm + kColW3 + lane_base, u);
+#pragma unroll
+            for (int o = 0; o < OUT; ++o) p[OFF_W3 + o * HID + row] = u[o];
+        }
+        if (w < 4) {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                loss += __shfl_xor_sync(0xffffffffu, loss, o);
+#pragma unroll
+                for (int c = 0; c < 3; ++c) db3[c] += __shfl_xor_sync(0xffffffffu, db3[c], o);
+            }
+            if (lane == 0) {
+                s.loss[w] = loss;
+                for (int c = 0; c < 3; ++c) s.db3[w][c] = db3[c];
+            }
+        }
+    } else if (t == 0) {
+        atomicAdd(err, 1u);
+    }
+    tc::fence_before_sync();
     __syncthreads();
-    if (threadIdx.x == 0) {
-        double s = 0.0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) s += sh[w];
-        atomicAdd(loss, s);
-    }
+    if (ok && t < OUT)
+        part[(size_t)blockIdx.x * NPARAM + OFF_B3 + t] =
+            t < 3 ? s.db3[0][t] + s.db3[1][t] + s.db3[2][t] + s.db3[3][t] : 0.0f;
+    if (ok && t == 0) ploss[blockIdx.x] = s.loss[0] + s.loss[1] + s.loss[2] + s.loss[3];
+    if (w == 0) tc::tmem_dealloc(s.taddr, kTrainTmem);
 }
 
-// dZ = dH * act'(Zb) (BF16 out).
-__global__ void k_act_back(int rows, int cols, const float *__restrict__ dH,
-                            const float *__restrict__ Zb, __nv_bfloat16 *__restrict__ dZ)
+// Sums the CTAs' partial gradients in their order, then Adam on the FP32
+// master weights and their BF16 copies; the batch's squared error is added
+// to *loss.  trunk = false: the output layer's rows of cmask alone.  The
+// first layer's bias has no gradient: it acts through the weight of the
+// constant feature 31.
+__global__ void __launch_bounds__(128)
+k_adam(int parts, const float *__restrict__ part, const double *__restrict__ ploss,
+       float *__restrict__ w, float *__restrict__ m, float *__restrict__ v, int cmask, bool trunk,
+       float lr, float b1t, float b2t, __nv_bfloat16 *__restrict__ wbf, double *__restrict__ loss)
 {
-    const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= (long long)rows * cols) return;
-    dZ[e] = __float2bfloat16(dH[e] * act_grad(Zb[e]));
-}
-
-// Column sums of a BF16 matrix (bias gradients), one thread per column.
-__global__ void k_colsum(int rows, int cols, const __nv_bfloat16 *__restrict__ D,
-                         float *__restrict__ out)
-{
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= cols) return;
-    float s = 0.0f;
-    for (int r = 0; r < rows; ++r) s += __bfloat162float(D[(size_t)r * cols + c]);
-    out[c] = s;
-}
-
-// Adam on the FP32 master weights (where `mask` is set), then BF16 copies.
-__global__ void k_adam(int n, float *__restrict__ w, const float *__restrict__ g,
-                       float *__restrict__ m, float *__restrict__ v, const unsigned char *mask,
-                       float lr, float b1t, float b2t, __nv_bfloat16 *__restrict__ wbf)
-{
+    pdl_enter();
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= n) return;
-    if (!mask || mask[e]) {
-        const float gg = g[e];
-        const float mm = 0.9f * m[e] + 0.1f * gg;
-        const float vv = 0.999f * v[e] + 0.001f * gg * gg;
+    if (e == 0) {
+        double a = 0.0;
+        for (int c = 0; c < parts; ++c) a += __ldcg(ploss + c);
+        *loss += a;
+    }
+    if (e >= NPARAM) return;
+    bool train = trunk;
+    if (!trunk && e >= OFF_W3)
+        train = (cmask >> (e >= OFF_B3 ? e - OFF_B3 : (e - OFF_W3) / HID)) & 1;
+    if (train) {
+        float g = 0.0f;
+        if (e < OFF_B1 || e >= OFF_W2) {
+#pragma unroll 8
+            for (int c = 0; c < parts; ++c) g += __ldcg(part + (size_t)c * NPARAM + e);
+        }
+        const float mm = 0.9f * m[e] + 0.1f * g;
+        const float vv = 0.999f * v[e] + 0.001f * g * g;
         m[e] = mm;
         v[e] = vv;
         w[e] -= lr * (mm / (1.0f - b1t)) / (sqrtf(vv / (1.0f - b2t)) + 1e-8f);
     }
     wbf[e] = __float2bfloat16(w[e]);
-}
-
-// Gathers a batch of rows of the sample set.
-__global__ void k_gather_rows(int rows, const int *__restrict__ idx,
-                              const __nv_bfloat16 *__restrict__ X, const float4 *__restrict__ T,
-                              __nv_bfloat16 *__restrict__ Xb, float4 *__restrict__ Tb)
-{
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= rows) return;
-    const int s = idx[r];
-    const uint4 *src = reinterpret_cast<const uint4 *>(X + (size_t)s * IN);
-    uint4 *dst = reinterpret_cast<uint4 *>(Xb + (size_t)r * IN);
-#pragma unroll
-    for (int q = 0; q < IN / 8; ++q) dst[q] = src[q];
-    Tb[r] = T[s];
 }
 
 __global__ void k_f32_to_bf16(int n, const float *__restrict__ in, __nv_bfloat16 *__restrict__ out)
@@ -774,7 +1006,7 @@ __global__ void k_wait_selftest(unsigned *__restrict__ gave_up)
 // The learned-relaxation model.
 struct LearnedModel {
     float *w = nullptr;         // FP32 master weights (device)
-    float *g = nullptr, *m = nullptr, *v = nullptr;
+    float *m = nullptr, *v = nullptr;
     __nv_bfloat16 *wbf = nullptr;
     int adam_t = 0;
     // samples
@@ -784,6 +1016,13 @@ struct LearnedModel {
     int nsamples = 0, cap = 0;
     unsigned calls = 0;
     unsigned *d_err = nullptr;
+    // training workspace, kept between calls: partial gradients and squared
+    // errors of a step's CTAs, the epoch's running sum (the last of `loss`),
+    // the epoch's sample order
+    float *part = nullptr;
+    double *loss = nullptr;
+    int *order = nullptr;
+    int parts_cap = 0, order_cap = 0;
     cudaStream_t stream = nullptr;
     unsigned long long seed = 0;
 };
@@ -805,6 +1044,7 @@ namespace {
 inline int nblk(long long n, int bs = 256) { return (int)((n + bs - 1) / bs); }
 
 size_t mlp_smem() { return sizeof(ml::MlpSmem) + 1024; }
+size_t train_smem() { return sizeof(ml::TrainSmem) + 1024; }
 // At least 60 KB, so that at most three GEMM CTAs (3 x 128 TMEM columns)
 // share an SM.
 size_t gemm_smem() { return std::max(sizeof(ml::GemmSmem) + 1024, (size_t)60 * 1024); }
@@ -814,6 +1054,7 @@ int configure_kernels()
     static bool done = false;
     if (done) return SPH_OK;
     LCUDA(cudaFuncSetAttribute(ml::k_mlp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mlp_smem()));
+    LCUDA(cudaFuncSetAttribute(ml::k_train, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)train_smem()));
     LCUDA(cudaFuncSetAttribute(ml::k_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gemm_smem()));
     done = true;
     return SPH_OK;
@@ -827,6 +1068,25 @@ int gemm(cudaStream_t st, int M, int N, int K, const __nv_bfloat16 *A, long long
     dim3 grid((M + 127) / 128, (N + BN - 1) / BN);
     ml::k_gemm<<<grid, 128, gemm_smem(), st>>>(M, N, K, A, sam, sak, B, sbn, sbk, C, ldc, BN, err);
     return cuda_fail(cudaGetLastError(), "gemm launch");
+}
+
+// A launch that may start while its predecessor's last CTAs still run; the
+// kernel waits for the predecessor's results in pdl_enter.
+template <typename... KArgs, typename... Args>
+void launch_pdl(void (*kern)(KArgs...), int grid, int block, size_t smem, cudaStream_t stream,
+                Args... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    (void)cudaLaunchKernelEx(&cfg, kern, args...);
 }
 
 int check_err(LearnedModel *l)
@@ -849,91 +1109,44 @@ int num_sms()
     return sms > 0 ? sms : 1;
 }
 
-// Training buffers for one batch size.
-struct TrainBufs {
-    int B = 0;
-    __nv_bfloat16 *Xb = nullptr, *H1 = nullptr, *H2 = nullptr, *dY = nullptr, *dZ2 = nullptr,
-                  *dZ1 = nullptr;
-    float4 *Tb = nullptr;
-    float *Z1 = nullptr, *Z2 = nullptr, *Y = nullptr, *dH2 = nullptr, *dH1 = nullptr;
-    int *idx = nullptr;
-    double *loss = nullptr;
-    unsigned char *mask = nullptr;
-    std::vector<void *> all;
-    template <class T>
-    int alloc(T **p, size_t n)
-    {
-        if (cudaMalloc((void **)p, n * sizeof(T)) != cudaSuccess) {
-            set_error("cudaMalloc for training buffers failed");
-            return SPH_ERR_ALLOC;
-        }
-        all.push_back(*p);
-        return SPH_OK;
-    }
-    ~TrainBufs()
-    {
-        for (void *p : all) cudaFree(p);
-    }
-};
-
-int make_bufs(TrainBufs &b, int B)
+// The training workspace for steps of `parts` CTAs and `rows` samples an epoch.
+int ensure_training(LearnedModel *l, int parts, int rows)
 {
-    using namespace ml;
-    b.B = B;
-    LTRY(b.alloc(&b.Xb, (size_t)B * IN));
-    LTRY(b.alloc(&b.Tb, (size_t)B));
-    LTRY(b.alloc(&b.Z1, (size_t)B * HID));
-    LTRY(b.alloc(&b.H1, (size_t)B * HID));
-    LTRY(b.alloc(&b.Z2, (size_t)B * HID));
-    LTRY(b.alloc(&b.H2, (size_t)B * HID));
-    LTRY(b.alloc(&b.Y, (size_t)B * OUT));
-    LTRY(b.alloc(&b.dY, (size_t)B * OUT));
-    LTRY(b.alloc(&b.dH2, (size_t)B * HID));
-    LTRY(b.alloc(&b.dZ2, (size_t)B * HID));
-    LTRY(b.alloc(&b.dH1, (size_t)B * HID));
-    LTRY(b.alloc(&b.dZ1, (size_t)B * HID));
-    LTRY(b.alloc(&b.idx, (size_t)B));
-    LTRY(b.alloc(&b.loss, (size_t)nblk(B) + 1));
-    LTRY(b.alloc(&b.mask, (size_t)NPARAM));
+    if (parts > l->parts_cap) {
+        cudaFree(l->part);
+        cudaFree(l->loss);
+        l->part = nullptr;
+        l->loss = nullptr;
+        l->parts_cap = 0;
+        LCUDA(cudaMalloc(&l->part, (size_t)parts * ml::NPARAM * sizeof(float)));
+        LCUDA(cudaMalloc(&l->loss, ((size_t)parts + 1) * sizeof(double)));
+        l->parts_cap = parts;
+    }
+    if (rows > l->order_cap) {
+        cudaFree(l->order);
+        l->order = nullptr;
+        l->order_cap = 0;
+        LCUDA(cudaMalloc(&l->order, (size_t)rows * sizeof(int)));
+        l->order_cap = rows;
+    }
     return SPH_OK;
 }
 
-// One forward + backward + Adam step on the batch in b.Xb / b.Tb.
-// cmask: outputs in the loss (bit 0, 1 displacement, bit 2 error);
-// trunk = false trains the output layer only.
-int train_batch(LearnedModel *l, TrainBufs &b, int cmask, bool trunk, float lr)
+// One forward + backward + Adam step on the samples order[0..batch) (batch a
+// multiple of 128).  cmask: outputs in the loss; trunk = false trains the
+// output layer only.
+int train_batch(LearnedModel *l, const int *order, int batch, int parts, int cmask, bool trunk,
+                float lr)
 {
     using namespace ml;
-    cudaStream_t st = l->stream;
-    const int B = b.B;
-    const __nv_bfloat16 *W1 = l->wbf + OFF_W1, *W2 = l->wbf + OFF_W2, *W3 = l->wbf + OFF_W3;
-    // forward
-    LTRY(gemm(st, B, HID, IN, b.Xb, IN, 1, W1, IN, 1, b.Z1, HID, l->d_err));
-    k_bias_act<<<nblk((long long)B * HID / 2), 256, 0, st>>>(B, HID, b.Z1, l->w + OFF_B1, b.H1);
-    LTRY(gemm(st, B, HID, HID, b.H1, HID, 1, W2, HID, 1, b.Z2, HID, l->d_err));
-    k_bias_act<<<nblk((long long)B * HID / 2), 256, 0, st>>>(B, HID, b.Z2, l->w + OFF_B2, b.H2);
-    LTRY(gemm(st, B, OUT, HID, b.H2, HID, 1, W3, HID, 1, b.Y, OUT, l->d_err));
-    k_out_grad<<<nblk(B), 256, 0, st>>>(B, b.Y, l->w + OFF_B3, b.Tb, cmask, b.dY, b.loss);
-    // backward: output layer
-    LCUDA(cudaMemsetAsync(l->g, 0, NPARAM * sizeof(float), st));
-    // dW3[o][h] = sum_b dY[b][o] H2[b][h]
-    LTRY(gemm(st, OUT, HID, B, b.dY, 1, OUT, b.H2, 1, HID, l->g + OFF_W3, HID, l->d_err));
-    k_colsum<<<1, OUT, 0, st>>>(B, OUT, b.dY, l->g + OFF_B3);
-    if (trunk) {
-        // dH2[b][h] = sum_o dY[b][o] W3[o][h]
-        LTRY(gemm(st, B, HID, OUT, b.dY, OUT, 1, W3, 1, HID, b.dH2, HID, l->d_err));
-        k_act_back<<<nblk((long long)B * HID), 256, 0, st>>>(B, HID, b.dH2, b.Z2, b.dZ2);
-        LTRY(gemm(st, HID, HID, B, b.dZ2, 1, HID, b.H1, 1, HID, l->g + OFF_W2, HID, l->d_err));
-        k_colsum<<<1, HID, 0, st>>>(B, HID, b.dZ2, l->g + OFF_B2);
-        LTRY(gemm(st, B, HID, HID, b.dZ2, HID, 1, W2, 1, HID, b.dH1, HID, l->d_err));
-        k_act_back<<<nblk((long long)B * HID), 256, 0, st>>>(B, HID, b.dH1, b.Z1, b.dZ1);
-        LTRY(gemm(st, HID, IN, B, b.dZ1, 1, HID, b.Xb, 1, IN, l->g + OFF_W1, IN, l->d_err));
-        // b1 stays zero: the first layer's bias is the weight of the constant feature 31
-    }
+    launch_pdl(k_train, parts, kTrainThreads, train_smem(), l->stream, batch / 128, order,
+               (const __nv_bfloat16 *)l->X, (const float4 *)l->T, (const __nv_bfloat16 *)l->wbf,
+               (const float *)l->w, cmask, trunk, l->part, l->loss, l->d_err);
     ++l->adam_t;
     const float b1t = powf(0.9f, (float)l->adam_t), b2t = powf(0.999f, (float)l->adam_t);
-    k_adam<<<nblk(NPARAM), 256, 0, st>>>(NPARAM, l->w, l->g, l->m, l->v, trunk ? nullptr : b.mask,
-                                         lr, b1t, b2t, l->wbf);
+    launch_pdl(k_adam, nblk(NPARAM, 128), 128, 0, l->stream, parts, (const float *)l->part,
+               (const double *)l->loss, l->w, l->m, l->v, cmask, trunk, lr, b1t, b2t, l->wbf,
+               l->loss + l->parts_cap);
     return cuda_fail(cudaGetLastError(), "training step");
 }
 
@@ -946,22 +1159,13 @@ int train_loop(LearnedModel *l, int first, int nsamples, int epochs, int batch, 
         set_error("%d training samples: at least 128 are needed", nsamples);
         return SPH_ERR_STATE;
     }
+    LTRY(configure_kernels());
     batch = std::max(128, std::min(batch, nsamples) / 128 * 128);
     const int per_epoch = nsamples / batch;
-    TrainBufs b;
-    LTRY(make_bufs(b, batch));
-    int *d_order = nullptr;
-    LTRY(b.alloc(&d_order, (size_t)per_epoch * batch));
-    if (!trunk) {
-        std::vector<unsigned char> mask(NPARAM, 0);
-        for (int o = 0; o < OUT; ++o)
-            if ((cmask >> o) & 1) {
-                for (int h = 0; h < HID; ++h) mask[OFF_W3 + o * HID + h] = 1;
-                mask[OFF_B3 + o] = 1;
-            }
-        LCUDA(cudaMemcpyAsync(b.mask, mask.data(), NPARAM, cudaMemcpyHostToDevice, l->stream));
-        LCUDA(cudaStreamSynchronize(l->stream));
-    }
+    // a CTA per tile of 128 samples, at most one per SM
+    const int parts = std::min(batch / 128, num_sms());
+    LTRY(ensure_training(l, parts, per_epoch * batch));
+    double *d_loss = l->loss + l->parts_cap;
     std::vector<int> order(nsamples);
     for (int i = 0; i < nsamples; ++i) order[i] = first + i;
     unsigned long long rng = l->seed * 0x9E3779B97F4A7C15ull + 17ull + (unsigned long long)l->adam_t;
@@ -975,16 +1179,13 @@ int train_loop(LearnedModel *l, int first, int nsamples, int epochs, int batch, 
     double last = 0.0;
     for (int ep = 0; ep < epochs; ++ep) {
         for (int i = nsamples - 1; i > 0; --i) std::swap(order[i], order[(int)(next() % (i + 1))]);
-        LCUDA(cudaMemcpyAsync(d_order, order.data(), (size_t)per_epoch * batch * sizeof(int),
+        LCUDA(cudaMemcpyAsync(l->order, order.data(), (size_t)per_epoch * batch * sizeof(int),
                               cudaMemcpyHostToDevice, l->stream));
-        LCUDA(cudaMemsetAsync(b.loss, 0, sizeof(double), l->stream));
-        for (int it = 0; it < per_epoch; ++it) {
-            ml::k_gather_rows<<<nblk(batch), 256, 0, l->stream>>>(
-                batch, d_order + (size_t)it * batch, l->X, l->T, b.Xb, b.Tb);
-            LTRY(train_batch(l, b, cmask, trunk, lr));
-        }
+        LCUDA(cudaMemsetAsync(d_loss, 0, sizeof(double), l->stream));
+        for (int it = 0; it < per_epoch; ++it)
+            LTRY(train_batch(l, l->order + (size_t)it * batch, batch, parts, cmask, trunk, lr));
         double acc = 0.0;
-        LCUDA(cudaMemcpyAsync(&acc, b.loss, sizeof(double), cudaMemcpyDeviceToHost, l->stream));
+        LCUDA(cudaMemcpyAsync(&acc, d_loss, sizeof(double), cudaMemcpyDeviceToHost, l->stream));
         LCUDA(cudaStreamSynchronize(l->stream));
         last = acc / ((double)per_epoch * batch);
     }
@@ -1122,7 +1323,6 @@ int sph_learned_create(sph_learned_t **out, int max_samples, unsigned long long 
     if (rc) return fail(rc);
     if ((rc = cuda_fail(cudaStreamCreateWithFlags(&l->stream, cudaStreamNonBlocking), "stream")) ||
         (rc = cuda_fail(cudaMalloc(&l->w, ml::NPARAM * sizeof(float)), "cudaMalloc")) ||
-        (rc = cuda_fail(cudaMalloc(&l->g, ml::NPARAM * sizeof(float)), "cudaMalloc")) ||
         (rc = cuda_fail(cudaMalloc(&l->m, ml::NPARAM * sizeof(float)), "cudaMalloc")) ||
         (rc = cuda_fail(cudaMalloc(&l->v, ml::NPARAM * sizeof(float)), "cudaMalloc")) ||
         (rc = cuda_fail(cudaMalloc(&l->wbf, ml::NPARAM * sizeof(__nv_bfloat16)), "cudaMalloc")) ||
@@ -1160,7 +1360,8 @@ int sph_learned_destroy(sph_learned_t *l)
 {
     if (!l) return SPH_OK;
     if (l->stream) cudaStreamSynchronize(l->stream);
-    void *ptrs[] = {l->w, l->g, l->m, l->v, l->wbf, l->d_err, l->X, l->T, l->slot};
+    void *ptrs[] = {l->w, l->m, l->v, l->wbf, l->d_err, l->X, l->T, l->slot, l->part,
+                    l->loss, l->order};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     if (l->stream) cudaStreamDestroy(l->stream);

@@ -219,6 +219,39 @@ __device__ __forceinline__ bool named_sync_and(int id, int count, bool v)
     return r != 0;
 }
 
+// An operand of tcgen05.mma in a tile staged with kmajor_offset (rows x
+// `cols`): as the matrix whose K runs along the tile's columns (K-major), or
+// along its rows (MN-major: the transposed matrix, read from the same tile).
+// The core matrix of 8 rows x 16 bytes is the same for both; only the two
+// strides change roles.  step: bytes from one K = 16 slice to the next.
+struct Operand {
+    uint32_t addr, lbo, sbo, step;
+    bool mn;
+};
+
+__device__ __forceinline__ Operand k_major(uint32_t addr, int cols)
+{
+    return {addr, (uint32_t)kCoreBytes, (uint32_t)(cols >> 3) * kCoreBytes, 2u * kCoreBytes, false};
+}
+
+__device__ __forceinline__ Operand mn_major(uint32_t addr, int cols)
+{
+    const uint32_t row = (uint32_t)(cols >> 3) * kCoreBytes;  // next 8 rows (8 of K)
+    return {addr, row, (uint32_t)kCoreBytes, 2u * row, true};
+}
+
+// D[128 x N] (+)= A[128 x K] . B[N x K]^T, K a multiple of 16; issued by one
+// thread, the caller commits.
+__device__ __forceinline__ void mma_operands(uint32_t tmem_d, const Operand &a, const Operand &b,
+                                             int N, int K, bool accumulate_first)
+{
+    const uint32_t idesc = idesc_bf16(128, N) | ((uint32_t)a.mn << 15) | ((uint32_t)b.mn << 16);
+    for (int k = 0; k < K / 16; ++k)
+        mma_bf16(tmem_d, smem_desc(a.addr + k * a.step, a.lbo, a.sbo),
+                 smem_desc(b.addr + k * b.step, b.lbo, b.sbo), idesc,
+                 (k > 0 || accumulate_first) ? 1u : 0u);
+}
+
 // D[128 x N] (+)= A[128 x K] . B[N x K]^T for operands staged in the
 // K-major layout at smem_a / smem_b (K a multiple of 16).  Issued by one
 // thread; the caller commits.

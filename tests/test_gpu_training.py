@@ -1,0 +1,91 @@
+"""The training kernels against a numpy restatement of the network's forward
+and backward pass and of Adam, at batches of one tile of 128 samples, of a
+few, and of more tiles than the GPU has SMs."""
+import numpy as np
+import pytest
+
+from sph_gb300 import LearnedModel, Simulation, scenes
+from test_gpu_learned import act_bf16, bf16
+
+pytestmark = pytest.mark.gpu
+
+
+def still_fluid(n, seed):
+    """A disordered block at rest without gravity or viscosity: its predicted
+    state is the state itself, so the samples' targets are the relaxation
+    displacements of the current positions."""
+    rng = np.random.default_rng(seed)
+    side = int(np.ceil(np.sqrt(n)))
+    i = np.arange(n)
+    x = (3.0 + 0.45 * (i % side) + rng.uniform(-0.15, 0.15, n)).astype(np.float32)
+    y = (3.0 + 0.45 * (i // side) + rng.uniform(-0.15, 0.15, n)).astype(np.float32)
+    size = int(np.ceil(0.45 * side)) + 6
+    p = scenes.Params(g=0.0, sigma=0.0, beta=0.0)
+    p.node_end_x = float(size)
+    z = np.zeros(n, np.float32)
+    return scenes.Scene(name="still", x=x, y=y, vx=z, vy=z.copy(), box=(0.0, float(size), 0.0, float(size)),
+                        params=p, spacing=1.0, size_x=size, size_y=size)
+
+
+def act_grad(z):
+    t = np.tanh(0.7978845608 * (z + 0.044715 * z ** 3))
+    return 1.0 + t + z * (1.0 - t * t) * 0.7978845608 * (1.0 + 0.134145 * z * z)
+
+
+def numpy_training(w, x, target, steps, lr):
+    """`steps` Adam steps on the whole of (x, target), operands rounded to
+    BF16 where the kernels round them, sums in 64 bits."""
+    r = lambda v: bf16(np.asarray(v, np.float32)).astype(np.float64)  # noqa: E731
+    p = {k: v.astype(np.float64).copy() for k, v in LearnedModel.unpack(w).items()}
+    m = {k: np.zeros_like(v) for k, v in p.items()}
+    v = {k: np.zeros_like(q) for k, q in p.items()}
+    losses = []
+    for t in range(1, steps + 1):
+        q = {k: r(a) for k, a in p.items()}
+        z1 = x @ q["W1"].T + q["b1"]
+        h1 = act_bf16(z1)
+        z2 = h1 @ q["W2"].T + q["b2"]
+        h2 = act_bf16(z2)
+        d = (h2 @ q["W3"].T + p["b3"])[:, :2] - target
+        losses.append(float((d * d).sum()) / len(x))
+        dy = np.zeros((len(x), LearnedModel.OUT))
+        dy[:, :2] = r(2.0 * d / len(x))
+        dz2 = r((dy @ q["W3"]) * act_grad(z2))
+        dz1 = r((dz2 @ q["W2"]) * act_grad(z1))
+        g = dict(W1=dz1.T @ x, b1=np.zeros(LearnedModel.HIDDEN), W2=dz2.T @ h1, b2=dz2.sum(0),
+                 W3=dy.T @ h2, b3=dy.sum(0))
+        for k in p:
+            m[k] = 0.9 * m[k] + 0.1 * g[k]
+            v[k] = 0.999 * v[k] + 0.001 * g[k] ** 2
+            p[k] -= lr * (m[k] / (1 - 0.9 ** t)) / (np.sqrt(v[k] / (1 - 0.999 ** t)) + 1e-8)
+    return np.concatenate([p[k].reshape(-1) for k in ("W1", "b1", "W2", "b2", "W3", "b3")]), losses
+
+
+@pytest.mark.parametrize("tiles", [1, 3, 157])
+def test_training_matches_numpy(cuda_lib, tiles):
+    rows, steps, lr = 128 * tiles, 3, 1e-3
+    sc = still_fluid(rows + 700, seed=tiles)
+    P = sc.params
+    with Simulation.from_scene(sc) as s, LearnedModel(rows, seed=2) as m:
+        f, count = s.learned_features()
+        dx, dy = s.probe_relaxation(P.as_dict())
+        assert m.collect(s) == rows  # the first rows eligible particles, in cell order
+        w0 = m.get_params()
+        w0 += np.random.default_rng(9).normal(0.0, 0.02, w0.shape).astype(np.float32)
+        m.set_params(w0)
+        losses = [m.train(1, rows, lr) for _ in range(steps)]  # one batch an epoch
+        w = m.get_params()
+    key = np.floor(sc.y).astype(np.int64) * sc.size_x + np.floor(sc.x).astype(np.int64)
+    order = np.argsort(key, kind="stable")
+    take = order[(count[order] >= 0) & (count[order] <= LearnedModel.MAX_NEIGHBORS)][:rows]
+    scale = P.smoothing_radius * P.time_step ** 2 * (P.k + P.k_near + P.k_spring)
+    target = np.stack([dx, dy], 1)[take].astype(np.float64) / scale
+    ref, ref_losses = numpy_training(w0, f[take].astype(np.float64), target, steps, lr)
+    # the kernels' tanh.approx differs from tanh by a BF16 unit (2^-8) here
+    # and there, so the gradients by a few 2^-8, and Adam moves a weight by
+    # lr times their normalised values: a wrong gradient is off by lr a step
+    assert np.allclose(losses, ref_losses, rtol=2e-2)
+    d = (w - ref) / (lr * steps)
+    assert np.sqrt(np.mean(d ** 2)) <= 0.05, np.sqrt(np.mean(d ** 2))
+    b1 = LearnedModel.unpack(w)["b1"]
+    assert np.array_equal(b1, LearnedModel.unpack(w0)["b1"])  # acts through the constant feature
