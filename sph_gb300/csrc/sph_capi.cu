@@ -9,6 +9,8 @@
 #include <cstring>
 #include <new>
 
+#include <unistd.h>
+
 #include "sph_internal.h"
 
 namespace sph {
@@ -81,6 +83,41 @@ static cudaError_t host_alloc(void **p, size_t bytes)
         }
     }
     return cudaHostAlloc(p, bytes, cudaHostAllocDefault);
+}
+
+static void touch_pages(char *p, size_t bytes, size_t page)
+{
+    if (bytes == 0) return;
+    *static_cast<volatile char *>(p) = 0;
+    for (uintptr_t a = ((uintptr_t)p / page + 1) * page; a < (uintptr_t)p + bytes; a += page)
+        *reinterpret_cast<volatile char *>(a) = 0;
+}
+
+PageToucher::PageToucher(void *p, size_t bytes)
+{
+    const long ps = sysconf(_SC_PAGESIZE);
+    const size_t page = ps > 0 ? (size_t)ps : 4096;
+    char *b = static_cast<char *>(p);
+    constexpr size_t kPerThread = (size_t)4 << 20;  // a thread costs about as much as 1 MB of faults
+    const int n = (int)std::min<size_t>(4, bytes / kPerThread);
+    size_t done = 0;
+    try {
+        threads_.reserve(4);
+        for (int k = 0; k < n; ++k) {
+            const size_t end = k == n - 1 ? bytes : bytes / n * (k + 1);
+            threads_.emplace_back(touch_pages, b + done, end - done, page);
+            done = end;
+        }
+    } catch (...) {  // no thread to be had: the rest is touched here
+    }
+    touch_pages(b + done, bytes - done, page);
+}
+
+void PageToucher::done()
+{
+    for (std::thread &t : threads_)
+        if (t.joinable()) t.join();
+    threads_.clear();
 }
 
 template <class T>

@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <thread>
 #include <vector>
 
 #include "sph_cuda.h"
@@ -204,6 +205,27 @@ inline Ctx make_ctx(const sph_cuda *h)
     c.maskx = h->long_masks ? h->maskx_c : nullptr;
     return c;
 }
+
+// Gives the pages of a caller's output buffer their memory before a
+// device-to-host copy overwrites ALL of it: a copy into pages that were
+// never touched takes its page faults from the GPU's side, 2 to 20 ms for
+// 32 MB against 0.2 ms into touched pages (GB300 with its Grace host).  A
+// touch is a plain store of 0 to a page: an access that reads first, atomics
+// included, maps the shared zero page, whose replacement then has to be
+// invalidated in the GPU's translations (10 ms for 32 MB).  Large buffers
+// are touched by a few threads beside whatever the caller does next (32 MB:
+// 1.1 ms on one thread, 0.4 ms on four).  done() must come before the copy.
+class PageToucher {
+public:
+    PageToucher(void *p, size_t bytes);
+    ~PageToucher() { done(); }
+    PageToucher(const PageToucher &) = delete;
+    PageToucher &operator=(const PageToucher &) = delete;
+    void done();
+
+private:
+    std::vector<std::thread> threads_;
+};
 
 // Core operations shared by the fast API and the legacy entry points.
 int ensure_scratch(sph_cuda *h, size_t bytes);

@@ -99,6 +99,7 @@ k_messages(Ctx c, const float4 *__restrict__ xr, const ulonglong2 *__restrict__ 
            const unsigned *__restrict__ occ_in, __nv_bfloat16 *__restrict__ feat,
            unsigned short *__restrict__ nbcount, unsigned *__restrict__ fb_count)
 {
+    pdl_enter();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i == 0 && fb_count) {  // both fallback counters of the step (fb_count, fb_long)
         fb_count[0] = 0u;
@@ -235,10 +236,10 @@ k_messages(Ctx c, const float4 *__restrict__ xr, const ulonglong2 *__restrict__ 
 #pragma unroll
     for (int q = 0; q < IN / 8; ++q) {
         uint4 v;
-        asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(v.x) : "f"(f[8 * q + 1]), "f"(f[8 * q + 0]));
-        asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(v.y) : "f"(f[8 * q + 3]), "f"(f[8 * q + 2]));
-        asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(v.z) : "f"(f[8 * q + 5]), "f"(f[8 * q + 4]));
-        asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(v.w) : "f"(f[8 * q + 7]), "f"(f[8 * q + 6]));
+        v.x = tc::pack_bf16x2(f[8 * q + 0], f[8 * q + 1]);
+        v.y = tc::pack_bf16x2(f[8 * q + 2], f[8 * q + 3]);
+        v.z = tc::pack_bf16x2(f[8 * q + 4], f[8 * q + 5]);
+        v.w = tc::pack_bf16x2(f[8 * q + 6], f[8 * q + 7]);
         row[q] = v;
     }
 }
@@ -291,32 +292,44 @@ static_assert(offsetof(MlpSmem, pipe) % 128 == 0 && sizeof(MlpPipe) % 128 == 0 &
               "pipeline tiles aligned");
 static_assert(sizeof(MlpSmem) + 1024 <= 227 * 1024, "fits the shared memory of one CTA");
 
+// A row-major BF16 matrix of `cols` columns into a K-major tile, 16 bytes
+// at a time.
+__device__ __forceinline__ void stage_matrix(unsigned char *tile, const __nv_bfloat16 *__restrict__ w,
+                                             int rows, int cols)
+{
+    const int chunks = cols >> 3;
+    const uint4 *src = reinterpret_cast<const uint4 *>(w);
+    for (int e = threadIdx.x; e < rows * chunks; e += blockDim.x) {
+        const int r = e / chunks, k = e % chunks;
+        *reinterpret_cast<uint4 *>(tile + tc::kmajor_offset(r, 8 * k, cols)) = __ldcg(src + e);
+    }
+}
+
+// The inference weights, in 16-byte pieces (with 2-byte ones this prologue
+// was 9 of the 13 us that a few rows took).
 __device__ __forceinline__ void stage_weights(MlpWeights &s, const __nv_bfloat16 *__restrict__ w,
                                               const float *__restrict__ wf)
 {
     const int t = threadIdx.x;
-    for (int e = t; e < HID * IN; e += blockDim.x) {
-        const int r = e / IN, k = e % IN;
-        const __nv_bfloat16 v =
-            k == IN - 1 ? __float2bfloat16(wf[OFF_W1 + e] + wf[OFF_B1 + r]) : w[OFF_W1 + e];
-        *reinterpret_cast<__nv_bfloat16 *>(s.w1 + tc::kmajor_offset(r, k, IN)) = v;
+    stage_matrix(s.w2, w + OFF_W2, HID, HID);
+    stage_matrix(s.w1, w + OFF_W1, HID, IN);
+    stage_matrix(s.w3, w + OFF_W3, OUT, HID);
+    const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+    for (int e = t; e < HID * 2; e += blockDim.x) {
+        const int r = e >> 1, k = 8 * (e & 1);
+        uint4 b = zero, o = zero;
+        if (k == 0) {
+            b.x = (uint32_t)__bfloat16_as_ushort(__float2bfloat16(__ldcg(wf + OFF_B2 + r)));
+            o.x = 0x3F80u;  // 1
+        }
+        *reinterpret_cast<uint4 *>(s.w2b + tc::kmajor_offset(r, k, 16)) = b;
+        *reinterpret_cast<uint4 *>(s.ones + tc::kmajor_offset(r, k, 16)) = o;
     }
-    for (int e = t; e < HID * HID; e += blockDim.x) {
-        const int r = e / HID, k = e % HID;
-        *reinterpret_cast<__nv_bfloat16 *>(s.w2 + tc::kmajor_offset(r, k, HID)) = w[OFF_W2 + e];
-    }
-    for (int e = t; e < HID * 16; e += blockDim.x) {
-        const int r = e / 16, k = e % 16;
-        *reinterpret_cast<__nv_bfloat16 *>(s.w2b + tc::kmajor_offset(r, k, 16)) =
-            __float2bfloat16(k == 0 ? wf[OFF_B2 + r] : 0.0f);
-        *reinterpret_cast<__nv_bfloat16 *>(s.ones + tc::kmajor_offset(r, k, 16)) =
-            __float2bfloat16(k == 0 ? 1.0f : 0.0f);
-    }
-    for (int e = t; e < OUT * HID; e += blockDim.x) {
-        const int r = e / HID, k = e % HID;
-        *reinterpret_cast<__nv_bfloat16 *>(s.w3 + tc::kmajor_offset(r, k, HID)) = w[OFF_W3 + e];
-    }
-    for (int e = t; e < OUT; e += blockDim.x) s.b3[e] = wf[OFF_B3 + e];
+    for (int e = t; e < OUT; e += blockDim.x) s.b3[e] = __ldcg(wf + OFF_B3 + e);
+    __syncthreads();  // column 31 of W1, staged above, takes the first bias
+    for (int r = t; r < HID; r += blockDim.x)
+        *reinterpret_cast<__nv_bfloat16 *>(s.w1 + tc::kmajor_offset(r, IN - 1, IN)) =
+            __float2bfloat16(__ldcg(wf + OFF_W1 + r * IN + IN - 1) + __ldcg(wf + OFF_B1 + r));
 }
 
 // Epilogue of a hidden layer in a pipeline: warp w (0..7 within it) takes
@@ -346,18 +359,31 @@ __device__ __forceinline__ void hidden_epilogue(unsigned char *hbuf, uint32_t ta
     }
 }
 
-// Half a feature row (16 BF16 = 32 bytes) of row tile*128 + (tp >> 1).
-__device__ __forceinline__ void load_feat(const __nv_bfloat16 *__restrict__ feat, int n, int tile,
-                                          int tp, uint4 &a, uint4 &b)
+// Half a feature row (16 values) of row tile*128 + (tp >> 1) as BF16: from
+// the step's BF16 rows, or (HOST_ROWS) from a caller's float rows.
+template <bool HOST_ROWS>
+__device__ __forceinline__ void load_feat(const void *__restrict__ feat, int n, int tile, int tp,
+                                          uint4 &a, uint4 &b)
 {
     const int gi = tile * 128 + (tp >> 1);
-    if (gi < n) {
-        const uint4 *src = reinterpret_cast<const uint4 *>(feat + (size_t)gi * IN) + 2 * (tp & 1);
+    a = make_uint4(0, 0, 0, 0);
+    b = a;
+    if (gi >= n) return;
+    if (!HOST_ROWS) {
+        const uint4 *src = reinterpret_cast<const uint4 *>(
+                               reinterpret_cast<const __nv_bfloat16 *>(feat) + (size_t)gi * IN) +
+                           2 * (tp & 1);
         a = __ldcs(src);
         b = __ldcs(src + 1);
     } else {
-        a = make_uint4(0, 0, 0, 0);
-        b = a;
+        const float4 *src = reinterpret_cast<const float4 *>(
+                                reinterpret_cast<const float *>(feat) + (size_t)gi * IN) +
+                            4 * (tp & 1);
+        const float4 f0 = __ldcs(src), f1 = __ldcs(src + 1), f2 = __ldcs(src + 2), f3 = __ldcs(src + 3);
+        a = make_uint4(tc::pack_bf16x2(f0.x, f0.y), tc::pack_bf16x2(f0.z, f0.w),
+                       tc::pack_bf16x2(f1.x, f1.y), tc::pack_bf16x2(f1.z, f1.w));
+        b = make_uint4(tc::pack_bf16x2(f2.x, f2.y), tc::pack_bf16x2(f2.z, f2.w),
+                       tc::pack_bf16x2(f3.x, f3.y), tc::pack_bf16x2(f3.z, f3.w));
     }
 }
 
@@ -369,10 +395,15 @@ __device__ __forceinline__ void store_feat(unsigned char *x, int tp, const uint4
 }
 
 // out[i] = (y0, y1, y2, 0) for n feature rows; tiles of 128 rows, pipeline
-// p of CTA b takes tiles (b kPipes + p) + k gridDim.x kPipes.  The next
-// tile's features are fetched while the current one runs.
+// p of CTA b takes tiles (p gridDim.x + b) + k gridDim.x kPipes: a few tiles
+// spread over as many SMs before a second pipeline of any starts.  The next
+// tile's features are fetched while the current one runs.  The weights are
+// staged before the wait for the predecessor: no kernel of a step writes
+// them.  HOST_ROWS: float rows in, rows of OUT floats (zeros after the
+// third) out.
+template <bool HOST_ROWS>
 __global__ void __launch_bounds__(kMlpThreads, 1)
-k_mlp(int n, const __nv_bfloat16 *__restrict__ feat, const __nv_bfloat16 *__restrict__ wbf,
+k_mlp(int n, const void *__restrict__ feat, const __nv_bfloat16 *__restrict__ wbf,
       const float *__restrict__ wf, float4 *__restrict__ out, unsigned *__restrict__ err)
 {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
@@ -392,10 +423,11 @@ k_mlp(int n, const __nv_bfloat16 *__restrict__ feat, const __nv_bfloat16 *__rest
     stage_weights(S.w, wbf, wf);
     const int ntiles = (n + 127) / 128;
     const int stride = gridDim.x * kPipes;
-    int tile = blockIdx.x * kPipes + p;
+    int tile = p * gridDim.x + blockIdx.x;
+    pdl_enter();
     {
         uint4 a, b;
-        load_feat(feat, n, tile, tp, a, b);
+        load_feat<HOST_ROWS>(feat, n, tile, tp, a, b);
         store_feat(P.x, tp, a, b);
     }
     tc::fence_async_smem();
@@ -418,7 +450,7 @@ k_mlp(int n, const __nv_bfloat16 *__restrict__ feat, const __nv_bfloat16 *__rest
         // tile: their DRAM latency hides behind the whole tile, not behind
         // layer 1 alone (6% off the kernel)
         uint4 na, nb;
-        load_feat(feat, n, tile + stride, tp, na, nb);
+        load_feat<HOST_ROWS>(feat, n, tile + stride, tp, na, nb);
         bool done = tc::mbar_wait(&P.mbar, phase);
         phase ^= 1u;
         tc::fence_after_sync();
@@ -457,8 +489,17 @@ k_mlp(int n, const __nv_bfloat16 *__restrict__ feat, const __nv_bfloat16 *__rest
             float v[16];
             tc::tmem_ld16(tacc + ((uint32_t)(32 * w) << 16), v);
             const int gi = tile * 128 + 32 * w + (tp & 31);
-            if (gi < n && done)
-                __stcs(out + gi, make_float4(v[0] + S.w.b3[0], v[1] + S.w.b3[1], v[2] + S.w.b3[2], 0.0f));
+            if (gi < n && done) {
+                const float4 y = make_float4(v[0] + S.w.b3[0], v[1] + S.w.b3[1], v[2] + S.w.b3[2], 0.0f);
+                if (!HOST_ROWS) {
+                    __stcs(out + gi, y);
+                } else {
+                    float4 *o = out + (size_t)gi * (OUT / 4);
+                    o[0] = y;
+#pragma unroll
+                    for (int q = 1; q < OUT / 4; ++q) o[q] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                }
+            }
         }
         store_feat(P.x, tp, na, nb);  // layer 1 consumed x long ago
         tc::fence_async_smem();
@@ -467,7 +508,12 @@ k_mlp(int n, const __nv_bfloat16 *__restrict__ feat, const __nv_bfloat16 *__rest
         tc::fence_after_sync();
         if (!ok) break;
     }
-    if (!ok && tp == 0) atomicAdd(err, 1u);
+    if (!ok && tp == 0) {
+        if (HOST_ROWS)
+            *reinterpret_cast<volatile unsigned *>(err) = 1u;  // page-locked host memory
+        else
+            atomicAdd(err, 1u);
+    }
     tc::fence_before_sync();
     __syncthreads();
     if (t < 32) tc::tmem_dealloc(S.w.taddr, kTmemCols);
@@ -610,18 +656,6 @@ struct alignas(128) TrainSmem {
     uint32_t taddr;
 };
 
-// A row-major BF16 matrix of `cols` columns into a K-major tile.
-__device__ __forceinline__ void stage_matrix(unsigned char *tile, const __nv_bfloat16 *__restrict__ w,
-                                             int rows, int cols)
-{
-    const int chunks = cols >> 3;
-    const uint4 *src = reinterpret_cast<const uint4 *>(w);
-    for (int e = threadIdx.x; e < rows * chunks; e += blockDim.x) {
-        const int r = e / chunks, k = e % chunks;
-        *reinterpret_cast<uint4 *>(tile + tc::kmajor_offset(r, 8 * k, cols)) = __ldcg(src + e);
-    }
-}
-
 // Makes the CTA's shared-memory writes visible to the tensor core and joins
 // the CTA; false once any thread's wait has given up.
 __device__ __forceinline__ bool join_for_mma(bool ok)
@@ -720,7 +754,7 @@ k_train(int tiles, const int *__restrict__ order, const __nv_bfloat16 *__restric
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
                 const int c = 8 * q + 2 * e;
-                asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(o[e]) : "f"(v[c + 1] * g[c + 1]), "f"(v[c] * g[c]));
+                o[e] = tc::pack_bf16x2(v[c] * g[c], v[c + 1] * g[c + 1]);
             }
             *reinterpret_cast<uint4 *>(h + tc::kmajor_offset(row, c0 + 8 * q, HID)) =
                 make_uint4(o[0], o[1], o[2], o[3]);
@@ -1023,6 +1057,14 @@ struct LearnedModel {
     double *loss = nullptr;
     int *order = nullptr;
     int parts_cap = 0, order_cap = 0;
+    // sph_learned_forward's workspace, kept between calls: two buffers of
+    // at most kForwardRows float rows and their outputs, the second stream,
+    // and a page-locked word that a wait that gave up sets
+    float *fwd_in[2] = {nullptr, nullptr};
+    float4 *fwd_out[2] = {nullptr, nullptr};
+    int fwd_cap[2] = {0, 0};
+    cudaStream_t stream2 = nullptr;
+    unsigned *h_err = nullptr;
     cudaStream_t stream = nullptr;
     unsigned long long seed = 0;
 };
@@ -1053,7 +1095,8 @@ int configure_kernels()
 {
     static bool done = false;
     if (done) return SPH_OK;
-    LCUDA(cudaFuncSetAttribute(ml::k_mlp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mlp_smem()));
+    LCUDA(cudaFuncSetAttribute(ml::k_mlp<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mlp_smem()));
+    LCUDA(cudaFuncSetAttribute(ml::k_mlp<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mlp_smem()));
     LCUDA(cudaFuncSetAttribute(ml::k_train, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)train_smem()));
     LCUDA(cudaFuncSetAttribute(ml::k_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gemm_smem()));
     done = true;
@@ -1107,6 +1150,30 @@ int num_sms()
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     return sms > 0 ? sms : 1;
+}
+
+// Rows of one piece of sph_learned_forward.
+constexpr int kForwardRows = 131072;
+
+// Buffer b of the forward workspace for `rows` rows.
+int ensure_forward(LearnedModel *l, int b, int rows)
+{
+    if (!l->h_err) {
+        LCUDA(cudaHostAlloc((void **)&l->h_err, sizeof(unsigned), cudaHostAllocMapped));
+        *l->h_err = 0u;
+    }
+    if (b == 1 && !l->stream2)
+        LCUDA(cudaStreamCreateWithFlags(&l->stream2, cudaStreamNonBlocking));
+    if (rows <= l->fwd_cap[b]) return SPH_OK;
+    cudaFree(l->fwd_in[b]);
+    cudaFree(l->fwd_out[b]);
+    l->fwd_in[b] = nullptr;
+    l->fwd_out[b] = nullptr;
+    l->fwd_cap[b] = 0;
+    LCUDA(cudaMalloc(&l->fwd_in[b], (size_t)rows * ml::IN * sizeof(float)));
+    LCUDA(cudaMalloc(&l->fwd_out[b], (size_t)rows * ml::OUT * sizeof(float)));
+    l->fwd_cap[b] = rows;
+    return SPH_OK;
 }
 
 // The training workspace for steps of `parts` CTAs and `rows` samples an epoch.
@@ -1200,10 +1267,12 @@ int train_loop(LearnedModel *l, int first, int nsamples, int epochs, int batch, 
 int launch_messages(sph_cuda *h, __nv_bfloat16 *feat, unsigned short *nbc)
 {
     if (h->n == 0) return SPH_OK;
-    (h->long_masks ? ml::k_messages<true> : ml::k_messages<false>)<<<nblk(h->n), kBlock, 0,
-                                                                      h->stream>>>(
-        make_ctx(h), h->xr_c, h->mask01_c, h->mask2_c, h->rows_c, h->prev_c, h->start_c,
-        &h->d_state->build_max_occ[SLOT_PREDICTED], feat, nbc, &h->d_state->fb_count);
+    launch_pdl(h->long_masks ? ml::k_messages<true> : ml::k_messages<false>, nblk(h->n), kBlock, 0,
+               h->stream, make_ctx(h), (const float4 *)h->xr_c, (const ulonglong2 *)h->mask01_c,
+               (const unsigned long long *)h->mask2_c, (const int4 *)h->rows_c,
+               (const float2 *)h->prev_c, (const int *)h->start_c,
+               (const unsigned *)&h->d_state->build_max_occ[SLOT_PREDICTED], feat, nbc,
+               &h->d_state->fb_count);
     return cuda_fail(cudaGetLastError(), "messages");
 }
 
@@ -1212,9 +1281,9 @@ int run_mlp(cudaStream_t st, LearnedModel *l, int n, const __nv_bfloat16 *feat, 
 {
     if (n == 0) return SPH_OK;
     LTRY(configure_kernels());
-    const int ntiles = (n + 127) / 128;
-    const int grid = std::min((ntiles + ml::kPipes - 1) / ml::kPipes, sms > 0 ? sms : num_sms());
-    ml::k_mlp<<<grid, ml::kMlpThreads, mlp_smem(), st>>>(n, feat, l->wbf, l->w, out, l->d_err);
+    const int grid = std::min((n + 127) / 128, sms > 0 ? sms : num_sms());
+    launch_pdl(ml::k_mlp<false>, grid, ml::kMlpThreads, mlp_smem(), st, n, (const void *)feat,
+               (const __nv_bfloat16 *)l->wbf, (const float *)l->w, out, l->d_err);
     return cuda_fail(cudaGetLastError(), "mlp launch");
 }
 
@@ -1360,10 +1429,13 @@ int sph_learned_destroy(sph_learned_t *l)
 {
     if (!l) return SPH_OK;
     if (l->stream) cudaStreamSynchronize(l->stream);
+    if (l->stream2) cudaStreamSynchronize(l->stream2);
     void *ptrs[] = {l->w, l->m, l->v, l->wbf, l->d_err, l->X, l->T, l->slot, l->part,
-                    l->loss, l->order};
+                    l->loss, l->order, l->fwd_in[0], l->fwd_in[1], l->fwd_out[0], l->fwd_out[1]};
     for (void *p : ptrs)
         if (p) cudaFree(p);
+    if (l->h_err) cudaFreeHost(l->h_err);
+    if (l->stream2) cudaStreamDestroy(l->stream2);
     if (l->stream) cudaStreamDestroy(l->stream);
     delete l;
     return SPH_OK;
@@ -1446,34 +1518,49 @@ int sph_learned_forward(sph_learned_t *l, const float *features, int n, float *o
         return SPH_ERR_INVALID;
     }
     if (n == 0) return SPH_OK;
-    std::vector<__nv_bfloat16> x((size_t)n * ml::IN);
-    for (size_t e = 0; e < x.size(); ++e) x[e] = __float2bfloat16(features[e]);
-    __nv_bfloat16 *dx = nullptr;
-    float4 *dy = nullptr;
-    int rc = SPH_OK;
-    if ((rc = cuda_fail(cudaMalloc(&dx, x.size() * 2), "cudaMalloc")) ||
-        (rc = cuda_fail(cudaMalloc(&dy, (size_t)n * sizeof(float4)), "cudaMalloc"))) {
-        cudaFree(dx);
-        return rc;
+    LTRY(configure_kernels());
+    // the caller's rows go to the device as they are, kForwardRows at a time
+    // on two streams, so that the copies of one piece can overlap the
+    // kernel and the copies of another
+    const int nbuf = n > kForwardRows ? 2 : 1;
+    // outputs that overlap the features: nothing may be written to them
+    // before every row is read
+    const bool overlap = (uintptr_t)out < (uintptr_t)(features + (size_t)n * ml::IN) &&
+                         (uintptr_t)features < (uintptr_t)(out + (size_t)n * ml::OUT);
+    std::vector<float> copy;
+    if (overlap && nbuf > 1) {
+        copy.assign(features, features + (size_t)n * ml::IN);
+        features = copy.data();
     }
-    cudaMemcpyAsync(dx, x.data(), x.size() * 2, cudaMemcpyHostToDevice, l->stream);
-    cudaMemsetAsync(l->d_err, 0, 4, l->stream);
-    rc = run_mlp(l->stream, l, n, dx, dy, 0);
-    std::vector<float4> y(n);
-    if (rc == SPH_OK) {
-        cudaMemcpyAsync(y.data(), dy, (size_t)n * sizeof(float4), cudaMemcpyDeviceToHost, l->stream);
-        rc = check_err(l);
+    for (int b = 0; b < nbuf; ++b) LTRY(ensure_forward(l, b, std::min(n, kForwardRows)));
+    PageToucher pages(out, overlap ? 0 : (size_t)n * ml::OUT * sizeof(float));
+    int rc = SPH_OK, k = 0;
+    for (int i0 = 0; i0 < n && rc == SPH_OK; i0 += kForwardRows, k ^= 1) {
+        const int rows = std::min(n - i0, kForwardRows);
+        cudaStream_t st = k ? l->stream2 : l->stream;
+        rc = cuda_fail(cudaMemcpyAsync(l->fwd_in[k], features + (size_t)i0 * ml::IN,
+                                       (size_t)rows * ml::IN * sizeof(float), cudaMemcpyHostToDevice, st),
+                       "feature rows");
+        if (rc != SPH_OK) break;
+        ml::k_mlp<true><<<std::min((rows + 127) / 128, num_sms()), ml::kMlpThreads, mlp_smem(), st>>>(
+            rows, l->fwd_in[k], l->wbf, l->w, l->fwd_out[k], l->h_err);
+        rc = cuda_fail(cudaGetLastError(), "mlp launch");
+        pages.done();
+        if (rc == SPH_OK)
+            rc = cuda_fail(cudaMemcpyAsync(out + (size_t)i0 * ml::OUT, l->fwd_out[k],
+                                           (size_t)rows * ml::OUT * sizeof(float),
+                                           cudaMemcpyDeviceToHost, st),
+                           "network outputs");
     }
-    if (rc == SPH_OK)
-        for (int i = 0; i < n; ++i) {
-            for (int o = 0; o < ml::OUT; ++o) out[(size_t)i * ml::OUT + o] = 0.0f;
-            out[(size_t)i * ml::OUT + 0] = y[i].x;
-            out[(size_t)i * ml::OUT + 1] = y[i].y;
-            out[(size_t)i * ml::OUT + 2] = y[i].z;
-        }
-    cudaFree(dx);
-    cudaFree(dy);
-    return rc;
+    const int rs = cuda_fail(cudaStreamSynchronize(l->stream), "forward");
+    const int rs2 = nbuf > 1 ? cuda_fail(cudaStreamSynchronize(l->stream2), "forward") : SPH_OK;
+    if (rc != SPH_OK || rs != SPH_OK || rs2 != SPH_OK) return rc != SPH_OK ? rc : rs != SPH_OK ? rs : rs2;
+    if (*l->h_err) {
+        *l->h_err = 0u;
+        set_error("tensor-core wait gave up (mbarrier not completed)");
+        return SPH_ERR_CUDA;
+    }
+    return SPH_OK;
 }
 
 int sph_learned_features(sph_cuda_t *h, float *features, int *counts)

@@ -200,6 +200,14 @@ __device__ __forceinline__ uint32_t act_bf16x2(float a, float b)
     return y;
 }
 
+// (a, b) rounded to a packed BF16 pair, a in the low half.
+__device__ __forceinline__ uint32_t pack_bf16x2(float a, float b)
+{
+    uint32_t x;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(x) : "f"(b), "f"(a));
+    return x;
+}
+
 // Named barrier over `count` threads (ids 1..15; 0 is __syncthreads).
 __device__ __forceinline__ void named_sync(int id, int count)
 {

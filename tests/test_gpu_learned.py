@@ -338,3 +338,24 @@ def test_bounded_wait_gives_up(cuda_lib):
     # the device still works afterwards
     A = np.ones((128, 32), np.float32)
     assert np.allclose(gemm_check(A, A[:16]), 32.0)
+
+
+def test_forward_pieces_and_overlap(cuda_lib):
+    """Rows split over the two forward buffers (kForwardRows rows a piece)
+    are the rows of a call on each part, also where the outputs overlap the
+    features in the caller's memory."""
+    import ctypes
+    from sph_gb300 import _lib
+    n = 2 * 131072 + 77
+    rng = np.random.default_rng(8)
+    x = rng.standard_normal((n, LearnedModel.IN)).astype(np.float32)
+    x[:, 31] = 1.0
+    with LearnedModel(0, seed=4) as m:
+        y = m.forward(x)
+        for a, b in ((0, 1), (0, 129), (131072 - 1, 131072 + 1), (n - 300, n)):
+            assert bits_equal(m.forward(x[a:b]), y[a:b])
+        buf = np.concatenate([x.reshape(-1), np.zeros(64, np.float32)])
+        fp = ctypes.POINTER(ctypes.c_float)
+        shifted = buf[48:]
+        _lib.check(cuda_lib.sph_learned_forward(m._l, buf.ctypes.data_as(fp), n, shifted.ctypes.data_as(fp)))
+        assert bits_equal(shifted[:n * LearnedModel.OUT].reshape(n, LearnedModel.OUT).copy(), y)
