@@ -240,6 +240,7 @@ int enqueue_step(sph_cuda *h, cudaEvent_t *events, int *nkernels,
 unsigned bounds_flags_kernels();  // checked builds (SPH_BOUNDS_CHECK): recorded index faults
 unsigned bounds_flags_learned();
 int enqueue_predicted_state(sph_cuda *h);       // first half of a step: C order + density
+int launch_prefix(sph_cuda *h, unsigned *in, int n, int *out);  // exclusive prefix sums, out[n] = total
 int launch_density_pass(sph_cuda *h);            // the density pass on the C order
 bool long_masks_supported();
 int launch_learned_passes(sph_cuda *h, cudaEvent_t *events);  // features + network (C order)

@@ -1836,6 +1836,11 @@ static int launch_scan(sph_cuda *h, unsigned *in, int M, int *out, unsigned *occ
     return SPH_OK;
 }
 
+int launch_prefix(sph_cuda *h, unsigned *in, int n, int *out)
+{
+    return launch_scan(h, in, n, out, nullptr, false, nullptr);
+}
+
 // The cell starts of a step's build (all M counters, zeroed after) into
 // `out` (M + 1 entries); the build's key producer counted its particles per
 // build tile into build_tiles, which the build's scatter zeroes again.

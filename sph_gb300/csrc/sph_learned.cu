@@ -944,16 +944,40 @@ __global__ void k_f32_to_bf16(int n, const float *__restrict__ in, __nv_bfloat16
 // sample collection and calibration
 // ---------------------------------------------------------------------------
 
-// Appends the rows of sorted slots sel[0..rows): features and targets
-// (plain displacement / s, error 0).
-__global__ void k_append(Ctx c, int rows, const int *__restrict__ sel,
-                         const __nv_bfloat16 *__restrict__ feat, const float2 *__restrict__ disp,
-                         __nv_bfloat16 *__restrict__ X, float4 *__restrict__ T,
-                         int *__restrict__ slot)
+// splitmix64 finaliser: the sample selection hash.
+__host__ __device__ __forceinline__ unsigned long long mix64(unsigned long long z)
 {
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= rows) return;
-    const int i = sel[r];
+    z += 0x9E3779B97F4A7C15ull;
+    z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
+    z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
+    return z ^ (z >> 31);
+}
+
+// 1 for each slot that is a sample: few enough neighbours and, for frac < 1,
+// the particle's hash below frac.
+__global__ void __launch_bounds__(kBlock)
+k_select(int n, const unsigned short *__restrict__ nbc, const int *__restrict__ ids,
+         unsigned long long salt, double frac, unsigned *__restrict__ flag)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    bool take = (int)nbc[i] <= MAXNB;
+    if (take && frac < 1.0)
+        take = (double)(mix64(salt ^ (unsigned long long)ids[i]) >> 11) * (1.0 / 9007199254740992.0) < frac;
+    flag[i] = take ? 1u : 0u;
+}
+
+// Appends the selected slots in slot order, `room` rows at most: row off[i]
+// takes slot i's features and targets (plain displacement / s, error 0).
+__global__ void __launch_bounds__(kBlock)
+k_append(Ctx c, int room, const unsigned *__restrict__ flag, const int *__restrict__ off,
+         const __nv_bfloat16 *__restrict__ feat, const float2 *__restrict__ disp,
+         __nv_bfloat16 *__restrict__ X, float4 *__restrict__ T, int *__restrict__ slot)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= c.n || !flag[i]) return;
+    const int r = off[i];
+    if (r >= room) return;
     const float s = out_scale(c.scenes + scene_of(c, i));
     const uint4 *src = reinterpret_cast<const uint4 *>(feat + (size_t)i * IN);
     uint4 *dst = reinterpret_cast<uint4 *>(X + (size_t)r * IN);
@@ -962,6 +986,36 @@ __global__ void k_append(Ctx c, int rows, const int *__restrict__ sel,
     const float2 d = disp[i];
     T[r] = make_float4(d.x / s, d.y / s, 0.0f, 1.0f);
     slot[r] = i;
+}
+
+// Feature rows (as floats) and neighbour counts (-1: always the plain
+// relaxation) of the particles with ids [lo, lo + m), by id: a thread per 8
+// features, so that a row's 64 bytes are read and its 128 written in full
+// sectors.  (On the host this conversion and scatter took 17 ns a particle;
+// 131,071 particles 2.4 -> 0.52 ms with the copies.)
+__global__ void __launch_bounds__(kBlock)
+k_rows_by_id(int n, int lo, int m, const int *__restrict__ ids,
+             const __nv_bfloat16 *__restrict__ feat, const unsigned short *__restrict__ nbc,
+             float *__restrict__ rows, int *__restrict__ counts)
+{
+    const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const long long i = e >> 2;
+    const int q = (int)(e & 3);
+    if (i >= n) return;
+    const int r = ids[i] - lo;
+    if (r < 0 || r >= m) return;
+    const uint4 v = __ldg(reinterpret_cast<const uint4 *>(feat + (size_t)i * IN) + q);
+    const uint32_t u[4] = {v.x, v.y, v.z, v.w};
+    float f[8];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        f[2 * k] = __uint_as_float(u[k] << 16);
+        f[2 * k + 1] = __uint_as_float(u[k] & 0xFFFF0000u);
+    }
+    float4 *dst = reinterpret_cast<float4 *>(rows + (size_t)r * IN) + 2 * q;
+    dst[0] = make_float4(f[0], f[1], f[2], f[3]);
+    dst[1] = make_float4(f[4], f[5], f[6], f[7]);
+    if (q == 0) counts[r] = nbc[i] == 65535 ? -1 : (int)nbc[i];
 }
 
 // Density at displaced positions pos + disp (sorted order) over the stencil
@@ -1151,6 +1205,9 @@ int num_sms()
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     return sms > 0 ? sms : 1;
 }
+
+// Particles of one piece of sph_learned_features.
+constexpr int kFeaturePiece = 262144;
 
 // Rows of one piece of sph_learned_forward.
 constexpr int kForwardRows = 131072;
@@ -1572,32 +1629,32 @@ int sph_learned_features(sph_cuda_t *h, float *features, int *counts)
     const int n = h->n;
     if (n == 0) return SPH_OK;
     LTRY(predicted_features(h, nullptr));
-    std::vector<__nv_bfloat16> f((size_t)n * ml::IN);
-    std::vector<unsigned short> cnt(n);
-    std::vector<int> ids(n);
-    LCUDA(cudaMemcpyAsync(f.data(), h->feat_c, f.size() * 2, cudaMemcpyDeviceToHost, h->stream));
-    LCUDA(cudaMemcpyAsync(cnt.data(), h->nbc_c, (size_t)n * 2, cudaMemcpyDeviceToHost, h->stream));
-    LCUDA(cudaMemcpyAsync(ids.data(), h->id_c, (size_t)n * 4, cudaMemcpyDeviceToHost, h->stream));
-    LCUDA(cudaStreamSynchronize(h->stream));
-    for (int i = 0; i < n; ++i) {
-        const int id = ids[i];
-        for (int e = 0; e < ml::IN; ++e)
-            features[(size_t)id * ml::IN + e] = __bfloat162float(f[(size_t)i * ml::IN + e]);
-        if (counts) counts[id] = cnt[i] == 65535 ? -1 : (int)cnt[i];
+    PageToucher row_pages(features, (size_t)n * ml::IN * sizeof(float));
+    PageToucher count_pages(counts, counts ? (size_t)n * sizeof(int) : 0);
+    // by id, kFeaturePiece particles at a time (a bounded scratch)
+    const int piece = std::min(n, kFeaturePiece);
+    LTRY(ensure_scratch(h, (size_t)piece * (ml::IN * sizeof(float) + sizeof(int)) + 256));
+    float *rows = (float *)h->d_scratch;
+    int *cnt = (int *)(rows + (size_t)piece * ml::IN);
+    for (int lo = 0; lo < n; lo += piece) {
+        const int m = std::min(piece, n - lo);
+        ml::k_rows_by_id<<<nblk(4ll * n), kBlock, 0, h->stream>>>(
+            n, lo, m, h->id_c, (const __nv_bfloat16 *)h->feat_c, h->nbc_c, rows, cnt);
+        LCUDA(cudaGetLastError());
+        row_pages.done();
+        LCUDA(cudaMemcpyAsync(features + (size_t)lo * ml::IN, rows, (size_t)m * ml::IN * sizeof(float),
+                              cudaMemcpyDeviceToHost, h->stream));
+        if (counts) {
+            count_pages.done();
+            LCUDA(cudaMemcpyAsync(counts + lo, cnt, (size_t)m * sizeof(int), cudaMemcpyDeviceToHost,
+                                  h->stream));
+        }
     }
+    LCUDA(cudaStreamSynchronize(h->stream));
     return SPH_OK;
 }
 
 namespace {
-
-// splitmix64 finaliser: the sample selection hash.
-unsigned long long mix64(unsigned long long z)
-{
-    z += 0x9E3779B97F4A7C15ull;
-    z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
-    z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
-    return z ^ (z >> 31);
-}
 
 // Samples of h's predicted state: features and plain displacements of the
 // selected particles appended at l->nsamples.  fraction >= 1 takes every
@@ -1608,12 +1665,16 @@ int collect_samples(LearnedModel *l, sph_cuda *h, float fraction, int *added)
     const int n = h->n;
     if (n == 0) return SPH_OK;
     LTRY(predicted_features(h, nullptr));
+    // scratch: displacements, selection flags and their prefix sums (16-byte
+    // aligned, as the scan needs them)
+    const size_t db = (((size_t)n * 8) + 255) & ~(size_t)255;
+    const size_t fb = (((size_t)n + 1) * 4 + 255) & ~(size_t)255;
+    LTRY(ensure_scratch(h, db + 2 * fb));
+    float2 *disp = (float2 *)h->d_scratch;
+    unsigned *flag = (unsigned *)((char *)h->d_scratch + db);
+    int *off = (int *)((char *)h->d_scratch + db + fb);
     // plain displacement (C order) through the learned relaxation with every
     // particle forced to fall back
-    const size_t db = (((size_t)n * 8) + 255) & ~(size_t)255;
-    LTRY(ensure_scratch(h, db + ((size_t)n + 1) * 4 + 256));
-    float2 *disp = (float2 *)h->d_scratch;
-    int *sel_d = (int *)((char *)h->d_scratch + db);
     const float thr = h->learned_thr;
     sph::LearnedModel *keep = h->learned;
     h->learned_thr = -1.0f;
@@ -1621,31 +1682,19 @@ int collect_samples(LearnedModel *l, sph_cuda *h, float fraction, int *added)
     h->learned_thr = thr;
     h->learned = keep;
     LTRY(rc);
-    std::vector<unsigned short> cnt(n);
-    std::vector<int> ids(n);
-    LCUDA(cudaMemcpyAsync(cnt.data(), h->nbc_c, (size_t)n * 2, cudaMemcpyDeviceToHost, h->stream));
-    LCUDA(cudaMemcpyAsync(ids.data(), h->id_c, (size_t)n * 4, cudaMemcpyDeviceToHost, h->stream));
-    LCUDA(cudaStreamSynchronize(h->stream));
-    const unsigned long long salt = mix64(l->seed ^ (0xA5A5A5A5ull + l->calls));
+    const unsigned long long salt = ml::mix64(l->seed ^ (0xA5A5A5A5ull + l->calls));
     const double frac = std::min(1.0, std::max(0.0, (double)fraction));
-    std::vector<int> sel;
-    sel.reserve(std::min(n, std::max(0, l->cap - l->nsamples)));
-    for (int i = 0; i < n && l->nsamples + (int)sel.size() < l->cap; ++i) {
-        if (cnt[i] > ml::MAXNB) continue;
-        if (frac < 1.0 &&
-            (double)(mix64(salt ^ (unsigned long long)ids[i]) >> 11) * (1.0 / 9007199254740992.0) >= frac)
-            continue;
-        sel.push_back(i);
-    }
-    const int rows = (int)sel.size();
-    if (rows > 0) {
-        LCUDA(cudaMemcpyAsync(sel_d, sel.data(), (size_t)rows * 4, cudaMemcpyHostToDevice, h->stream));
-        ml::k_append<<<nblk(rows), kBlock, 0, h->stream>>>(
-            make_ctx(h), rows, sel_d, (const __nv_bfloat16 *)h->feat_c, disp,
-            l->X + (size_t)l->nsamples * ml::IN, l->T + l->nsamples, l->slot + l->nsamples);
-        LCUDA(cudaGetLastError());
-        LCUDA(cudaStreamSynchronize(h->stream));
-    }
+    const int room = std::max(0, l->cap - l->nsamples);
+    ml::k_select<<<nblk(n), kBlock, 0, h->stream>>>(n, h->nbc_c, h->id_c, salt, frac, flag);
+    LTRY(launch_prefix(h, flag, n, off));
+    ml::k_append<<<nblk(n), kBlock, 0, h->stream>>>(
+        make_ctx(h), room, flag, off, (const __nv_bfloat16 *)h->feat_c, disp,
+        l->X + (size_t)l->nsamples * ml::IN, l->T + l->nsamples, l->slot + l->nsamples);
+    LCUDA(cudaGetLastError());
+    int total = 0;
+    LCUDA(cudaMemcpyAsync(&total, off + n, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+    LCUDA(cudaStreamSynchronize(h->stream));
+    const int rows = std::min(total, room);
     l->nsamples += rows;
     ++l->calls;
     *added = rows;

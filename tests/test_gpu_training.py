@@ -89,3 +89,36 @@ def test_training_matches_numpy(cuda_lib, tiles):
     assert np.sqrt(np.mean(d ** 2)) <= 0.05, np.sqrt(np.mean(d ** 2))
     b1 = LearnedModel.unpack(w)["b1"]
     assert np.array_equal(b1, LearnedModel.unpack(w0)["b1"])  # acts through the constant feature
+
+
+def splitmix64(z):
+    m = (1 << 64) - 1
+    z = (z + 0x9E3779B97F4A7C15) & m
+    z = ((z ^ (z >> 30)) * 0xBF58476D1CE4E5B9) & m
+    z = ((z ^ (z >> 27)) * 0x94D049BB133111EB) & m
+    return z ^ (z >> 31)
+
+
+@pytest.mark.parametrize("n", [1, 255, 4097])
+def test_collected_samples_and_feature_rows(cuda_lib, n):
+    """The number of samples of each collection is that of the selection
+    rule (few enough neighbours, the particle's hash below the fraction),
+    cut at the model's capacity; feature rows come by id."""
+    sc = still_fluid(n, seed=n)
+    seed, fraction = 5, 0.4
+    cap = n + n // 3
+    with Simulation.from_scene(sc) as s, LearnedModel(cap, seed=seed) as m:
+        f, count = s.learned_features()
+        ok = (count >= 0) & (count <= LearnedModel.MAX_NEIGHBORS)
+        held = 0
+        for call in range(4):
+            salt = splitmix64(seed ^ (0xA5A5A5A5 + call))
+            u = np.array([(splitmix64(salt ^ i) >> 11) / 2.0 ** 53 for i in range(n)])
+            want = min(int((ok & (u < fraction)).sum()), cap - held)
+            assert m.collect(s, fraction) == want
+            held += want
+            assert m.num_samples == held
+    assert np.all(f[:, 31] == 1.0)
+    # row of particle i against particle i's own neighbour count
+    got = np.rint(f[:, 7] * LearnedModel.MAX_NEIGHBORS)
+    assert np.all(np.abs(got - np.minimum(count, LearnedModel.MAX_NEIGHBORS)) <= 0.25)
