@@ -386,9 +386,10 @@ static int build_handle(sph_cuda **out, std::vector<Scene> &&scenes, int capacit
     h->ntiles = (int)((scan_items + kScanTile - 1) / kScanTile);
     h->npartials = 148 * 2;
     const size_t nwords = (M + 31) / 32 + 1;
-    if ((rc = dalloc(&h->pos_a, N)) || (rc = dalloc(&h->vel_a, N)) || (rc = dalloc(&h->id_a, N)) ||
+    // the sorted positions are read up to kRowPad past their end (hit_mask32)
+    if ((rc = dalloc(&h->pos_a, N + kRowPad)) || (rc = dalloc(&h->vel_a, N)) || (rc = dalloc(&h->id_a, N)) ||
         (rc = dalloc(&h->pos_b, N)) || (rc = dalloc(&h->prev_b, N)) ||
-        (rc = dalloc(&h->vel_b, N)) || (rc = dalloc(&h->kr_b, N)) || (rc = dalloc(&h->pos_c, N)) ||
+        (rc = dalloc(&h->vel_b, N)) || (rc = dalloc(&h->kr_b, N)) || (rc = dalloc(&h->pos_c, N + kRowPad)) ||
         (rc = dalloc(&h->prev_c, N)) || (rc = dalloc(&h->xr_c, N)) ||
         (rc = dalloc(&h->mask01_c, N)) || (rc = dalloc(&h->mask2_c, N)) || (rc = dalloc(&h->rows_c, N)) ||
         (rc = dalloc(&h->id_c, N)) || (rc = dalloc(&h->tmp_id, N)) ||
@@ -1180,10 +1181,6 @@ int sph_cuda_set_launch_shapes(sph_cuda_t *h, const int *shapes)
 int sph_cuda_set_long_row_masks(sph_cuda_t *h, int on)
 {
     SPH_TRY(check_handle(h));
-    if (on && !long_masks_supported()) {
-        set_error("long-row masks are not built with the shared-memory staged gathers");
-        return SPH_ERR_UNSUPPORTED;
-    }
     if (on && !h->maskx_c) SPH_TRY(dalloc(&h->maskx_c, 3 * (size_t)h->capacity + 3));
     if ((on != 0) != h->long_masks) {
         SPH_CUDA(cudaStreamSynchronize(h->stream));
@@ -1265,28 +1262,26 @@ int sph_cuda_autotune(sph_cuda_t *h, int trial_steps, int *shapes_out)
     // then the long-row hit masks, on or off, the same way (they pay where
     // stencil rows of more than 64 candidates are common, and cost a little
     // where they are not)
-    if (long_masks_supported()) {
-        const bool was = h->long_masks;
-        if (sph_cuda_set_long_row_masks(h, 1) == SPH_OK) {
-            std::vector<float> t[2];
-            for (int r = 0; r < trial_steps; ++r)
-                for (int v = 0; v < 2; ++v) {
-                    h->long_masks = v != 0;
-                    destroy_graph(h);
-                    SPH_TRY(run_steps(h, 1));
-                    SPH_CUDA(cudaEventRecord(h->timer[0], h->stream));
-                    SPH_TRY(run_steps(h, 1));
-                    SPH_CUDA(cudaEventRecord(h->timer[1], h->stream));
-                    SPH_CUDA(cudaEventSynchronize(h->timer[1]));
-                    float ms = 0.0f;
-                    SPH_CUDA(cudaEventElapsedTime(&ms, h->timer[0], h->timer[1]));
-                    t[v].push_back(ms);
-                }
-            for (auto &v : t) std::sort(v.begin(), v.end());
-            h->long_masks = t[1][t[1].size() / 2] < t[0][t[0].size() / 2];
-        } else {
-            h->long_masks = was;
-        }
+    const bool was = h->long_masks;
+    if (sph_cuda_set_long_row_masks(h, 1) == SPH_OK) {
+        std::vector<float> t[2];
+        for (int r = 0; r < trial_steps; ++r)
+            for (int v = 0; v < 2; ++v) {
+                h->long_masks = v != 0;
+                destroy_graph(h);
+                SPH_TRY(run_steps(h, 1));
+                SPH_CUDA(cudaEventRecord(h->timer[0], h->stream));
+                SPH_TRY(run_steps(h, 1));
+                SPH_CUDA(cudaEventRecord(h->timer[1], h->stream));
+                SPH_CUDA(cudaEventSynchronize(h->timer[1]));
+                float ms = 0.0f;
+                SPH_CUDA(cudaEventElapsedTime(&ms, h->timer[0], h->timer[1]));
+                t[v].push_back(ms);
+            }
+        for (auto &v : t) std::sort(v.begin(), v.end());
+        h->long_masks = t[1][t[1].size() / 2] < t[0][t[0].size() / 2];
+    } else {
+        h->long_masks = was;
     }
     destroy_graph(h);
     if (shapes_out) SPH_TRY(sph_cuda_get_launch_shapes(h, shapes_out));

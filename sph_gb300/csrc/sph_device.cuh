@@ -91,10 +91,44 @@ __device__ __forceinline__ unsigned cell_key(float x, float y, const SG &g)
     return (unsigned)(g.c_off + (k < g.ncells ? (int)k : g.ncells));
 }
 
-// checkVelocity, fluid.c:613-625
+// checkVelocity, fluid.c:613-625.  A NaN passes through, as it fails both of
+// the reference's comparisons: min and max in their NaN-propagating forms,
+// two instructions where two compare-and-selects are four.
 __device__ __forceinline__ float clamp5(float v)
 {
-    return v > 5.0f ? 5.0f : (v < -5.0f ? -5.0f : v);
+    asm("min.NaN.f32 %0, %0, 0f40A00000;" : "+f"(v));   //  5
+    asm("max.NaN.f32 %0, %0, 0fC0A00000;" : "+f"(v));   // -5
+    return v;
+}
+
+// Approximate reciprocal root of a normal number (or zero): rsqrtf without
+// its scaling of subnormal inputs, the same bits for all others.
+__device__ __forceinline__ float rsqrt_normal(float x)
+{
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+constexpr float kMinNormal = 1.17549435e-38f;
+
+// The cell column and row of a key in the scene's grid.
+__device__ __forceinline__ void cell_of_key(unsigned key, const SG &g, int &gx, int &gy)
+{
+    const int lk = (int)key - g.c_off;
+    gy = lk / g.size_x;
+    gx = lk - gy * g.size_x;
+}
+
+// The same of a position whose key is in the grid: from the position's own
+// floors, as cell_key takes them, without the integer division (about 20
+// instructions); a column beyond the grid's width aliases into later rows
+// as its key does.
+__device__ __forceinline__ void cell_of(float2 p, unsigned key, const SG &g, int &gx, int &gy)
+{
+    const bool p2 = g.inv != 0.0f;
+    gx = (int)floorf(p2 ? __fmul_rn(p.x, g.inv) : __fdiv_rn(p.x, g.spacing));
+    gy = (int)floorf(p2 ? __fmul_rn(p.y, g.inv) : __fdiv_rn(p.y, g.spacing));
+    if (gx >= g.size_x) cell_of_key(key, g, gx, gy);
 }
 
 // boundaryConditions, fluid.c:656-744.  Rounded step by step (no fused
@@ -228,9 +262,8 @@ __device__ __forceinline__ void for_each_candidate(unsigned key, const int *__re
                                                    const SG &g, bool capped, int max_bucket,
                                                    int n, F &&f)
 {
-    const int lk = (int)key - g.c_off;
-    const int gy = lk / g.size_x;
-    const int gx = lk - gy * g.size_x;
+    int gx, gy;
+    cell_of_key(key, g, gx, gy);
     const int x0 = gx > 0 ? gx - 1 : 0;
     const int x1 = gx + 1 < g.size_x ? gx + 1 : g.size_x - 1;
     const int y0 = gy > 0 ? gy - 1 : 0;
@@ -263,15 +296,14 @@ __device__ __forceinline__ bool searchable(unsigned key, int slot, const int *__
     return !capped || slot - __ldg(start + key) < max_bucket;
 }
 
-// The three stencil rows of a cell (slot 0: gy-1, 1: gy, 2: gy+1), each the
+// The three stencil rows of the cell of a position with key `key` (slot 0: gy-1, 1: gy, 2: gy+1), each the
 // contiguous range [a[r], a[r] + len[r]) of sorted slots (empty outside the
 // grid).  Valid when no cell overflowed its bucket cap.
-__device__ __forceinline__ void stencil_rows(unsigned key, const int *__restrict__ start,
+__device__ __forceinline__ void stencil_rows(float2 p, unsigned key, const int *__restrict__ start,
                                              const SG &g, int (&a)[3], int (&len)[3], int n)
 {
-    const int lk = (int)key - g.c_off;
-    const int gy = lk / g.size_x;
-    const int gx = lk - gy * g.size_x;
+    int gx, gy;
+    cell_of(p, key, g, gx, gy);
     const int x0 = gx > 0 ? gx - 1 : 0;
     const int x1 = gx + 1 < g.size_x ? gx + 1 : g.size_x - 1;
 #pragma unroll
@@ -289,91 +321,6 @@ __device__ __forceinline__ void stencil_rows(unsigned key, const int *__restrict
                 len[r] = 0;
         }
     }
-}
-
-// ---------------------------------------------------------------------------
-// CTA staging of stencil rows in shared memory
-// ---------------------------------------------------------------------------
-
-// The particles of a CTA are consecutive in cell order, so the stencil rows
-// its threads read are three short, heavily overlapping runs of slots: for
-// each row r, the union of the threads' ranges [lo, hi) is one contiguous run
-// a little longer than the CTA.  stage_rows copies those three runs of `src`
-// into shared memory once (coalesced 8- or 16-byte loads), so that every
-// neighbour read of the gather that follows is a shared-memory load instead
-// of an L1/L2 round trip.  Each thread passes its own ranges (lo = INT_MAX,
-// hi = INT_MIN for a row it does not read); every thread of the CTA must
-// call it (it has two CTA barriers).  Returns true when the runs fit `cap`
-// elements, in which case slot j of row r is at sm[j + delta[r]] (and, when
-// a second array src2 is given, at sm2[j + delta[r]]); otherwise nothing is
-// staged and the gather reads global memory as before.
-constexpr int kStageWarpsMax = kMaxBlock / 32;
-
-__device__ __forceinline__ int warp_min_i(int v)
-{
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = min(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
-}
-
-__device__ __forceinline__ int warp_max_i(int v)
-{
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
-}
-
-template <class T, class U = T>
-__device__ __forceinline__ bool stage_rows(const int (&lo)[3], const int (&hi)[3],
-                                           const T *__restrict__ src, T *sm, int cap,
-                                           int (&delta)[3], const U *__restrict__ src2 = nullptr,
-                                           U *sm2 = nullptr)
-{
-    __shared__ int4 s_red[kStageWarpsMax][2];  // per warp: (lo0, lo1, lo2, -), (hi0, hi1, hi2, -)
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    int l[3], h[3];
-#pragma unroll
-    for (int r = 0; r < 3; ++r) {
-        l[r] = warp_min_i(lo[r]);
-        h[r] = warp_max_i(hi[r]);
-    }
-    if (lane == 0) {
-        s_red[warp][0] = make_int4(l[0], l[1], l[2], 0);
-        s_red[warp][1] = make_int4(h[0], h[1], h[2], 0);
-    }
-    __syncthreads();
-    // every thread combines the per-warp words itself (no second reduction barrier)
-#pragma unroll
-    for (int r = 0; r < 3; ++r) {
-        l[r] = INT_MAX;
-        h[r] = INT_MIN;
-    }
-    for (int w = 0; w < nw; ++w) {
-        const int4 a = s_red[w][0], b = s_red[w][1];
-        l[0] = min(l[0], a.x); l[1] = min(l[1], a.y); l[2] = min(l[2], a.z);
-        h[0] = max(h[0], b.x); h[1] = max(h[1], b.y); h[2] = max(h[2], b.z);
-    }
-    int len[3], off[3], total = 0;
-#pragma unroll
-    for (int r = 0; r < 3; ++r) {
-        len[r] = h[r] > l[r] ? h[r] - l[r] : 0;
-        off[r] = total;
-        total += len[r];
-        delta[r] = off[r] - l[r];
-    }
-    const bool ok = total <= cap;  // the same in every thread of the CTA
-    if (ok) {
-#pragma unroll
-        for (int r = 0; r < 3; ++r)
-            for (int k = threadIdx.x; k < len[r]; k += blockDim.x) {
-                sm[off[r] + k] = src[l[r] + k];
-                if (src2) sm2[off[r] + k] = src2[l[r] + k];
-            }
-    }
-    // also when nothing was staged: s_red and sm are reused by the CTA's
-    // next call only after every thread has passed this barrier
-    __syncthreads();
-    return ok;
 }
 
 constexpr int kMaskRow = 64;  // candidates per stencil row recorded in a hit mask
@@ -413,6 +360,84 @@ __device__ __forceinline__ void walk_mask(unsigned long long m, int base, int n,
             dp = d;
             have = true;
         }
+    }
+    if (have) visit(jp, dp);
+}
+
+// The same over the masks of a particle's three stencil rows, with the record
+// in flight carried from row to row: the pipeline is drained once per
+// particle, not once per row (relax_update 182 -> 178 us at 4,194,304
+// particles early in the dam break, 205 -> 199 us compressed).
+template <class T, class Load, class Visit>
+__device__ __forceinline__ void walk_rows(const unsigned long long (&m)[3], const int (&base)[3],
+                                          int n, Load load, Visit visit)
+{
+    bool have = false;
+    int jp = 0;
+    T dp{};
+#pragma unroll
+    for (int r = 0; r < 3; ++r)
+#pragma unroll
+        for (int hh = 0; hh < 2; ++hh) {
+            unsigned b = hh ? (unsigned)(m[r] >> 32) : (unsigned)m[r];
+            while (b) {
+                const int j = base[r] + 32 * hh + __ffs(b) - 1;
+                b &= b - 1u;
+                if (!in_bounds(j, n, kBadSlot)) continue;
+                const T d = load(j);
+                if (have) visit(jp, dp);
+                jp = j;
+                dp = d;
+                have = true;
+            }
+        }
+    if (have) visit(jp, dp);
+}
+
+// The hit bits (r2 <= h2) of the n <= 32 candidates from `row` on.  Blocks of
+// U candidates are loaded and tested without a remainder: the last block may
+// read up to U - 1 positions past the row (the sorted position arrays have
+// kRowPad more than their particles), whose bits are cut off at the end.
+// Eight loads in flight and no remainder loop: with an unrolled-by-four
+// loop and its remainder the viscosity pass took 226 us, so 218 us
+// (4,194,304 particles).
+template <int U>
+__device__ __forceinline__ unsigned hit_mask32(const float2 *__restrict__ row, int n, float2 mp,
+                                               float h2)
+{
+    static_assert(U <= kRowPad && 32 % U == 0, "block of candidates");
+    unsigned m = 0u;
+    for (int t = 0; t < n; t += U) {
+        float2 q[U];
+#pragma unroll
+        for (int k = 0; k < U; ++k) q[k] = __ldg(row + t + k);
+        unsigned b = 0u;
+#pragma unroll
+        for (int k = 0; k < U; ++k) {
+            float2 e;
+            if (dist2_packed(mp, q[k], e) <= h2) b |= 1u << k;
+        }
+        m |= b << t;
+    }
+    return n < 32 ? m & ((1u << n) - 1u) : m;
+}
+
+// Visits the set bits of a 32-bit mask as walk_mask does.
+template <class T, class Load, class Visit>
+__device__ __forceinline__ void walk_mask32(unsigned b, int base, int n, Load load, Visit visit)
+{
+    bool have = false;
+    int jp = 0;
+    T dp{};
+    while (b) {
+        const int j = base + __ffs(b) - 1;
+        b &= b - 1u;
+        if (!in_bounds(j, n, kBadSlot)) continue;
+        const T d = load(j);
+        if (have) visit(jp, dp);
+        jp = j;
+        dp = d;
+        have = true;
     }
     if (have) visit(jp, dp);
 }

@@ -70,6 +70,7 @@ struct DevState {
 
 enum BuildSlot { SLOT_PREDICTED = 0, SLOT_RELAXED = 1, SLOT_UPLOAD = 2, SLOT_PROBE = 3 };
 
+constexpr int kRowPad = 8;          // positions readable past the end of a sorted array
 constexpr int kScanThreads = 256;
 constexpr int kScanItems = 16;                        // per thread
 constexpr int kScanTile = kScanThreads * kScanItems;  // cells per scan tile
@@ -242,7 +243,6 @@ unsigned bounds_flags_learned();
 int enqueue_predicted_state(sph_cuda *h);       // first half of a step: C order + density
 int launch_prefix(sph_cuda *h, unsigned *in, int n, int *out);  // exclusive prefix sums, out[n] = total
 int launch_density_pass(sph_cuda *h);            // the density pass on the C order
-bool long_masks_supported();
 int launch_learned_passes(sph_cuda *h, cudaEvent_t *events);  // features + network (C order)
 int launch_learned_relax(sph_cuda *h, float2 *probe_out, cudaEvent_t *events = nullptr);
 void free_learned_buffers(sph_cuda *h);

@@ -29,36 +29,12 @@
 #include "sph_device.cuh"
 #include "sph_learned.h"
 
-// Unroll factors of the candidate filter loops and the relaxation's
-// register budget (tuned on GB300).
-#ifndef SPH_VISC_UNROLL
-#define SPH_VISC_UNROLL 4
-#endif
-#ifndef SPH_DENS_UNROLL
-#define SPH_DENS_UNROLL 2
-#endif
-#ifndef SPH_RELAX_MIN_BLOCKS
-#define SPH_RELAX_MIN_BLOCKS 4  // resident 256-thread CTAs per SM the relaxation is built for
-#endif
-#ifndef SPH_RELAX_SMEM
-#define SPH_RELAX_SMEM 0  // relaxation reads its stencil rows from a shared-memory copy
-#endif
-#ifndef SPH_DENS_SMEM
-#define SPH_DENS_SMEM 0   // density pass likewise
-#endif
-#ifndef SPH_VISC_SMEM
-#define SPH_VISC_SMEM 0   // viscosity pass likewise
-#endif
-
 namespace sph {
-// Shared-memory elements a gather CTA stages per thread of the CTA (the
-// three stencil-row runs of a CTA in one grid row are about 3.2 per thread).
-#ifndef SPH_STAGE_PER_THREAD
-#define SPH_STAGE_PER_THREAD 4
-#endif
-constexpr int kStagePerThread = SPH_STAGE_PER_THREAD;
-constexpr int kViscUnroll = SPH_VISC_UNROLL;
-constexpr int kDensUnroll = SPH_DENS_UNROLL;
+// Unroll factors of the candidate loops (tuned on GB300): the blocks of a
+// mark-then-walk scan (hit_mask32), and the single-phase loop of the density
+// pass's long rows.
+constexpr int kMarkUnroll = 8;
+constexpr int kDensLongUnroll = 4;
 }  // namespace sph
 
 namespace sph {
@@ -615,154 +591,22 @@ k_keys(Ctx c, const float2 *__restrict__ pos, uint2 *__restrict__ kr, unsigned *
 // pass 1: gravity + viscosity (gather) + predict + boundary + cell key
 // ---------------------------------------------------------------------------
 
-// apply_gravity (fluid.c:398-413), viscosity_impluses (fluid.c:416-478) in
-// gather form, predict_positions (fluid.c:507-523) with boundaryConditions.
-// Gather form of the viscosity: dv_i = -1/2 sum_j clamp5(I_ij),
-// I_ij = dt (1 - r/h)(sigma u + beta u^2) (x_j - x_i)/r for u > 0,
-// u = ((v_i - v_j).(x_j - x_i))/r, all from the velocities after gravity.
-// PROBE writes dv instead of advancing.
-// STAGED: every thread of the CTA calls this (valid = false for a thread
-// without a particle), and the CTA first copies the union of its stencil
-// rows' positions and velocities to shared memory (sm_p, sm_v; cap
-// elements each; stage_rows).
-template <bool PROBE, bool STAGED = false>
-__device__ __forceinline__ void viscosity_predict_one(
-    int i, const Ctx &c, const DevState *__restrict__ st, const float2 *__restrict__ pos,
-    const float2 *__restrict__ vel, const int *__restrict__ start, bool capped,
-    float2 *__restrict__ pos_out, float2 *__restrict__ prev_out, uint2 *__restrict__ kr_out,
-    unsigned *__restrict__ cnt, float2 *__restrict__ probe_out, int *tile_made = nullptr,
-    bool valid = true, float2 *sm_p = nullptr, float2 *sm_v = nullptr, int cap = 0)
+// The end of a particle's viscosity pass: gravity and the impulses' sum dv on
+// its velocity v0, predict_positions with boundaryConditions, and the
+// predicted position's cell key counted into its build.
+__device__ __forceinline__ void viscosity_finish(int i, const Ctx &c, const Scene *S, const SG &g,
+                                                 float2 p, float2 v0, float2 dv,
+                                                 float2 *__restrict__ pos_out,
+                                                 float2 *__restrict__ prev_out,
+                                                 uint2 *__restrict__ kr_out,
+                                                 unsigned *__restrict__ cnt, int *tile_made)
 {
-    const Scene *S = c.scenes + (valid ? scene_of(c, i) : 0);
-    const SG g = load_grid(S);
     const float dt = __ldg(&S->P.time_step);
     const float gdt = __fmul_rn(-__ldg(&S->P.g), dt);
-    const float hh = __ldg(&S->P.smoothing_radius);
-    const float h2 = __fmul_rn(hh, hh);
-    const float h_recip = __fdiv_rn(1.0f, hh);
-    const float sigma = __ldg(&S->P.sigma), beta = __ldg(&S->P.beta);
-    const float dt_h = dt * h_recip;
-
-    const float2 p = valid ? pos[i] : make_float2(-1.0f, -1.0f);
-    const float2 v0 = valid ? vel[i] : make_float2(0.0f, 0.0f);  // before gravity: velocity differences need none
-    float2 v = make_float2(v0.x, __fadd_rn(v0.y, gdt));
-    float2 dv = make_float2(0.0f, 0.0f);
-    const unsigned key = cell_key(p.x, p.y, g);
-    // One pair's impulse on this particle; self (and any coincident
-    // particle) has r2 == 0 and gives none, as u is NaN in the reference for
-    // r == 0 (fluid.c:446-451).  IN_RANGE: the caller has established
-    // r2 <= h2 (a hit-mask walk recomputes the same r2).
-    const float2 mp = make_float2(-p.x, -p.y);
-    auto impulse_core = [&](const float4 &d, bool in_range) {
-        float2 e;
-        const float r2 = dist2_packed(mp, make_float2(d.x, d.y), e);
-        const float qx = e.x, qy = e.y;
-        if ((!in_range && r2 > h2) || r2 == 0.0f) return;
-        const float r_recip = rsqrtf(r2);
-        const float r = r2 * r_recip;
-        // gravity adds the same amount to both velocities: the difference
-        // is taken before it (one packed subtraction)
-        const float2 w = __fadd2_rn(v0, make_float2(-d.z, -d.w));
-        const float u0 = (w.x * qx + w.y * qy) * r_recip;
-        // only approaching pairs (u > 0) push; the others run the same
-        // instructions with u = 0, whose impulse is +-0 and leaves dv's bits
-        // as they are (no divergent branch: about half the pairs of every
-        // warp approach)
-        const float u = u0 > 0.0f ? u0 : 0.0f;
-        // dt (1 - r/h) (sigma u + beta u^2) = (dt - (dt/h) r) u (sigma + beta u)
-        const float imp = fmaf(-dt_h, r, dt) * u * fmaf(beta, u, sigma);
-        // per component imp * q * r_recip, clamped, halved and subtracted
-        // (packed FP32x2, each operation rounded as the scalar form)
-        const float2 t = __fmul2_rn(__fmul2_rn(make_float2(imp, imp), e),
-                                    make_float2(r_recip, r_recip));
-        dv = __ffma2_rn(make_float2(-0.5f, -0.5f), make_float2(clamp5(t.x), clamp5(t.y)), dv);
-    };
-    auto impulse_with = [&](const float4 &d) { impulse_core(d, false); };
-    auto load_pv = [&](int j) {
-        const float2 q = __ldg(pos + j), w = __ldg(vel + j);
-        return make_float4(q.x, q.y, w.x, w.y);
-    };
-    auto impulse = [&](int j) { impulse_with(load_pv(j)); };
-    const bool search = valid && (PROBE || st->lists_valid) &&
-                        searchable(key, i, start, g, capped, c.max_bucket);
-    int ra[3] = {0, 0, 0}, rl[3] = {0, 0, 0};
-    if (search && !capped) stencil_rows(key, start, g, ra, rl, c.n);
-    const bool masked = search && !capped && rl[0] <= kMaskRow && rl[1] <= kMaskRow &&
-                        rl[2] <= kMaskRow;
-    int d[3] = {0, 0, 0};
-    bool staged = false;
-    if (STAGED) {
-        int lo[3], hi[3];
-#pragma unroll
-        for (int r = 0; r < 3; ++r) {
-            const bool use = masked && rl[r] > 0;
-            lo[r] = use ? ra[r] : INT_MAX;
-            hi[r] = use ? ra[r] + rl[r] : INT_MIN;
-        }
-        staged = stage_rows(lo, hi, pos, sm_p, cap, d, vel, sm_v);
-    }
-    if (!valid) return;
-    if (masked) {
-        // two phases: a cheap scan marks the neighbours of each stencil
-        // row, then only they pay for the impulse (less SIMT waste)
-        auto two_phase = [&](auto SMc, const float2 *bp, const float2 *bv) {
-            constexpr bool SM = decltype(SMc)::value;
-            unsigned long long m[3];
-#pragma unroll
-            for (int r = 0; r < 3; ++r) {
-                const float2 *row = bp + ra[r] + (SM ? d[r] : 0);
-                auto at = [&](int t) { return SM ? row[t] : __ldg(row + t); };
-                const int len = rl[r];
-                // 32-bit halves: cheaper bit operations than one 64-bit mask
-                unsigned lo = 0u, hi = 0u;
-                const int n0 = min(len, 32);
-#pragma unroll kViscUnroll
-                for (int t = 0; t < n0; ++t) {
-                    float2 e;
-                    const float r2 = dist2_packed(mp, at(t), e);
-                    // self and coincident particles are marked too; the
-                    // impulse skips them (r2 == 0)
-                    lo |= (unsigned)(r2 <= h2) << t;
-                }
-#pragma unroll kViscUnroll
-                for (int t = 32; t < len; ++t) {
-                    float2 e;
-                    const float r2 = dist2_packed(mp, at(t), e);
-                    hi |= (unsigned)(r2 <= h2) << (t - 32);
-                }
-                m[r] = ((unsigned long long)hi << 32) | lo;
-            }
-            m[1] &= ~(1ull << (i - ra[1]));  // self
-#pragma unroll
-            for (int r = 0; r < 3; ++r) {
-                const int dd = SM ? d[r] : 0;
-                walk_mask<float4>(
-                    m[r], ra[r], c.n,
-                    [&](int j) {
-                        if (SM) {
-                            const float2 q = bp[j + dd], w = bv[j + dd];
-                            return make_float4(q.x, q.y, w.x, w.y);
-                        }
-                        return load_pv(j);
-                    },
-                    [&](int, const float4 &dq) { impulse_core(dq, true); });
-            }
-        };
-        if (STAGED && staged)
-            two_phase(std::integral_constant<bool, true>(), sm_p, sm_v);
-        else
-            two_phase(std::integral_constant<bool, false>(), pos, vel);
-    } else if (search) {
-        for_each_candidate(key, start, g, capped, c.max_bucket, c.n, impulse);
-    }
-    if (PROBE) {
-        probe_out[i] = dv;
-        return;
-    }
-    v.x = __fadd_rn(v.x, dv.x);
-    v.y = __fadd_rn(v.y, dv.y);
-    float nx = __fadd_rn(p.x, __fmul_rn(v.x, dt));
-    float ny = __fadd_rn(p.y, __fmul_rn(v.y, dt));
+    const float vx = __fadd_rn(v0.x, dv.x);
+    const float vy = __fadd_rn(__fadd_rn(v0.y, gdt), dv.y);
+    float nx = __fadd_rn(p.x, __fmul_rn(vx, dt));
+    float ny = __fadd_rn(p.y, __fmul_rn(vy, dt));
     boundary_of(nx, ny, S);
     const unsigned k2 = cell_key(nx, ny, g);
     unsigned rank = 0u;
@@ -778,28 +622,108 @@ __device__ __forceinline__ void viscosity_predict_one(
     kr_out[i] = make_uint2(k2, rank);
 }
 
-// The viscosity pass with the CTA's stencil rows (positions and velocities)
-// staged in shared memory.
-template <bool PERSIST>
-__global__ void __maxnreg__(48)
-k_viscosity_predict_sm(Ctx c, const DevState *__restrict__ st, const float2 *__restrict__ pos,
-                       const float2 *__restrict__ vel, const int *__restrict__ start,
-                       const unsigned *__restrict__ occ_in, unsigned *occ_reset,
-                       float2 *__restrict__ pos_out, float2 *__restrict__ prev_out,
-                       uint2 *__restrict__ kr_out, unsigned *__restrict__ cnt)
+// apply_gravity (fluid.c:398-413), viscosity_impluses (fluid.c:416-478) in
+// gather form, predict_positions (fluid.c:507-523) with boundaryConditions.
+// Gather form of the viscosity: dv_i = -1/2 sum_j clamp5(I_ij),
+// I_ij = dt (1 - r/h)(sigma u + beta u^2) (x_j - x_i)/r for u > 0,
+// u = ((v_i - v_j).(x_j - x_i))/r, all from the velocities after gravity.
+// PROBE writes dv instead of advancing.
+template <bool PROBE>
+__device__ __forceinline__ void viscosity_predict_one(
+    int i, const Ctx &c, const DevState *__restrict__ st, const float2 *__restrict__ pos,
+    const float2 *__restrict__ vel, const int *__restrict__ start, bool capped,
+    float2 *__restrict__ pos_out, float2 *__restrict__ prev_out, uint2 *__restrict__ kr_out,
+    unsigned *__restrict__ cnt, float2 *__restrict__ probe_out, int *tile_made = nullptr)
 {
-    extern __shared__ float2 sm_pv[];
-    pdl_enter();
-    if (blockIdx.x == 0 && threadIdx.x == 0) *occ_reset = 0u;
-    const bool capped = *occ_in > (unsigned)c.max_bucket;
-    const int cap = kStagePerThread * (int)blockDim.x;
-    const int ntiles = (c.n + blockDim.x - 1) / blockDim.x;
-    for (int tile = blockIdx.x; tile < ntiles; tile += PERSIST ? gridDim.x : ntiles) {
-        const int i = tile * blockDim.x + threadIdx.x;
-        viscosity_predict_one<false, true>(i, c, st, pos, vel, start, capped, pos_out, prev_out,
-                                           kr_out, cnt, nullptr, nullptr, i < c.n, sm_pv,
-                                           sm_pv + cap, cap);
+    const Scene *S = c.scenes + scene_of(c, i);
+    const SG g = load_grid(S);
+    const float dt = __ldg(&S->P.time_step);
+    const float hh = __ldg(&S->P.smoothing_radius);
+    const float h2 = __fmul_rn(hh, hh);
+    const float h_recip = __fdiv_rn(1.0f, hh);
+    const float sigma = __ldg(&S->P.sigma), beta = __ldg(&S->P.beta);
+    const float dt_h = dt * h_recip;
+
+    const float2 p = pos[i];
+    const float2 v0 = vel[i];  // before gravity: velocity differences need none
+    float2 dv = make_float2(0.0f, 0.0f);
+    const unsigned key = cell_key(p.x, p.y, g);
+    // One pair's impulse on this particle; self (and any coincident
+    // particle) has r2 == 0 and gives none, as u is NaN in the reference for
+    // r == 0 (fluid.c:446-451).  in_range: the caller has established
+    // r2 <= h2 (a hit-mask walk recomputes the same r2).
+    const float2 mp = make_float2(-p.x, -p.y);
+    auto impulse = [&](const float4 &d, bool in_range) {
+        float2 e;
+        const float r2 = dist2_packed(mp, make_float2(d.x, d.y), e);
+        const float qx = e.x, qy = e.y;
+        if (!in_range && r2 > h2) return;
+        float r_recip = rsqrt_normal(r2);
+        if (r2 < kMinNormal) {
+            if (r2 == 0.0f) return;
+            r_recip = rsqrtf(r2);
+        }
+        const float r = r2 * r_recip;
+        // gravity adds the same amount to both velocities: the difference
+        // is taken before it (one packed subtraction)
+        const float2 w = __fadd2_rn(v0, make_float2(-d.z, -d.w));
+        const float u0 = (w.x * qx + w.y * qy) * r_recip;
+        // only approaching pairs (u > 0) push; the others run the same
+        // instructions with u = 0, whose impulse is +-0 and leaves dv's bits
+        // as they are (no divergent branch: about half the pairs of every
+        // warp approach)
+        const float u = fmaxf(u0, 0.0f);  // 0 for a NaN
+        // dt (1 - r/h) (sigma u + beta u^2) = (dt - (dt/h) r) u (sigma + beta u)
+        const float imp = fmaf(-dt_h, r, dt) * u * fmaf(beta, u, sigma);
+        // per component imp * q * r_recip, clamped, halved and subtracted
+        // (packed FP32x2, each operation rounded as the scalar form)
+        const float2 t = __fmul2_rn(__fmul2_rn(make_float2(imp, imp), e),
+                                    make_float2(r_recip, r_recip));
+        dv = __ffma2_rn(make_float2(-0.5f, -0.5f), make_float2(clamp5(t.x), clamp5(t.y)), dv);
+    };
+    auto load_pv = [&](int j) {
+        const float2 q = __ldg(pos + j), w = __ldg(vel + j);
+        return make_float4(q.x, q.y, w.x, w.y);
+    };
+    if ((PROBE || st->lists_valid) && searchable(key, i, start, g, capped, c.max_bucket)) {
+        if (!capped) {
+            // two phases per 32 candidates of a stencil row: a cheap scan
+            // marks the neighbours, then only they pay for the impulse
+            // (less SIMT waste).  A piece at a time, a row of any length
+            // takes the same path: with whole rows marked first, rows of
+            // more than 64 candidates had every one of them run through the
+            // impulse (512-scene ensemble of compressed scenes: 20% of the
+            // particles).  4,194,304 particles: 236 -> 207 us early in the
+            // dam break, 285 -> 264 us compressed.
+            int ra[3], rl[3];
+            stencil_rows(p, key, start, g, ra, rl, c.n);
+#pragma unroll
+            for (int r = 0; r < 3; ++r) {
+                auto piece = [&](int a, int n) {
+                    unsigned m = hit_mask32<kMarkUnroll>(pos + a, n, mp, h2);
+                    // self is marked too; its impulse would be none
+                    if (r == 1 && (unsigned)(i - a) < 32u) m &= ~(1u << (i - a));
+                    walk_mask32<float4>(m, a, c.n, load_pv,
+                                        [&](int, const float4 &dq) { impulse(dq, true); });
+                };
+                // one piece as straight code: nearly every row (2% off the pass)
+                if (rl[r] <= 32) {
+                    piece(ra[r], rl[r]);
+                } else {
+#pragma unroll 1
+                    for (int c0 = 0; c0 < rl[r]; c0 += 32) piece(ra[r] + c0, min(rl[r] - c0, 32));
+                }
+            }
+        } else {
+            for_each_candidate(key, start, g, true, c.max_bucket, c.n,
+                               [&](int j) { impulse(load_pv(j), false); });
+        }
     }
+    if (PROBE) {
+        probe_out[i] = dv;
+        return;
+    }
+    viscosity_finish(i, c, S, g, p, v0, dv, pos_out, prev_out, kr_out, cnt, tile_made);
 }
 
 // 48 registers: more resident warps than the compiler's free choice (55),
@@ -839,122 +763,96 @@ k_viscosity_predict(Ctx c, const DevState *__restrict__ st, const float2 *__rest
 // candidates that are neighbours (r2 <= h2, self excluded), which the
 // relaxation pass of the same positions walks instead of the whole stencil.
 // The candidate filter of one particle over its three stencil rows (slots
-// [ra[r], ra[r] + rl[r])), reading the rows from global memory or, SM, from
-// the CTA's shared-memory copy (slot j of row r at base[j + d[r]]).
+// [ra[r], ra[r] + rl[r])).  Rows of up to 32 candidates are marked first and
+// the marked ones walked: the terms are run for the hits alone, where one
+// loop over the candidates runs them for nearly every candidate of a warp
+// (some lane hits).  Longer rows keep the one loop: there the lanes of a
+// warp are mostly of one cell and read the same candidate at a time, which a
+// walk over each lane's own hits does not.  4,194,304 particles: 182 -> 147
+// us early in the dam break, 201 -> 182 us compressed; two phases for rows
+// of any length 162 and 197 us.
 // mx (long-row masks): where the hit bits of candidates kMaskRow..
 // 2 kMaskRow - 1 of each row go (3 words; null: nowhere).
-template <bool SM>
 __device__ __forceinline__ void density_filter(int i, float2 mp, float h2, float h_recip,
                                                const int (&ra)[3], const int (&rl)[3],
-                                               const float2 *base, const int (&d)[3],
-                                               float2 &ab, unsigned long long (&m)[3],
+                                               const float2 *__restrict__ pos, float2 &ab,
+                                               unsigned long long (&m)[3],
                                                unsigned long long *mx = nullptr)
 {
-    // the particle's own slot in its row (row 1): never a neighbour of
-    // itself (hash.c pairs distinct particles only)
-    const int self = i - ra[1];
 #pragma unroll
     for (int r = 0; r < 3; ++r) {
-        const float2 *row = base + ra[r] + (SM ? d[r] : 0);
-        auto at = [&](int t) { return SM ? row[t] : __ldg(row + t); };
         const int len = rl[r];
-        unsigned mh[2] = {0u, 0u};  // 32-bit halves of the row's hit mask
-#pragma unroll
-        for (int hh = 0; hh < 2; ++hh) {
-            const int t1 = hh == 0 ? min(len, 32) : min(len, kMaskRow);
-#pragma unroll kDensUnroll
-            for (int t = 32 * hh; t < t1; ++t) {
+        if (len <= 32) {
+            const float2 *row = pos + ra[r];
+            unsigned b = hit_mask32<kMarkUnroll>(row, len, mp, h2);
+            if (r == 1) b &= ~(1u << (i - ra[1]));
+            m[r] = b;
+            while (b) {
+                const int t = __ffs(b) - 1;
+                b &= b - 1u;
                 float2 e;
-                const float r2 = dist2_packed(mp, at(t), e);
-                if (r2 <= h2 && (r != 1 || t != self)) {
-                    mh[hh] |= 1u << (t & 31);
+                add_density(ab, dist2_packed(mp, __ldg(row + t), e), h_recip);
+            }
+            continue;
+        }
+        unsigned long long w0 = 0ull, w1 = 0ull;
+        for (int c0 = 0; c0 < len; c0 += 32) {
+            const int a = ra[r] + c0, n = min(len - c0, 32);
+            const float2 *row = pos + a;
+            unsigned b = 0u;
+#pragma unroll kDensLongUnroll
+            for (int t = 0; t < n; ++t) {
+                float2 e;
+                const float r2 = dist2_packed(mp, __ldg(row + t), e);
+                if (r2 <= h2 && (r != 1 || a + t != i)) {
+                    b |= 1u << t;
                     add_density(ab, r2, h_recip);
                 }
             }
+            if (c0 < kMaskRow) w0 |= (unsigned long long)b << c0;
+            else if (c0 < 2 * kMaskRow) w1 |= (unsigned long long)b << (c0 - kMaskRow);
         }
-        // rows longer than the mask: with long-row masks the next kMaskRow
-        // candidates' bits go to mx; the rest have no mask bits (the
-        // relaxation then walks the whole stencil)
-        int t2 = kMaskRow;
-        if (mx != nullptr && len > kMaskRow) {
-            unsigned long long hx = 0ull;
-            t2 = min(len, 2 * kMaskRow);
-            for (int t = kMaskRow; t < t2; ++t) {
-                float2 e;
-                const float r2 = dist2_packed(mp, at(t), e);
-                if (r2 <= h2 && (r != 1 || t != self)) {
-                    hx |= 1ull << (t - kMaskRow);
-                    add_density(ab, r2, h_recip);
-                }
-            }
-            mx[r] = hx;
-        }
-        for (int t = t2; t < len; ++t) {
-            float2 e;
-            const float r2 = dist2_packed(mp, at(t), e);
-            if (r2 <= h2 && (r != 1 || t != self)) add_density(ab, r2, h_recip);
-        }
-        m[r] = ((unsigned long long)mh[1] << 32) | mh[0];
+        m[r] = w0;
+        if (mx != nullptr && len > kMaskRow) mx[r] = w1;
     }
 }
 
-// STAGED: every thread of the CTA calls this (also those with no particle,
-// valid = false), and the CTA first copies the union of its stencil rows to
-// shared memory `sm` (cap elements; stage_rows).
 // LM: long-row masks (rows of up to 2 kMaskRow candidates recorded as
 // kRowsMasked2, their second masks in c.maskx).
-template <bool STAGED = false, bool LM = false>
+template <bool LM = false>
 __device__ __forceinline__ void density_one(int i, const Ctx &c, const float2 *__restrict__ pos,
                                             const int *__restrict__ start, bool capped,
                                             float4 *__restrict__ xr_out,
                                             ulonglong2 *__restrict__ mask01,
                                             unsigned long long *__restrict__ mask2,
-                                            int4 *__restrict__ rows_out, bool valid = true,
-                                            float2 *sm = nullptr, int cap = 0)
+                                            int4 *__restrict__ rows_out)
 {
-    const Scene *S = c.scenes + (valid ? scene_of(c, i) : 0);
+    const Scene *S = c.scenes + scene_of(c, i);
     const SG g = load_grid(S);
     const float hh = __ldg(&S->P.smoothing_radius);
     const float h2 = __fmul_rn(hh, hh);
     const float h_recip = __fdiv_rn(1.0f, hh);
-    const float2 p = valid ? pos[i] : make_float2(-1.0f, -1.0f);
+    const float2 p = pos[i];
     const float2 mp = make_float2(-p.x, -p.y);
     const unsigned key = cell_key(p.x, p.y, g);
     float2 ab = make_float2(0.0f, 0.0f);  // (rho, rho_near)
     unsigned long long m[3] = {0ull, 0ull, 0ull};
     int4 rec = make_int4(0, 0, 0, kRowsNone);
-    const bool search = valid && searchable(key, i, start, g, capped, c.max_bucket);
-    int ra[3] = {0, 0, 0}, rl[3] = {0, 0, 0};
-    if (search && !capped) stencil_rows(key, start, g, ra, rl, c.n);
-    int d[3] = {0, 0, 0};
-    bool staged = false;
-    if (STAGED) {
-        int lo[3], hi[3];
-#pragma unroll
-        for (int r = 0; r < 3; ++r) {
-            const bool use = search && !capped && rl[r] > 0;
-            lo[r] = use ? ra[r] : INT_MAX;
-            hi[r] = use ? ra[r] + rl[r] : INT_MIN;
-        }
-        staged = stage_rows(lo, hi, pos, sm, cap, d);
-    }
-    if (!valid) return;
-    if (search) {
+    if (searchable(key, i, start, g, capped, c.max_bucket)) {
         rec.w = kRowsFull;
         if (!capped) {
+            int ra[3], rl[3];
+            stencil_rows(p, key, start, g, ra, rl, c.n);
             unsigned long long *mx = nullptr;
             if (rl[0] <= kMaskRow && rl[1] <= kMaskRow && rl[2] <= kMaskRow) {
                 rec = make_int4(ra[0], ra[1], ra[2], kRowsMasked);
-            } else if (LM && !STAGED && c.maskx && rl[0] <= 2 * kMaskRow &&
-                       rl[1] <= 2 * kMaskRow && rl[2] <= 2 * kMaskRow) {
+            } else if (LM && c.maskx && rl[0] <= 2 * kMaskRow && rl[1] <= 2 * kMaskRow &&
+                       rl[2] <= 2 * kMaskRow) {
                 rec = make_int4(ra[0], ra[1], ra[2], kRowsMasked2);
                 mx = c.maskx + 3 * (size_t)i;
                 mx[0] = mx[1] = mx[2] = 0ull;  // rows of kMaskRow or fewer leave theirs
             }
-            if (STAGED && staged)
-                density_filter<true>(i, mp, h2, h_recip, ra, rl, sm, d, ab, m);
-            else
-                density_filter<false>(i, mp, h2, h_recip, ra, rl, pos, d, ab, m, LM ? mx : nullptr);
+            density_filter(i, mp, h2, h_recip, ra, rl, pos, ab, m, LM ? mx : nullptr);
         } else {
             for_each_candidate(key, start, g, true, c.max_bucket, c.n, [&](int j) {
                 if (j == i) return;
@@ -971,33 +869,10 @@ __device__ __forceinline__ void density_one(int i, const Ctx &c, const float2 *_
     if (rows_out) rows_out[i] = rec;
 }
 
-// The density pass with the CTA's stencil rows staged in shared memory
-// (one tile of blockDim.x particles per CTA, or grid-stride over tiles).
-template <bool PERSIST>
-__global__ void __launch_bounds__(kMaxBlock, 4)
-k_density_sm(Ctx c, const float2 *__restrict__ pos, const int *__restrict__ start,
-             const unsigned *__restrict__ occ_in, float4 *__restrict__ xr_out,
-             ulonglong2 *__restrict__ mask01, unsigned long long *__restrict__ mask2,
-             int4 *__restrict__ rows_out)
-{
-    extern __shared__ float2 sm_pos[];
-    pdl_enter();
-    const bool capped = *occ_in > (unsigned)c.max_bucket;
-    const int ntiles = (c.n + blockDim.x - 1) / blockDim.x;
-    for (int tile = blockIdx.x; tile < ntiles; tile += PERSIST ? gridDim.x : ntiles) {
-        const int i = tile * blockDim.x + threadIdx.x;
-        density_one<true>(i, c, pos, start, capped, xr_out, mask01, mask2, rows_out, i < c.n,
-                          sm_pos, kStagePerThread * (int)blockDim.x);
-    }
-}
-
 // 32 registers (four 512-thread CTAs' worth per SM): full occupancy for this
 // issue-bound pass outweighs the few spilled values of its rare paths.
-#ifndef SPH_DENS_MIN_BLOCKS
-#define SPH_DENS_MIN_BLOCKS 4  // resident 512-thread CTAs per SM the density pass is built for
-#endif
 template <bool PERSIST, bool LM = false>
-__global__ void __launch_bounds__(kMaxBlock, SPH_DENS_MIN_BLOCKS)
+__global__ void __launch_bounds__(kMaxBlock, 4)
 k_density_t(Ctx c, const float2 *__restrict__ pos, const int *__restrict__ start,
             const unsigned *__restrict__ occ_in, float4 *__restrict__ xr_out,
             ulonglong2 *__restrict__ mask01, unsigned long long *__restrict__ mask2,
@@ -1008,11 +883,11 @@ k_density_t(Ctx c, const float2 *__restrict__ pos, const int *__restrict__ start
     const int i0 = blockIdx.x * blockDim.x + threadIdx.x;
     if (!PERSIST) {
         if (i0 < c.n)
-            density_one<false, LM>(i0, c, pos, start, capped, xr_out, mask01, mask2, rows_out);
+            density_one<LM>(i0, c, pos, start, capped, xr_out, mask01, mask2, rows_out);
         return;
     }
     for (int i = i0; i < c.n; i += gridDim.x * blockDim.x)
-        density_one<false, LM>(i, c, pos, start, capped, xr_out, mask01, mask2, rows_out);
+        density_one<LM>(i, c, pos, start, capped, xr_out, mask01, mask2, rows_out);
 }
 
 // One density launch per block (the form other translation units call).
@@ -1109,14 +984,15 @@ __device__ __forceinline__ bool relax_pair_term(const WalkConsts &c, float2 p, f
 {
     // d = q - p: the negated pair offset, rounded as p - q is
     const float r2 = dist2_packed(make_float2(-p.x, -p.y), make_float2(q.x, q.y), d);
+    float r_recip = rsqrt_normal(r2);
     if (r2 <= 2e-12f) {
         // r <= 1e-6 (rare): the owner of the pair is nudged (fluid.c:583-586)
         const float r = r2 > 0.0f ? __fsqrt_rn(r2) : 0.0f;
         if (j != i && r <= 0.000001f && owns_pair_of(S, p, ids, i, make_float2(q.x, q.y), j))
             ++nudges;
         if (!(r > 0.0f)) return false;
+        r_recip = rsqrtf(r2);
     }
-    const float r_recip = rsqrtf(r2);
     const float r = r2 * r_recip;
     const float ratio = r * c.h_recip;
     if (!(ratio < 1.0f)) return false;
@@ -1161,14 +1037,6 @@ struct LearnedIn {
     bool defer = false;  // leave the fallback particles to a second pass
 };
 
-// Where a masked walk reads its neighbours' (x, y, rho, rho_near) records:
-// global memory, or the CTA's shared-memory copy of its stencil rows
-// (stage_rows: slot j of row r at sm[j + d[r]]).
-struct RowsIn {
-    const float4 *sm = nullptr;
-    int d[3] = {0, 0, 0};
-};
-
 // The end of a particle's relaxation: x += the displacement and the owner's
 // nudges, boundaryConditions, then updateVelocity (fluid.c:627-653):
 // v = (x - x_prev)/dt clamped to +-5, and the new position's cell key
@@ -1210,8 +1078,7 @@ __device__ __forceinline__ void relax_update_one(
     const float2 *__restrict__ prev, const int *__restrict__ ids, const int *__restrict__ start,
     bool capped, float2 *__restrict__ pos_out, float2 *__restrict__ vel_out,
     uint2 *__restrict__ kr_out, unsigned *__restrict__ cnt, float2 *__restrict__ probe_out,
-    const LearnedIn &L = LearnedIn(), bool *used_net = nullptr, int *tile_made = nullptr,
-    const RowsIn &R = RowsIn())
+    const LearnedIn &L = LearnedIn(), bool *used_net = nullptr, int *tile_made = nullptr)
 {
     const Scene *S = cx.scenes + scene_of(cx, i);
     const SG g = load_grid(S);
@@ -1267,7 +1134,7 @@ __device__ __forceinline__ void relax_update_one(
             mode = kRowsNone;
         } else if (!capped) {
             int rl[3];
-            stencil_rows(key, start, g, ra, rl, cx.n);
+            stencil_rows(p, key, start, g, ra, rl, cx.n);
             if (rl[0] <= kMaskRow && rl[1] <= kMaskRow && rl[2] <= kMaskRow) {
                 mode = kRowsMasked;
             } else if (LONG_ROWS) {
@@ -1312,25 +1179,9 @@ __device__ __forceinline__ void relax_update_one(
     } else if (mode == kRowsMasked) {
         const ulonglong2 m01 = kHoist ? m01h : mask01[i];
         const unsigned long long mm[3] = {m01.x, m01.y, kHoist ? m2h : mask2[i]};
-        if (R.sm) {
-#pragma unroll
-            for (int r = 0; r < 3; ++r) {
-                const float4 *row = R.sm + R.d[r];
-                walk_mask<float4>(
-                    mm[r], ra[r], cx.n, [&](int j) { return row[j]; },
-                    [&](int j, const float4 &q) {
-                        relax_pair_walk(wc, p, q, i, j, S, ids, acc, nudges);
-                    });
-            }
-        } else {
-#pragma unroll
-            for (int r = 0; r < 3; ++r)
-                walk_mask<float4>(
-                    mm[r], ra[r], cx.n, [&](int j) { return __ldg(xr + j); },
-                    [&](int j, const float4 &q) {
-                        relax_pair_walk(wc, p, q, i, j, S, ids, acc, nudges);
-                    });
-        }
+        walk_rows<float4>(
+            mm, ra, cx.n, [&](int j) { return __ldg(xr + j); },
+            [&](int j, const float4 &q) { relax_pair_walk(wc, p, q, i, j, S, ids, acc, nudges); });
     } else if (mode == kRowsFull) {
         for_each_candidate(key, start, g, capped, cx.max_bucket, cx.n, [&](int j) {
             if (j == i) return;
@@ -1348,57 +1199,8 @@ __device__ __forceinline__ void relax_update_one(
 }
 
 
-// The slot ranges a thread's masked walk reads (stage_rows' lo, hi): for row
-// r, [ra[r], ra[r] + index of the highest hit + 1); nothing for rows without
-// hits or particles that do not walk masks.
-__device__ __forceinline__ void mask_ranges(int4 rw, unsigned long long m0, unsigned long long m1,
-                                            unsigned long long m2, int (&lo)[3], int (&hi)[3])
-{
-    const int ra[3] = {rw.x, rw.y, rw.z};
-    const unsigned long long mm[3] = {m0, m1, m2};
-#pragma unroll
-    for (int r = 0; r < 3; ++r) {
-        const bool use = rw.w == kRowsMasked && mm[r] != 0ull;
-        lo[r] = use ? ra[r] : INT_MAX;
-        hi[r] = use ? ra[r] + 64 - __clzll(mm[r]) : INT_MIN;
-    }
-}
-
-template <bool PROBE, bool PERSIST = false>
-__global__ void __launch_bounds__(kBlock, SPH_RELAX_MIN_BLOCKS)
-k_relax_update_sm(Ctx c, const float4 *__restrict__ xr, const ulonglong2 *__restrict__ mask01,
-                  const unsigned long long *__restrict__ mask2, const int4 *__restrict__ rows,
-                  const float2 *__restrict__ prev,
-                  const int *__restrict__ ids, const int *__restrict__ start,
-                  const unsigned *__restrict__ occ_in, unsigned *occ_reset,
-                  float2 *__restrict__ pos_out, float2 *__restrict__ vel_out,
-                  uint2 *__restrict__ kr_out, unsigned *__restrict__ cnt,
-                  float2 *__restrict__ probe_out)
-{
-    extern __shared__ float4 sm_rows[];
-    pdl_enter();
-    if (!PROBE && blockIdx.x == 0 && threadIdx.x == 0) *occ_reset = 0u;
-    const bool capped = *occ_in > (unsigned)c.max_bucket;
-    const int ntiles = (c.n + blockDim.x - 1) / blockDim.x;
-    for (int tile = blockIdx.x; tile < ntiles; tile += PERSIST ? gridDim.x : ntiles) {
-        const int i = tile * blockDim.x + threadIdx.x;
-        int lo[3] = {INT_MAX, INT_MAX, INT_MAX}, hi[3] = {INT_MIN, INT_MIN, INT_MIN};
-        if (i < c.n) {
-            const int4 rw = __ldg(rows + i);
-            const ulonglong2 m01 = __ldg(mask01 + i);
-            mask_ranges(rw, m01.x, m01.y, __ldg(mask2 + i), lo, hi);
-        }
-        RowsIn R;
-        if (stage_rows(lo, hi, xr, sm_rows, kStagePerThread * (int)blockDim.x, R.d)) R.sm = sm_rows;
-        if (i < c.n)
-            relax_update_one<PROBE>(i, c, xr, mask01, mask2, rows, prev, ids, start, capped,
-                                    pos_out, vel_out, kr_out, cnt, probe_out, LearnedIn(), nullptr,
-                                    nullptr, R);
-    }
-}
-
 template <bool PROBE, bool PERSIST = false, bool LM = false>
-__global__ void __launch_bounds__(kBlock, SPH_RELAX_MIN_BLOCKS)
+__global__ void __launch_bounds__(kBlock, 4)
 k_relax_update(Ctx c, const float4 *__restrict__ xr, const ulonglong2 *__restrict__ mask01,
                const unsigned long long *__restrict__ mask2, const int4 *__restrict__ rows,
                const float2 *__restrict__ prev,
@@ -1512,7 +1314,7 @@ __device__ __forceinline__ void relax_warp_one(
     const unsigned key = cell_key(p.x, p.y, g);
     if (searchable(key, i, start, g, false, cx.max_bucket)) {
         int ra[3], rl[3];
-        stencil_rows(key, start, g, ra, rl, cx.n);
+        stencil_rows(p, key, start, g, ra, rl, cx.n);
         const float2 mp = make_float2(-p.x, -p.y);
         for (int r = 0; r < 3; ++r) {
             for (int c0 = 0; c0 < rl[r]; c0 += 32) {
@@ -1876,15 +1678,6 @@ static void enqueue_predict_sort(sph_cuda *h, Mark &mark)
     const Ctx c = make_ctx(h);
     DevState *st = h->d_state;
     {
-#if SPH_VISC_SMEM
-        auto kv = h->shape[0].persistent ? k_viscosity_predict_sm<true>
-                                         : k_viscosity_predict_sm<false>;
-        const size_t smem = 2 * (size_t)kStagePerThread * h->shape[0].block * sizeof(float2);
-        launch_step(kv, gather_grid(h, h->shape[0]), h->shape[0].block, smem, h->stream, c,
-                    (const DevState *)st, (const float2 *)h->pos_a, (const float2 *)h->vel_a,
-                    (const int *)h->start_a, (const unsigned *)&st->build_max_occ[SLOT_RELAXED],
-                    &st->build_max_occ[SLOT_PREDICTED], h->pos_b, h->prev_b, h->kr_b, h->cnt);
-#else
         auto kv = h->shape[0].persistent ? k_viscosity_predict<false, true>
                                          : k_viscosity_predict<false, false>;
         launch_step(kv, gather_grid(h, h->shape[0]), h->shape[0].block, 0, h->stream, c,
@@ -1892,7 +1685,6 @@ static void enqueue_predict_sort(sph_cuda *h, Mark &mark)
                     (const int *)h->start_a, (const unsigned *)&st->build_max_occ[SLOT_RELAXED],
                     &st->build_max_occ[SLOT_PREDICTED], h->pos_b, h->prev_b, h->kr_b, h->cnt,
                     (float2 *)nullptr);
-#endif
     }
     mark();
     enqueue_cell_starts(h, h->start_c, &st->build_max_occ[SLOT_PREDICTED]);
@@ -1912,24 +1704,15 @@ static void enqueue_predict_sort(sph_cuda *h, Mark &mark)
 static void enqueue_density(sph_cuda *h)
 {
     DevState *st = h->d_state;
-#if SPH_DENS_SMEM
-    auto kd = h->shape[1].persistent ? k_density_sm<true> : k_density_sm<false>;
-    const size_t smem = (size_t)kStagePerThread * h->shape[1].block * sizeof(float2);
-#else
     auto kd = h->shape[1].persistent
                   ? (h->long_masks ? k_density_t<true, true> : k_density_t<true, false>)
                   : (h->long_masks ? k_density_t<false, true> : k_density_t<false, false>);
     const size_t smem = 0;
-#endif
     launch_step(kd, gather_grid(h, h->shape[1]), h->shape[1].block, smem, h->stream, make_ctx(h),
                 (const float2 *)h->pos_c, (const int *)h->start_c,
                 (const unsigned *)&st->build_max_occ[SLOT_PREDICTED], h->xr_c, h->mask01_c,
                 h->mask2_c, h->rows_c);
 }
-
-// Whether this build's gathers support long-row hit masks (not with the
-// shared-memory staged forms).
-bool long_masks_supported() { return !(SPH_DENS_SMEM || SPH_RELAX_SMEM); }
 
 // The density pass of a step (the learned step's features start with it).
 int launch_density_pass(sph_cuda *h)
@@ -2024,18 +1807,12 @@ int enqueue_step(sph_cuda *h, cudaEvent_t *events, int *nkernels, const tunable_
     } else {
         enqueue_density(h);
         mark();
-#if SPH_RELAX_SMEM
-        auto kr = h->shape[2].persistent ? k_relax_update_sm<false, true>
-                                         : k_relax_update_sm<false, false>;
-        const size_t smem = (size_t)kStagePerThread * h->shape[2].block * sizeof(float4);
-#else
         auto kr = h->shape[2].persistent
                       ? (h->long_masks ? k_relax_update<false, true, true>
                                        : k_relax_update<false, true, false>)
                       : (h->long_masks ? k_relax_update<false, false, true>
                                        : k_relax_update<false, false, false>);
         const size_t smem = 0;
-#endif
         launch_step(kr, gather_grid(h, h->shape[2]), h->shape[2].block, smem, h->stream, c,
                     (const float4 *)h->xr_c, (const ulonglong2 *)h->mask01_c,
                     (const unsigned long long *)h->mask2_c, (const int4 *)h->rows_c,

@@ -92,7 +92,7 @@ struct NbRec {
 // nudges) or in an overflowing bucket gets count 65535: it always takes the
 // plain relaxation.  Block 0 resets the step's fallback-list counters.
 template <bool LM>
-__global__ void __maxnreg__(48)
+__global__ void __maxnreg__(56)
 k_messages(Ctx c, const float4 *__restrict__ xr, const ulonglong2 *__restrict__ mask01,
            const unsigned long long *__restrict__ mask2, const int4 *__restrict__ rows,
            const float2 *__restrict__ prev, const int *__restrict__ start,
@@ -132,10 +132,13 @@ k_messages(Ctx c, const float4 *__restrict__ xr, const ulonglong2 *__restrict__ 
     auto visit = [&](int, const NbRec &d) {
         float2 e;  // q - p
         const float r2 = dist2_packed(mp, make_float2(d.q.x, d.q.y), e);
-        const float rinv = rsqrtf(r2);
-        const float ratio = r2 * rinv * h_recip;
+        float rinv = rsqrt_normal(r2);
         ++count;
-        degenerate |= r2 <= 2e-12f;
+        if (r2 <= 2e-12f) {
+            degenerate = true;
+            rinv = rsqrtf(r2);
+        }
+        const float ratio = r2 * rinv * h_recip;
         if (ratio < 1.0f) {
             const float omr = 1.0f - ratio;
             const float omr2 = omr * omr;
@@ -165,8 +168,7 @@ k_messages(Ctx c, const float4 *__restrict__ xr, const ulonglong2 *__restrict__ 
     if (!capped && rw.w == kRowsMasked) {
         const int ra[3] = {rw.x, rw.y, rw.z};
         const unsigned long long mm[3] = {m01.x, m01.y, m2};
-#pragma unroll
-        for (int r = 0; r < 3; ++r) walk_mask<NbRec>(mm[r], ra[r], c.n, load, visit);
+        walk_rows<NbRec>(mm, ra, c.n, load, visit);
     } else if (LM && !capped && rw.w == kRowsMasked2) {
         // long-row masks: each row's two masks in slot order
         const int ra[3] = {rw.x, rw.y, rw.z};
