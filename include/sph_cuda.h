@@ -139,7 +139,10 @@ int sph_cuda_scene_diagnostics(sph_cuda_t *h, double *out);
 /* Launch shapes of the three gather kernels (viscosity_predict, density,
  * relax_update): shapes[2k] threads per block, shapes[2k+1] 0 for one block
  * per tile of particles or the number of resident blocks per SM for a
- * persistent grid-stride launch.  Any shape gives the same results. */
+ * persistent grid-stride launch.  Any shape gives the same results.  At the
+ * default shape {256, 0} a handle of at most 40,000 particles runs its
+ * gathers with several lanes per particle; any other shape asks for one
+ * thread per particle. */
 int sph_cuda_set_launch_shapes(sph_cuda_t *h, const int *shapes);
 int sph_cuda_get_launch_shapes(sph_cuda_t *h, int *shapes);
 

@@ -1390,6 +1390,347 @@ k_relax_fallback(Ctx c, const float4 *__restrict__ xr, const ulonglong2 *__restr
 }
 
 // ---------------------------------------------------------------------------
+// the gathers with G lanes per particle (small handles)
+// ---------------------------------------------------------------------------
+
+// One thread per particle leaves the GPU nearly idle where there are few
+// particles: a pass then takes as long as one thread needs for its densest
+// particle's candidates, one after another (3,000 particles, dense: 16-30 us
+// a gather at 1-2% of the issue slots).  Here G lanes of a warp share a
+// particle: they load and test G candidates of a stencil row at once and
+// evaluate the hits' terms side by side; the terms are then added in slot
+// order from shuffles, by every lane, with the very operations of the
+// one-thread passes -- bit for bit the same sums.  A lane whose candidate
+// is no hit takes no part in the additions.
+//
+// All lanes of a warp run the same loops (bounds are maxima over its
+// groups), so that every shuffle and vote is converged; groups past the last
+// particle have empty rows.
+template <int G>
+struct Group {
+    static_assert(G == 8 || G == 16 || G == 32, "lanes per particle");
+    static constexpr unsigned kFull = 0xffffffffu;
+    int lane, gl, base;
+    __device__ __forceinline__ Group()
+    {
+        lane = threadIdx.x & 31;
+        gl = lane & (G - 1);
+        base = lane & ~(G - 1);
+    }
+    // the group's bits of a warp vote
+    __device__ __forceinline__ unsigned ballot(bool p) const
+    {
+        const unsigned b = __ballot_sync(kFull, p);
+        return G == 32 ? b : (b >> base) & ((1u << (G & 31)) - 1u);
+    }
+    __device__ __forceinline__ static int max_over_warp(int v) { return __reduce_max_sync(kFull, v); }
+    // visits the set bits of `hits` (the group's lanes) in increasing order:
+    // f(source lane, whether this group still has one)
+    template <class F>
+    __device__ __forceinline__ void ordered(unsigned hits, F &&f) const
+    {
+        const int iters = G == 32 ? __popc(hits) : max_over_warp(__popc(hits));
+#pragma unroll 4
+        for (int k = 0; k < iters; ++k) {
+            const bool on = hits != 0u;
+            const int src = base + (on ? __ffs(hits) - 1 : 0);
+            hits &= hits - 1u;
+            f(src, on);
+        }
+    }
+};
+
+// Particle i's viscosity pass by the group (every lane of the warp calls it;
+// `valid` per group; no overflowing buckets).
+template <int G>
+__device__ __forceinline__ void viscosity_group_one(
+    const Group<G> &g, int i, bool valid, const Ctx &c, const DevState *__restrict__ st,
+    const float2 *__restrict__ pos, const float2 *__restrict__ vel, const int *__restrict__ start,
+    float2 *__restrict__ pos_out, float2 *__restrict__ prev_out, uint2 *__restrict__ kr_out,
+    unsigned *__restrict__ cnt)
+{
+    const Scene *S = c.scenes + scene_of(c, i);
+    const SG sg = load_grid(S);
+    const float2 p = __ldg(pos + i), v0 = __ldg(vel + i);
+    const float dt = __ldg(&S->P.time_step);
+    const float hh = __ldg(&S->P.smoothing_radius);
+    const float h2 = __fmul_rn(hh, hh);
+    const float dt_h = dt * __fdiv_rn(1.0f, hh);
+    const float sigma = __ldg(&S->P.sigma), beta = __ldg(&S->P.beta);
+    const unsigned key = cell_key(p.x, p.y, sg);
+    int ra[3] = {0, 0, 0}, rl[3] = {0, 0, 0};
+    if (valid && st->lists_valid && searchable(key, i, start, sg, false, c.max_bucket))
+        stencil_rows(p, key, start, sg, ra, rl, c.n);
+    const float2 mp = make_float2(-p.x, -p.y);
+    float2 dv = make_float2(0.0f, 0.0f);
+    // the rows' first candidates, requested together
+    float2 q0[3], w0[3];
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+        q0[r] = w0[r] = make_float2(0.0f, 0.0f);
+        if (g.gl < rl[r]) {
+            q0[r] = __ldg(pos + ra[r] + g.gl);
+            w0[r] = __ldg(vel + ra[r] + g.gl);
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+        const int len = Group<G>::max_over_warp(rl[r]);
+        for (int t0 = 0; t0 < len; t0 += G) {
+            const int t = t0 + g.gl;
+            float2 q = q0[r], w = w0[r];
+            if (t0 > 0 && t < rl[r]) {
+                q = __ldg(pos + ra[r] + t);
+                w = __ldg(vel + ra[r] + t);
+            }
+            float2 e;
+            const float r2 = dist2_packed(mp, q, e);
+            float cx = 0.0f, cy = 0.0f;
+            bool push = false;
+            if (t < rl[r] && r2 <= h2 && r2 != 0.0f) {
+                // as viscosity_predict_one; a pair that does not approach
+                // (u <= 0) adds +-0 there and nothing here
+                const float r_recip = rsqrtf(r2);
+                const float rr = r2 * r_recip;
+                const float2 dw = __fadd2_rn(v0, make_float2(-w.x, -w.y));
+                const float u = (dw.x * e.x + dw.y * e.y) * r_recip;
+                push = u > 0.0f;
+                const float imp = fmaf(-dt_h, rr, dt) * u * fmaf(beta, u, sigma);
+                const float2 m = __fmul2_rn(__fmul2_rn(make_float2(imp, imp), e),
+                                            make_float2(r_recip, r_recip));
+                cx = clamp5(m.x);
+                cy = clamp5(m.y);
+            }
+            g.ordered(g.ballot(push), [&](int src, bool on) {
+                const float sx = __shfl_sync(Group<G>::kFull, cx, src);
+                const float sy = __shfl_sync(Group<G>::kFull, cy, src);
+                if (on) dv = __ffma2_rn(make_float2(-0.5f, -0.5f), make_float2(sx, sy), dv);
+            });
+        }
+    }
+    if (valid && g.gl == 0)
+        viscosity_finish(i, c, S, sg, p, v0, dv, pos_out, prev_out, kr_out, cnt, nullptr);
+}
+
+template <int G>
+__global__ void __launch_bounds__(kBlock)
+k_viscosity_group(Ctx c, const DevState *__restrict__ st, const float2 *__restrict__ pos,
+                  const float2 *__restrict__ vel, const int *__restrict__ start,
+                  const unsigned *__restrict__ occ_in, unsigned *occ_reset,
+                  float2 *__restrict__ pos_out, float2 *__restrict__ prev_out,
+                  uint2 *__restrict__ kr_out, unsigned *__restrict__ cnt)
+{
+    pdl_enter();
+    const int th = blockIdx.x * blockDim.x + threadIdx.x;
+    if (th == 0) *occ_reset = 0u;
+    const bool capped = *occ_in > (unsigned)c.max_bucket;
+    const Group<G> g;
+    const bool valid = th / G < c.n;
+    const int i = valid ? th / G : c.n - 1;
+    if (capped) {  // overflowing buckets (pathological): the one-thread form
+        if (valid && g.gl == 0)
+            viscosity_predict_one<false>(i, c, st, pos, vel, start, true, pos_out, prev_out, kr_out,
+                                         cnt, nullptr);
+        return;
+    }
+    viscosity_group_one<G>(g, i, valid, c, st, pos, vel, start, pos_out, prev_out, kr_out, cnt);
+}
+
+template <int G, bool LM>
+__device__ __forceinline__ void density_group_one(
+    const Group<G> &g, int i, bool valid, const Ctx &c, const float2 *__restrict__ pos,
+    const int *__restrict__ start, float4 *__restrict__ xr_out, ulonglong2 *__restrict__ mask01,
+    unsigned long long *__restrict__ mask2, int4 *__restrict__ rows_out)
+{
+    const Scene *S = c.scenes + scene_of(c, i);
+    const SG sg = load_grid(S);
+    const float2 p = __ldg(pos + i);
+    const float hh = __ldg(&S->P.smoothing_radius);
+    const float h2 = __fmul_rn(hh, hh);
+    const float h_recip = __fdiv_rn(1.0f, hh);
+    const float2 mp = make_float2(-p.x, -p.y);
+    const unsigned key = cell_key(p.x, p.y, sg);
+    const bool search = valid && searchable(key, i, start, sg, false, c.max_bucket);
+    int ra[3] = {0, 0, 0}, rl[3] = {0, 0, 0};
+    if (search) stencil_rows(p, key, start, sg, ra, rl, c.n);
+    float2 ab = make_float2(0.0f, 0.0f);
+    unsigned long long m[3] = {0ull, 0ull, 0ull}, mx[3] = {0ull, 0ull, 0ull};
+    float2 q0[3];
+#pragma unroll
+    for (int r = 0; r < 3; ++r)
+        q0[r] = g.gl < rl[r] ? __ldg(pos + ra[r] + g.gl) : make_float2(0.0f, 0.0f);
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+        const int len = Group<G>::max_over_warp(rl[r]);
+        for (int t0 = 0; t0 < len; t0 += G) {
+            const int t = t0 + g.gl;
+            float2 q = q0[r];
+            if (t0 > 0 && t < rl[r]) q = __ldg(pos + ra[r] + t);
+            float2 e;
+            const float r2 = dist2_packed(mp, q, e);
+            const bool hit = t < rl[r] && r2 <= h2 && ra[r] + t != i;
+            float2 term = make_float2(0.0f, 0.0f);
+            if (hit) add_density(term, r2, h_recip);  // 0 + x: the term itself
+            const unsigned bits = g.ballot(hit);
+            if (t0 < kMaskRow) m[r] |= (unsigned long long)bits << t0;
+            else if (LM && t0 < 2 * kMaskRow) mx[r] |= (unsigned long long)bits << (t0 - kMaskRow);
+            g.ordered(bits, [&](int src, bool on) {
+                const float ta = __shfl_sync(Group<G>::kFull, term.x, src);
+                const float tb = __shfl_sync(Group<G>::kFull, term.y, src);
+                if (on) ab = __fadd2_rn(ab, make_float2(ta, tb));
+            });
+        }
+    }
+    if (!valid || g.gl != 0) return;
+    int4 rec = make_int4(0, 0, 0, kRowsNone);
+    if (search) {
+        rec.w = kRowsFull;
+        if (rl[0] <= kMaskRow && rl[1] <= kMaskRow && rl[2] <= kMaskRow) {
+            rec = make_int4(ra[0], ra[1], ra[2], kRowsMasked);
+        } else if (LM && c.maskx && rl[0] <= 2 * kMaskRow && rl[1] <= 2 * kMaskRow &&
+                   rl[2] <= 2 * kMaskRow) {
+            rec = make_int4(ra[0], ra[1], ra[2], kRowsMasked2);
+            unsigned long long *x = c.maskx + 3 * (size_t)i;
+            x[0] = mx[0]; x[1] = mx[1]; x[2] = mx[2];
+        }
+    }
+    xr_out[i] = make_float4(p.x, p.y, ab.x, ab.y);
+    mask01[i] = make_ulonglong2(m[0], m[1]);
+    mask2[i] = m[2];
+    rows_out[i] = rec;
+}
+
+template <int G, bool LM>
+__global__ void __launch_bounds__(kBlock)
+k_density_group(Ctx c, const float2 *__restrict__ pos, const int *__restrict__ start,
+                const unsigned *__restrict__ occ_in, float4 *__restrict__ xr_out,
+                ulonglong2 *__restrict__ mask01, unsigned long long *__restrict__ mask2,
+                int4 *__restrict__ rows_out)
+{
+    pdl_enter();
+    const bool capped = *occ_in > (unsigned)c.max_bucket;
+    const int th = blockIdx.x * blockDim.x + threadIdx.x;
+    const Group<G> g;
+    const bool valid = th / G < c.n;
+    const int i = valid ? th / G : c.n - 1;
+    if (capped) {
+        if (valid && g.gl == 0)
+            density_one(i, c, pos, start, true, xr_out, mask01, mask2, rows_out);
+        return;
+    }
+    density_group_one<G, LM>(g, i, valid, c, pos, start, xr_out, mask01, mask2, rows_out);
+}
+
+template <int G, bool LM>
+__device__ __forceinline__ void relax_group_one(
+    const Group<G> &g, int i, bool valid, const Ctx &c, const float4 *__restrict__ xr,
+    const ulonglong2 *__restrict__ mask01, const unsigned long long *__restrict__ mask2,
+    const int4 *__restrict__ rows, const float2 *__restrict__ prev, const int *__restrict__ ids,
+    const int *__restrict__ start, float2 *__restrict__ pos_out, float2 *__restrict__ vel_out,
+    uint2 *__restrict__ kr_out, unsigned *__restrict__ cnt)
+{
+    // the particle's record, masks and rows, requested together
+    const float4 me = __ldg(xr + i);
+    const int4 rw = __ldg(rows + i);
+    const ulonglong2 m01 = __ldg(mask01 + i);
+    const unsigned long long m2 = __ldg(mask2 + i);
+    asm volatile("prefetch.global.L1 [%0];" ::"l"(prev + i));
+    const Scene *S = c.scenes + scene_of(c, i);
+    const RelaxConsts rc = relax_consts(S);
+    const float2 p = make_float2(me.x, me.y);
+    const WalkConsts wc = walk_consts(rc, me);
+    // the rows to visit: with hit masks only the hits are loaded (the
+    // distance test below holds for exactly those), else every candidate
+    int ra[3] = {rw.x, rw.y, rw.z}, rl[3] = {0, 0, 0};
+    unsigned long long lo[3] = {~0ull, ~0ull, ~0ull}, hi[3] = {~0ull, ~0ull, ~0ull};
+    const int mode = valid ? rw.w : kRowsNone;
+    if (mode == kRowsMasked || (LM && mode == kRowsMasked2)) {
+        lo[0] = m01.x; lo[1] = m01.y; lo[2] = m2;
+        hi[0] = hi[1] = hi[2] = 0ull;
+        if (LM && mode == kRowsMasked2) {
+            const unsigned long long *x = c.maskx + 3 * (size_t)i;
+#pragma unroll
+            for (int r = 0; r < 3; ++r) hi[r] = __ldg(x + r);
+        }
+#pragma unroll
+        for (int r = 0; r < 3; ++r) rl[r] = hi[r] ? 128 - __clzll(hi[r]) : lo[r] ? 64 - __clzll(lo[r]) : 0;
+    } else if (mode != kRowsNone) {
+        const SG sg = load_grid(S);
+        const unsigned key = cell_key(p.x, p.y, sg);
+        ra[0] = ra[1] = ra[2] = 0;
+        if (searchable(key, i, start, sg, false, c.max_bucket))
+            stencil_rows(p, key, start, sg, ra, rl, c.n);
+    }
+    const bool masked = mode != kRowsFull;
+    auto wanted = [&](int r, int t) {
+        if (t >= rl[r]) return false;
+        if (!masked) return ra[r] + t != i;
+        return t < 64 ? ((lo[r] >> t) & 1ull) != 0ull : LM && ((hi[r] >> (t - 64)) & 1ull) != 0ull;
+    };
+    float4 q0[3];
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+        q0[r] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (wanted(r, g.gl) && in_bounds(ra[r] + g.gl, c.n, kBadSlot)) q0[r] = __ldg(xr + ra[r] + g.gl);
+    }
+    float2 acc = make_float2(0.0f, 0.0f);
+    int nudges = 0;
+    const float2 mp = make_float2(-p.x, -p.y);
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+        const int len = Group<G>::max_over_warp(rl[r]);
+        for (int t0 = 0; t0 < len; t0 += G) {
+            const int t = t0 + g.gl, j = ra[r] + t;
+            float s = 0.0f;
+            float2 d = make_float2(0.0f, 0.0f);
+            bool apply = false;
+            if (wanted(r, t) && in_bounds(j, c.n, kBadSlot)) {
+                const float4 q = t0 > 0 ? __ldg(xr + j) : q0[r];
+                float2 e;
+                if (dist2_packed(mp, make_float2(q.x, q.y), e) <= rc.h2)
+                    apply = relax_pair_term(wc, p, q, i, j, S, ids, s, d, nudges);
+            }
+            g.ordered(g.ballot(apply), [&](int src, bool on) {
+                const float ss = __shfl_sync(Group<G>::kFull, s, src);
+                const float dx = __shfl_sync(Group<G>::kFull, d.x, src);
+                const float dy = __shfl_sync(Group<G>::kFull, d.y, src);
+                if (on) acc = __ffma2_rn(make_float2(-ss, -ss), make_float2(dx, dy), acc);
+            });
+        }
+    }
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1) nudges += __shfl_xor_sync(Group<G>::kFull, nudges, o);
+    if (valid && g.gl == 0)
+        relax_finish(i, c, S, p, acc, nudges, prev, pos_out, vel_out, kr_out, cnt, nullptr);
+}
+
+template <int G, bool LM>
+__global__ void __launch_bounds__(kBlock)
+k_relax_group(Ctx c, const float4 *__restrict__ xr, const ulonglong2 *__restrict__ mask01,
+              const unsigned long long *__restrict__ mask2, const int4 *__restrict__ rows,
+              const float2 *__restrict__ prev, const int *__restrict__ ids,
+              const int *__restrict__ start, const unsigned *__restrict__ occ_in,
+              unsigned *occ_reset, float2 *__restrict__ pos_out, float2 *__restrict__ vel_out,
+              uint2 *__restrict__ kr_out, unsigned *__restrict__ cnt)
+{
+    pdl_enter();
+    const int th = blockIdx.x * blockDim.x + threadIdx.x;
+    if (th == 0) *occ_reset = 0u;
+    const bool capped = *occ_in > (unsigned)c.max_bucket;
+    const Group<G> g;
+    const bool valid = th / G < c.n;
+    const int i = valid ? th / G : c.n - 1;
+    if (capped) {
+        if (valid && g.gl == 0)
+            relax_update_one<false>(i, c, xr, mask01, mask2, rows, prev, ids, start, true, pos_out,
+                                    vel_out, kr_out, cnt, nullptr);
+        return;
+    }
+    relax_group_one<G, LM>(g, i, valid, c, xr, mask01, mask2, rows, prev, ids, start, pos_out,
+                           vel_out, kr_out, cnt);
+}
+
+// ---------------------------------------------------------------------------
 // state I/O, diagnostics, neighbour lists
 // ---------------------------------------------------------------------------
 
@@ -1669,6 +2010,34 @@ static const char *const kLearnedKernelNames[] = {
     "cell_starts_2",     "cell_scatter_2", "cell_permute_2"};
 static const int kLearnedStepKernels = 11;
 
+// Lanes per particle of gather k.  The lines lie where the times of the two
+// neighbouring choices cross (dam breaks, early and compressed): the fewer
+// the particles, the more lanes it takes to fill the GPU; beyond ~40,000 one
+// thread per particle fills it, and the shared form's votes and shuffles
+// cost more than they save (the relaxation, whose one-thread walk has the
+// least to do per neighbour, first).  Microseconds a step early / compressed,
+// one thread against this: 3,000 particles 98 / 89 against 37 / 37, 10,000
+// 87 / 125 against 47 / 59, 30,000 88 / 143 against 61 / 90; at 65,536, 8
+// lanes take 89 / 132 against 89 / 139.  A launch shape other than the
+// default asks for the one-thread kernels.
+static int gather_lanes(const sph_cuda *h, int k)
+{
+    if (h->shape[k].block != kBlock || h->shape[k].persistent != 0) return 1;
+    const int n = h->n;
+    return n <= 5000 ? 32 : n <= 14000 ? 16 : n <= (k == 2 ? 30000 : 40000) ? 8 : 1;
+}
+
+// f(std::integral_constant<int, G>) for the G lanes of a group kernel.
+template <class F>
+static void with_lanes(int lanes, F &&f)
+{
+    switch (lanes) {
+    case 32: f(std::integral_constant<int, 32>()); break;
+    case 16: f(std::integral_constant<int, 16>()); break;
+    default: f(std::integral_constant<int, 8>()); break;
+    }
+}
+
 // Viscosity + prediction, the rebuild into the C order (kernels 0-3 of a step).
 template <class Mark>
 static void enqueue_predict_sort(sph_cuda *h, Mark &mark)
@@ -1677,7 +2046,16 @@ static void enqueue_predict_sort(sph_cuda *h, Mark &mark)
     const int nb = blocks_for(n);
     const Ctx c = make_ctx(h);
     DevState *st = h->d_state;
-    {
+    const int lanes = gather_lanes(h, 0);
+    if (lanes > 1) {
+        with_lanes(lanes, [&](auto G) {
+            launch_step(k_viscosity_group<G.value>, blocks_for(n * G.value), kBlock, 0, h->stream, c,
+                        (const DevState *)st, (const float2 *)h->pos_a, (const float2 *)h->vel_a,
+                        (const int *)h->start_a,
+                        (const unsigned *)&st->build_max_occ[SLOT_RELAXED],
+                        &st->build_max_occ[SLOT_PREDICTED], h->pos_b, h->prev_b, h->kr_b, h->cnt);
+        });
+    } else {
         auto kv = h->shape[0].persistent ? k_viscosity_predict<false, true>
                                          : k_viscosity_predict<false, false>;
         launch_step(kv, gather_grid(h, h->shape[0]), h->shape[0].block, 0, h->stream, c,
@@ -1704,6 +2082,17 @@ static void enqueue_predict_sort(sph_cuda *h, Mark &mark)
 static void enqueue_density(sph_cuda *h)
 {
     DevState *st = h->d_state;
+    const int lanes = gather_lanes(h, 1);
+    if (lanes > 1) {
+        with_lanes(lanes, [&](auto G) {
+            launch_step(h->long_masks ? k_density_group<G.value, true> : k_density_group<G.value, false>,
+                        blocks_for(h->n * G.value), kBlock, 0, h->stream, make_ctx(h),
+                        (const float2 *)h->pos_c, (const int *)h->start_c,
+                        (const unsigned *)&st->build_max_occ[SLOT_PREDICTED], h->xr_c, h->mask01_c,
+                        h->mask2_c, h->rows_c);
+        });
+        return;
+    }
     auto kd = h->shape[1].persistent
                   ? (h->long_masks ? k_density_t<true, true> : k_density_t<true, false>)
                   : (h->long_masks ? k_density_t<false, true> : k_density_t<false, false>);
@@ -1807,19 +2196,33 @@ int enqueue_step(sph_cuda *h, cudaEvent_t *events, int *nkernels, const tunable_
     } else {
         enqueue_density(h);
         mark();
-        auto kr = h->shape[2].persistent
-                      ? (h->long_masks ? k_relax_update<false, true, true>
-                                       : k_relax_update<false, true, false>)
-                      : (h->long_masks ? k_relax_update<false, false, true>
-                                       : k_relax_update<false, false, false>);
-        const size_t smem = 0;
-        launch_step(kr, gather_grid(h, h->shape[2]), h->shape[2].block, smem, h->stream, c,
-                    (const float4 *)h->xr_c, (const ulonglong2 *)h->mask01_c,
-                    (const unsigned long long *)h->mask2_c, (const int4 *)h->rows_c,
-                    (const float2 *)h->prev_c, (const int *)h->id_c, (const int *)h->start_c,
-                    (const unsigned *)&st->build_max_occ[SLOT_PREDICTED],
-                    &st->build_max_occ[SLOT_RELAXED], h->pos_b, h->vel_b, h->kr_b, h->cnt,
-                    (float2 *)nullptr);
+        const int lanes = gather_lanes(h, 2);
+        if (lanes > 1) {
+            with_lanes(lanes, [&](auto G) {
+                launch_step(h->long_masks ? k_relax_group<G.value, true> : k_relax_group<G.value, false>,
+                            blocks_for(n * G.value), kBlock, 0, h->stream, c,
+                            (const float4 *)h->xr_c, (const ulonglong2 *)h->mask01_c,
+                            (const unsigned long long *)h->mask2_c, (const int4 *)h->rows_c,
+                            (const float2 *)h->prev_c, (const int *)h->id_c,
+                            (const int *)h->start_c,
+                            (const unsigned *)&st->build_max_occ[SLOT_PREDICTED],
+                            &st->build_max_occ[SLOT_RELAXED], h->pos_b, h->vel_b, h->kr_b, h->cnt);
+            });
+        } else {
+            auto kr = h->shape[2].persistent
+                          ? (h->long_masks ? k_relax_update<false, true, true>
+                                           : k_relax_update<false, true, false>)
+                          : (h->long_masks ? k_relax_update<false, false, true>
+                                           : k_relax_update<false, false, false>);
+            const size_t smem = 0;
+            launch_step(kr, gather_grid(h, h->shape[2]), h->shape[2].block, smem, h->stream, c,
+                        (const float4 *)h->xr_c, (const ulonglong2 *)h->mask01_c,
+                        (const unsigned long long *)h->mask2_c, (const int4 *)h->rows_c,
+                        (const float2 *)h->prev_c, (const int *)h->id_c, (const int *)h->start_c,
+                        (const unsigned *)&st->build_max_occ[SLOT_PREDICTED],
+                        &st->build_max_occ[SLOT_RELAXED], h->pos_b, h->vel_b, h->kr_b, h->cnt,
+                        (float2 *)nullptr);
+        }
         mark();
     }
     enqueue_cell_starts(h, h->start_a, &st->build_max_occ[SLOT_RELAXED]);
