@@ -150,22 +150,25 @@ int ensure_stage(sph_cuda *h, size_t bytes)
     return SPH_OK;
 }
 
-static void destroy_graph(sph_cuda *h)
+void destroy_graph(sph_cuda *h)
 {
     if (h->exec) cudaGraphExecDestroy(h->exec);
+    if (h->exec_many) cudaGraphExecDestroy(h->exec_many);
     if (h->graph) cudaGraphDestroy(h->graph);
     h->exec = nullptr;
+    h->exec_many = nullptr;
     h->graph = nullptr;
     h->graph_n = -1;
+    h->many_calls = 0;
 }
 
-// One step as a graph (captured on the handle's stream).
-static int capture_step(sph_cuda *h)
+// `steps` steps as a graph (captured on the handle's stream).
+static int capture_steps(sph_cuda *h, int steps, cudaGraph_t *out, int *nk)
 {
-    destroy_graph(h);
+    *out = nullptr;
     SPH_CUDA(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
-    int nk = 0;
-    int rc = enqueue_step(h, nullptr, &nk);
+    int rc = SPH_OK;
+    for (int t = 0; t < steps && rc == SPH_OK; ++t) rc = enqueue_step(h, nullptr, nk);
     cudaGraph_t g = nullptr;
     const cudaError_t ce = cudaStreamEndCapture(h->stream, &g);
     if (rc != SPH_OK) {
@@ -173,8 +176,17 @@ static int capture_step(sph_cuda *h)
         return rc;
     }
     SPH_CUDA(ce);
-    h->graph = g;
-    SPH_CUDA(cudaGraphInstantiate(&h->exec, g, 0));
+    *out = g;
+    return SPH_OK;
+}
+
+// One step as a graph.
+static int capture_step(sph_cuda *h)
+{
+    destroy_graph(h);
+    int nk = 0;
+    SPH_TRY(capture_steps(h, 1, &h->graph, &nk));
+    SPH_CUDA(cudaGraphInstantiate(&h->exec, h->graph, 0));
     h->graph_n = h->n;
     h->launches_per_step = nk;
     return SPH_OK;
@@ -203,7 +215,26 @@ int run_steps(sph_cuda *h, int nsteps)
 {
     if (h->n == 0) return SPH_OK;
     if (h->graph_n != h->n) SPH_TRY(capture_step(h));
-    for (int t = 0; t < nsteps; ++t) SPH_CUDA(cudaGraphLaunch(h->exec, h->stream));
+    // Steps launched together start each step's first kernel by programmatic
+    // launch too and save the gap between graph launches (a frame of four
+    // steps of 3,000 particles: 157 -> 150 us).  Made once a handle has shown
+    // that it runs frames: the capture costs about as much as ten of them
+    // save, so it is not put on the first calls.
+    int t = 0;
+    if (nsteps >= kManySteps) {
+        if (!h->exec_many && ++h->many_calls == kManyCalls) {
+            cudaGraph_t g = nullptr;
+            int nk = 0;
+            SPH_TRY(capture_steps(h, kManySteps, &g, &nk));
+            const cudaError_t ie = cudaGraphInstantiate(&h->exec_many, g, 0);
+            cudaGraphDestroy(g);
+            SPH_CUDA(ie);
+        }
+        if (h->exec_many)
+            for (; t + kManySteps <= nsteps; t += kManySteps)
+                SPH_CUDA(cudaGraphLaunch(h->exec_many, h->stream));
+    }
+    for (; t < nsteps; ++t) SPH_CUDA(cudaGraphLaunch(h->exec, h->stream));
     return SPH_OK;
 }
 

@@ -89,6 +89,8 @@ constexpr int kBlock = 256;                           // default particle-kernel
 constexpr int kMaxBlock = 512;                        // largest block an autotuner may pick
 constexpr int kRankScanMax = 1024;  // cells above this population use atomic order
 constexpr int kMaxKernelsPerStep = 16;
+constexpr int kManySteps = 4;       // steps of a handle's multi-step graph (a frame's sub-steps)
+constexpr int kManyCalls = 8;       // the call of that many steps or more that makes it
 constexpr int kGathers = 3;         // viscosity_predict, density, relax_update
 
 // Launch shape of one gather kernel: threads per block, and 0 for one block
@@ -174,6 +176,10 @@ struct sph_cuda {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     int graph_n = -1;
+    // several steps as one graph, for calls that run that many with the same
+    // tunables (made at the kManyCalls-th such call; null: not yet)
+    cudaGraphExec_t exec_many = nullptr;
+    int many_calls = 0;
     cudaEvent_t timer[2] = {nullptr, nullptr};
     int launches_per_step = 0;
 
@@ -249,5 +255,6 @@ void free_learned_buffers(sph_cuda *h);
 const char *step_kernel_name(const sph_cuda *h, int k);
 int step_kernel_count(const sph_cuda *h);
 int run_steps(sph_cuda *h, int nsteps);
+void destroy_graph(sph_cuda *h);
 
 }  // namespace sph

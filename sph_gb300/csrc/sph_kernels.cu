@@ -490,15 +490,18 @@ k_permute(int n, const uint2 *__restrict__ kr, const int *__restrict__ start,
 // (strided by the block size, so the loads stay coalesced), their loads
 // issued together, so that each thread has K dependent chains (key -> cell
 // start -> slot) in flight instead of one.
+//
+// What a kernel reads of kernels before its predecessor it requests ahead of
+// the wait for the predecessor (their results are complete: the predecessor
+// waited for them before this kernel could start), past L1 (ld.cg), so that
+// its first loads overlap the predecessor's tail.
 template <int K>
 __global__ void __launch_bounds__(kBlock)
 k_scatter_ids_x(int n, const uint2 *__restrict__ kr, const int *__restrict__ id_src,
                 const int *__restrict__ start, int *__restrict__ tmp, unsigned *tile_cnt,
                 int ntiles)
 {
-    pdl_enter();
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
-    for (int t = g; t < ntiles; t += gridDim.x * blockDim.x) tile_cnt[t] = 0u;
     const int i0 = blockIdx.x * blockDim.x * K + threadIdx.x;
     uint2 k[K];
     int id[K], st[K];
@@ -506,10 +509,12 @@ k_scatter_ids_x(int n, const uint2 *__restrict__ kr, const int *__restrict__ id_
     for (int j = 0; j < K; ++j) {
         const int i = i0 + j * blockDim.x;
         if (i < n) {
-            k[j] = kr[i];
-            id[j] = id_src ? id_src[i] : i;
+            k[j] = __ldcg(kr + i);
+            id[j] = id_src ? __ldcg(id_src + i) : i;
         }
     }
+    pdl_enter();
+    for (int t = g; t < ntiles; t += gridDim.x * blockDim.x) tile_cnt[t] = 0u;
 #pragma unroll
     for (int j = 0; j < K; ++j)
         if (i0 + j * (int)blockDim.x < n) st[j] = __ldg(start + k[j].x);
@@ -529,11 +534,6 @@ k_permute_x(int n, const uint2 *__restrict__ kr, const int *__restrict__ start,
             int *__restrict__ id_dst, float2 *__restrict__ a_dst, float2 *__restrict__ b_dst,
             DevState *__restrict__ end_step)
 {
-    pdl_enter();
-    if (end_step && blockIdx.x == 0 && threadIdx.x == 0) {
-        end_step->lists_valid = 1u;
-        end_step->steps += 1ull;
-    }
     const int i0 = blockIdx.x * blockDim.x * K + threadIdx.x;
     uint2 k[K];
     int id[K], s0[K], s1[K];
@@ -542,18 +542,23 @@ k_permute_x(int n, const uint2 *__restrict__ kr, const int *__restrict__ start,
     for (int j = 0; j < K; ++j) {
         const int i = i0 + j * blockDim.x;
         if (i < n) {
-            k[j] = kr[i];
-            id[j] = id_src ? id_src[i] : i;
-            a[j] = a_src[i];
-            if (b_src) b[j] = b_src[i];
+            k[j] = __ldcg(kr + i);
+            id[j] = id_src ? __ldcg(id_src + i) : i;
+            a[j] = __ldcg(a_src + i);
+            if (b_src) b[j] = __ldcg(b_src + i);
         }
     }
 #pragma unroll
     for (int j = 0; j < K; ++j)
         if (i0 + j * (int)blockDim.x < n) {
-            s0[j] = __ldg(start + k[j].x);
-            s1[j] = __ldg(start + k[j].x + 1);
+            s0[j] = __ldcg(start + k[j].x);
+            s1[j] = __ldcg(start + k[j].x + 1);
         }
+    pdl_enter();
+    if (end_step && blockIdx.x == 0 && threadIdx.x == 0) {
+        end_step->lists_valid = 1u;
+        end_step->steps += 1ull;
+    }
 #pragma unroll
     for (int j = 0; j < K; ++j) {
         if (i0 + j * (int)blockDim.x >= n) continue;

@@ -1814,12 +1814,7 @@ int sph_cuda_set_learned(sph_cuda_t *h, sph_learned_t *l, float threshold)
     h->learned_thr = threshold;
     const unsigned long long zero[2] = {0ull, 0ull};
     LCUDA(cudaMemcpy(&h->d_state->learned_steps, zero, sizeof(zero), cudaMemcpyHostToDevice));
-    // the step graph changes
-    if (h->exec) cudaGraphExecDestroy(h->exec);
-    if (h->graph) cudaGraphDestroy(h->graph);
-    h->exec = nullptr;
-    h->graph = nullptr;
-    h->graph_n = -1;
+    destroy_graph(h);  // the step changes
     return SPH_OK;
 }
 
