@@ -270,8 +270,8 @@ class Simulation:
         """The render rank's liquid image of the current particles:
         (height, width, 3) uint8, top row first; with alpha=True also the
         blurred half-resolution alpha texture (bottom row first)."""
-        rgb = np.zeros((height, width, 3), np.uint8)
-        a = np.zeros((height // 2, width // 2), np.uint8) if alpha else None
+        rgb = np.empty((height, width, 3), np.uint8)
+        a = np.empty((height // 2, width // 2), np.uint8) if alpha else None
         check(lib().sph_cuda_render_liquid(self._h, int(width), int(height), rgb.ctypes.data,
                                            a.ctypes.data if alpha else None))
         return (rgb, a) if alpha else rgb
@@ -393,8 +393,8 @@ def render_liquid(coords: np.ndarray, width: int = 1920, height: int = 1080):
     """The liquid image (and the half-resolution alpha texture) from packed
     short coordinates [n, 2] (sph_render_liquid)."""
     c = np.ascontiguousarray(coords, np.int16)
-    rgb = np.zeros((height, width, 3), np.uint8)
-    a = np.zeros((height // 2, width // 2), np.uint8)
+    rgb = np.empty((height, width, 3), np.uint8)
+    a = np.empty((height // 2, width // 2), np.uint8)
     check(lib().sph_render_liquid(c.ctypes.data_as(_lib.c_short_p), int(c.shape[0]), int(width),
                                   int(height), rgb.ctypes.data, a.ctypes.data))
     return rgb, a

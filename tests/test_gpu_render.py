@@ -42,3 +42,20 @@ def test_image_edges_and_crowding(cuda_lib):
     compare(pts, 500, 300)
     rgb, a = render_liquid(np.zeros((0, 2), np.int16), 64, 32)
     assert rgb.max() == 0 and a.max() == 0
+
+
+@pytest.mark.parametrize("n,W,H", [(65535, 322, 214), (65536, 322, 214), (65537, 640, 360), (70001, 127, 250),
+                                   (66000, 2, 2), (65600, 1001, 9)])
+def test_two_pass_splat_and_row_widths(cuda_lib, n, W, H):
+    """Around the particle count from which the splat runs in two passes, with
+    rows that end on a word and rows that do not: a crowd that fills texels
+    and blocks, a thin rest, and points on the image's border.  The splat is
+    integer arithmetic: one pass over the same points in two halves of the
+    saturated range gives the same texture, so the whole image equals the
+    restatement's wherever its blurred alpha does."""
+    rng = np.random.default_rng(n)
+    crowd = rng.normal(0.0, 6000.0, (n - 3000, 2)).clip(-32767, 32767)
+    thin = rng.integers(-32767, 32768, (2990, 2))
+    border = [[-32767, -32767], [32767, 32767], [32767, -32767], [-32767, 32767], [0, 32767], [32767, 0],
+              [0, -32767], [-32767, 0], [-32768, 5], [5, -32768]]
+    compare(np.concatenate([crowd, thin, border]).astype(np.int16)[rng.permutation(n)], W, H)
