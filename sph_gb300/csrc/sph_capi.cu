@@ -19,7 +19,8 @@ namespace sph {
 int launch_unpermute(sph_cuda *h, float2 *out);
 int launch_pack(sph_cuda *h, short2 *out);
 int launch_diagnostics(sph_cuda *h, double *d_out);
-int launch_scene_diagnostics(sph_cuda *h, double *d_out);
+int launch_scene_diagnostics(sph_cuda *h, double *d_out, double *partials);
+int scene_diagnostic_pieces(const sph_cuda *h);
 int launch_probe(sph_cuda *h, int which, void *scratch, float2 *out);
 size_t probe_scratch_bytes(int n);
 int launch_half_lists(sph_cuda *h, unsigned *d_counts, int *d_off, int *d_ids, bool write);
@@ -1053,8 +1054,9 @@ int sph_cuda_scene_diagnostics(sph_cuda_t *h, double *out)
         return SPH_OK;
     }
     const size_t b = (size_t)h->nscenes * 3 * sizeof(double);
-    SPH_TRY(ensure_scratch(h, b + 16));
-    SPH_TRY(launch_scene_diagnostics(h, (double *)h->d_scratch));
+    SPH_TRY(ensure_scratch(h, b * (1 + (size_t)scene_diagnostic_pieces(h)) + 16));
+    double *d_out = (double *)h->d_scratch;
+    SPH_TRY(launch_scene_diagnostics(h, d_out, d_out + 3 * (size_t)h->nscenes));
     SPH_CUDA(cudaMemcpyAsync(out, h->d_scratch, b, cudaMemcpyDeviceToHost, h->stream));
     SPH_CUDA(cudaStreamSynchronize(h->stream));
     return SPH_OK;
