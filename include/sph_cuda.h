@@ -317,7 +317,7 @@ int sph_cuda_probe_viscosity(sph_cuda_t *h, const tunable_parameters *tp, float 
  * max_bucket_size and max_neighbors; tp gives smoothing_radius.
  *
  * Allocates nothing: every intermediate lives in one fixed-size device
- * array inside the library (about 7 MB, held on every GPU that loads the
+ * array inside the library (about 4 MB, held on every GPU that loads the
  * library until the process exits).  Rejects n > SPH_STATIC_MAX_PARTICLES
  * and size_x * size_y > SPH_STATIC_MAX_CELLS with SPH_ERR_CAPACITY.
  * Each call outside stream capture looks up that array's device address (a

@@ -42,15 +42,24 @@ struct SG {
     int size_x, size_y, ncells, c_off;
 };
 
+// 1/spacing for a power of two whose reciprocal is normal too, else 0.
+__host__ __device__ __forceinline__ float exact_reciprocal(float spacing)
+{
+    union {
+        float f;
+        unsigned u;
+    } v{spacing};
+    const unsigned e = (v.u >> 23) & 0xFFu;
+    if ((v.u & 0x807FFFFFu) != 0u || e <= 1u || e >= 253u) return 0.0f;
+    v.u = (254u - e) << 23;
+    return v.f;
+}
+
 __device__ __forceinline__ SG load_grid(const Scene *__restrict__ S)
 {
     SG g;
     g.spacing = __ldg(&S->spacing);
-    const unsigned b = __float_as_uint(g.spacing);
-    const unsigned e = (b >> 23) & 0xFFu;
-    // a normal power of two whose reciprocal is normal too
-    g.inv = ((b & 0x807FFFFFu) == 0u && e > 1u && e < 253u) ? __uint_as_float((254u - e) << 23)
-                                                           : 0.0f;
+    g.inv = exact_reciprocal(g.spacing);
     g.size_x = __ldg(&S->size_x);
     g.size_y = __ldg(&S->size_y);
     g.ncells = __ldg(&S->ncells);

@@ -103,6 +103,17 @@ struct Shape {
 
 struct LearnedModel;
 
+// The arrays of sph_cuda_density_static, in its fixed scratch.
+struct StaticArrays {
+    Scene *scene;
+    int *p_off;
+    unsigned *nocell, *cnt, *tile_cnt;
+    DevState *state;
+    int *start, *tmp, *id_s;
+    float2 *pos_in, *pos_s;
+    uint2 *kr;
+};
+
 }  // namespace sph
 
 // The handle.  Arrays named by the order they are kept in:
@@ -248,6 +259,8 @@ unsigned bounds_flags_kernels();  // checked builds (SPH_BOUNDS_CHECK): recorded
 unsigned bounds_flags_learned();
 int enqueue_predicted_state(sph_cuda *h);       // first half of a step: C order + density
 int launch_prefix(sph_cuda *h, unsigned *in, int n, int *out);  // exclusive prefix sums, out[n] = total
+int launch_static_density(const Scene &sc, const StaticArrays &a, const float *x, const float *y,
+                          float *rho, float *rho_near, cudaStream_t st);
 int launch_density_pass(sph_cuda *h);            // the density pass on the C order
 int launch_learned_passes(sph_cuda *h, cudaEvent_t *events);  // features + network (C order)
 int launch_learned_relax(sph_cuda *h, float2 *probe_out, cudaEvent_t *events = nullptr);

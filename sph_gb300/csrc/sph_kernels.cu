@@ -822,15 +822,29 @@ __device__ __forceinline__ void density_filter(int i, float2 mp, float h2, float
     }
 }
 
+// Where a density pass by itself puts its results: by particle id.
+struct DensityById {
+    const int *ids;
+    float *rho, *rho_near;
+    __device__ __forceinline__ void put(int i, float2 ab) const
+    {
+        const int id = __ldg(ids + i);
+        rho[id] = ab.x;
+        rho_near[id] = ab.y;
+    }
+};
+
 // LM: long-row masks (rows of up to 2 kMaskRow candidates recorded as
-// kRowsMasked2, their second masks in c.maskx).
-template <bool LM = false>
+// kRowsMasked2, their second masks in c.maskx).  BY_ID: the densities alone,
+// to `by_id` (no record, masks or rows).
+template <bool LM = false, bool BY_ID = false>
 __device__ __forceinline__ void density_one(int i, const Ctx &c, const float2 *__restrict__ pos,
                                             const int *__restrict__ start, bool capped,
                                             float4 *__restrict__ xr_out,
                                             ulonglong2 *__restrict__ mask01,
                                             unsigned long long *__restrict__ mask2,
-                                            int4 *__restrict__ rows_out)
+                                            int4 *__restrict__ rows_out,
+                                            const DensityById &by_id = DensityById())
 {
     const Scene *S = c.scenes + scene_of(c, i);
     const SG g = load_grid(S);
@@ -867,6 +881,10 @@ __device__ __forceinline__ void density_one(int i, const Ctx &c, const float2 *_
                 add_density(ab, r2, h_recip);
             });
         }
+    }
+    if (BY_ID) {
+        by_id.put(i, ab);
+        return;
     }
     xr_out[i] = make_float4(p.x, p.y, ab.x, ab.y);
     mask01[i] = make_ulonglong2(m[0], m[1]);
@@ -1541,11 +1559,12 @@ k_viscosity_group(Ctx c, const DevState *__restrict__ st, const float2 *__restri
     viscosity_group_one<G>(g, i, valid, c, st, pos, vel, start, pos_out, prev_out, kr_out, cnt);
 }
 
-template <int G, bool LM>
+template <int G, bool LM, bool BY_ID = false>
 __device__ __forceinline__ void density_group_one(
     const Group<G> &g, int i, bool valid, const Ctx &c, const float2 *__restrict__ pos,
     const int *__restrict__ start, float4 *__restrict__ xr_out, ulonglong2 *__restrict__ mask01,
-    unsigned long long *__restrict__ mask2, int4 *__restrict__ rows_out)
+    unsigned long long *__restrict__ mask2, int4 *__restrict__ rows_out,
+    const DensityById &by_id = DensityById())
 {
     const Scene *S = c.scenes + scene_of(c, i);
     const SG sg = load_grid(S);
@@ -1587,6 +1606,10 @@ __device__ __forceinline__ void density_group_one(
         }
     }
     if (!valid || g.gl != 0) return;
+    if (BY_ID) {
+        by_id.put(i, ab);
+        return;
+    }
     int4 rec = make_int4(0, 0, 0, kRowsNone);
     if (search) {
         rec.w = kRowsFull;
@@ -2046,11 +2069,15 @@ static const int kLearnedStepKernels = 11;
 // 87 / 125 against 47 / 59, 30,000 88 / 143 against 61 / 90; at 65,536, 8
 // lanes take 89 / 132 against 89 / 139.  A launch shape other than the
 // default asks for the one-thread kernels.
+static int lanes_for(int n, int k)
+{
+    return n <= 5000 ? 32 : n <= 14000 ? 16 : n <= (k == 2 ? 30000 : 40000) ? 8 : 1;
+}
+
 static int gather_lanes(const sph_cuda *h, int k)
 {
     if (h->shape[k].block != kBlock || h->shape[k].persistent != 0) return 1;
-    const int n = h->n;
-    return n <= 5000 ? 32 : n <= 14000 ? 16 : n <= (k == 2 ? 30000 : 40000) ? 8 : 1;
+    return lanes_for(h->n, k);
 }
 
 // f(std::integral_constant<int, G>) for the G lanes of a group kernel.
@@ -2486,6 +2513,122 @@ int launch_half_lists(sph_cuda *h, unsigned *d_counts, int *d_off, int *d_ids, b
                                                          nullptr, d_off, d_ids);
     }
     return cuda_fail(cudaGetLastError(), "half lists");
+}
+
+// ---------------------------------------------------------------------------
+// the density of caller-owned arrays (sph_cuda_density_static)
+// ---------------------------------------------------------------------------
+
+// Everything a call starts from: zero counters and tile counts, a fresh
+// state, the scene table and its no-cell bitmap.
+__global__ void __launch_bounds__(kBlock)
+k_static_init(Scene s, StaticArrays a, int ntiles)
+{
+    pdl_trigger();  // the keys may fetch the caller's positions meanwhile
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, nt = gridDim.x * blockDim.x;
+    const int M = s.ncells + 1;
+    for (int i = t; i < M; i += nt) a.cnt[i] = 0u;
+    for (int i = t; i < ntiles; i += nt) a.tile_cnt[i] = 0u;
+    for (int i = t; i < (M + 31) / 32; i += nt)
+        a.nocell[i] = i == s.ncells >> 5 ? 1u << (s.ncells & 31) : 0u;
+    if (t == 0) {
+        *a.scene = s;
+        a.p_off[0] = 0;
+        a.p_off[1] = s.n;
+        *a.state = DevState{};
+    }
+}
+
+// Positions and cell keys of the caller's arrays.
+__global__ void __launch_bounds__(kBlock)
+k_static_keys(Ctx c, SG g, const float *__restrict__ x, const float *__restrict__ y,
+              float2 *__restrict__ pos, uint2 *__restrict__ kr, unsigned *__restrict__ cnt)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    float2 p = make_float2(0.0f, 0.0f);
+    if (i < c.n) p = make_float2(__ldg(x + i), __ldg(y + i));  // the caller's: complete before the call
+    pdl_enter();
+    if (i >= c.n) return;
+    const unsigned key = cell_key(p.x, p.y, g);
+    unsigned rank = 0u;
+    if (in_bounds(key, c.M, kBadKey)) {
+        rank = atomicAdd(cnt + key, 1u);
+        add_tile_count(c.tile_cnt, key);
+    }
+    pos[i] = p;
+    kr[i] = make_uint2(key, rank);
+}
+
+template <int G>
+__global__ void __launch_bounds__(kBlock)
+k_density_static(Ctx c, const float2 *__restrict__ pos, const int *__restrict__ start,
+                 const unsigned *__restrict__ occ_in, DensityById by_id)
+{
+    pdl_enter();
+    const bool capped = *occ_in > (unsigned)c.max_bucket;
+    const int th = blockIdx.x * blockDim.x + threadIdx.x;
+    if constexpr (G > 1) {
+        const Group<G> g;
+        const bool valid = th / G < c.n;
+        const int i = valid ? th / G : c.n - 1;
+        if (!capped) {
+            density_group_one<G, false, true>(g, i, valid, c, pos, start, nullptr, nullptr, nullptr,
+                                              nullptr, by_id);
+        } else if (valid && g.gl == 0) {
+            density_one<false, true>(i, c, pos, start, true, nullptr, nullptr, nullptr, nullptr, by_id);
+        }
+    } else if (th < c.n) {
+        density_one<false, true>(th, c, pos, start, capped, nullptr, nullptr, nullptr, nullptr, by_id);
+    }
+}
+
+// Six kernels, the first launched as usual, each of the others while its
+// predecessor still runs (programmatic launch): zeroing, keys, cell starts,
+// scatter, permute, density by id.  With three memsets, nine kernels and a
+// full drain between each two, 65,521 particles took 58 us, so 23 us.
+int launch_static_density(const Scene &sc, const StaticArrays &a, const float *x, const float *y,
+                          float *rho, float *rho_near, cudaStream_t st)
+{
+    Ctx c;
+    c.scenes = a.scene;
+    c.p_off = a.p_off;
+    c.nscenes = 1;
+    c.n = sc.n;
+    c.max_bucket = sc.max_bucket;
+    c.M = sc.ncells + 1;
+    c.tile_cnt = a.tile_cnt;
+    SG g;
+    g.spacing = sc.spacing;
+    g.inv = exact_reciprocal(sc.spacing);
+    g.size_x = sc.size_x;
+    g.size_y = sc.size_y;
+    g.ncells = sc.ncells;
+    g.c_off = 0;
+    const int n = sc.n, nb = blocks_for(n), nbx = blocks_for(n, kBlock * kBuildPerThread);
+    const int ntiles = (c.M + kBuildTile - 1) / kBuildTile;
+    unsigned *occ = &a.state->build_max_occ[SLOT_PROBE];
+    k_static_init<<<blocks_for(c.M, kBlock * 4), kBlock, 0, st>>>(sc, a, ntiles);
+    launch_step(k_static_keys, nb, kBlock, 0, st, c, g, x, y, a.pos_in, a.kr, a.cnt);
+    launch_step(k_cell_starts, ntiles, kBuildThreads, 0, st, a.cnt, c.M, (const unsigned *)a.nocell,
+                (const unsigned *)a.tile_cnt, a.start, a.state, occ, sc.max_bucket, sc.max_neighbors);
+    launch_step(k_scatter_ids_x<kBuildPerThread>, nbx, kBlock, 0, st, n, (const uint2 *)a.kr,
+                (const int *)nullptr, (const int *)a.start, a.tmp, a.tile_cnt, ntiles);
+    launch_step(k_permute_x<kBuildPerThread>, nbx, kBlock, 0, st, n, (const uint2 *)a.kr,
+                (const int *)a.start, (const int *)a.tmp, (const int *)nullptr,
+                (const float2 *)a.pos_in, (const float2 *)nullptr, a.id_s, a.pos_s,
+                (float2 *)nullptr, (DevState *)nullptr);
+    const DensityById by_id{a.id_s, rho, rho_near};
+    const int lanes = lanes_for(n, 1);
+    if (lanes > 1) {
+        with_lanes(lanes, [&](auto G) {
+            launch_step(k_density_static<G.value>, blocks_for(n * G.value), kBlock, 0, st, c,
+                        (const float2 *)a.pos_s, (const int *)a.start, (const unsigned *)occ, by_id);
+        });
+    } else {
+        launch_step(k_density_static<1>, nb, kBlock, 0, st, c, (const float2 *)a.pos_s,
+                    (const int *)a.start, (const unsigned *)occ, by_id);
+    }
+    return cuda_fail(cudaGetLastError(), "sph_cuda_density_static launch");
 }
 
 }  // namespace sph

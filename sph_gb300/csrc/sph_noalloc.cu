@@ -9,34 +9,12 @@
 // fluid.c:527-539) of caller-owned device arrays, keeping every intermediate
 // (cell keys, histogram, cell starts, sorted copies) in the file-scope array
 // below, whose size is fixed at compile time.  Every GPU that loads the
-// library holds that array (about 7 MB) until the process exits.
+// library holds that array (about 4 MB) until the process exits.
 #include <mutex>
 
 #include "sph_internal.h"
 
 namespace sph {
-
-// Kernels of sph_kernels.cu, launched here unchanged.
-__global__ void k_keys(Ctx c, const float2 *__restrict__ pos, uint2 *__restrict__ kr,
-                       unsigned *__restrict__ cnt, unsigned *occ_reset);
-__global__ void k_scan_reduce(const unsigned *__restrict__ in, int M,
-                              const unsigned *__restrict__ nocell, int *__restrict__ tile_sums,
-                              DevState *__restrict__ st, unsigned *occ, int max_bucket,
-                              int max_neighbors);
-__global__ void k_scan_apply(unsigned *__restrict__ in, int M, const int *__restrict__ tile_sums,
-                             int *__restrict__ out, int zero_input);
-__global__ void k_scatter_ids(int n, const uint2 *__restrict__ kr, const int *__restrict__ id_src,
-                              const int *__restrict__ start, int *__restrict__ tmp,
-                              unsigned *tile_cnt, int ntiles);
-__global__ void k_permute(int n, const uint2 *__restrict__ kr, const int *__restrict__ start,
-                          const int *__restrict__ tmp, const int *__restrict__ id_src,
-                          const float2 *__restrict__ a_src, const float2 *__restrict__ b_src,
-                          int *__restrict__ id_dst, float2 *__restrict__ a_dst,
-                          float2 *__restrict__ b_dst, DevState *__restrict__ end_step);
-__global__ void k_density(Ctx c, const float2 *__restrict__ pos, const int *__restrict__ start,
-                          const unsigned *__restrict__ occ_in, float4 *__restrict__ xr_out,
-                          ulonglong2 *__restrict__ mask01, unsigned long long *__restrict__ mask2,
-                          int4 *__restrict__ rows_out);
 
 namespace {
 
@@ -45,7 +23,7 @@ constexpr size_t up(size_t b) { return (b + kAlign - 1) / kAlign * kAlign; }
 
 constexpr size_t kN = SPH_STATIC_MAX_PARTICLES;
 constexpr size_t kC = SPH_STATIC_MAX_CELLS;
-constexpr size_t kTiles = ((kC + 1 > kN ? kC + 1 : kN) + 1 + kScanTile - 1) / kScanTile;
+constexpr size_t kTiles = (kC + 1 + kBuildTile - 1) / kBuildTile;
 
 // Layout of the scratch array (byte offsets, each 256-byte aligned).
 constexpr size_t kNocellWords = (kC + 1 + 31) / 32 + 1;
@@ -61,10 +39,9 @@ constexpr size_t kOffKr = kOffPosIn + up(kN * sizeof(float2));
 constexpr size_t kOffTmp = kOffKr + up(kN * sizeof(uint2));
 constexpr size_t kOffPosS = kOffTmp + up(kN * sizeof(int));
 constexpr size_t kOffIdS = kOffPosS + up(kN * sizeof(float2));
-constexpr size_t kOffXr = kOffIdS + up(kN * sizeof(int));
-constexpr size_t kOffM01 = kOffXr + up(kN * sizeof(float4));
-constexpr size_t kOffM2 = kOffM01 + up(kN * sizeof(ulonglong2));
-constexpr size_t kScratchBytes = kOffM2 + up(kN * sizeof(unsigned long long));
+constexpr size_t kScratchBytes = kOffIdS + up(kN * sizeof(int));
+// the sorted positions are read up to kRowPad past their end
+static_assert(kScratchBytes - kOffIdS >= kRowPad * sizeof(float2), "padding after the sorted positions");
 
 }  // namespace
 
@@ -108,38 +85,6 @@ int scratch_address(cudaStream_t stream, void **out)
     }
     *out = g_scratch_addr[dev];
     return SPH_OK;
-}
-
-// The one-scene table of the call: scene record, slot offsets {0, n} and
-// the scene's no-cell bucket in the (cleared) no-cell bitmap.
-__global__ void k_static_scene(Scene s)
-{
-    *reinterpret_cast<Scene *>(g_static_scratch + kOffScene) = s;
-    int *p_off = reinterpret_cast<int *>(g_static_scratch + kOffPoff);
-    p_off[0] = 0;
-    p_off[1] = s.n;
-    unsigned *bits = reinterpret_cast<unsigned *>(g_static_scratch + kOffNocell);
-    bits[s.ncells >> 5] |= 1u << (s.ncells & 31);
-}
-
-__global__ void __launch_bounds__(kBlock)
-k_static_gather(int n, const float *__restrict__ x, const float *__restrict__ y,
-                float2 *__restrict__ pos)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) pos[i] = make_float2(x[i], y[i]);
-}
-
-__global__ void __launch_bounds__(kBlock)
-k_static_scatter(int n, const int *__restrict__ ids, const float4 *__restrict__ xr,
-                 float *__restrict__ rho, float *__restrict__ rho_near)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float4 v = xr[i];
-    const int id = ids[i];
-    rho[id] = v.z;
-    rho_near[id] = v.w;
 }
 
 // The counters of the last call's cell build, into caller device memory.
@@ -209,21 +154,19 @@ extern "C" int sph_cuda_density_static(const float *x, const float *y, int n,
     if (n == 0) return SPH_OK;
 
     char *base = static_cast<char *>(base_v);
-    const Scene *scene = reinterpret_cast<const Scene *>(base + kOffScene);
-    const int *p_off = reinterpret_cast<const int *>(base + kOffPoff);
-    unsigned *nocell = reinterpret_cast<unsigned *>(base + kOffNocell);
-    DevState *state = reinterpret_cast<DevState *>(base + kOffState);
-    unsigned *cnt = reinterpret_cast<unsigned *>(base + kOffCnt);
-    int *start = reinterpret_cast<int *>(base + kOffStart);
-    int *tiles = reinterpret_cast<int *>(base + kOffTiles);
-    float2 *pos_in = reinterpret_cast<float2 *>(base + kOffPosIn);
-    uint2 *kr = reinterpret_cast<uint2 *>(base + kOffKr);
-    int *tmp = reinterpret_cast<int *>(base + kOffTmp);
-    float2 *pos_s = reinterpret_cast<float2 *>(base + kOffPosS);
-    int *id_s = reinterpret_cast<int *>(base + kOffIdS);
-    float4 *xr = reinterpret_cast<float4 *>(base + kOffXr);
-    ulonglong2 *m01 = reinterpret_cast<ulonglong2 *>(base + kOffM01);
-    unsigned long long *m2 = reinterpret_cast<unsigned long long *>(base + kOffM2);
+    StaticArrays a;
+    a.scene = reinterpret_cast<Scene *>(base + kOffScene);
+    a.p_off = reinterpret_cast<int *>(base + kOffPoff);
+    a.nocell = reinterpret_cast<unsigned *>(base + kOffNocell);
+    a.state = reinterpret_cast<DevState *>(base + kOffState);
+    a.cnt = reinterpret_cast<unsigned *>(base + kOffCnt);
+    a.start = reinterpret_cast<int *>(base + kOffStart);
+    a.tile_cnt = reinterpret_cast<unsigned *>(base + kOffTiles);
+    a.pos_in = reinterpret_cast<float2 *>(base + kOffPosIn);
+    a.kr = reinterpret_cast<uint2 *>(base + kOffKr);
+    a.tmp = reinterpret_cast<int *>(base + kOffTmp);
+    a.pos_s = reinterpret_cast<float2 *>(base + kOffPosS);
+    a.id_s = reinterpret_cast<int *>(base + kOffIdS);
 
     Scene sc{};
     sc.P = *tp;
@@ -236,38 +179,6 @@ extern "C" int sph_cuda_density_static(const float *x, const float *y, int n,
     sc.n = n;
     sc.max_bucket = (int)grid->max_bucket_size;
     sc.max_neighbors = (int)grid->max_neighbors;
-    Ctx c;
-    c.scenes = scene;
-    c.p_off = p_off;
-    c.nscenes = 1;
-    c.n = n;
-    c.max_bucket = sc.max_bucket;
-    c.M = (int)cells + 1;
-
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
-    const int M = sc.ncells + 1;
-    const int nt = (M + kScanTile - 1) / kScanTile;
-    const int nb = (n + kBlock - 1) / kBlock;
-    // The array keeps the previous call's contents: the histogram and the
-    // counters must start from zero.
-    rc = cuda_fail(cudaMemsetAsync(cnt, 0, (size_t)M * sizeof(unsigned), s), "cudaMemsetAsync");
-    if (rc != SPH_OK) return rc;
-    rc = cuda_fail(cudaMemsetAsync(state, 0, sizeof(DevState), s), "cudaMemsetAsync");
-    if (rc != SPH_OK) return rc;
-    rc = cuda_fail(cudaMemsetAsync(nocell, 0, ((size_t)M + 31) / 32 * sizeof(unsigned), s),
-                   "cudaMemsetAsync");
-    if (rc != SPH_OK) return rc;
-    unsigned *occ = &state->build_max_occ[SLOT_PROBE];
-    k_static_scene<<<1, 1, 0, s>>>(sc);
-    k_static_gather<<<nb, kBlock, 0, s>>>(n, x, y, pos_in);
-    k_keys<<<nb, kBlock, 0, s>>>(c, pos_in, kr, cnt, occ);
-    k_scan_reduce<<<nt, kScanThreads, 0, s>>>(cnt, M, nocell, tiles, state, occ, sc.max_bucket,
-                                              sc.max_neighbors);
-    k_scan_apply<<<nt, kScanThreads, 0, s>>>(cnt, M, tiles, start, 1);
-    k_scatter_ids<<<nb, kBlock, 0, s>>>(n, kr, nullptr, start, tmp, nullptr, 0);
-    k_permute<<<nb, kBlock, 0, s>>>(n, kr, start, tmp, nullptr, pos_in, nullptr, id_s, pos_s,
-                                    nullptr, nullptr);
-    k_density<<<nb, kBlock, 0, s>>>(c, pos_s, start, occ, xr, m01, m2, nullptr);
-    k_static_scatter<<<nb, kBlock, 0, s>>>(n, id_s, xr, density, density_near);
-    return cuda_fail(cudaGetLastError(), "sph_cuda_density_static launch");
+    return launch_static_density(sc, a, x, y, density, density_near,
+                                 static_cast<cudaStream_t>(stream));
 }
