@@ -9,6 +9,7 @@
 #include <cstring>
 #include <new>
 
+#include <sys/mman.h>
 #include <unistd.h>
 
 #include "sph_internal.h"
@@ -23,7 +24,8 @@ int launch_scene_diagnostics(sph_cuda *h, double *d_out, double *partials);
 int scene_diagnostic_pieces(const sph_cuda *h);
 int launch_probe(sph_cuda *h, int which, void *scratch, float2 *out);
 size_t probe_scratch_bytes(int n);
-int launch_half_lists(sph_cuda *h, unsigned *d_counts, int *d_off, int *d_ids, bool write);
+int launch_half_list_counts(sph_cuda *h, unsigned *d_counts, int *d_off);
+int launch_half_lists(sph_cuda *h, const int *d_off, int *d_ids, long long lo, long long m);
 const char *kernel_name(int k);
 int step_kernel_count();
 
@@ -96,20 +98,34 @@ static void touch_pages(char *p, size_t bytes, size_t page)
 
 PageToucher::PageToucher(void *p, size_t bytes)
 {
+    if (bytes == 0) return;
     const long ps = sysconf(_SC_PAGESIZE);
     const size_t page = ps > 0 ? (size_t)ps : 4096;
     char *b = static_cast<char *>(p);
     constexpr size_t kPerThread = (size_t)4 << 20;  // a thread costs about as much as 1 MB of faults
-    const int n = (int)std::min<size_t>(4, bytes / kPerThread);
     size_t done = 0;
+    if (bytes < kPerThread / 4) {
+        touch_pages(b, bytes, page);
+        return;
+    }
     try {
+        // pages that have their memory (a buffer used before) need nothing
+        char *first = reinterpret_cast<char *>((uintptr_t)p / page * page);
+        std::vector<unsigned char> resident(((uintptr_t)b + bytes - (uintptr_t)first + page - 1) / page);
+        size_t missing = resident.size();
+        if (mincore(first, (uintptr_t)b + bytes - (uintptr_t)first, resident.data()) == 0) {
+            missing = 0;
+            for (unsigned char r : resident) missing += !(r & 1u);
+            if (missing == 0) return;
+        }
+        const int n = (int)std::min<size_t>(4, missing * page / kPerThread);
         threads_.reserve(4);
         for (int k = 0; k < n; ++k) {
             const size_t end = k == n - 1 ? bytes : bytes / n * (k + 1);
             threads_.emplace_back(touch_pages, b + done, end - done, page);
             done = end;
         }
-    } catch (...) {  // no thread to be had: the rest is touched here
+    } catch (...) {  // no memory or thread to be had: the rest is touched here
     }
     touch_pages(b + done, bytes - done, page);
 }
@@ -1062,6 +1078,9 @@ int sph_cuda_scene_diagnostics(sph_cuda_t *h, double *out)
     return SPH_OK;
 }
 
+// Entries of one piece of sph_cuda_neighbor_lists (64 MB of scratch at most).
+static constexpr long long kListPiece = 16ll << 20;
+
 int sph_cuda_neighbor_lists(sph_cuda_t *h, int *counts, int *ids, long long max_total,
                             long long *total)
 {
@@ -1073,17 +1092,25 @@ int sph_cuda_neighbor_lists(sph_cuda_t *h, int *counts, int *ids, long long max_
     const int n = h->n;
     *total = 0;
     if (n == 0) return SPH_OK;
-    // scratch: counts (n+1 words) | offsets (n+1 ints), each 256-byte aligned
+    // scratch: counts (n words) | offsets (n + 1 ints) | a piece of the lists,
+    // each 256-byte aligned
     const size_t part = (((size_t)(n + 1) * sizeof(int)) + 255) & ~(size_t)255;
-    SPH_TRY(ensure_scratch(h, 2 * part));
+    const long long piece = ids ? std::min(std::max(max_total, 0ll), kListPiece) : 0;
+    SPH_TRY(ensure_scratch(h, 2 * part + (size_t)piece * sizeof(int)));
     unsigned *d_counts = (unsigned *)h->d_scratch;
     int *d_off = (int *)((char *)h->d_scratch + part);
-    SPH_CUDA(cudaMemsetAsync(d_counts, 0, (size_t)(n + 1) * sizeof(unsigned), h->stream));
-    SPH_TRY(launch_half_lists(h, d_counts, d_off, nullptr, false));
-    SPH_CUDA(cudaMemcpyAsync(counts, d_counts, (size_t)n * sizeof(int), cudaMemcpyDeviceToHost,
-                             h->stream));
+    int *d_ids = (int *)((char *)h->d_scratch + 2 * part);
+    SPH_TRY(launch_half_list_counts(h, d_counts, d_off));
+    // the first piece (nearly always all of them) is written before the host
+    // has seen the total: the GPU does not wait for the question whether the
+    // caller's buffer holds it
+    if (piece > 0) SPH_TRY(launch_half_lists(h, d_off, d_ids, 0, piece));
+    PageToucher count_pages(counts, (size_t)n * sizeof(int));
     int tot = 0;
     SPH_CUDA(cudaMemcpyAsync(&tot, d_off + n, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+    count_pages.done();
+    SPH_CUDA(cudaMemcpyAsync(counts, d_counts, (size_t)n * sizeof(int), cudaMemcpyDeviceToHost,
+                             h->stream));
     SPH_CUDA(cudaStreamSynchronize(h->stream));
     *total = tot;
     if (tot > max_total || (!ids && tot > 0)) {
@@ -1091,16 +1118,15 @@ int sph_cuda_neighbor_lists(sph_cuda_t *h, int *counts, int *ids, long long max_
         return SPH_ERR_CAPACITY;
     }
     if (tot == 0) return SPH_OK;
-    int *d_ids = nullptr;
-    SPH_CUDA(cudaMallocAsync((void **)&d_ids, (size_t)tot * sizeof(int), h->stream));
-    int rc = launch_half_lists(h, nullptr, d_off, d_ids, true);
-    if (rc == SPH_OK)
-        rc = cuda_fail(cudaMemcpyAsync(ids, d_ids, (size_t)tot * sizeof(int),
-                                       cudaMemcpyDeviceToHost, h->stream),
-                       "list copy");
-    cudaFreeAsync(d_ids, h->stream);
-    if (rc == SPH_OK) rc = cuda_fail(cudaStreamSynchronize(h->stream), "list sync");
-    return rc;
+    PageToucher id_pages(ids, (size_t)tot * sizeof(int));
+    id_pages.done();
+    for (long long lo = 0; lo < tot; lo += piece) {
+        if (lo > 0) SPH_TRY(launch_half_lists(h, d_off, d_ids, lo, piece));
+        SPH_CUDA(cudaMemcpyAsync(ids + lo, d_ids, (size_t)std::min<long long>(piece, tot - lo) * sizeof(int),
+                                 cudaMemcpyDeviceToHost, h->stream));
+    }
+    SPH_CUDA(cudaStreamSynchronize(h->stream));
+    return SPH_OK;
 }
 
 static int probe(sph_cuda *h, const tunable_parameters *tp, int which, float *a, float *b)

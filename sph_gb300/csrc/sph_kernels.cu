@@ -1924,12 +1924,14 @@ k_diag_scenes_final(Ctx c, int pieces, const double *__restrict__ partials, doub
 // The reference's half list of one particle, in its order (hash.c:169-234):
 // later members of its own cell, then the forward cells (0,+1), (+1,-1),
 // (+1,0), (+1,+1), each in id order, r2 <= h2, cut at max_neighbors.
-// WRITE = false counts, WRITE = true writes ids at out + off[id].
+// WRITE = false counts, WRITE = true writes the entries at off[id], those of
+// them in [lo, lo + m), to out[entry - lo].
 template <bool WRITE>
 __global__ void __launch_bounds__(kBlock)
 k_half_lists(Ctx c, const float2 *__restrict__ pos, const int *__restrict__ ids,
              const int *__restrict__ start, const unsigned *__restrict__ occ_in,
-             unsigned *__restrict__ counts, const int *__restrict__ off, int *__restrict__ out)
+             unsigned *__restrict__ counts, const int *__restrict__ off, int *__restrict__ out,
+             long long lo, long long m)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= c.n) return;
@@ -1943,7 +1945,8 @@ k_half_lists(Ctx c, const float2 *__restrict__ pos, const int *__restrict__ ids,
     const unsigned key = cell_key(p.x, p.y, g);
     const int myid = ids[i];
     int cnum = 0;
-    int *dst = WRITE ? out + off[myid] : nullptr;
+    const long long first = WRITE ? off[myid] - lo : 0;
+    if (WRITE && (first >= m || off[myid + 1] - lo <= 0)) return;
     if (searchable(key, i, start, g, capped, c.max_bucket)) {
         const int lk = (int)key - g.c_off;
         const int gy = lk / g.size_x, gx = lk - gy * g.size_x;
@@ -1959,7 +1962,7 @@ k_half_lists(Ctx c, const float2 *__restrict__ pos, const int *__restrict__ ids,
                 const float2 q = pos[j];
                 if (dist2(p.x - q.x, p.y - q.y) > h2) continue;
                 if (cnum < max_neighbors) {
-                    if (WRITE) dst[cnum] = ids[j];
+                    if (WRITE && first + cnum >= 0 && first + cnum < m) out[first + cnum] = ids[j];
                     ++cnum;
                 }
             }
@@ -2494,24 +2497,26 @@ int launch_probe(sph_cuda *h, int which, void *scratch, float2 *out)
     return cuda_fail(cudaGetLastError(), "probe");
 }
 
-// Half lists in the reference's order on the A state.  d_counts: n + 1
-// words, d_off: n + 1 ints (both 16-byte aligned).
-int launch_half_lists(sph_cuda *h, unsigned *d_counts, int *d_off, int *d_ids, bool write)
+// Half lists in the reference's order on the A state: the counts by id and
+// their prefix sums (d_counts: n words, d_off: n + 1 ints, both 16-byte
+// aligned), or the entries [lo, lo + m) of the lists.
+int launch_half_list_counts(sph_cuda *h, unsigned *d_counts, int *d_off)
 {
     const int n = h->n;
     if (n == 0) return SPH_OK;
-    const int nb = blocks_for(n);
-    const Ctx c = make_ctx(h);
-    const unsigned *occ = &h->d_state->build_max_occ[SLOT_RELAXED];
-    if (!write) {
-        k_half_lists<false><<<nb, kBlock, 0, h->stream>>>(c, h->pos_a, h->id_a, h->start_a, occ,
-                                                          d_counts, nullptr, nullptr);
-        const int rc = launch_scan(h, d_counts, n, d_off, nullptr, false, nullptr);
-        if (rc != SPH_OK) return rc;
-    } else {
-        k_half_lists<true><<<nb, kBlock, 0, h->stream>>>(c, h->pos_a, h->id_a, h->start_a, occ,
-                                                         nullptr, d_off, d_ids);
-    }
+    k_half_lists<false><<<blocks_for(n), kBlock, 0, h->stream>>>(
+        make_ctx(h), h->pos_a, h->id_a, h->start_a, &h->d_state->build_max_occ[SLOT_RELAXED], d_counts,
+        nullptr, nullptr, 0, 0);
+    const int rc = launch_scan(h, d_counts, n, d_off, nullptr, false, nullptr);
+    return rc != SPH_OK ? rc : cuda_fail(cudaGetLastError(), "half list counts");
+}
+
+int launch_half_lists(sph_cuda *h, const int *d_off, int *d_ids, long long lo, long long m)
+{
+    if (h->n == 0) return SPH_OK;
+    k_half_lists<true><<<blocks_for(h->n), kBlock, 0, h->stream>>>(
+        make_ctx(h), h->pos_a, h->id_a, h->start_a, &h->d_state->build_max_occ[SLOT_RELAXED], nullptr,
+        d_off, d_ids, lo, m);
     return cuda_fail(cudaGetLastError(), "half lists");
 }
 
