@@ -35,6 +35,12 @@ namespace sph {
 // pass's long rows.
 constexpr int kMarkUnroll = 8;
 constexpr int kDensLongUnroll = 4;
+// The learned step's fallback pass: CTAs resident per SM, and how many times
+// over its grid fills the GPU (it knows its particles on the device only; with
+// one filling a list a little longer than the grid had threads left most of
+// them idle in the second turn: 94 -> 78 us at 130,000 particles).
+constexpr int kFallbackCtas = 4;
+constexpr int kFallbackWaves = 2;
 }  // namespace sph
 
 namespace sph {
@@ -990,30 +996,57 @@ __device__ __forceinline__ WalkConsts walk_consts(const RelaxConsts &c, float4 m
     return wc;
 }
 
-__device__ __noinline__ bool owns_pair_of(const Scene *S, float2 p, const int *__restrict__ ids,
-                                          int i, float2 q, int j)
+// Whether the pair of particle i (cell `key`) with slot j, r2 <= 2e-12, is one
+// whose owner i is nudged (fluid.c:583-586): r <= 1e-6 and i holds it.
+__device__ __noinline__ bool is_nudge(int i, int j, const Scene *S, const float4 *__restrict__ xr,
+                                      const int *__restrict__ ids)
 {
+    if (j == i) return false;
+    const float4 me = __ldg(xr + i), q = __ldg(xr + j);
+    float2 e;
+    const float r2 = dist2_packed(make_float2(-me.x, -me.y), make_float2(q.x, q.y), e);
+    const float r = r2 > 0.0f ? __fsqrt_rn(r2) : 0.0f;
+    if (!(r <= 0.000001f)) return false;
     const SG g = load_grid(S);
-    return owns_pair(cell_key(p.x, p.y, g), ids[i], q, ids[j], g);
+    return owns_pair(cell_key(me.x, me.y, g), ids[i], make_float2(q.x, q.y), ids[j], g);
 }
 
-// The pair term of one neighbour (r2 <= h2 known): returns whether it
-// displaces the particle, by s (p - q) with d = q - p (the caller adds
-// -s d with one packed FMA), and counts a nudge of the pair's owner.
-__device__ __forceinline__ bool relax_pair_term(const WalkConsts &c, float2 p, float4 q, int i,
-                                                int j, const Scene *S,
-                                                const int *__restrict__ ids, float &s, float2 &d,
-                                                int &nudges)
+// The nudges of particle i, searched for again once its walk has met a pair
+// that may be one -- out of line, so that neither the ids nor the scene are
+// live across the walks.
+__device__ __noinline__ int count_nudges(int i, const Scene *S, const float4 *__restrict__ xr,
+                                         const int *__restrict__ ids, const int *__restrict__ start,
+                                         bool capped, int max_bucket, int n)
+{
+    const SG g = load_grid(S);
+    const float hh = __ldg(&S->P.smoothing_radius), h2 = __fmul_rn(hh, hh);
+    const float4 me = __ldg(xr + i);
+    const float2 mp = make_float2(-me.x, -me.y);
+    const unsigned key = cell_key(me.x, me.y, g);
+    int nudges = 0;
+    if (!searchable(key, i, start, g, capped, max_bucket)) return 0;
+    for_each_candidate(key, start, g, capped, max_bucket, n, [&](int j) {
+        const float4 q = __ldg(xr + j);
+        float2 e;
+        const float r2 = dist2_packed(mp, make_float2(q.x, q.y), e);
+        if (r2 <= 2e-12f && r2 <= h2 && is_nudge(i, j, S, xr, ids)) ++nudges;
+    });
+    return nudges;
+}
+
+// The pair term of one neighbour (r2 <= h2 known, not the particle itself):
+// returns whether it displaces the particle, by s (p - q) with d = q - p (the
+// caller adds -s d with one packed FMA); `rare` is set by a pair that may be
+// a nudge (r <= 1e-6).
+__device__ __forceinline__ bool relax_pair_term(const WalkConsts &c, float2 p, float4 q, float &s,
+                                                float2 &d, bool &rare)
 {
     // d = q - p: the negated pair offset, rounded as p - q is
     const float r2 = dist2_packed(make_float2(-p.x, -p.y), make_float2(q.x, q.y), d);
     float r_recip = rsqrt_normal(r2);
     if (r2 <= 2e-12f) {
-        // r <= 1e-6 (rare): the owner of the pair is nudged (fluid.c:583-586)
-        const float r = r2 > 0.0f ? __fsqrt_rn(r2) : 0.0f;
-        if (j != i && r <= 0.000001f && owns_pair_of(S, p, ids, i, make_float2(q.x, q.y), j))
-            ++nudges;
-        if (!(r > 0.0f)) return false;
+        rare = true;
+        if (!(r2 > 0.0f)) return false;
         r_recip = rsqrtf(r2);
     }
     const float r = r2 * r_recip;
@@ -1026,15 +1059,65 @@ __device__ __forceinline__ bool relax_pair_term(const WalkConsts &c, float2 p, f
     return true;
 }
 
-__device__ __forceinline__ void relax_pair_walk(const WalkConsts &c, float2 p, float4 q, int i,
-                                                int j, const Scene *S,
-                                                const int *__restrict__ ids, float2 &a,
-                                                int &nudges)
+__device__ __forceinline__ void relax_pair_walk(const WalkConsts &c, float2 p, float4 q, float2 &a,
+                                                bool &rare)
 {
     float s;
     float2 d;
-    if (relax_pair_term(c, p, q, i, j, S, ids, s, d, nudges))
+    if (relax_pair_term(c, p, q, s, d, rare))
         a = __ffma2_rn(make_float2(-s, -s), d, a);  // += s (p - q), per component
+}
+
+// The displacement of a particle whose rows have no hit masks (a row too long
+// for them, or an overflowing bucket), in slot order, 32 candidates marked
+// and walked at a time.  Out of line: compiled into the relaxation it cost
+// the masked walk its registers.
+struct ColdSum {
+    float x, y;
+    int rare;
+};
+__device__ __noinline__ ColdSum relax_unmasked(int i, const Scene *S, const float4 *__restrict__ xr,
+                                               const int *__restrict__ start, bool capped,
+                                               int max_bucket, int n)
+{
+    const SG g = load_grid(S);
+    const RelaxConsts c = relax_consts(S);
+    const float4 me = __ldg(xr + i);
+    const WalkConsts wc = walk_consts(c, me);
+    const float2 p = make_float2(me.x, me.y), mp = make_float2(-me.x, -me.y);
+    float2 acc = make_float2(0.0f, 0.0f);
+    bool rare = false;
+    auto visit = [&](int, const float4 &q) { relax_pair_walk(wc, p, q, acc, rare); };
+    const unsigned key = cell_key(p.x, p.y, g);
+    if (searchable(key, i, start, g, capped, max_bucket)) {
+        if (!capped) {
+            int ra[3], rl[3];
+            stencil_rows(p, key, start, g, ra, rl, n);
+#pragma unroll 1
+            for (int r = 0; r < 3; ++r)
+#pragma unroll 1
+                for (int c0 = 0; c0 < rl[r]; c0 += 32) {
+                    const int a = ra[r] + c0, m = min(rl[r] - c0, 32);
+                    unsigned b = 0u;
+#pragma unroll 4
+                    for (int t = 0; t < m; ++t) {
+                        const float4 q = __ldg(xr + a + t);
+                        float2 e;
+                        if (dist2_packed(mp, make_float2(q.x, q.y), e) <= c.h2) b |= 1u << t;
+                    }
+                    if (r == 1 && (unsigned)(i - a) < 32u) b &= ~(1u << (i - a));
+                    walk_mask32<float4>(b, a, n, [&](int j) { return __ldg(xr + j); }, visit);
+                }
+        } else {
+            for_each_candidate(key, start, g, true, max_bucket, n, [&](int j) {
+                if (j == i) return;
+                const float4 q = __ldg(xr + j);
+                if (dist2(p.x - q.x, p.y - q.y) > c.h2) return;
+                visit(j, q);
+            });
+        }
+    }
+    return {acc.x, acc.y, rare ? 1 : 0};
 }
 
 // double_density_relaxation (fluid.c:541-611) in gather form:
@@ -1094,7 +1177,7 @@ __device__ __forceinline__ void relax_finish(int i, const Ctx &cx, const Scene *
     kr_out[i] = make_uint2(k2, rank);
 }
 
-template <bool PROBE, bool LEARNED = false, bool LONG_ROWS = false, bool LM = false>
+template <bool PROBE, bool LEARNED = false, bool LM = false>
 __device__ __forceinline__ void relax_update_one(
     int i, const Ctx &cx, const float4 *__restrict__ xr, const ulonglong2 *__restrict__ mask01,
     const unsigned long long *__restrict__ mask2, const int4 *__restrict__ rows,
@@ -1104,9 +1187,6 @@ __device__ __forceinline__ void relax_update_one(
     const LearnedIn &L = LearnedIn(), bool *used_net = nullptr, int *tile_made = nullptr)
 {
     const Scene *S = cx.scenes + scene_of(cx, i);
-    const SG g = load_grid(S);
-    const RelaxConsts c = relax_consts(S);
-
     const float4 me = xr[i];
     // the plain pass requests the hit masks with the record and prefetches
     // the previous position, so that their DRAM latencies overlap instead of
@@ -1114,25 +1194,24 @@ __device__ __forceinline__ void relax_update_one(
     // relax_finish reads the previous position): 7% off this latency-bound
     // pass
     constexpr bool kHoist = !LEARNED;
-    ulonglong2 m01h = make_ulonglong2(0ull, 0ull);
-    unsigned long long m2h = 0ull;
-    if (kHoist && rows) {
-        m01h = __ldg(mask01 + i);
-        m2h = __ldg(mask2 + i);
-        asm volatile("prefetch.global.L1 [%0];" ::"l"(prev + i));
+    ulonglong2 m01 = make_ulonglong2(0ull, 0ull);
+    unsigned long long m2 = 0ull;
+    if (kHoist) {
+        m01 = __ldg(mask01 + i);
+        m2 = __ldg(mask2 + i);
+        if (!PROBE) asm volatile("prefetch.global.L1 [%0];" ::"l"(prev + i));
     }
     const float2 p = make_float2(me.x, me.y);
-    const WalkConsts wc = walk_consts(c, me);
     float2 acc = make_float2(0.0f, 0.0f);  // the displacement
-    int nudges = 0;
-    bool net = false;
+    bool rare = false, net = false;
     if (LEARNED) {
         // the network's output requested with the count (not after it), and
         // the previous position prefetched for relax_finish: one DRAM latency
         // for a network particle instead of three in a row
         const float4 y = __ldg(L.net + i);
-        asm volatile("prefetch.global.L1 [%0];" ::"l"(prev + i));
+        if (!PROBE) asm volatile("prefetch.global.L1 [%0];" ::"l"(prev + i));
         if ((int)__ldg(L.nbc + i) <= L.max_nb && y.z <= L.thr_pct) {
+            const RelaxConsts c = relax_consts(S);
             const float s = c.hh * c.dt2 * (c.k + c.k_near + 2.0f * c.half_spring);
             acc = make_float2(y.x * s, y.y * s);
             net = true;
@@ -1140,79 +1219,40 @@ __device__ __forceinline__ void relax_update_one(
     }
     if (LEARNED && used_net) *used_net = net;
     if (LEARNED && !net && L.defer) return;
-    // the density pass's row record: the stencil rows' first slots, so the
-    // walk needs neither the cell key nor the cell starts (without one, the
-    // rows are found here)
-    int mode = net ? kRowsNone : kRowsFull;
-    int ra[3] = {0, 0, 0};
-    if (!net && rows) {
+    if (!net) {
+        // the density pass's row record: the stencil rows' first slots, so
+        // the walk needs neither the cell key nor the cell starts
         const int4 rw = __ldg(rows + i);
-        mode = rw.w;
-        ra[0] = rw.x; ra[1] = rw.y; ra[2] = rw.z;
-    }
-    unsigned key = 0u;
-    if (mode == kRowsFull) {
-        key = cell_key(p.x, p.y, g);
-        if (!searchable(key, i, start, g, capped, cx.max_bucket)) {
-            mode = kRowsNone;
-        } else if (!capped) {
-            int rl[3];
-            stencil_rows(p, key, start, g, ra, rl, cx.n);
-            if (rl[0] <= kMaskRow && rl[1] <= kMaskRow && rl[2] <= kMaskRow) {
-                mode = kRowsMasked;
-            } else if (LONG_ROWS) {
-                // a row longer than one mask (dense cells): filter and walk
-                // 64 candidates at a time, in slot order -- for the fallback
-                // pass, whose particles are the dense ones (in the full pass
-                // the extra code costs the common path more than it saves)
-                const float2 mp = make_float2(-p.x, -p.y);
-                auto xr_pos = [&](int j) {
-                    const float4 q = __ldg(xr + j);
-                    return make_float2(q.x, q.y);
-                };
-                for (int r = 0; r < 3; ++r)
-                    walk_row_hits<float4>(
-                        ra[r], rl[r], r == 1 ? i : -1, cx.n, mp, c.h2, xr_pos,
-                        [&](int j) { return __ldg(xr + j); },
-                        [&](int j, const float4 &q) {
-                            relax_pair_walk(wc, p, q, i, j, S, ids, acc, nudges);
-                        });
-                mode = kRowsNone;
+        const int ra[3] = {rw.x, rw.y, rw.z};
+        if (rw.w == kRowsMasked || (LM && rw.w == kRowsMasked2)) {
+            const WalkConsts wc = walk_consts(relax_consts(S), me);
+            if (!kHoist) {
+                m01 = __ldg(mask01 + i);
+                m2 = __ldg(mask2 + i);
             }
+            const unsigned long long mm[3] = {m01.x, m01.y, m2};
+            auto load = [&](int j) { return __ldg(xr + j); };
+            auto visit = [&](int, const float4 &q) { relax_pair_walk(wc, p, q, acc, rare); };
+            if (!LM || rw.w == kRowsMasked) {
+                walk_rows<float4>(mm, ra, cx.n, load, visit);
+            } else {
+                // rows of up to 2 kMaskRow candidates: each row's two masks in
+                // slot order (the visiting order of the whole-stencil walk)
+                const unsigned long long *mx = cx.maskx + 3 * (size_t)i;
+                const unsigned long long mh[3] = {__ldg(mx), __ldg(mx + 1), __ldg(mx + 2)};
+#pragma unroll
+                for (int r = 0; r < 3; ++r) {
+                    walk_mask<float4>(mm[r], ra[r], cx.n, load, visit);
+                    walk_mask<float4>(mh[r], ra[r] + kMaskRow, cx.n, load, visit);
+                }
+            }
+        } else if (rw.w != kRowsNone) {
+            const ColdSum r = relax_unmasked(i, S, xr, start, capped, cx.max_bucket, cx.n);
+            acc = make_float2(r.x, r.y);
+            rare = r.rare != 0;
         }
     }
-    if (LM && mode == kRowsMasked2) {
-        // rows of up to 2 kMaskRow candidates: each row's two masks in slot
-        // order (the visiting order of the whole-stencil walk)
-        const ulonglong2 m01 = kHoist ? m01h : mask01[i];
-        const unsigned long long mm[3] = {m01.x, m01.y, kHoist ? m2h : mask2[i]};
-        const unsigned long long *mx = cx.maskx + 3 * (size_t)i;
-        const unsigned long long mh[3] = {__ldg(mx), __ldg(mx + 1), __ldg(mx + 2)};
-#pragma unroll
-        for (int r = 0; r < 3; ++r) {
-#pragma unroll
-            for (int q = 0; q < 2; ++q)
-                walk_mask<float4>(
-                    q ? mh[r] : mm[r], ra[r] + q * kMaskRow, cx.n,
-                    [&](int j) { return __ldg(xr + j); },
-                    [&](int j, const float4 &qv) {
-                        relax_pair_walk(wc, p, qv, i, j, S, ids, acc, nudges);
-                    });
-        }
-    } else if (mode == kRowsMasked) {
-        const ulonglong2 m01 = kHoist ? m01h : mask01[i];
-        const unsigned long long mm[3] = {m01.x, m01.y, kHoist ? m2h : mask2[i]};
-        walk_rows<float4>(
-            mm, ra, cx.n, [&](int j) { return __ldg(xr + j); },
-            [&](int j, const float4 &q) { relax_pair_walk(wc, p, q, i, j, S, ids, acc, nudges); });
-    } else if (mode == kRowsFull) {
-        for_each_candidate(key, start, g, capped, cx.max_bucket, cx.n, [&](int j) {
-            if (j == i) return;
-            const float4 q = __ldg(xr + j);
-            if (dist2(p.x - q.x, p.y - q.y) > c.h2) return;
-            relax_pair_walk(wc, p, q, i, j, S, ids, acc, nudges);
-        });
-    }
+    const int nudges = rare ? count_nudges(i, S, xr, ids, start, capped, cx.max_bucket, cx.n) : 0;
     if (PROBE) {
         const float nd = (float)nudges * 0.000001f;
         probe_out[i] = make_float2(acc.x + nd, acc.y + nd);
@@ -1221,9 +1261,12 @@ __device__ __forceinline__ void relax_update_one(
     relax_finish(i, cx, S, p, acc, nudges, prev, pos_out, vel_out, kr_out, cnt, tile_made);
 }
 
-
+// 48 registers: 40 resident warps per SM instead of 32 (64 registers) for
+// this latency-bound pass; what the rare paths would need is out of line
+// (4,194,304 particles: 178 -> 160 us early in the dam break, 227 -> 209 us
+// compressed).
 template <bool PROBE, bool PERSIST = false, bool LM = false>
-__global__ void __launch_bounds__(kBlock, 4)
+__global__ void __maxnreg__(48)
 k_relax_update(Ctx c, const float4 *__restrict__ xr, const ulonglong2 *__restrict__ mask01,
                const unsigned long long *__restrict__ mask2, const int4 *__restrict__ rows,
                const float2 *__restrict__ prev,
@@ -1239,13 +1282,13 @@ k_relax_update(Ctx c, const float4 *__restrict__ xr, const ulonglong2 *__restric
     const bool capped = *occ_in > (unsigned)c.max_bucket;
     if (!PERSIST) {
         if (i0 < c.n)
-            relax_update_one<PROBE, false, false, LM>(i0, c, xr, mask01, mask2, rows, prev, ids,
+            relax_update_one<PROBE, false, LM>(i0, c, xr, mask01, mask2, rows, prev, ids,
                                                       start, capped, pos_out, vel_out, kr_out,
                                                       cnt, probe_out);
         return;
     }
     for (int i = i0; i < c.n; i += gridDim.x * blockDim.x)
-        relax_update_one<PROBE, false, false, LM>(i, c, xr, mask01, mask2, rows, prev, ids, start,
+        relax_update_one<PROBE, false, LM>(i, c, xr, mask01, mask2, rows, prev, ids, start,
                                                   capped, pos_out, vel_out, kr_out, cnt,
                                                   probe_out);
 }
@@ -1276,7 +1319,7 @@ k_relax_learned(Ctx c, const float4 *__restrict__ xr, const ulonglong2 *__restri
     L.defer = !PROBE;
     int t = -1;
     if (i < c.n)
-        relax_update_one<PROBE, true, false, LM>(i, c, xr, mask01, mask2, rows, prev, ids, start, capped, pos_out,
+        relax_update_one<PROBE, true, LM>(i, c, xr, mask01, mask2, rows, prev, ids, start, capped, pos_out,
                                       vel_out, kr_out, cnt, probe_out, L, &used, &t);
     if (PROBE) return;
     if (c.tile_cnt) cta_tile_count(c.tile_cnt, t);
@@ -1303,115 +1346,6 @@ k_relax_learned(Ctx c, const float4 *__restrict__ xr, const ulonglong2 *__restri
     }
 }
 
-// The plain relaxation and update of particle i by a whole warp: the lanes
-// test 32 stencil candidates at a time and evaluate the pair terms of the
-// hits in parallel; the displacement is then accumulated from them in slot
-// order, row by row, with the same packed FMA as the one-thread walk, so the
-// result is bit for bit the one-thread result (the plain step's).  Lane 0
-// finishes the particle.  The learned step's fallback particles are its
-// dense ones (long stencil rows): one thread each made them a long tail.
-__device__ __forceinline__ void relax_warp_one(
-    int i, const Ctx &cx, const float4 *__restrict__ xr, const ulonglong2 *__restrict__ mask01,
-    const unsigned long long *__restrict__ mask2, const int4 *__restrict__ rows,
-    const float2 *__restrict__ prev, const int *__restrict__ ids, const int *__restrict__ start,
-    bool capped, float2 *__restrict__ pos_out, float2 *__restrict__ vel_out,
-    uint2 *__restrict__ kr_out, unsigned *__restrict__ cnt)
-{
-    const unsigned lane = threadIdx.x & 31u;
-    if (capped) {
-        // overflowing buckets (pathological): the one-thread form
-        if (lane == 0)
-            relax_update_one<false, false, true>(i, cx, xr, mask01, mask2, rows, prev, ids, start,
-                                                 capped, pos_out, vel_out, kr_out, cnt, nullptr);
-        return;
-    }
-    const Scene *S = cx.scenes + scene_of(cx, i);
-    const SG g = load_grid(S);
-    const RelaxConsts c = relax_consts(S);
-    const float h2 = c.h2;
-    const float4 me = xr[i];
-    const float2 p = make_float2(me.x, me.y);
-    const WalkConsts wc = walk_consts(c, me);  // as relax_update_one's
-    float2 acc = make_float2(0.0f, 0.0f);
-    int nudges = 0;
-    const unsigned key = cell_key(p.x, p.y, g);
-    if (searchable(key, i, start, g, false, cx.max_bucket)) {
-        int ra[3], rl[3];
-        stencil_rows(p, key, start, g, ra, rl, cx.n);
-        const float2 mp = make_float2(-p.x, -p.y);
-        for (int r = 0; r < 3; ++r) {
-            for (int c0 = 0; c0 < rl[r]; c0 += 32) {
-                const int t = c0 + (int)lane;
-                const int j = ra[r] + t;
-                float s = 0.0f;
-                float2 d = make_float2(0.0f, 0.0f);
-                bool apply = false;
-                if (t < rl[r] && j != i && in_bounds(j, cx.n, kBadSlot)) {
-                    const float4 q = __ldg(xr + j);
-                    float2 e;
-                    if (dist2_packed(mp, make_float2(q.x, q.y), e) <= h2)
-                        apply = relax_pair_term(wc, p, q, i, j, S, ids, s, d, nudges);
-                }
-                unsigned hits = __ballot_sync(0xffffffffu, apply);
-                while (hits) {
-                    const int b = __ffs(hits) - 1;
-                    hits &= hits - 1u;
-                    const float sb = __shfl_sync(0xffffffffu, s, b);
-                    const float dx = __shfl_sync(0xffffffffu, d.x, b);
-                    const float dy = __shfl_sync(0xffffffffu, d.y, b);
-                    acc = __ffma2_rn(make_float2(-sb, -sb), make_float2(dx, dy), acc);
-                }
-            }
-        }
-        nudges = __reduce_add_sync(0xffffffffu, nudges);
-    }
-    if (lane == 0) relax_finish(i, cx, S, p, acc, nudges, prev, pos_out, vel_out, kr_out, cnt,
-                                nullptr);
-}
-
-// The fallback particles of a learned step: the plain relaxation + update
-// for each slot on fb_list -- one thread per particle for those at its front
-// (rows within the hit masks), then one warp per particle for those at its
-// back (a row too long for a mask: the densest, whose one-thread walks were
-// the long tail).  Grid-stride loops: the counts are known on the device
-// only.  Block 0 adds the counts to the fallback statistics.
-template <bool LM = false>
-__global__ void __launch_bounds__(kBlock, 4)
-k_relax_fallback(Ctx c, const float4 *__restrict__ xr, const ulonglong2 *__restrict__ mask01,
-                 const unsigned long long *__restrict__ mask2, const int4 *__restrict__ rows,
-                 const float2 *__restrict__ prev,
-                 const int *__restrict__ ids, const int *__restrict__ start,
-                 const unsigned *__restrict__ occ_in, float2 *__restrict__ pos_out,
-                 float2 *__restrict__ vel_out, uint2 *__restrict__ kr_out,
-                 unsigned *__restrict__ cnt, DevState *st, const int *__restrict__ fb_list)
-{
-    const unsigned total = st->fb_count, total_long = st->fb_long;
-    if (blockIdx.x == 0 && threadIdx.x == 0)
-        atomicAdd(&st->learned_fallback, (unsigned long long)(total + total_long));
-    const bool capped = *occ_in > (unsigned)c.max_bucket;
-    const unsigned t0 = blockIdx.x * blockDim.x + threadIdx.x;
-    const unsigned nt = gridDim.x * blockDim.x;
-    for (unsigned k = t0; k < total; k += nt)
-        relax_update_one<false, false, true, LM>(fb_list[k], c, xr, mask01, mask2, rows, prev,
-                                                 ids, start, capped, pos_out, vel_out, kr_out,
-                                                 cnt, nullptr);
-    // the long-row particles: a warp each when they are few enough for one
-    // pass of the grid's warps (the long tail of a step with a few dense
-    // spots), else a thread each (many dense particles: a warp each would
-    // leave most of them waiting).  Both sum in slot order: the same bits.
-    const unsigned w0 = t0 >> 5, nw = nt >> 5;
-    if (total_long <= nw) {
-        for (unsigned k = w0; k < total_long; k += nw)
-            relax_warp_one(fb_list[c.n - 1 - (int)k], c, xr, mask01, mask2, rows, prev, ids,
-                           start, capped, pos_out, vel_out, kr_out, cnt);
-    } else {
-        for (unsigned k = t0; k < total_long; k += nt)
-            relax_update_one<false, false, true, LM>(fb_list[c.n - 1 - (int)k], c, xr, mask01,
-                                                     mask2, rows, prev, ids, start, capped,
-                                                     pos_out, vel_out, kr_out, cnt, nullptr);
-    }
-}
-
 // ---------------------------------------------------------------------------
 // the gathers with G lanes per particle (small handles)
 // ---------------------------------------------------------------------------
@@ -1431,7 +1365,7 @@ k_relax_fallback(Ctx c, const float4 *__restrict__ xr, const ulonglong2 *__restr
 // particle have empty rows.
 template <int G>
 struct Group {
-    static_assert(G == 8 || G == 16 || G == 32, "lanes per particle");
+    static_assert(G == 4 || G == 8 || G == 16 || G == 32, "lanes per particle");
     static constexpr unsigned kFull = 0xffffffffu;
     int lane, gl, base;
     __device__ __forceinline__ Group()
@@ -1715,8 +1649,11 @@ __device__ __forceinline__ void relax_group_one(
             if (wanted(r, t) && in_bounds(j, c.n, kBadSlot)) {
                 const float4 q = t0 > 0 ? __ldg(xr + j) : q0[r];
                 float2 e;
-                if (dist2_packed(mp, make_float2(q.x, q.y), e) <= rc.h2)
-                    apply = relax_pair_term(wc, p, q, i, j, S, ids, s, d, nudges);
+                if (dist2_packed(mp, make_float2(q.x, q.y), e) <= rc.h2) {
+                    bool rare = false;
+                    apply = relax_pair_term(wc, p, q, s, d, rare);
+                    if (rare && is_nudge(i, j, S, xr, ids)) ++nudges;
+                }
             }
             g.ordered(g.ballot(apply), [&](int src, bool on) {
                 const float ss = __shfl_sync(Group<G>::kFull, s, src);
@@ -1756,6 +1693,51 @@ k_relax_group(Ctx c, const float4 *__restrict__ xr, const ulonglong2 *__restrict
     }
     relax_group_one<G, LM>(g, i, valid, c, xr, mask01, mask2, rows, prev, ids, start, pos_out,
                            vel_out, kr_out, cnt);
+}
+
+// The fallback particles of a learned step: the plain relaxation + update for
+// each slot on fb_list (those with hit masks from its front, those with a row
+// too long for them from its back).  They are the densest particles, with the
+// longest walks of all, and mostly too few to fill the GPU with a thread
+// each: 32 or 4 lanes a particle while the grid holds them in one pass, else
+// a thread each (at two passes of 4 lanes the threads are the faster).  The
+// same bits either way.  The dam break's 1,048,576 particles: 26,000 on the
+// list 61 -> 35 us, 90,000 72 -> 53 us.  Grid-stride loops: the counts are
+// known on the device only.  Block 0 adds them to the fallback statistics.
+template <bool LM>
+__global__ void __launch_bounds__(kBlock, kFallbackCtas)
+k_relax_fallback(Ctx c, const float4 *__restrict__ xr, const ulonglong2 *__restrict__ mask01,
+                 const unsigned long long *__restrict__ mask2, const int4 *__restrict__ rows,
+                 const float2 *__restrict__ prev,
+                 const int *__restrict__ ids, const int *__restrict__ start,
+                 const unsigned *__restrict__ occ_in, float2 *__restrict__ pos_out,
+                 float2 *__restrict__ vel_out, uint2 *__restrict__ kr_out,
+                 unsigned *__restrict__ cnt, DevState *st, const int *__restrict__ fb_list)
+{
+    const unsigned front = st->fb_count, total = front + st->fb_long;
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+        atomicAdd(&st->learned_fallback, (unsigned long long)total);
+    const bool capped = *occ_in > (unsigned)c.max_bucket;
+    const unsigned t0 = blockIdx.x * blockDim.x + threadIdx.x;
+    const unsigned nt = gridDim.x * blockDim.x, resident = nt / kFallbackWaves;
+    auto slot_of = [&](unsigned k) { return fb_list[k < front ? (int)k : c.n - 1 - (int)(k - front)]; };
+    auto by_groups = [&](auto G) {
+        const Group<G.value> g;
+        const unsigned k = t0 / G.value, k0 = (t0 & ~31u) / G.value;
+        if (k0 >= total) return;  // the whole warp
+        const bool valid = k < total;
+        relax_group_one<G.value, LM>(g, slot_of(valid ? k : k0), valid, c, xr, mask01, mask2, rows, prev,
+                                     ids, start, pos_out, vel_out, kr_out, cnt);
+    };
+    if (!capped && total <= resident / 32) {
+        by_groups(std::integral_constant<int, 32>());
+    } else if (!capped && total <= resident / 4) {
+        by_groups(std::integral_constant<int, 4>());
+    } else {
+        for (unsigned k = t0; k < total; k += nt)
+            relax_update_one<false, false, LM>(slot_of(k), c, xr, mask01, mask2, rows, prev, ids, start,
+                                               capped, pos_out, vel_out, kr_out, cnt, nullptr);
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -2210,7 +2192,7 @@ int launch_learned_relax(sph_cuda *h, float2 *probe_out, cudaEvent_t *events)
         &st->build_max_occ[SLOT_RELAXED], h->pos_b, h->vel_b, h->kr_b, h->cnt, nullptr, L, st,
         h->fb_list);
     if (events) cudaEventRecord(events[0], h->stream);
-    const int fb_blocks = std::min(nb, 4 * h->num_sms);
+    const int fb_blocks = kFallbackWaves * kFallbackCtas * h->num_sms;
     (lm ? k_relax_fallback<true> : k_relax_fallback<false>)<<<fb_blocks, kBlock, 0, h->stream>>>(
         c, h->xr_c, h->mask01_c, h->mask2_c, h->rows_c, h->prev_c, h->id_c, h->start_c, occ,
         h->pos_b, h->vel_b, h->kr_b, h->cnt, st, h->fb_list);

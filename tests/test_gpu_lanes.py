@@ -7,7 +7,7 @@ import numpy as np
 import pytest
 
 from conftest import bits_equal
-from sph_gb300 import Simulation, scenes
+from sph_gb300 import LearnedModel, Simulation, scenes
 
 pytestmark = pytest.mark.gpu
 
@@ -50,3 +50,22 @@ def test_lanes_give_the_one_thread_results(cuda_lib, n, lattice, h, long_masks):
     for k in (0, 1):
         for f in FIELDS:
             assert bits_equal(out[0][k][f], out[1][k][f]), (k, f)
+
+
+@pytest.mark.parametrize("n", [1, 4000, 16384, 50000, 320000])
+@pytest.mark.parametrize("lattice", [0.5, 0.14])
+def test_learned_fallback_by_lanes_is_the_plain_step(cuda_lib, n, lattice):
+    """Every particle on the learned step's fallback list, from lists of 32
+    and 4 lanes a particle to more than the pass has threads: the plain
+    step's bits, coincident pairs included."""
+    sc = block(n, lattice, 1.0)
+    P = sc.params.as_dict()
+    with Simulation.from_scene(sc) as plain, Simulation.from_scene(sc) as learned, LearnedModel(0, seed=1) as m:
+        plain.set_launch_shapes(ONE_THREAD)
+        learned.set_learned(m, threshold=-1.0)
+        for s in (plain, learned):
+            s.step(P, 5)
+        a, b = plain.download(), learned.download()
+        assert learned.learned_counts() == (0, 5 * n)
+    for f in FIELDS:
+        assert bits_equal(a[f], b[f]), f
