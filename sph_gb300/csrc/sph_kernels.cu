@@ -30,11 +30,18 @@
 #include "sph_learned.h"
 
 namespace sph {
+// Stencil rows of up to kShortRow candidates have their hits marked first and
+// then walked, longer ones are gathered in one loop over the candidates
+// (density_filter and viscosity_long_rows say why; with the line at 20 to 28
+// the dam break's 1,048,576 particles lost 2-8% of the viscosity pass and the
+// other states stayed within 1%).
+constexpr int kShortRow = 32;
 // Unroll factors of the candidate loops (tuned on GB300): the blocks of a
-// mark-then-walk scan (hit_mask32), and the single-phase loop of the density
-// pass's long rows.
+// mark-then-walk scan (hit_mask32), and the single-phase loops of the density
+// and viscosity passes' long rows.
 constexpr int kMarkUnroll = 8;
 constexpr int kDensLongUnroll = 4;
+constexpr int kViscLongUnroll = 8;
 // The learned step's fallback pass: CTAs resident per SM, and how many times
 // over its grid fills the GPU (it knows its particles on the device only; with
 // one filling a list a little longer than the grid had threads left most of
@@ -633,6 +640,109 @@ __device__ __forceinline__ void viscosity_finish(int i, const Ctx &c, const Scen
     kr_out[i] = make_uint2(k2, rank);
 }
 
+// The scene constants of a pair's viscosity impulse, and the impulse itself.
+struct ViscConsts {
+    float h2, dt, dt_h, sigma, beta;
+};
+
+__device__ __forceinline__ ViscConsts visc_consts(const Scene *S)
+{
+    ViscConsts c;
+    c.dt = __ldg(&S->P.time_step);
+    const float hh = __ldg(&S->P.smoothing_radius);
+    c.h2 = __fmul_rn(hh, hh);
+    c.dt_h = c.dt * __fdiv_rn(1.0f, hh);
+    c.sigma = __ldg(&S->P.sigma);
+    c.beta = __ldg(&S->P.beta);
+    return c;
+}
+
+// One neighbour's impulse on the particle at -mp with velocity v0, added to
+// dv; d = (position, velocity), r2 <= h2 known, velocities before gravity
+// (which adds the same amount to both).  Self (and any coincident particle)
+// has r2 == 0 and gives none, as u is NaN in the reference for r == 0
+// (fluid.c:446-451).
+__device__ __forceinline__ void visc_impulse(const ViscConsts &c, float2 e, float r2, float2 v0,
+                                             float2 dvel, float2 &dv)
+{
+    float r_recip = rsqrt_normal(r2);
+    if (r2 < kMinNormal) {
+        if (r2 == 0.0f) return;
+        r_recip = rsqrtf(r2);
+    }
+    const float r = r2 * r_recip;
+    const float2 w = __fadd2_rn(v0, make_float2(-dvel.x, -dvel.y));
+    const float u0 = (w.x * e.x + w.y * e.y) * r_recip;
+    // only approaching pairs (u > 0) push; the others run the same
+    // instructions with u = 0, whose impulse is +-0 and leaves dv's bits
+    // as they are (no divergent branch: about half the pairs of every
+    // warp approach)
+    const float u = fmaxf(u0, 0.0f);  // 0 for a NaN
+    // dt (1 - r/h) (sigma u + beta u^2) = (dt - (dt/h) r) u (sigma + beta u)
+    const float imp = fmaf(-c.dt_h, r, c.dt) * u * fmaf(c.beta, u, c.sigma);
+    // per component imp * q * r_recip, clamped, halved and subtracted
+    // (packed FP32x2, each operation rounded as the scalar form)
+    const float2 t = __fmul2_rn(__fmul2_rn(make_float2(imp, imp), e),
+                                make_float2(r_recip, r_recip));
+    dv = __ffma2_rn(make_float2(-0.5f, -0.5f), make_float2(clamp5(t.x), clamp5(t.y)), dv);
+}
+
+// The sum of a particle with a stencil row of more than 32 candidates, or
+// with an overflowing bucket somewhere: rows of up to 32 marked and walked,
+// longer ones in one loop over the candidates (the lanes of a warp are then
+// mostly of one cell and read the same candidate at a time, which a walk over
+// each lane's own hits does not: the dam break's 1,048,576 particles
+// compressed: all rows marked and walked 218 us, this 187 us; 64 scenes 231
+// and 220 us).  Out of line:
+// compiled into the pass it cost the short rows' walk its registers.
+__device__ __noinline__ float2 viscosity_long_rows(int i, const Scene *S,
+                                                   const float2 *__restrict__ pos,
+                                                   const float2 *__restrict__ vel,
+                                                   const int *__restrict__ start, bool capped,
+                                                   int max_bucket, int n)
+{
+    const SG g = load_grid(S);
+    const ViscConsts vc = visc_consts(S);
+    const float2 p = __ldg(pos + i), v0 = __ldg(vel + i);
+    const float2 mp = make_float2(-p.x, -p.y);
+    const unsigned key = cell_key(p.x, p.y, g);
+    float2 dv = make_float2(0.0f, 0.0f);
+    if (capped) {
+        for_each_candidate(key, start, g, true, max_bucket, n, [&](int j) {
+            const float2 q = __ldg(pos + j);
+            float2 e;
+            const float r2 = dist2_packed(mp, q, e);
+            if (!(r2 > vc.h2)) visc_impulse(vc, e, r2, v0, __ldg(vel + j), dv);
+        });
+        return dv;
+    }
+    auto one = [&](int j) {
+        const float2 q = __ldg(pos + j), w = __ldg(vel + j);
+        float2 e;
+        const float r2 = dist2_packed(mp, q, e);
+        if (r2 <= vc.h2) visc_impulse(vc, e, r2, v0, w, dv);
+    };
+    int ra[3], rl[3];
+    stencil_rows(p, key, start, g, ra, rl, n);
+#pragma unroll 1
+    for (int r = 0; r < 3; ++r) {
+        const int a = ra[r], l = rl[r];
+        if (l <= kShortRow) {
+            unsigned b = hit_mask32<kMarkUnroll>(pos + a, l, mp, vc.h2);
+            if (r == 1) b &= ~(1u << (i - a));
+            while (b) {
+                const int j = a + __ffs(b) - 1;
+                b &= b - 1u;
+                one(j);
+            }
+        } else {
+#pragma unroll kViscLongUnroll
+            for (int j = a; j < a + l; ++j) one(j);
+        }
+    }
+    return dv;
+}
+
 // apply_gravity (fluid.c:398-413), viscosity_impluses (fluid.c:416-478) in
 // gather form, predict_positions (fluid.c:507-523) with boundaryConditions.
 // Gather form of the viscosity: dv_i = -1/2 sum_j clamp5(I_ij),
@@ -648,86 +758,35 @@ __device__ __forceinline__ void viscosity_predict_one(
 {
     const Scene *S = c.scenes + scene_of(c, i);
     const SG g = load_grid(S);
-    const float dt = __ldg(&S->P.time_step);
-    const float hh = __ldg(&S->P.smoothing_radius);
-    const float h2 = __fmul_rn(hh, hh);
-    const float h_recip = __fdiv_rn(1.0f, hh);
-    const float sigma = __ldg(&S->P.sigma), beta = __ldg(&S->P.beta);
-    const float dt_h = dt * h_recip;
-
     const float2 p = pos[i];
-    const float2 v0 = vel[i];  // before gravity: velocity differences need none
+    const float2 v0 = vel[i];  // before gravity
     float2 dv = make_float2(0.0f, 0.0f);
     const unsigned key = cell_key(p.x, p.y, g);
-    // One pair's impulse on this particle; self (and any coincident
-    // particle) has r2 == 0 and gives none, as u is NaN in the reference for
-    // r == 0 (fluid.c:446-451).  in_range: the caller has established
-    // r2 <= h2 (a hit-mask walk recomputes the same r2).
-    const float2 mp = make_float2(-p.x, -p.y);
-    auto impulse = [&](const float4 &d, bool in_range) {
-        float2 e;
-        const float r2 = dist2_packed(mp, make_float2(d.x, d.y), e);
-        const float qx = e.x, qy = e.y;
-        if (!in_range && r2 > h2) return;
-        float r_recip = rsqrt_normal(r2);
-        if (r2 < kMinNormal) {
-            if (r2 == 0.0f) return;
-            r_recip = rsqrtf(r2);
-        }
-        const float r = r2 * r_recip;
-        // gravity adds the same amount to both velocities: the difference
-        // is taken before it (one packed subtraction)
-        const float2 w = __fadd2_rn(v0, make_float2(-d.z, -d.w));
-        const float u0 = (w.x * qx + w.y * qy) * r_recip;
-        // only approaching pairs (u > 0) push; the others run the same
-        // instructions with u = 0, whose impulse is +-0 and leaves dv's bits
-        // as they are (no divergent branch: about half the pairs of every
-        // warp approach)
-        const float u = fmaxf(u0, 0.0f);  // 0 for a NaN
-        // dt (1 - r/h) (sigma u + beta u^2) = (dt - (dt/h) r) u (sigma + beta u)
-        const float imp = fmaf(-dt_h, r, dt) * u * fmaf(beta, u, sigma);
-        // per component imp * q * r_recip, clamped, halved and subtracted
-        // (packed FP32x2, each operation rounded as the scalar form)
-        const float2 t = __fmul2_rn(__fmul2_rn(make_float2(imp, imp), e),
-                                    make_float2(r_recip, r_recip));
-        dv = __ffma2_rn(make_float2(-0.5f, -0.5f), make_float2(clamp5(t.x), clamp5(t.y)), dv);
-    };
-    auto load_pv = [&](int j) {
-        const float2 q = __ldg(pos + j), w = __ldg(vel + j);
-        return make_float4(q.x, q.y, w.x, w.y);
-    };
     if ((PROBE || st->lists_valid) && searchable(key, i, start, g, capped, c.max_bucket)) {
-        if (!capped) {
-            // two phases per 32 candidates of a stencil row: a cheap scan
-            // marks the neighbours, then only they pay for the impulse
-            // (less SIMT waste).  A piece at a time, a row of any length
-            // takes the same path: with whole rows marked first, rows of
-            // more than 64 candidates had every one of them run through the
-            // impulse (512-scene ensemble of compressed scenes: 20% of the
-            // particles).  4,194,304 particles: 236 -> 207 us early in the
-            // dam break, 285 -> 264 us compressed.
-            int ra[3], rl[3];
-            stencil_rows(p, key, start, g, ra, rl, c.n);
-#pragma unroll
-            for (int r = 0; r < 3; ++r) {
-                auto piece = [&](int a, int n) {
-                    unsigned m = hit_mask32<kMarkUnroll>(pos + a, n, mp, h2);
-                    // self is marked too; its impulse would be none
-                    if (r == 1 && (unsigned)(i - a) < 32u) m &= ~(1u << (i - a));
-                    walk_mask32<float4>(m, a, c.n, load_pv,
-                                        [&](int, const float4 &dq) { impulse(dq, true); });
-                };
-                // one piece as straight code: nearly every row (2% off the pass)
-                if (rl[r] <= 32) {
-                    piece(ra[r], rl[r]);
-                } else {
-#pragma unroll 1
-                    for (int c0 = 0; c0 < rl[r]; c0 += 32) piece(ra[r] + c0, min(rl[r] - c0, 32));
-                }
-            }
+        int ra[3] = {0, 0, 0}, rl[3] = {0, 0, 0};
+        if (!capped) stencil_rows(p, key, start, g, ra, rl, c.n);
+        if (!capped && max(rl[0], max(rl[1], rl[2])) <= kShortRow) {
+            // two phases: a cheap scan marks the neighbours of the stencil
+            // rows, then only they pay for the impulse (less SIMT waste)
+            const ViscConsts vc = visc_consts(S);
+            const float2 mp = make_float2(-p.x, -p.y);
+            const unsigned b0 = hit_mask32<kMarkUnroll>(pos + ra[0], rl[0], mp, vc.h2);
+            const unsigned b1 = hit_mask32<kMarkUnroll>(pos + ra[1], rl[1], mp, vc.h2) &
+                                ~(1u << (i - ra[1]));  // not the particle itself
+            const unsigned b2 = hit_mask32<kMarkUnroll>(pos + ra[2], rl[2], mp, vc.h2);
+            walk_three<float4>(
+                b0, ra[0], b1, ra[1], b2, ra[2], c.n,
+                [&](int j) {
+                    const float2 q = __ldg(pos + j), w = __ldg(vel + j);
+                    return make_float4(q.x, q.y, w.x, w.y);
+                },
+                [&](int, const float4 &d) {
+                    float2 e;
+                    const float r2 = dist2_packed(mp, make_float2(d.x, d.y), e);
+                    visc_impulse(vc, e, r2, v0, make_float2(d.z, d.w), dv);
+                });
         } else {
-            for_each_candidate(key, start, g, true, c.max_bucket, c.n,
-                               [&](int j) { impulse(load_pv(j), false); });
+            dv = viscosity_long_rows(i, S, pos, vel, start, capped, c.max_bucket, c.n);
         }
     }
     if (PROBE) {
@@ -774,26 +833,49 @@ k_viscosity_predict(Ctx c, const DevState *__restrict__ st, const float2 *__rest
 // candidates that are neighbours (r2 <= h2, self excluded), which the
 // relaxation pass of the same positions walks instead of the whole stencil.
 // The candidate filter of one particle over its three stencil rows (slots
-// [ra[r], ra[r] + rl[r])).  Rows of up to 32 candidates are marked first and
-// the marked ones walked: the terms are run for the hits alone, where one
-// loop over the candidates runs them for nearly every candidate of a warp
-// (some lane hits).  Longer rows keep the one loop: there the lanes of a
+// [ra[r], ra[r] + rl[r])).  Rows of up to kShortRow candidates are marked
+// first and the marked ones walked: the terms are run for the hits alone,
+// where one loop over the candidates runs them for nearly every candidate of a
+// warp (some lane hits).  Longer rows keep the one loop: there the lanes of a
 // warp are mostly of one cell and read the same candidate at a time, which a
-// walk over each lane's own hits does not.  4,194,304 particles: 182 -> 147
-// us early in the dam break, 201 -> 182 us compressed; two phases for rows
-// of any length 162 and 197 us.
+// walk over each lane's own hits does not.  4,194,304 particles: one loop for
+// every row 182 us early in the dam break and 201 us compressed, this 143 and
+// 176 us; two phases for rows of any length 162 and 197 us.
 // mx (long-row masks): where the hit bits of candidates kMaskRow..
 // 2 kMaskRow - 1 of each row go (3 words; null: nowhere).
 __device__ __forceinline__ void density_filter(int i, float2 mp, float h2, float h_recip,
                                                const int (&ra)[3], const int (&rl)[3],
-                                               const float2 *__restrict__ pos, float2 &ab,
+                                               const float2 *__restrict__ pos, int n, float2 &ab,
                                                unsigned long long (&m)[3],
                                                unsigned long long *mx = nullptr)
 {
+    if (max(rl[0], max(rl[1], rl[2])) <= kShortRow) {
+        unsigned b0 = hit_mask32<kMarkUnroll>(pos + ra[0], rl[0], mp, h2);
+        unsigned b1 = hit_mask32<kMarkUnroll>(pos + ra[1], rl[1], mp, h2) &
+                      ~(1u << (i - ra[1]));  // not the particle itself
+        unsigned b2 = hit_mask32<kMarkUnroll>(pos + ra[2], rl[2], mp, h2);
+        m[0] = b0;
+        m[1] = b1;
+        m[2] = b2;
+        // walk_three without the record in flight, for which this pass has
+        // no registers
+        int a0 = ra[0], a1 = ra[1], a2 = ra[2];
+        if (!b1) { b1 = b2; a1 = a2; b2 = 0u; }
+        if (!b0) { b0 = b1; a0 = a1; b1 = b2; a1 = a2; b2 = 0u; }
+        while (b0) {
+            const int j = a0 + __ffs(b0) - 1;
+            b0 &= b0 - 1u;
+            if (!b0) { b0 = b1; a0 = a1; b1 = b2; a1 = a2; b2 = 0u; }
+            if (!in_bounds(j, n, kBadSlot)) continue;
+            float2 e;
+            add_density(ab, dist2_packed(mp, __ldg(pos + j), e), h_recip);
+        }
+        return;
+    }
 #pragma unroll
     for (int r = 0; r < 3; ++r) {
         const int len = rl[r];
-        if (len <= 32) {
+        if (len <= kShortRow) {
             const float2 *row = pos + ra[r];
             unsigned b = hit_mask32<kMarkUnroll>(row, len, mp, h2);
             if (r == 1) b &= ~(1u << (i - ra[1]));
@@ -877,7 +959,7 @@ __device__ __forceinline__ void density_one(int i, const Ctx &c, const float2 *_
                 mx = c.maskx + 3 * (size_t)i;
                 mx[0] = mx[1] = mx[2] = 0ull;  // rows of kMaskRow or fewer leave theirs
             }
-            density_filter(i, mp, h2, h_recip, ra, rl, pos, ab, m, LM ? mx : nullptr);
+            density_filter(i, mp, h2, h_recip, ra, rl, pos, c.n, ab, m, LM ? mx : nullptr);
         } else {
             for_each_candidate(key, start, g, true, c.max_bucket, c.n, [&](int j) {
                 if (j == i) return;
