@@ -214,6 +214,12 @@ __device__ __forceinline__ void named_sync(int id, int count)
     asm volatile("bar.sync %0, %1;" :: "r"(id), "r"(count) : "memory");
 }
 
+// Arrival at a named barrier that other threads wait at, without waiting.
+__device__ __forceinline__ void named_arrive(int id, int count)
+{
+    asm volatile("bar.arrive %0, %1;" :: "r"(id), "r"(count) : "memory");
+}
+
 // Named barrier that also ANDs a predicate over the participating threads.
 __device__ __forceinline__ bool named_sync_and(int id, int count, bool v)
 {

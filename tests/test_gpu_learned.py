@@ -359,3 +359,18 @@ def test_forward_pieces_and_overlap(cuda_lib):
         shifted = buf[48:]
         _lib.check(cuda_lib.sph_learned_forward(m._l, buf.ctypes.data_as(fp), n, shifted.ctypes.data_as(fp)))
         assert bits_equal(shifted[:n * LearnedModel.OUT].reshape(n, LearnedModel.OUT).copy(), y)
+
+
+@pytest.mark.parametrize("extra", [-1, 0, 1])
+@pytest.mark.parametrize("pipes", [1, 2, 3, 4, 6, 7])
+def test_forward_rows_over_the_pipelines(cuda_lib, pipes, extra):
+    """Row counts at which the last pipelines of the network kernel have a
+    tile less than their partners, or none: the rows of calls of one tile."""
+    import torch
+    n = 128 * (pipes * torch.cuda.get_device_properties(0).multi_processor_count + extra)
+    x = np.random.default_rng(pipes).standard_normal((n, LearnedModel.IN)).astype(np.float32)
+    x[:, 31] = 1.0
+    with LearnedModel(0, seed=6) as m:
+        y = m.forward(x)
+        for a in (0, 128 * 5, n // 256 * 128, n - 256, n - 128):
+            assert bits_equal(m.forward(x[a:a + 128]), y[a:a + 128]), a
