@@ -137,6 +137,33 @@ void PageToucher::done()
     threads_.clear();
 }
 
+void *host_in_place(const void *p, size_t bytes, size_t align, bool write)
+{
+    if (bytes == 0 || bytes > kInPlaceBytes || (uintptr_t)p % align != 0) return nullptr;
+    int dev = 0, shared_tables = 0;
+    cudaPointerAttributes at{};
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&shared_tables, cudaDevAttrPageableMemoryAccessUsesHostPageTables,
+                               dev) != cudaSuccess ||
+        cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return nullptr;
+    }
+    if (!shared_tables || (at.type != cudaMemoryTypeUnregistered && at.type != cudaMemoryTypeHost))
+        return nullptr;
+    const long ps = sysconf(_SC_PAGESIZE);
+    const size_t page = ps > 0 ? (size_t)ps : 4096;
+    char *b = static_cast<char *>(const_cast<void *>(p));
+    if (write) {
+        touch_pages(b, bytes, page);
+    } else {
+        (void)*static_cast<volatile const char *>(b);
+        for (uintptr_t a = ((uintptr_t)b / page + 1) * page; a < (uintptr_t)b + bytes; a += page)
+            (void)*reinterpret_cast<volatile const char *>(a);
+    }
+    return at.type == cudaMemoryTypeHost ? at.devicePointer : b;
+}
+
 template <class T>
 static int dalloc(T **p, size_t count)
 {
@@ -312,6 +339,7 @@ static void free_all(sph_cuda *h)
         if (h->copy_ev[k]) cudaEventDestroy(h->copy_ev[k]);
     }
     if (h->copy_stream) cudaStreamDestroy(h->copy_stream);
+    if (h->upload_ev) cudaEventDestroy(h->upload_ev);
     void *ptrs[] = {h->pos_a, h->vel_a, h->id_a, h->pos_b, h->prev_b, h->vel_b, h->kr_b,
                     h->pos_c, h->prev_c, h->xr_c, h->mask01_c, h->mask2_c, h->maskx_c, h->rows_c, h->id_c,
                     h->tmp_id, h->cnt, h->start_a, h->start_c, h->tile_sums, h->build_tiles, h->d_scenes,
@@ -427,6 +455,8 @@ static int build_handle(sph_cuda **out, std::vector<Scene> &&scenes, int capacit
     rc = cuda_fail(cudaStreamCreateWithFlags(&h->own_stream, cudaStreamNonBlocking),
                    "cudaStreamCreate");
     if (rc) return fail(rc);
+    rc = cuda_fail(cudaEventCreateWithFlags(&h->upload_ev, cudaEventDisableTiming), "event");
+    if (rc) return fail(rc);
     h->stream = h->own_stream;
     const size_t N = (size_t)capacity;
     const size_t M = (size_t)h->M;
@@ -491,8 +521,8 @@ static int build_handle(sph_cuda **out, std::vector<Scene> &&scenes, int capacit
 }
 
 // The common tail of every upload: the particle count, a fresh device state,
-// zero tile counts and the sort into the A order (upload_soa_device).
-static int upload_finish(sph_cuda *h, int n)
+// zero tile counts and the sort into the A order (upload_device).
+static int upload_finish(sph_cuda *h, int n, const UploadSource &src = UploadSource())
 {
     if (h->nscenes == 1 && h->scenes[0].n != n) {
         h->scenes[0].n = n;
@@ -500,8 +530,9 @@ static int upload_finish(sph_cuda *h, int n)
     }
     h->n = n;
     SPH_CUDA(cudaMemsetAsync(h->d_state, 0, sizeof(DevState), h->stream));
-    SPH_TRY(upload_soa_device(h, n));
-    SPH_CUDA(cudaStreamSynchronize(h->stream));  // the caller's buffers are free again
+    SPH_TRY(upload_device(h, n, src));
+    // the caller's buffers are free again (the sort goes on behind the call)
+    SPH_CUDA(cudaEventSynchronize(h->upload_ev));
     return SPH_OK;
 }
 
@@ -706,8 +737,8 @@ int sph_cuda_upload(sph_cuda_t *h, fluid_particle *const *ptrs, int n)
     });
 }
 
-// The caller's contiguous arrays go to the device as they are (one copy
-// each, no host-side repacking) and a kernel lays them out.
+// The caller's contiguous arrays go to the device as they are (read in place,
+// or one copy each; no host-side repacking) and a kernel lays them out.
 int sph_cuda_upload_particles(sph_cuda_t *h, const fluid_particle *ps, int n)
 {
     SPH_TRY(check_handle(h));
@@ -717,14 +748,14 @@ int sph_cuda_upload_particles(sph_cuda_t *h, const fluid_particle *ps, int n)
     }
     SPH_TRY(check_n(h, n));
     SPH_CUDA(cudaStreamSynchronize(h->stream));
+    UploadSource src;
     if (n > 0) {
         const size_t b = (size_t)n * sizeof(fluid_particle);
         SPH_TRY(ensure_scratch(h, b));
-        auto *recs = static_cast<fluid_particle *>(h->d_scratch);
-        SPH_CUDA(cudaMemcpyAsync(recs, ps, b, cudaMemcpyHostToDevice, h->stream));
-        SPH_TRY(launch_upload_layout(h, n, nullptr, nullptr, nullptr, nullptr, recs));
+        SPH_CUDA(cudaMemcpyAsync(h->d_scratch, ps, b, cudaMemcpyHostToDevice, h->stream));
+        src.recs = static_cast<fluid_particle *>(h->d_scratch);
     }
-    return upload_finish(h, n);
+    return upload_finish(h, n, src);
 }
 
 int sph_cuda_upload_soa(sph_cuda_t *h, const float *x, const float *y, const float *vx,
@@ -737,19 +768,24 @@ int sph_cuda_upload_soa(sph_cuda_t *h, const float *x, const float *y, const flo
     }
     SPH_TRY(check_n(h, n));
     SPH_CUDA(cudaStreamSynchronize(h->stream));
+    UploadSource src;
     if (n > 0) {
-        // the A-state arrays are free until the sort rewrites them
+        // in place, or into the A-state arrays, which are free until the sort
+        // rewrites them
         const size_t b = (size_t)n * sizeof(float);
-        float *dx = reinterpret_cast<float *>(h->pos_a), *dy = dx + n;
-        float *dvx = reinterpret_cast<float *>(h->vel_a), *dvy = dvx + n;
-        SPH_CUDA(cudaMemcpyAsync(dx, x, b, cudaMemcpyHostToDevice, h->stream));
-        SPH_CUDA(cudaMemcpyAsync(dy, y, b, cudaMemcpyHostToDevice, h->stream));
-        if (vx) SPH_CUDA(cudaMemcpyAsync(dvx, vx, b, cudaMemcpyHostToDevice, h->stream));
-        if (vy) SPH_CUDA(cudaMemcpyAsync(dvy, vy, b, cudaMemcpyHostToDevice, h->stream));
-        SPH_TRY(launch_upload_layout(h, n, dx, dy, vx ? dvx : nullptr, vy ? dvy : nullptr,
-                                     nullptr));
+        float *pos = reinterpret_cast<float *>(h->pos_a), *vel = reinterpret_cast<float *>(h->vel_a);
+        float *const spare[4] = {pos, pos + n, vel, vel + n};
+        const float *const from[4] = {x, y, vx, vy};
+        const float **const at[4] = {&src.x, &src.y, &src.vx, &src.vy};
+        for (int k = 0; k < 4; ++k) {
+            if (!from[k]) continue;
+            *at[k] = static_cast<const float *>(host_in_place(from[k], b, sizeof(float), false));
+            if (*at[k]) continue;
+            *at[k] = spare[k];
+            SPH_CUDA(cudaMemcpyAsync(spare[k], from[k], b, cudaMemcpyHostToDevice, h->stream));
+        }
     }
-    return upload_finish(h, n);
+    return upload_finish(h, n, src);
 }
 
 int sph_cuda_step(sph_cuda_t *h, const tunable_parameters *tp, int nsteps)
@@ -833,8 +869,8 @@ int sph_cuda_download_particles(sph_cuda_t *h, fluid_particle *ps, int n)
     return SPH_OK;
 }
 
-// Laid out on the device and copied straight into the caller's arrays (no
-// host-side repacking).
+// Laid out on the device, into the caller's arrays themselves or copied
+// straight into them (no host-side repacking).
 int sph_cuda_download_soa(sph_cuda_t *h, float *x, float *y, float *vx, float *vy, float *rho,
                           float *rho_near, int n)
 {
@@ -849,12 +885,24 @@ int sph_cuda_download_soa(sph_cuda_t *h, float *x, float *y, float *vx, float *v
     float2 *s = static_cast<float2 *>(h->d_scratch);
     float *cols = reinterpret_cast<float *>(s + 5 * (size_t)n);
     SPH_TRY(launch_unpermute(h, s));
-    SPH_TRY(launch_split_soa(h, n, s, cols));
-    float *dst[6] = {x, y, vx, vy, rho, rho_near};
+    float *const dst[6] = {x, y, vx, vy, rho, rho_near};
+    SoaColumns out;
+    bool copied[6] = {}, apart = true;  // columns that overlap: the later one is what remains
     for (int k = 0; k < 6; ++k)
-        if (dst[k])
-            SPH_CUDA(cudaMemcpyAsync(dst[k], cols + k * (size_t)n, col, cudaMemcpyDeviceToHost,
-                                     h->stream));
+        for (int l = 0; l < k; ++l)
+            apart = apart && !(dst[k] && dst[l] && (uintptr_t)dst[k] < (uintptr_t)dst[l] + col &&
+                               (uintptr_t)dst[l] < (uintptr_t)dst[k] + col);
+    for (int k = 0; k < 6; ++k) {
+        out.c[k] = nullptr;
+        if (!dst[k]) continue;
+        if (apart) out.c[k] = static_cast<float *>(host_in_place(dst[k], col, sizeof(float), true));
+        copied[k] = !out.c[k];
+        if (copied[k]) out.c[k] = cols + k * (size_t)n;
+    }
+    SPH_TRY(launch_split_soa(h, n, s, out));
+    for (int k = 0; k < 6; ++k)
+        if (copied[k])
+            SPH_CUDA(cudaMemcpyAsync(dst[k], out.c[k], col, cudaMemcpyDeviceToHost, h->stream));
     SPH_CUDA(cudaStreamSynchronize(h->stream));
     return SPH_OK;
 }
@@ -867,9 +915,12 @@ int sph_cuda_pack_coords_short(sph_cuda_t *h, short *coords, int n)
         return SPH_ERR_INVALID;
     }
     const size_t b = (size_t)n * sizeof(short2);
-    SPH_TRY(ensure_scratch(h, b + 16));
-    SPH_TRY(launch_pack(h, (short2 *)h->d_scratch));
-    if (n > 0) SPH_CUDA(cudaMemcpyAsync(coords, h->d_scratch, b, cudaMemcpyDeviceToHost, h->stream));
+    // scattered by id: beyond kInPlacePack bytes a copy is the faster
+    void *const own = b <= kInPlacePack ? host_in_place(coords, b, sizeof(short2), true) : nullptr;
+    if (!own) SPH_TRY(ensure_scratch(h, b + 16));
+    SPH_TRY(launch_pack(h, (short2 *)(own ? own : h->d_scratch)));
+    if (n > 0 && !own)
+        SPH_CUDA(cudaMemcpyAsync(coords, h->d_scratch, b, cudaMemcpyDeviceToHost, h->stream));
     SPH_CUDA(cudaStreamSynchronize(h->stream));
     return SPH_OK;
 }
@@ -1004,11 +1055,7 @@ int sph_cuda_rebuild_neighbors(sph_cuda_t *h)
     SPH_TRY(check_handle(h));
     // The sorted state always carries the cell lists of its current
     // positions, so the relation exists already: enable it.
-    const unsigned one = 1u;
-    SPH_CUDA(cudaMemcpyAsync(&h->d_state->lists_valid, &one, sizeof(one), cudaMemcpyHostToDevice,
-                             h->stream));
-    SPH_CUDA(cudaStreamSynchronize(h->stream));
-    return SPH_OK;
+    return launch_enable_lists(h);
 }
 
 int sph_cuda_synchronize(sph_cuda_t *h)

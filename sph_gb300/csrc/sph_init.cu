@@ -116,7 +116,7 @@ extern "C" int sph_cuda_init_lattice(sph_cuda_t *h, const sph_lattice_block *blo
         if (rc) return rc;
     }
     rc = cuda_fail(cudaMemsetAsync(h->d_state, 0, sizeof(DevState), h->stream), "state");
-    if (!rc) rc = upload_soa_device(h, n);
+    if (!rc) rc = upload_device(h, n);
     if (!rc) rc = cuda_fail(cudaStreamSynchronize(h->stream), "sync");
     return rc;
 }

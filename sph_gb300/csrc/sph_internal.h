@@ -200,6 +200,7 @@ struct sph_cuda {
     short2 *d_coords[2] = {nullptr, nullptr};
     cudaEvent_t pack_ev[2] = {nullptr, nullptr};
     cudaEvent_t copy_ev[2] = {nullptr, nullptr};
+    cudaEvent_t upload_ev = nullptr;  // the last upload's source has been read
     const void *copy_dst[2] = {nullptr, nullptr};
     int pack_slot = 0;
 };
@@ -248,10 +249,39 @@ private:
 // Core operations shared by the fast API and the legacy entry points.
 int ensure_scratch(sph_cuda *h, size_t bytes);
 int ensure_stage(sph_cuda *h, size_t bytes);
-int upload_soa_device(sph_cuda *h, int n);  // pos_b/vel_b (id order) + xr_c -> state
-int launch_upload_layout(sph_cuda *h, int n, const float *x, const float *y, const float *vx,
-                         const float *vy, const fluid_particle *recs);
-int launch_split_soa(sph_cuda *h, int n, const float2 *rec, float *out);
+
+// The caller's host memory [p, p + bytes) as a kernel can reach it, or null
+// where it has to be copied: kernels of a GPU that shares the host's page
+// tables read and write pageable memory (and page-locked memory) in place.
+// Every page is touched here first, so that a bad range faults on the host,
+// as a copy of it would, and no page fault is left to the GPU.  `write`: the
+// kernel overwrites ALL of it.  A copy by the runtime costs about 10 us of the
+// host's time besides its bytes.  Columns of kInPlaceBytes at most, copied /
+// in place: upload of four at 65,536 particles 100 / 40 us, at 1,048,576 (4
+// MB a column) 196 / 132, download of six 91 / 41 and 238 / 207, at 2,097,152
+// 394 / 439.  Packed coordinates, which are written by id, up to kInPlacePack:
+// 65,536 particles 18.5 / 16 us, 262,144 23 / 27.  Feature rows up to
+// kInPlaceRows: 1,024 rows 43 / 26 us, 8,192 59 / 49, 16,384 78 / 86.
+constexpr size_t kInPlaceBytes = (size_t)4 << 20;
+constexpr size_t kInPlacePack = (size_t)256 << 10;
+constexpr size_t kInPlaceRows = (size_t)1 << 20;
+void *host_in_place(const void *p, size_t bytes, size_t align, bool write);
+
+// Particles to upload, where a kernel reads them: arrays (vx, vy may be null:
+// zero), or the reference's records, or (all null) pos_b, vel_b, prev_c and
+// xr_c filled already, in id order.
+struct UploadSource {
+    const float *x = nullptr, *y = nullptr, *vx = nullptr, *vy = nullptr;
+    const fluid_particle *recs = nullptr;
+};
+int upload_device(sph_cuda *h, int n, const UploadSource &src = UploadSource());
+
+// Columns by id (x, y, vx, vy, rho, rho_near) for launch_split_soa; null: not wanted.
+struct SoaColumns {
+    float *c[6];
+};
+int launch_split_soa(sph_cuda *h, int n, const float2 *rec, const SoaColumns &out);
+int launch_enable_lists(sph_cuda *h);
 int set_scene_params(sph_cuda *h, int scene, const tunable_parameters *tp);
 int enqueue_step(sph_cuda *h, cudaEvent_t *events, int *nkernels,
                  const tunable_parameters *mid_tp = nullptr);

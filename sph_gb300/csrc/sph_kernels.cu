@@ -172,72 +172,39 @@ __device__ __forceinline__ unsigned block_exclusive_scan(unsigned v, unsigned *s
 // cell build: histogram scan, scatter, permute
 // ---------------------------------------------------------------------------
 
-// Per-tile sums of the histogram, and occupancy statistics of the in-grid
-// cells (`nocell` has a bit set for every scene's no-cell bucket).
+// Per-tile sums.
 __global__ void __launch_bounds__(kScanThreads)
-k_scan_reduce(const unsigned *__restrict__ in, int M, const unsigned *__restrict__ nocell,
-              int *__restrict__ tile_sums, DevState *__restrict__ st, unsigned *occ,
-              int max_bucket, int max_neighbors)
+k_scan_reduce(const unsigned *__restrict__ in, int M, int *__restrict__ tile_sums)
 {
-    __shared__ unsigned sh_s[kScanThreads / 32], sh_m[kScanThreads / 32];
-    __shared__ unsigned long long sh_e[kScanThreads / 32], sh_o[kScanThreads / 32];
+    __shared__ unsigned sh_s[kScanThreads / 32];
     const int base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
-    unsigned s = 0, mx = 0;
-    unsigned long long excess = 0, outside = 0;
-    unsigned v[kScanItems];
+    unsigned s = 0;
     if (base + kScanItems <= M) {
         const uint4 *p = reinterpret_cast<const uint4 *>(in + base);
 #pragma unroll
         for (int q = 0; q < kScanItems / 4; ++q) {
             const uint4 t = p[q];
-            v[4 * q] = t.x; v[4 * q + 1] = t.y; v[4 * q + 2] = t.z; v[4 * q + 3] = t.w;
+            s += t.x + t.y + t.z + t.w;
         }
     } else {
 #pragma unroll
-        for (int e = 0; e < kScanItems; ++e) v[e] = base + e < M ? in[base + e] : 0u;
-    }
-    // the thread's 16 counters lie in one 32-bit word of the no-cell bitmap
-    const unsigned bits = (nocell && base < M) ? (__ldg(nocell + (base >> 5)) >> (base & 31)) : 0u;
-#pragma unroll
-    for (int e = 0; e < kScanItems; ++e) {
-        s += v[e];
-        if ((bits >> e) & 1u) {
-            outside += v[e];
-        } else {
-            mx = max(mx, v[e]);
-            if (v[e] > (unsigned)max_bucket) excess += v[e] - max_bucket;
-        }
+        for (int e = 0; e < kScanItems; ++e) s += base + e < M ? in[base + e] : 0u;
     }
     s = warp_sum(s);
-    mx = warp_max(mx);
-    excess = warp_sum(excess);
-    outside = warp_sum(outside);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (lane == 0) { sh_s[warp] = s; sh_m[warp] = mx; sh_e[warp] = excess; sh_o[warp] = outside; }
+    if (lane == 0) sh_s[warp] = s;
     __syncthreads();
     if (threadIdx.x == 0) {
-        unsigned ts = 0, tm = 0;
-        unsigned long long te = 0, to = 0;
-        for (int w = 0; w < kScanThreads / 32; ++w) {
-            ts += sh_s[w]; tm = max(tm, sh_m[w]); te += sh_e[w]; to += sh_o[w];
-        }
+        unsigned ts = 0;
+        for (int w = 0; w < kScanThreads / 32; ++w) ts += sh_s[w];
         tile_sums[blockIdx.x] = (int)ts;
-        if (occ) {
-            atomicMax(occ, tm);
-            atomicMax(&st->max_occ, tm);
-            if (te) atomicAdd(&st->bucket_overflow, te);
-            if (to) atomicAdd(&st->out_of_grid, to);
-            const unsigned m = tm < (unsigned)max_bucket ? tm : (unsigned)max_bucket;
-            if (m > 0 && 5u * m - 1u > (unsigned)max_neighbors) atomicOr(&st->list_cap_risk, 1u);
-        }
     }
 }
 
-// Exclusive scan: out[i] = sum(in[0..i)), out[M] = total.  Zeroes `in` when
-// asked (the histogram must be zero before the next build).
+// Exclusive scan: out[i] = sum(in[0..i)), out[M] = total.
 __global__ void __launch_bounds__(kScanThreads)
-k_scan_apply(unsigned *__restrict__ in, int M, const int *__restrict__ tile_sums,
-             int *__restrict__ out, int zero_input)
+k_scan_apply(const unsigned *__restrict__ in, int M, const int *__restrict__ tile_sums,
+             int *__restrict__ out)
 {
     __shared__ unsigned sh[kScanThreads / 32];
     __shared__ unsigned sh_prefix;
@@ -286,18 +253,12 @@ k_scan_apply(unsigned *__restrict__ in, int M, const int *__restrict__ tile_sums
             t.w = (int)run; run += v[4 * q + 3];
             o[q] = t;
         }
-        if (zero_input) {
-            uint4 *p = reinterpret_cast<uint4 *>(in + base);
-#pragma unroll
-            for (int q = 0; q < kScanItems / 4; ++q) p[q] = make_uint4(0, 0, 0, 0);
-        }
     } else {
 #pragma unroll
         for (int e = 0; e < kScanItems; ++e) {
             if (base + e < M) {
                 out[base + e] = (int)run;
                 run += v[e];
-                if (zero_input) in[base + e] = 0u;
             }
         }
     }
@@ -448,61 +409,14 @@ k_cell_starts(unsigned *__restrict__ in, int M, const unsigned *__restrict__ noc
     }
 }
 
-// Scratch slot per particle: cell start + arrival rank.
-__global__ void __launch_bounds__(kBlock)
-k_scatter_ids(int n, const uint2 *__restrict__ kr, const int *__restrict__ id_src,
-              const int *__restrict__ start, int *__restrict__ tmp, unsigned *tile_cnt, int ntiles)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    // the build's tile counts have been read (k_cell_starts): zero them for
-    // the next build
-    for (int t = i; t < ntiles; t += gridDim.x * blockDim.x) tile_cnt[t] = 0u;
-    if (i >= n) return;
-    const uint2 k = kr[i];
-    const int d = __ldg(start + k.x) + (int)k.y;
-    if (in_bounds(d, n, kBadScatter)) tmp[d] = id_src ? id_src[i] : i;
-}
-
-// Final position = cell start + number of cell members with a smaller id, so
-// that each cell holds its particles in id order -- the order hash.c:153-163
-// inserts them into a bucket (pointer-array order).
-__global__ void __launch_bounds__(kBlock)
-k_permute(int n, const uint2 *__restrict__ kr, const int *__restrict__ start,
-          const int *__restrict__ tmp, const int *__restrict__ id_src,
-          const float2 *__restrict__ a_src, const float2 *__restrict__ b_src,
-          int *__restrict__ id_dst, float2 *__restrict__ a_dst, float2 *__restrict__ b_dst,
-          DevState *__restrict__ end_step)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (end_step && i == 0) {
-        // last kernel of a step: the neighbour relation of the new positions
-        // now exists (viscosity is on from the next step), one more step done
-        end_step->lists_valid = 1u;
-        end_step->steps += 1ull;
-    }
-    if (i >= n) return;
-    const uint2 k = kr[i];
-    const int s0 = __ldg(start + k.x), s1 = __ldg(start + k.x + 1);
-    const int myid = id_src ? id_src[i] : i;
-    int r;
-    if (s1 - s0 <= kRankScanMax) {
-        r = 0;
-        for (int j = s0; j < s1; ++j)
-            if (in_bounds(j, n, kBadScatter)) r += __ldg(tmp + j) < myid;
-    } else {
-        r = (int)k.y;  // pathological cell: arrival order
-    }
-    const int d = s0 + r;
-    if (!in_bounds(d, n, kBadScatter)) return;
-    id_dst[d] = myid;
-    a_dst[d] = a_src[i];
-    if (b_src) b_dst[d] = b_src[i];
-}
-
-// The step's forms of k_scatter_ids and k_permute: K particles per thread
-// (strided by the block size, so the loads stay coalesced), their loads
-// issued together, so that each thread has K dependent chains (key -> cell
-// start -> slot) in flight instead of one.
+// Scatter and permutation of a build.  The scatter puts each particle's id
+// into its scratch slot (cell start + arrival rank); the permutation's slot is
+// the cell start + the number of cell members with a smaller id, so that each
+// cell holds its particles in id order -- the order hash.c:153-163 inserts
+// them into a bucket (pointer-array order).  K particles per thread (strided
+// by the block size, so the loads stay coalesced), their loads issued
+// together, so that each thread has K dependent chains (key -> cell start ->
+// slot) in flight instead of one.
 //
 // What a kernel reads of kernels before its predecessor it requests ahead of
 // the wait for the predecessor (their results are complete: the predecessor
@@ -527,6 +441,8 @@ k_scatter_ids_x(int n, const uint2 *__restrict__ kr, const int *__restrict__ id_
         }
     }
     pdl_enter();
+    // the build's tile counts have been read (k_cell_starts): zero them for
+    // the next build
     for (int t = g; t < ntiles; t += gridDim.x * blockDim.x) tile_cnt[t] = 0u;
 #pragma unroll
     for (int j = 0; j < K; ++j)
@@ -569,6 +485,8 @@ k_permute_x(int n, const uint2 *__restrict__ kr, const int *__restrict__ start,
         }
     pdl_enter();
     if (end_step && blockIdx.x == 0 && threadIdx.x == 0) {
+        // last kernel of a step: the neighbour relation of the new positions
+        // now exists (viscosity is on from the next step), one more step done
         end_step->lists_valid = 1u;
         end_step->steps += 1ull;
     }
@@ -589,20 +507,6 @@ k_permute_x(int n, const uint2 *__restrict__ kr, const int *__restrict__ start,
         a_dst[d] = a[j];
         if (b_src) b_dst[d] = b[j];
     }
-}
-
-// Cell keys of uploaded positions (id order, no step before them).
-__global__ void __launch_bounds__(kBlock)
-k_keys(Ctx c, const float2 *__restrict__ pos, uint2 *__restrict__ kr, unsigned *__restrict__ cnt,
-       unsigned *occ_reset)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i == 0 && occ_reset) *occ_reset = 0u;
-    if (i >= c.n) return;
-    const SG g = load_grid(c.scenes + scene_of(c, i));
-    const float2 p = pos[i];
-    const unsigned key = cell_key(p.x, p.y, g);
-    kr[i] = make_uint2(key, in_bounds(key, c.M, kBadKey) ? atomicAdd(cnt + key, 1u) : 0u);
 }
 
 // ---------------------------------------------------------------------------
@@ -1868,14 +1772,6 @@ k_by_id(int n, const int *__restrict__ ids, const float2 *__restrict__ in, float
     out[ids[i]] = in[i];
 }
 
-// Identity id map for the *_c slots that download reads before the first step.
-__global__ void __launch_bounds__(kBlock)
-k_iota(int n, int *__restrict__ ids)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) ids[i] = i;
-}
-
 // Pixel-space shorts for the render rank (fluid.c:360-361), by id.
 __global__ void __launch_bounds__(kBlock)
 k_pack_coords(Ctx c, const int *__restrict__ id_a, const float2 *__restrict__ pos_a,
@@ -2077,8 +1973,7 @@ static inline dim3 gather_grid(const sph_cuda *h, const Shape &s)
 
 // Exclusive scan of `in` (M entries) into out (M + 1 entries).  Both arrays
 // must be 16-byte aligned: the scan kernels move 16-byte vectors.
-static int launch_scan(sph_cuda *h, unsigned *in, int M, int *out, unsigned *occ, bool zero,
-                       const unsigned *nocell)
+int launch_prefix(sph_cuda *h, unsigned *in, int M, int *out)
 {
     if (((uintptr_t)in | (uintptr_t)out) & 15u) {
         set_error("internal: scan arrays not 16-byte aligned");
@@ -2089,15 +1984,9 @@ static int launch_scan(sph_cuda *h, unsigned *in, int M, int *out, unsigned *occ
         set_error("internal: scan of %d items exceeds the tile buffer", M);
         return SPH_ERR_INVALID;
     }
-    k_scan_reduce<<<tiles, kScanThreads, 0, h->stream>>>(in, M, nocell, h->tile_sums, h->d_state,
-                                                         occ, h->max_bucket, h->max_neighbors);
-    k_scan_apply<<<tiles, kScanThreads, 0, h->stream>>>(in, M, h->tile_sums, out, zero ? 1 : 0);
+    k_scan_reduce<<<tiles, kScanThreads, 0, h->stream>>>(in, M, h->tile_sums);
+    k_scan_apply<<<tiles, kScanThreads, 0, h->stream>>>(in, M, h->tile_sums, out);
     return SPH_OK;
-}
-
-int launch_prefix(sph_cuda *h, unsigned *in, int n, int *out)
-{
-    return launch_scan(h, in, n, out, nullptr, false, nullptr);
 }
 
 // The cell starts of a step's build (all M counters, zeroed after) into
@@ -2112,6 +2001,22 @@ static void enqueue_cell_starts(sph_cuda *h, int *out, unsigned *occ)
     launch_step(k_cell_starts, build_tiles_of(h), kBuildThreads, 0, h->stream, h->cnt, h->M,
                 (const unsigned *)h->d_nocell, (const unsigned *)h->build_tiles, out, h->d_state,
                 occ, h->max_bucket, h->max_neighbors);
+}
+
+// Scatter and permutation of pos_b / vel_b (ids id_c, keys kr_b) into the A
+// order by start_a; `end_step`: they end a step.  between() comes between.
+template <class F>
+static void enqueue_a_order(sph_cuda *h, DevState *end_step, F &&between)
+{
+    const int n = h->n, nbx = blocks_for(n, kBlock * kBuildPerThread);
+    launch_step(k_scatter_ids_x<kBuildPerThread>, nbx, kBlock, 0, h->stream, n,
+                (const uint2 *)h->kr_b, (const int *)h->id_c, (const int *)h->start_a, h->tmp_id,
+                h->build_tiles, build_tiles_of(h));
+    between();
+    launch_step(k_permute_x<kBuildPerThread>, nbx, kBlock, 0, h->stream, n,
+                (const uint2 *)h->kr_b, (const int *)h->start_a, (const int *)h->tmp_id,
+                (const int *)h->id_c, (const float2 *)h->pos_b, (const float2 *)h->vel_b,
+                h->id_a, h->pos_a, h->vel_a, end_step);
 }
 
 static const char *const kKernelNames[] = {
@@ -2347,15 +2252,7 @@ int enqueue_step(sph_cuda *h, cudaEvent_t *events, int *nkernels, const tunable_
     }
     enqueue_cell_starts(h, h->start_a, &st->build_max_occ[SLOT_RELAXED]);
     mark();
-    const int nbx = blocks_for(n, kBlock * kBuildPerThread);
-    launch_step(k_scatter_ids_x<kBuildPerThread>, nbx, kBlock, 0, h->stream, n,
-                (const uint2 *)h->kr_b, (const int *)h->id_c, (const int *)h->start_a, h->tmp_id,
-                h->build_tiles, build_tiles_of(h));
-    mark();
-    launch_step(k_permute_x<kBuildPerThread>, nbx, kBlock, 0, h->stream, n,
-                (const uint2 *)h->kr_b, (const int *)h->start_a, (const int *)h->tmp_id,
-                (const int *)h->id_c, (const float2 *)h->pos_b, (const float2 *)h->vel_b,
-                h->id_a, h->pos_a, h->vel_a, st);
+    enqueue_a_order(h, st, mark);
     mark();
     if (nkernels) *nkernels = e - 1;
     return cuda_fail(cudaGetLastError(), "step launch");
@@ -2378,100 +2275,96 @@ int step_kernel_count(const sph_cuda *h)
     return (h && h->learned) ? kLearnedStepKernels : kStepKernels;
 }
 
-// Host-layout particles, already on the device, -> the upload arrays in id
-// order: pos_b, vel_b, prev_c and xr_c = (x, y, rho, rho_near).  From
-// structure-of-arrays (vx, vy may be null: zero) or from the reference's
-// fluid_particle records.
+// Particles to upload -> the upload arrays in id order (pos_b, vel_b, prev_c
+// and xr_c = (x, y, rho, rho_near)), from structure-of-arrays (vx, vy may be
+// null: zero), from the reference's fluid_particle records, or in place
+// already, with their cell keys counted into the build that sorts them, in
+// one kernel (layout, ids and keys were three, and the sort that followed
+// four more without programmatic launch).
 __global__ void __launch_bounds__(kBlock)
-k_upload_soa(int n, const float *__restrict__ x, const float *__restrict__ y,
-             const float *__restrict__ vx, const float *__restrict__ vy, float2 *__restrict__ pos,
-             float2 *__restrict__ vel, float2 *__restrict__ prev, float4 *__restrict__ xr)
+k_upload(Ctx c, UploadSource src, float2 *__restrict__ pos, float2 *__restrict__ vel,
+         float2 *__restrict__ prev, float4 *__restrict__ xr, int *__restrict__ id,
+         uint2 *__restrict__ kr, unsigned *__restrict__ cnt, unsigned *occ_reset)
 {
+    pdl_enter();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float px = x[i], py = y[i];
-    pos[i] = make_float2(px, py);
-    vel[i] = make_float2(vx ? vx[i] : 0.0f, vy ? vy[i] : 0.0f);
-    prev[i] = make_float2(px, py);
-    xr[i] = make_float4(px, py, 0.0f, 0.0f);
-}
-
-__global__ void __launch_bounds__(kBlock)
-k_upload_records(int n, const fluid_particle *__restrict__ ps, float2 *__restrict__ pos,
-                 float2 *__restrict__ vel, float2 *__restrict__ prev, float4 *__restrict__ xr)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const fluid_particle &p = ps[i];
-    pos[i] = make_float2(p.x, p.y);
-    vel[i] = make_float2(p.v_x, p.v_y);
-    prev[i] = make_float2(p.x_prev, p.y_prev);
-    xr[i] = make_float4(p.x, p.y, p.density, p.density_near);
-}
-
-// Launches one of the two above on device copies of the caller's arrays
-// (x, y, vx, vy or recs; the others null).
-int launch_upload_layout(sph_cuda *h, int n, const float *x, const float *y, const float *vx,
-                         const float *vy, const fluid_particle *recs)
-{
-    if (n == 0) return SPH_OK;
-    const int nb = blocks_for(n);
-    if (recs)
-        k_upload_records<<<nb, kBlock, 0, h->stream>>>(n, recs, h->pos_b, h->vel_b, h->prev_c,
-                                                       h->xr_c);
-    else
-        k_upload_soa<<<nb, kBlock, 0, h->stream>>>(n, x, y, vx, vy, h->pos_b, h->vel_b, h->prev_c,
-                                                   h->xr_c);
-    return cuda_fail(cudaGetLastError(), "upload layout");
+    if (i == 0) *occ_reset = 0u;
+    int t = -1;
+    if (i < c.n) {
+        float2 p;
+        if (src.x) {
+            p = make_float2(src.x[i], src.y[i]);
+            pos[i] = p;
+            vel[i] = make_float2(src.vx ? src.vx[i] : 0.0f, src.vy ? src.vy[i] : 0.0f);
+            prev[i] = p;
+            xr[i] = make_float4(p.x, p.y, 0.0f, 0.0f);
+        } else if (src.recs) {
+            const fluid_particle &q = src.recs[i];
+            p = make_float2(q.x, q.y);
+            pos[i] = p;
+            vel[i] = make_float2(q.v_x, q.v_y);
+            prev[i] = make_float2(q.x_prev, q.y_prev);
+            xr[i] = make_float4(q.x, q.y, q.density, q.density_near);
+        } else {
+            p = pos[i];
+        }
+        id[i] = i;
+        const unsigned key = cell_key(p.x, p.y, load_grid(c.scenes + scene_of(c, i)));
+        unsigned rank = 0u;
+        if (in_bounds(key, c.M, kBadKey)) {
+            rank = atomicAdd(cnt + key, 1u);
+            t = (int)(key / (unsigned)kBuildTile);
+        }
+        kr[i] = make_uint2(key, rank);
+    }
+    cta_tile_count(c.tile_cnt, t);
 }
 
 // The id-order records of k_unpermute (pos, vel, prev, (rho, rho_near),
 // pressures; n float2 each) -> six float arrays x, y, vx, vy, rho, rho_near
-// (n each, in that order), for copies straight into the caller's arrays.
+// (n each; null: not wanted), which may be the caller's own.
 __global__ void __launch_bounds__(kBlock)
-k_split_soa(int n, const float2 *__restrict__ rec, float *__restrict__ out)
+k_split_soa(int n, const float2 *__restrict__ rec, SoaColumns out)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const size_t m = (size_t)n;
     const float2 p = rec[i], v = rec[m + i], r = rec[3 * m + i];
-    out[i] = p.x;
-    out[m + i] = p.y;
-    out[2 * m + i] = v.x;
-    out[3 * m + i] = v.y;
-    out[4 * m + i] = r.x;
-    out[5 * m + i] = r.y;
+    const float f[6] = {p.x, p.y, v.x, v.y, r.x, r.y};
+#pragma unroll
+    for (int k = 0; k < 6; ++k)
+        if (out.c[k]) out.c[k][i] = f[k];
 }
 
-int launch_split_soa(sph_cuda *h, int n, const float2 *rec, float *out)
+int launch_split_soa(sph_cuda *h, int n, const float2 *rec, const SoaColumns &out)
 {
     if (n == 0) return SPH_OK;
     k_split_soa<<<blocks_for(n), kBlock, 0, h->stream>>>(n, rec, out);
     return cuda_fail(cudaGetLastError(), "split");
 }
 
-// Upload tail: pos_b / vel_b (id order) -> sorted A state; prev_c / xr_c
-// already hold the uploaded values in id order.
-int upload_soa_device(sph_cuda *h, int n)
+__global__ void k_enable_lists(DevState *st) { st->lists_valid = 1u; }
+
+int launch_enable_lists(sph_cuda *h)
 {
-    const int nb = blocks_for(n);
+    k_enable_lists<<<1, 1, 0, h->stream>>>(h->d_state);
+    return cuda_fail(cudaGetLastError(), "neighbour lists");
+}
+
+// Uploaded particles -> sorted A state; prev_c / xr_c hold the uploaded values
+// in id order.
+int upload_device(sph_cuda *h, int n, const UploadSource &src)
+{
+    if (n == 0) return SPH_OK;
     DevState *st = h->d_state;
-    if (n > 0) {
-        // a fresh state starts every step's build from zero tile counts,
-        // whatever an interrupted step left
-        cudaMemsetAsync(h->build_tiles, 0, (size_t)h->ntiles * sizeof(unsigned), h->stream);
-        k_iota<<<nb, kBlock, 0, h->stream>>>(n, h->id_c);
-        k_keys<<<nb, kBlock, 0, h->stream>>>(make_ctx(h), h->pos_b, h->kr_b, h->cnt,
-                                             &st->build_max_occ[SLOT_RELAXED]);
-        const int rc = launch_scan(h, h->cnt, h->M, h->start_a, &st->build_max_occ[SLOT_RELAXED],
-                                   true, h->d_nocell);
-        if (rc != SPH_OK) return rc;
-        k_scatter_ids<<<nb, kBlock, 0, h->stream>>>(n, h->kr_b, nullptr, h->start_a, h->tmp_id,
-                                                    nullptr, 0);
-        k_permute<<<nb, kBlock, 0, h->stream>>>(n, h->kr_b, h->start_a, h->tmp_id, nullptr,
-                                                h->pos_b, h->vel_b, h->id_a, h->pos_a, h->vel_a,
-                                                nullptr);
-    }
+    // a fresh state starts every step's build from zero tile counts,
+    // whatever an interrupted step left
+    cudaMemsetAsync(h->build_tiles, 0, (size_t)h->ntiles * sizeof(unsigned), h->stream);
+    launch_step(k_upload, blocks_for(n), kBlock, 0, h->stream, make_ctx(h), src, h->pos_b, h->vel_b,
+                h->prev_c, h->xr_c, h->id_c, h->kr_b, h->cnt, &st->build_max_occ[SLOT_RELAXED]);
+    cudaEventRecord(h->upload_ev, h->stream);  // the source has been read
+    enqueue_cell_starts(h, h->start_a, &st->build_max_occ[SLOT_RELAXED]);
+    enqueue_a_order(h, nullptr, [] {});
     return cuda_fail(cudaGetLastError(), "upload kernels");
 }
 
@@ -2571,7 +2464,7 @@ int launch_half_list_counts(sph_cuda *h, unsigned *d_counts, int *d_off)
     k_half_lists<false><<<blocks_for(n), kBlock, 0, h->stream>>>(
         make_ctx(h), h->pos_a, h->id_a, h->start_a, &h->d_state->build_max_occ[SLOT_RELAXED], d_counts,
         nullptr, nullptr, 0, 0);
-    const int rc = launch_scan(h, d_counts, n, d_off, nullptr, false, nullptr);
+    const int rc = launch_prefix(h, d_counts, n, d_off);
     return rc != SPH_OK ? rc : cuda_fail(cudaGetLastError(), "half list counts");
 }
 

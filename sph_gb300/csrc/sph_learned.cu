@@ -1654,20 +1654,30 @@ int sph_learned_forward(sph_learned_t *l, const float *features, int n, float *o
         features = copy.data();
     }
     for (int b = 0; b < nbuf; ++b) LTRY(ensure_forward(l, b, std::min(n, kForwardRows)));
-    PageToucher pages(out, overlap ? 0 : (size_t)n * ml::OUT * sizeof(float));
+    // a few rows: read and written in the caller's memory (kInPlaceRows)
+    const size_t in_bytes = (size_t)n * ml::IN * sizeof(float), out_bytes = (size_t)n * ml::OUT * sizeof(float);
+    const float *own_in = nullptr;
+    float4 *own_out = nullptr;
+    if (!overlap && in_bytes <= kInPlaceRows) {
+        own_in = static_cast<const float *>(host_in_place(features, in_bytes, 16, false));
+        own_out = static_cast<float4 *>(host_in_place(out, out_bytes, 16, true));
+    }
+    PageToucher pages(out, overlap || own_out ? 0 : out_bytes);
     int rc = SPH_OK, k = 0;
     for (int i0 = 0; i0 < n && rc == SPH_OK; i0 += kForwardRows, k ^= 1) {
         const int rows = std::min(n - i0, kForwardRows);
         cudaStream_t st = k ? l->stream2 : l->stream;
-        rc = cuda_fail(cudaMemcpyAsync(l->fwd_in[k], features + (size_t)i0 * ml::IN,
-                                       (size_t)rows * ml::IN * sizeof(float), cudaMemcpyHostToDevice, st),
-                       "feature rows");
+        if (!own_in)
+            rc = cuda_fail(cudaMemcpyAsync(l->fwd_in[k], features + (size_t)i0 * ml::IN,
+                                           (size_t)rows * ml::IN * sizeof(float),
+                                           cudaMemcpyHostToDevice, st),
+                           "feature rows");
         if (rc != SPH_OK) break;
         ml::k_mlp<true><<<std::min((rows + 127) / 128, num_sms()), ml::kMlpThreads, mlp_smem(), st>>>(
-            rows, l->fwd_in[k], l->wbf, l->w, l->fwd_out[k], l->h_err);
+            rows, own_in ? own_in : l->fwd_in[k], l->wbf, l->w, own_out ? own_out : l->fwd_out[k], l->h_err);
         rc = cuda_fail(cudaGetLastError(), "mlp launch");
         pages.done();
-        if (rc == SPH_OK)
+        if (rc == SPH_OK && !own_out)
             rc = cuda_fail(cudaMemcpyAsync(out + (size_t)i0 * ml::OUT, l->fwd_out[k],
                                            (size_t)rows * ml::OUT * sizeof(float),
                                            cudaMemcpyDeviceToHost, st),
