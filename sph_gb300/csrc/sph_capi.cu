@@ -139,7 +139,7 @@ void PageToucher::done()
 
 void *host_in_place(const void *p, size_t bytes, size_t align, bool write)
 {
-    if (bytes == 0 || bytes > kInPlaceBytes || (uintptr_t)p % align != 0) return nullptr;
+    if (bytes == 0 || (uintptr_t)p % align != 0) return nullptr;
     int dev = 0, shared_tables = 0;
     cudaPointerAttributes at{};
     if (cudaGetDevice(&dev) != cudaSuccess ||
@@ -151,12 +151,13 @@ void *host_in_place(const void *p, size_t bytes, size_t align, bool write)
     }
     if (!shared_tables || (at.type != cudaMemoryTypeUnregistered && at.type != cudaMemoryTypeHost))
         return nullptr;
-    const long ps = sysconf(_SC_PAGESIZE);
-    const size_t page = ps > 0 ? (size_t)ps : 4096;
     char *b = static_cast<char *>(const_cast<void *>(p));
     if (write) {
-        touch_pages(b, bytes, page);
+        PageToucher pages(b, bytes);
+        pages.done();
     } else {
+        const long ps = sysconf(_SC_PAGESIZE);
+        const size_t page = ps > 0 ? (size_t)ps : 4096;
         (void)*static_cast<volatile const char *>(b);
         for (uintptr_t a = ((uintptr_t)b / page + 1) * page; a < (uintptr_t)b + bytes; a += page)
             (void)*reinterpret_cast<volatile const char *>(a);
@@ -779,7 +780,8 @@ int sph_cuda_upload_soa(sph_cuda_t *h, const float *x, const float *y, const flo
         const float **const at[4] = {&src.x, &src.y, &src.vx, &src.vy};
         for (int k = 0; k < 4; ++k) {
             if (!from[k]) continue;
-            *at[k] = static_cast<const float *>(host_in_place(from[k], b, sizeof(float), false));
+            if (b <= kInPlaceBytes)
+                *at[k] = static_cast<const float *>(host_in_place(from[k], b, sizeof(float), false));
             if (*at[k]) continue;
             *at[k] = spare[k];
             SPH_CUDA(cudaMemcpyAsync(spare[k], from[k], b, cudaMemcpyHostToDevice, h->stream));
@@ -895,7 +897,8 @@ int sph_cuda_download_soa(sph_cuda_t *h, float *x, float *y, float *vx, float *v
     for (int k = 0; k < 6; ++k) {
         out.c[k] = nullptr;
         if (!dst[k]) continue;
-        if (apart) out.c[k] = static_cast<float *>(host_in_place(dst[k], col, sizeof(float), true));
+        if (apart && col <= kInPlaceBytes)
+            out.c[k] = static_cast<float *>(host_in_place(dst[k], col, sizeof(float), true));
         copied[k] = !out.c[k];
         if (copied[k]) out.c[k] = cols + k * (size_t)n;
     }

@@ -34,6 +34,31 @@ __device__ __forceinline__ void pdl_enter()
     pdl_trigger();
 }
 
+// Launches one kernel of a step on the handle's stream.  With SPH_PDL it is
+// a programmatic dependent launch: the kernel may start launching while
+// its predecessor's last CTAs still run, and waits for the predecessor's
+// results in pdl_enter (in stream capture this becomes a programmatic edge
+// of the step's graph).
+#ifndef SPH_PDL
+#define SPH_PDL 1
+#endif
+template <typename... KArgs, typename... Args>
+inline void launch_step(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem,
+                        cudaStream_t stream, Args &&...args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = SPH_PDL ? 1 : 0;
+    (void)cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
+}
+
 // A scene's grid, as the cell keys and stencils use it.  inv is 1/spacing
 // when spacing is a power of two (then x / spacing == x * inv exactly: both
 // round the same real number), 0 otherwise.

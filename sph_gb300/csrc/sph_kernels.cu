@@ -1937,31 +1937,6 @@ k_half_lists(Ctx c, const float2 *__restrict__ pos, const int *__restrict__ ids,
 
 static inline int blocks_for(int n, int bs = kBlock) { return (n + bs - 1) / bs; }
 
-// Launches one kernel of a step on the handle's stream.  With SPH_PDL it is
-// a programmatic dependent launch: the kernel may start launching while
-// its predecessor's last CTAs still run, and waits for the predecessor's
-// results in pdl_enter (in stream capture this becomes a programmatic edge
-// of the step's graph).
-#ifndef SPH_PDL
-#define SPH_PDL 1
-#endif
-template <typename... KArgs, typename... Args>
-static void launch_step(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem,
-                        cudaStream_t stream, Args &&...args)
-{
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = SPH_PDL ? 1 : 0;
-    (void)cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
-}
-
 // Grid of a gather launch for shape s.
 static inline dim3 gather_grid(const sph_cuda *h, const Shape &s)
 {

@@ -1230,25 +1230,6 @@ int gemm(cudaStream_t st, int M, int N, int K, const __nv_bfloat16 *A, long long
     return cuda_fail(cudaGetLastError(), "gemm launch");
 }
 
-// A launch that may start while its predecessor's last CTAs still run; the
-// kernel waits for the predecessor's results in pdl_enter.
-template <typename... KArgs, typename... Args>
-void launch_pdl(void (*kern)(KArgs...), int grid, int block, size_t smem, cudaStream_t stream,
-                Args... args)
-{
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(block);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    (void)cudaLaunchKernelEx(&cfg, kern, args...);
-}
-
 int check_err(LearnedModel *l)
 {
     unsigned e = 0;
@@ -1326,12 +1307,12 @@ int train_batch(LearnedModel *l, const int *order, int batch, int parts, int cma
                 float lr)
 {
     using namespace ml;
-    launch_pdl(k_train, parts, kTrainThreads, train_smem(), l->stream, batch / 128, order,
+    launch_step(k_train, parts, kTrainThreads, train_smem(), l->stream, batch / 128, order,
                (const __nv_bfloat16 *)l->X, (const float4 *)l->T, (const __nv_bfloat16 *)l->wbf,
                (const float *)l->w, cmask, trunk, l->part, l->loss, l->d_err);
     ++l->adam_t;
     const float b1t = powf(0.9f, (float)l->adam_t), b2t = powf(0.999f, (float)l->adam_t);
-    launch_pdl(k_adam, nblk(NPARAM, 128), 128, 0, l->stream, parts, (const float *)l->part,
+    launch_step(k_adam, nblk(NPARAM, 128), 128, 0, l->stream, parts, (const float *)l->part,
                (const double *)l->loss, l->w, l->m, l->v, cmask, trunk, lr, b1t, b2t, l->wbf,
                l->loss + l->parts_cap);
     return cuda_fail(cudaGetLastError(), "training step");
@@ -1388,7 +1369,7 @@ int train_loop(LearnedModel *l, int first, int nsamples, int epochs, int batch, 
 int launch_messages(sph_cuda *h, __nv_bfloat16 *feat, unsigned short *nbc, int max_nb)
 {
     if (h->n == 0) return SPH_OK;
-    launch_pdl(h->long_masks ? ml::k_messages<true> : ml::k_messages<false>, nblk(h->n), kBlock, 0,
+    launch_step(h->long_masks ? ml::k_messages<true> : ml::k_messages<false>, nblk(h->n), kBlock, 0,
                h->stream, make_ctx(h), (const float4 *)h->xr_c, (const ulonglong2 *)h->mask01_c,
                (const unsigned long long *)h->mask2_c, (const int4 *)h->rows_c,
                (const float2 *)h->prev_c, (const int *)h->start_c,
@@ -1403,7 +1384,7 @@ int run_mlp(cudaStream_t st, LearnedModel *l, int n, const __nv_bfloat16 *feat, 
     if (n == 0) return SPH_OK;
     LTRY(configure_kernels());
     const int grid = std::min((n + 127) / 128, sms > 0 ? sms : num_sms());
-    launch_pdl(ml::k_mlp<false>, grid, ml::kMlpThreads, mlp_smem(), st, n, (const void *)feat,
+    launch_step(ml::k_mlp<false>, grid, ml::kMlpThreads, mlp_smem(), st, n, (const void *)feat,
                (const __nv_bfloat16 *)l->wbf, (const float *)l->w, out, l->d_err);
     return cuda_fail(cudaGetLastError(), "mlp launch");
 }

@@ -24,7 +24,7 @@
 // so images are kept bottom row first until the final file order.
 #include <cmath>
 
-#include "sph_internal.h"
+#include "sph_device.cuh"
 
 namespace sph {
 namespace render {
@@ -72,18 +72,29 @@ __device__ __forceinline__ void splat_row(const Sprite &s, int y, int pitch, flo
     const int xa = max(s.x0, (int)floorf(s.cx - 0.5f - half));
     const int xb = min(s.x1, (int)ceilf(s.cx - 0.5f + half));
     unsigned *row = acc + (size_t)y * pitch;
-    for (int x4 = xa & ~3; x4 <= xb; x4 += 4) {
-        const uint4 t = __ldcg(reinterpret_cast<const uint4 *>(row + x4));
-        if (min(min(t.x, t.y), min(t.z, t.w)) >= 255u) continue;
-        const unsigned have[4] = {t.x, t.y, t.z, t.w};
+    // kGroup x 4 texels requested together (1,048,576 particles' image: with
+    // one 4 us more, with five, a whole row, 3 us more: the later texels have
+    // filled up by the time the first ones are done)
+    constexpr int kGroup = 2;
+    for (int g4 = xa & ~3; g4 <= xb; g4 += 4 * kGroup) {
+        uint4 t[kGroup];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const int x = x4 + k;
-            const float dx = ((float)x + 0.5f - s.cx) * inv;
-            const float r2 = dx * dx + dy * dy;
-            if (r2 > 0.34f || x < xa || x > xb || have[k] >= 255u) continue;
-            const int v = __float2int_rn((1.0f - 3.0f * r2) * 255.0f);
-            if (v > 0) atomicAdd(row + x, (unsigned)v);
+        for (int q = 0; q < kGroup; ++q)
+            t[q] = g4 + 4 * q <= xb ? __ldcg(reinterpret_cast<const uint4 *>(row + g4 + 4 * q))
+                                    : make_uint4(255u, 255u, 255u, 255u);
+#pragma unroll
+        for (int q = 0; q < kGroup; ++q) {
+            if (min(min(t[q].x, t[q].y), min(t[q].z, t[q].w)) >= 255u) continue;
+            const unsigned have[4] = {t[q].x, t[q].y, t[q].z, t[q].w};
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const int x = g4 + 4 * q + k;
+                const float dx = ((float)x + 0.5f - s.cx) * inv;
+                const float r2 = dx * dx + dy * dy;
+                if (r2 > 0.34f || x < xa || x > xb || have[k] >= 255u) continue;
+                const int v = __float2int_rn((1.0f - 3.0f * r2) * 255.0f);
+                if (v > 0) atomicAdd(row + x, (unsigned)v);
+            }
         }
     }
 }
@@ -104,9 +115,10 @@ __global__ void __launch_bounds__(256)
 k_splat(int n, int step, const short2 *__restrict__ coords, int w, int h, float radius, int pitch,
         unsigned *__restrict__ acc, const unsigned *__restrict__ full, int words_x)
 {
+    pdl_enter();
     const long long th = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const long long t = th / LANES;
-    const long long i = full ? t + t / (step - 1) + 1 : t * step;
+    const unsigned t = (unsigned)(th / LANES);  // below 2^31, as n is
+    const long long i = full ? (long long)t + t / (unsigned)(step - 1) + 1 : (long long)t * step;
     if (i >= n) return;
     const Sprite s = sprite_of(coords[i], w, h, radius);
     if (s.x0 > s.x1) return;
@@ -134,6 +146,7 @@ __global__ void __launch_bounds__(256)
 k_full_blocks(int w, int h, int pitch, const unsigned *__restrict__ acc, unsigned *__restrict__ full,
               int words_x)
 {
+    pdl_enter();
     const int bx = blockIdx.x * blockDim.x + threadIdx.x, by = blockIdx.y;
     bool all = bx * kBlk < w;
     for (int y = by * kBlk; y < min(h, (by + 1) * kBlk) && all; ++y)
@@ -172,6 +185,7 @@ template <bool VERTICAL, class T>
 __global__ void k_blur(int w, int h, int pitch, const T *__restrict__ in,
                        unsigned char *__restrict__ out)
 {
+    pdl_enter();
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
     const int y = blockIdx.y;
     if (x >= w || y >= h) return;
@@ -223,24 +237,40 @@ __device__ __forceinline__ unsigned composite_pixel(int X, int Y, int W, int H, 
            (unsigned)(unsigned char)__float2int_rn(b * 255.0f) << 16;
 }
 
-// The image, top row first.  A thread makes four pixels of a row and stores
-// their 12 bytes as three words where the width keeps every row's start on a
-// word (WORDS), else a thread per pixel and byte stores.
+// The image, top row first.  A thread makes four pixels of a row where the
+// width keeps every row's start on a word (WORDS), else one, with byte stores.
+// The image may be the caller's own memory (kInPlaceImage).
 template <bool WORDS>
-__global__ void k_composite(int W, int H, int w, int h, const unsigned char *__restrict__ a,
-                            unsigned char *__restrict__ rgb)
+__global__ void __launch_bounds__(256)
+k_composite(int W, int H, int w, int h, const unsigned char *__restrict__ a,
+            unsigned char *__restrict__ rgb)
 {
+    pdl_enter();
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     const int Y = blockIdx.y;
     if (WORDS) {
-        if (4 * q >= W) return;
-        unsigned c[4];
+        // four pixels a thread, the CTA's bytes by way of shared memory, so
+        // that they leave in whole 16-byte pieces
+        __shared__ uint4 stage[192];
+        if (4 * q < W) {
+            unsigned c[4];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) c[k] = composite_pixel(4 * q + k, Y, W, H, w, h, a);
-        unsigned *p = reinterpret_cast<unsigned *>(rgb + ((size_t)(H - 1 - Y) * W + 4 * q) * 3);
-        p[0] = c[0] | c[1] << 24;
-        p[1] = c[1] >> 8 | c[2] << 16;
-        p[2] = c[2] >> 16 | c[3] << 8;
+            for (int k = 0; k < 4; ++k) c[k] = composite_pixel(4 * q + k, Y, W, H, w, h, a);
+            unsigned *p = reinterpret_cast<unsigned *>(stage) + 3 * threadIdx.x;
+            p[0] = c[0] | c[1] << 24;
+            p[1] = c[1] >> 8 | c[2] << 16;
+            p[2] = c[2] >> 16 | c[3] << 8;
+        }
+        __syncthreads();
+        constexpr int kBytes = 4 * 3 * 256;  // a CTA's share of the row
+        const int at = blockIdx.x * kBytes, bytes = min(kBytes, W * 3 - at);
+        unsigned char *row = rgb + (size_t)(H - 1 - Y) * W * 3 + at;
+        if (W % 16 == 0) {
+            if (16 * (int)threadIdx.x < bytes) reinterpret_cast<uint4 *>(row)[threadIdx.x] = stage[threadIdx.x];
+        } else {
+            for (int e = threadIdx.x; 4 * e < bytes; e += blockDim.x)
+                reinterpret_cast<unsigned *>(row)[e] = reinterpret_cast<unsigned *>(stage)[e];
+        }
     } else {
         if (q >= W) return;
         const unsigned c = composite_pixel(q, Y, W, H, w, h, a);
@@ -285,8 +315,15 @@ static RenderScratch render_layout(int W, int H)
 
 static size_t render_scratch(int W, int H) { return render_layout(W, H).total; }
 
-static int render_device(cudaStream_t st, const short2 *coords, int n, int W, int H,
-                         unsigned char *d_rgb, unsigned char *scratch, unsigned char **alpha)
+static int render_clear(cudaStream_t st, int W, int H, unsigned char *scratch)
+{
+    const RenderScratch lay = render_layout(W, H);
+    return cuda_fail(cudaMemsetAsync(scratch + lay.acc, 0, (size_t)lay.pitch * (H / 2) * 4, st), "clear");
+}
+
+// After render_clear: the blurred reduced alpha from device coordinates.
+static int render_alpha(cudaStream_t st, const short2 *coords, int n, int W, int H,
+                        unsigned char *scratch, unsigned char **alpha)
 {
     using namespace render;
     const int w = W / 2, h = H / 2;
@@ -294,8 +331,6 @@ static int render_device(cudaStream_t st, const short2 *coords, int n, int W, in
     unsigned *acc = reinterpret_cast<unsigned *>(scratch + lay.acc);
     unsigned *full = reinterpret_cast<unsigned *>(scratch + lay.full);
     unsigned char *t0 = scratch + lay.t0, *t1 = scratch + lay.t1;
-    int rc = cuda_fail(cudaMemsetAsync(acc, 0, (size_t)lay.pitch * h * 4, st), "clear");
-    if (rc) return rc;
     const float radius = 0.5f * ((float)W * 0.020f / 2.0f);
     auto blocks = [](long long k) { return (int)((k + 255) / 256); };
     // two passes where the particles are many enough for full blocks to be
@@ -303,25 +338,35 @@ static int render_device(cudaStream_t st, const short2 *coords, int n, int W, in
     constexpr int kSample = 64;
     if (n >= kSplatTwoPass) {
         const int first = (n + kSample - 1) / kSample;
-        k_splat<8><<<blocks((long long)first * 8), 256, 0, st>>>(
-            n, kSample, coords, w, h, radius, lay.pitch, acc, nullptr, 0);
-        k_full_blocks<<<dim3((lay.words_x * 32 + 255) / 256, lay.blocks_y), 256, 0, st>>>(
-            w, h, lay.pitch, acc, full, lay.words_x);
-        k_splat<1><<<blocks((long long)(n - first) * 1), 256, 0, st>>>(
-            n, kSample, coords, w, h, radius, lay.pitch, acc, full, lay.words_x);
+        launch_step(k_splat<8>, blocks((long long)first * 8), 256, 0, st, n, kSample, coords, w, h, radius,
+                    lay.pitch, acc, (const unsigned *)nullptr, 0);
+        launch_step(k_full_blocks, dim3((lay.words_x * 32 + 255) / 256, lay.blocks_y), 256, 0, st, w, h,
+                    lay.pitch, (const unsigned *)acc, full, lay.words_x);
+        launch_step(k_splat<1>, blocks((long long)(n - first) * 1), 256, 0, st, n, kSample, coords, w, h, radius,
+                    lay.pitch, acc, (const unsigned *)full, lay.words_x);
     } else if (n > 0) {
-        k_splat<8><<<blocks((long long)n * 8), 256, 0, st>>>(n, 1, coords, w, h, radius,
-                                                                       lay.pitch, acc, nullptr, 0);
+        launch_step(k_splat<8>, blocks((long long)n * 8), 256, 0, st, n, 1, coords, w, h, radius, lay.pitch, acc,
+                    (const unsigned *)nullptr, 0);
     }
     const dim3 rows((w + 255) / 256, h);
-    k_blur<true><<<rows, 256, 0, st>>>(w, h, lay.pitch, (const unsigned *)acc, t1);
-    k_blur<false><<<rows, 256, 0, st>>>(w, h, w, (const unsigned char *)t1, t0);
-    if (W % 4 == 0)
-        k_composite<true><<<dim3((W / 4 + 255) / 256, H), 256, 0, st>>>(W, H, w, h, t0, d_rgb);
-    else
-        k_composite<false><<<dim3((W + 255) / 256, H), 256, 0, st>>>(W, H, w, h, t0, d_rgb);
+    launch_step(k_blur<true, unsigned>, rows, 256, 0, st, w, h, lay.pitch, (const unsigned *)acc, t1);
+    launch_step(k_blur<false, unsigned char>, rows, 256, 0, st, w, h, w, (const unsigned char *)t1, t0);
     *alpha = t0;
     return cuda_fail(cudaGetLastError(), "render");
+}
+
+static int render_composite(cudaStream_t st, const unsigned char *alpha, int W, int H,
+                            unsigned char *rgb)
+{
+    using namespace render;
+    const int w = W / 2, h = H / 2;
+    if (W % 4 == 0)
+        launch_step(k_composite<true>, dim3((W / 4 + 255) / 256, H), 256, 0, st, W, H, w, h,
+                    alpha, rgb);
+    else
+        launch_step(k_composite<false>, dim3((W + 255) / 256, H), 256, 0, st, W, H, w, h,
+                    alpha, rgb);
+    return cuda_fail(cudaGetLastError(), "composite");
 }
 
 static int check_size(int W, int H)
@@ -363,7 +408,9 @@ int sph_render_liquid(const short *coords, int n, int width, int height, unsigne
         if (n > 0)
             rc = cuda_fail(cudaMemcpyAsync(d_coords, coords, (size_t)n * 4, cudaMemcpyHostToDevice, st),
                            "coords");
-        if (!rc) rc = render_device(st, d_coords, n, width, height, d_rgb, scratch, &d_alpha);
+        if (!rc) rc = render_clear(st, width, height, scratch);
+        if (!rc) rc = render_alpha(st, d_coords, n, width, height, scratch, &d_alpha);
+        if (!rc) rc = render_composite(st, d_alpha, width, height, d_rgb);
         if (!rc) rc = cuda_fail(cudaMemcpyAsync(rgb, d_rgb, img, cudaMemcpyDeviceToHost, st), "image");
         if (!rc && alpha)
             rc = cuda_fail(cudaMemcpyAsync(alpha, d_alpha, m, cudaMemcpyDeviceToHost, st), "alpha");
@@ -393,14 +440,25 @@ int sph_cuda_render_liquid(sph_cuda_t *h, int width, int height, unsigned char *
     unsigned char *base = (unsigned char *)h->d_scratch;
     short2 *d_coords = reinterpret_cast<short2 *>(base);
     unsigned char *d_rgb = base + cb, *scratch = d_rgb + ib, *d_alpha = nullptr;
+    rc = render_clear(h->stream, width, height, scratch);
+    if (rc) return rc;
     if (n > 0) {
         rc = launch_pack(h, d_coords);
         if (rc) return rc;
     }
-    rc = render_device(h->stream, d_coords, n, width, height, d_rgb, scratch, &d_alpha);
-    PageToucher pages(rgb, img);  // while the kernels run
-    pages.done();
-    if (!rc) rc = cuda_fail(cudaMemcpyAsync(rgb, d_rgb, img, cudaMemcpyDeviceToHost, h->stream), "image");
+    rc = render_alpha(h->stream, d_coords, n, width, height, scratch, &d_alpha);
+    if (rc) return rc;
+    // composed in the caller's memory where the stores are whole 16-byte pieces
+    unsigned char *own = nullptr;
+    if (width % 16 == 0 && img <= kInPlaceImage)
+        own = static_cast<unsigned char *>(host_in_place(rgb, img, 16, true));
+    rc = render_composite(h->stream, d_alpha, width, height, own ? own : d_rgb);
+    if (!own) {
+        PageToucher pages(rgb, img);  // while the kernels run
+        pages.done();
+        if (!rc)
+            rc = cuda_fail(cudaMemcpyAsync(rgb, d_rgb, img, cudaMemcpyDeviceToHost, h->stream), "image");
+    }
     if (!rc && alpha)
         rc = cuda_fail(cudaMemcpyAsync(alpha, d_alpha, m, cudaMemcpyDeviceToHost, h->stream), "alpha");
     if (!rc) rc = cuda_fail(cudaStreamSynchronize(h->stream), "sync");

@@ -8,7 +8,7 @@ import numpy as np
 import pytest
 
 from conftest import bits_equal
-from sph_gb300 import LearnedModel, Simulation, _lib, scenes
+from sph_gb300 import LearnedModel, Simulation, _lib, render_liquid, scenes
 
 pytestmark = pytest.mark.gpu
 
@@ -102,3 +102,19 @@ def test_forward(cuda_lib, n, place):
         _lib.check(cuda_lib.sph_learned_forward(m._l, ptr(a), n, ptr(y)))
         big = np.concatenate([x, np.zeros((20000, LearnedModel.IN), np.float32)])  # copied
         assert bits_equal(y.copy().view(np.float32).reshape(n, -1), m.forward(big)[:n])
+
+
+@pytest.mark.parametrize("W,H", [(16, 2), (32, 33), (48, 20), (1024, 9), (1040, 9), (2064, 5), (36, 21), (34, 11), (35, 12)])
+@pytest.mark.parametrize("offset", [0, 4, 1])
+def test_image(cuda_lib, W, H, offset):
+    """Rows of whole 16-byte pieces, of words and of neither, in the caller's
+    memory or copied to it: the image of the same coordinates through a
+    buffer of the library's own."""
+    sc = random_scene(3000)
+    with Simulation.from_scene(sc) as s:
+        want = render_liquid(s.pack_coords(), W, H)[0]
+        raw = at_byte(np.full((H, W, 3), 77, np.uint8), offset)
+        up = ctypes.POINTER(ctypes.c_ubyte)
+        _lib.check(cuda_lib.sph_cuda_render_liquid(s.handle, W, H, ctypes.cast(raw.ctypes.data, up),
+                                                   ctypes.cast(None, up)))
+        assert np.array_equal(raw.reshape(H, W, 3), want)
