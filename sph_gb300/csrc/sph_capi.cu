@@ -24,8 +24,9 @@ int launch_scene_diagnostics(sph_cuda *h, double *d_out, double *partials);
 int scene_diagnostic_pieces(const sph_cuda *h);
 int launch_probe(sph_cuda *h, int which, void *scratch, float2 *out);
 size_t probe_scratch_bytes(int n);
-int launch_half_list_counts(sph_cuda *h, unsigned *d_counts, int *d_off);
-int launch_half_lists(sph_cuda *h, const int *d_off, int *d_ids, long long lo, long long m);
+int launch_half_list_counts(sph_cuda *h, unsigned *d_counts, int *d_off, int *total_out);
+int launch_half_lists(sph_cuda *h, const int *d_off, int *d_ids, long long lo, long long m,
+                      unsigned *counts_out = nullptr);
 const char *kernel_name(int k);
 int step_kernel_count();
 
@@ -340,7 +341,7 @@ static void free_all(sph_cuda *h)
         if (h->copy_ev[k]) cudaEventDestroy(h->copy_ev[k]);
     }
     if (h->copy_stream) cudaStreamDestroy(h->copy_stream);
-    if (h->upload_ev) cudaEventDestroy(h->upload_ev);
+    if (h->host_ev) cudaEventDestroy(h->host_ev);
     void *ptrs[] = {h->pos_a, h->vel_a, h->id_a, h->pos_b, h->prev_b, h->vel_b, h->kr_b,
                     h->pos_c, h->prev_c, h->xr_c, h->mask01_c, h->mask2_c, h->maskx_c, h->rows_c, h->id_c,
                     h->tmp_id, h->cnt, h->start_a, h->start_c, h->tile_sums, h->build_tiles, h->d_scenes,
@@ -456,7 +457,7 @@ static int build_handle(sph_cuda **out, std::vector<Scene> &&scenes, int capacit
     rc = cuda_fail(cudaStreamCreateWithFlags(&h->own_stream, cudaStreamNonBlocking),
                    "cudaStreamCreate");
     if (rc) return fail(rc);
-    rc = cuda_fail(cudaEventCreateWithFlags(&h->upload_ev, cudaEventDisableTiming), "event");
+    rc = cuda_fail(cudaEventCreateWithFlags(&h->host_ev, cudaEventDisableTiming), "event");
     if (rc) return fail(rc);
     h->stream = h->own_stream;
     const size_t N = (size_t)capacity;
@@ -533,7 +534,7 @@ static int upload_finish(sph_cuda *h, int n, const UploadSource &src = UploadSou
     SPH_CUDA(cudaMemsetAsync(h->d_state, 0, sizeof(DevState), h->stream));
     SPH_TRY(upload_device(h, n, src));
     // the caller's buffers are free again (the sort goes on behind the call)
-    SPH_CUDA(cudaEventSynchronize(h->upload_ev));
+    SPH_CUDA(cudaEventSynchronize(h->host_ev));
     return SPH_OK;
 }
 
@@ -1150,18 +1151,28 @@ int sph_cuda_neighbor_lists(sph_cuda_t *h, int *counts, int *ids, long long max_
     unsigned *d_counts = (unsigned *)h->d_scratch;
     int *d_off = (int *)((char *)h->d_scratch + part);
     int *d_ids = (int *)((char *)h->d_scratch + 2 * part);
-    SPH_TRY(launch_half_list_counts(h, d_counts, d_off));
+    // the total comes with the prefix sums: the host goes on from there while
+    // the GPU writes the lists, and the counts into the caller's memory
+    SPH_TRY(ensure_stage(h, 256));
+    volatile int *stage_total = static_cast<int *>(h->h_stage);
+    const size_t cb = (size_t)n * sizeof(int);
+    unsigned *own = nullptr;
+    if (piece > 0 && cb <= kInPlaceBytes)
+        own = static_cast<unsigned *>(host_in_place(counts, cb, sizeof(int), true));
+    SPH_TRY(launch_half_list_counts(h, d_counts, d_off, static_cast<int *>(h->h_stage)));
+    SPH_CUDA(cudaEventRecord(h->host_ev, h->stream));
     // the first piece (nearly always all of them) is written before the host
     // has seen the total: the GPU does not wait for the question whether the
     // caller's buffer holds it
-    if (piece > 0) SPH_TRY(launch_half_lists(h, d_off, d_ids, 0, piece));
-    PageToucher count_pages(counts, (size_t)n * sizeof(int));
-    int tot = 0;
-    SPH_CUDA(cudaMemcpyAsync(&tot, d_off + n, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
-    count_pages.done();
-    SPH_CUDA(cudaMemcpyAsync(counts, d_counts, (size_t)n * sizeof(int), cudaMemcpyDeviceToHost,
-                             h->stream));
-    SPH_CUDA(cudaStreamSynchronize(h->stream));
+    if (piece > 0) SPH_TRY(launch_half_lists(h, d_off, d_ids, 0, piece, own));
+    if (!own) {
+        PageToucher count_pages(counts, cb);
+        count_pages.done();
+        SPH_CUDA(cudaMemcpyAsync(counts, d_counts, cb, cudaMemcpyDeviceToHost, h->stream));
+    }
+    SPH_CUDA(cudaEventSynchronize(h->host_ev));
+    const int tot = *stage_total;
+    if (tot > max_total || !ids || tot == 0) SPH_CUDA(cudaStreamSynchronize(h->stream));
     *total = tot;
     if (tot > max_total || (!ids && tot > 0)) {
         set_error("neighbour list buffer holds %lld entries, %d needed", max_total, tot);

@@ -200,7 +200,7 @@ struct sph_cuda {
     short2 *d_coords[2] = {nullptr, nullptr};
     cudaEvent_t pack_ev[2] = {nullptr, nullptr};
     cudaEvent_t copy_ev[2] = {nullptr, nullptr};
-    cudaEvent_t upload_ev = nullptr;  // the last upload's source has been read
+    cudaEvent_t host_ev = nullptr;  // the host goes on here, beside the rest of a call's kernels
     const void *copy_dst[2] = {nullptr, nullptr};
     int pack_slot = 0;
 };
@@ -291,7 +291,9 @@ int enqueue_step(sph_cuda *h, cudaEvent_t *events, int *nkernels,
 unsigned bounds_flags_kernels();  // checked builds (SPH_BOUNDS_CHECK): recorded index faults
 unsigned bounds_flags_learned();
 int enqueue_predicted_state(sph_cuda *h);       // first half of a step: C order + density
-int launch_prefix(sph_cuda *h, unsigned *in, int n, int *out);  // exclusive prefix sums, out[n] = total
+// Exclusive prefix sums, out[n] = total, and with `total` there too (it may be
+// page-locked host memory).
+int launch_prefix(sph_cuda *h, unsigned *in, int n, int *out, int *total = nullptr);
 int launch_static_density(const Scene &sc, const StaticArrays &a, const float *x, const float *y,
                           float *rho, float *rho_near, cudaStream_t st);
 int launch_density_pass(sph_cuda *h);            // the density pass on the C order

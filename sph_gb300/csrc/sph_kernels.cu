@@ -176,6 +176,7 @@ __device__ __forceinline__ unsigned block_exclusive_scan(unsigned v, unsigned *s
 __global__ void __launch_bounds__(kScanThreads)
 k_scan_reduce(const unsigned *__restrict__ in, int M, int *__restrict__ tile_sums)
 {
+    pdl_enter();
     __shared__ unsigned sh_s[kScanThreads / 32];
     const int base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
     unsigned s = 0;
@@ -201,11 +202,13 @@ k_scan_reduce(const unsigned *__restrict__ in, int M, int *__restrict__ tile_sum
     }
 }
 
-// Exclusive scan: out[i] = sum(in[0..i)), out[M] = total.
+// Exclusive scan: out[i] = sum(in[0..i)), out[M] = total, which goes to
+// total_out too (if any).
 __global__ void __launch_bounds__(kScanThreads)
 k_scan_apply(const unsigned *__restrict__ in, int M, const int *__restrict__ tile_sums,
-             int *__restrict__ out)
+             int *__restrict__ out, int *__restrict__ total_out)
 {
+    pdl_enter();
     __shared__ unsigned sh[kScanThreads / 32];
     __shared__ unsigned sh_prefix;
     // prefix of all earlier tiles
@@ -262,7 +265,10 @@ k_scan_apply(const unsigned *__restrict__ in, int M, const int *__restrict__ til
             }
         }
     }
-    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == blockDim.x - 1) out[M] = (int)(prefix + total);
+    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == blockDim.x - 1) {
+        out[M] = (int)(prefix + total);
+        if (total_out) *total_out = (int)(prefix + total);
+    }
 }
 
 // Cell starts of a step's build in one pass over the counters: the key
@@ -1885,7 +1891,8 @@ k_diag_scenes_final(Ctx c, int pieces, const double *__restrict__ partials, doub
 // later members of its own cell, then the forward cells (0,+1), (+1,-1),
 // (+1,0), (+1,+1), each in id order, r2 <= h2, cut at max_neighbors.
 // WRITE = false counts, WRITE = true writes the entries at off[id], those of
-// them in [lo, lo + m), to out[entry - lo].
+// them in [lo, lo + m), to out[entry - lo] (and the counts, if asked, in the
+// order of their ids, as suits host memory).
 template <bool WRITE>
 __global__ void __launch_bounds__(kBlock)
 k_half_lists(Ctx c, const float2 *__restrict__ pos, const int *__restrict__ ids,
@@ -1893,8 +1900,10 @@ k_half_lists(Ctx c, const float2 *__restrict__ pos, const int *__restrict__ ids,
              unsigned *__restrict__ counts, const int *__restrict__ off, int *__restrict__ out,
              long long lo, long long m)
 {
+    pdl_enter();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= c.n) return;
+    if (WRITE && counts) counts[i] = (unsigned)(off[i + 1] - off[i]);
     const Scene *S = c.scenes + scene_of(c, i);
     const SG g = load_grid(S);
     const float hh = __ldg(&S->P.smoothing_radius);
@@ -1948,7 +1957,7 @@ static inline dim3 gather_grid(const sph_cuda *h, const Shape &s)
 
 // Exclusive scan of `in` (M entries) into out (M + 1 entries).  Both arrays
 // must be 16-byte aligned: the scan kernels move 16-byte vectors.
-int launch_prefix(sph_cuda *h, unsigned *in, int M, int *out)
+int launch_prefix(sph_cuda *h, unsigned *in, int M, int *out, int *total)
 {
     if (((uintptr_t)in | (uintptr_t)out) & 15u) {
         set_error("internal: scan arrays not 16-byte aligned");
@@ -1959,8 +1968,10 @@ int launch_prefix(sph_cuda *h, unsigned *in, int M, int *out)
         set_error("internal: scan of %d items exceeds the tile buffer", M);
         return SPH_ERR_INVALID;
     }
-    k_scan_reduce<<<tiles, kScanThreads, 0, h->stream>>>(in, M, h->tile_sums);
-    k_scan_apply<<<tiles, kScanThreads, 0, h->stream>>>(in, M, h->tile_sums, out);
+    launch_step(k_scan_reduce, tiles, kScanThreads, 0, h->stream, (const unsigned *)in, M,
+                h->tile_sums);
+    launch_step(k_scan_apply, tiles, kScanThreads, 0, h->stream, (const unsigned *)in, M,
+                (const int *)h->tile_sums, out, total);
     return SPH_OK;
 }
 
@@ -2337,7 +2348,7 @@ int upload_device(sph_cuda *h, int n, const UploadSource &src)
     cudaMemsetAsync(h->build_tiles, 0, (size_t)h->ntiles * sizeof(unsigned), h->stream);
     launch_step(k_upload, blocks_for(n), kBlock, 0, h->stream, make_ctx(h), src, h->pos_b, h->vel_b,
                 h->prev_c, h->xr_c, h->id_c, h->kr_b, h->cnt, &st->build_max_occ[SLOT_RELAXED]);
-    cudaEventRecord(h->upload_ev, h->stream);  // the source has been read
+    cudaEventRecord(h->host_ev, h->stream);  // the source has been read
     enqueue_cell_starts(h, h->start_a, &st->build_max_occ[SLOT_RELAXED]);
     enqueue_a_order(h, nullptr, [] {});
     return cuda_fail(cudaGetLastError(), "upload kernels");
@@ -2431,24 +2442,27 @@ int launch_probe(sph_cuda *h, int which, void *scratch, float2 *out)
 
 // Half lists in the reference's order on the A state: the counts by id and
 // their prefix sums (d_counts: n words, d_off: n + 1 ints, both 16-byte
-// aligned), or the entries [lo, lo + m) of the lists.
-int launch_half_list_counts(sph_cuda *h, unsigned *d_counts, int *d_off)
+// aligned; total_out: as launch_prefix), or the entries [lo, lo + m) of the
+// lists (and, with counts_out, the counts once more, for host memory).
+int launch_half_list_counts(sph_cuda *h, unsigned *d_counts, int *d_off, int *total_out)
 {
     const int n = h->n;
     if (n == 0) return SPH_OK;
     k_half_lists<false><<<blocks_for(n), kBlock, 0, h->stream>>>(
         make_ctx(h), h->pos_a, h->id_a, h->start_a, &h->d_state->build_max_occ[SLOT_RELAXED], d_counts,
         nullptr, nullptr, 0, 0);
-    const int rc = launch_prefix(h, d_counts, n, d_off);
+    const int rc = launch_prefix(h, d_counts, n, d_off, total_out);
     return rc != SPH_OK ? rc : cuda_fail(cudaGetLastError(), "half list counts");
 }
 
-int launch_half_lists(sph_cuda *h, const int *d_off, int *d_ids, long long lo, long long m)
+int launch_half_lists(sph_cuda *h, const int *d_off, int *d_ids, long long lo, long long m,
+                      unsigned *counts_out)
 {
     if (h->n == 0) return SPH_OK;
-    k_half_lists<true><<<blocks_for(h->n), kBlock, 0, h->stream>>>(
-        make_ctx(h), h->pos_a, h->id_a, h->start_a, &h->d_state->build_max_occ[SLOT_RELAXED], nullptr,
-        d_off, d_ids, lo, m);
+    launch_step(k_half_lists<true>, blocks_for(h->n), kBlock, 0, h->stream, make_ctx(h),
+                (const float2 *)h->pos_a, (const int *)h->id_a, (const int *)h->start_a,
+                (const unsigned *)&h->d_state->build_max_occ[SLOT_RELAXED], counts_out, d_off,
+                d_ids, lo, m);
     return cuda_fail(cudaGetLastError(), "half lists");
 }
 
