@@ -30,9 +30,9 @@
 #include "sph_learned.h"
 
 namespace sph {
-// Stencil rows of up to kShortRow candidates have their hits marked first and
-// then walked, longer ones are gathered in one loop over the candidates
-// (density_filter and viscosity_long_rows say why; with the line at 20 to 28
+// Particles whose stencil rows have up to kShortRow candidates have their hits
+// marked first and then walked, the others are gathered in one loop over the
+// candidates (density_filter and viscosity_long_rows say why; with the line at 20 to 28
 // the dam break's 1,048,576 particles lost 2-8% of the viscosity pass and the
 // other states stayed within 1%).
 constexpr int kShortRow = 32;
@@ -597,14 +597,13 @@ __device__ __forceinline__ void visc_impulse(const ViscConsts &c, float2 e, floa
     dv = __ffma2_rn(make_float2(-0.5f, -0.5f), make_float2(clamp5(t.x), clamp5(t.y)), dv);
 }
 
-// The sum of a particle with a stencil row of more than 32 candidates, or
-// with an overflowing bucket somewhere: rows of up to 32 marked and walked,
-// longer ones in one loop over the candidates (the lanes of a warp are then
-// mostly of one cell and read the same candidate at a time, which a walk over
-// each lane's own hits does not: the dam break's 1,048,576 particles
-// compressed: all rows marked and walked 218 us, this 187 us; 64 scenes 231
-// and 220 us).  Out of line:
-// compiled into the pass it cost the short rows' walk its registers.
+// The sum of a particle with a stencil row of more than kShortRow candidates,
+// or with an overflowing bucket somewhere, in one loop over the candidates:
+// the lanes of a warp are then mostly of one cell and read the same candidate
+// at a time, which a walk over each lane's own hits does not (the dam break's
+// 1,048,576 particles, compressed: all rows marked and walked 218 us, this 187
+// us; 64 compressed scenes 231 and 217 us).  Out of line: compiled into the
+// pass it cost the short rows' walk its registers.
 __device__ __noinline__ float2 viscosity_long_rows(int i, const Scene *S,
                                                    const float2 *__restrict__ pos,
                                                    const float2 *__restrict__ vel,
@@ -637,18 +636,8 @@ __device__ __noinline__ float2 viscosity_long_rows(int i, const Scene *S,
 #pragma unroll 1
     for (int r = 0; r < 3; ++r) {
         const int a = ra[r], l = rl[r];
-        if (l <= kShortRow) {
-            unsigned b = hit_mask32<kMarkUnroll>(pos + a, l, mp, vc.h2);
-            if (r == 1) b &= ~(1u << (i - a));
-            while (b) {
-                const int j = a + __ffs(b) - 1;
-                b &= b - 1u;
-                one(j);
-            }
-        } else {
 #pragma unroll kViscLongUnroll
-            for (int j = a; j < a + l; ++j) one(j);
-        }
+        for (int j = a; j < a + l; ++j) one(j);
     }
     return dv;
 }
@@ -746,7 +735,7 @@ k_viscosity_predict(Ctx c, const DevState *__restrict__ st, const float2 *__rest
 // [ra[r], ra[r] + rl[r])).  Rows of up to kShortRow candidates are marked
 // first and the marked ones walked: the terms are run for the hits alone,
 // where one loop over the candidates runs them for nearly every candidate of a
-// warp (some lane hits).  Longer rows keep the one loop: there the lanes of a
+// warp (some lane hits).  Particles with a longer row keep the one loop: there the lanes of a
 // warp are mostly of one cell and read the same candidate at a time, which a
 // walk over each lane's own hits does not.  4,194,304 particles: one loop for
 // every row 182 us early in the dam break and 201 us compressed, this 143 and
@@ -785,19 +774,6 @@ __device__ __forceinline__ void density_filter(int i, float2 mp, float h2, float
 #pragma unroll
     for (int r = 0; r < 3; ++r) {
         const int len = rl[r];
-        if (len <= kShortRow) {
-            const float2 *row = pos + ra[r];
-            unsigned b = hit_mask32<kMarkUnroll>(row, len, mp, h2);
-            if (r == 1) b &= ~(1u << (i - ra[1]));
-            m[r] = b;
-            while (b) {
-                const int t = __ffs(b) - 1;
-                b &= b - 1u;
-                float2 e;
-                add_density(ab, dist2_packed(mp, __ldg(row + t), e), h_recip);
-            }
-            continue;
-        }
         unsigned long long w0 = 0ull, w1 = 0ull;
         for (int c0 = 0; c0 < len; c0 += 32) {
             const int a = ra[r] + c0, n = min(len - c0, 32);
