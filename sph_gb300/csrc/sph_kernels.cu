@@ -582,7 +582,7 @@ __device__ __forceinline__ void visc_impulse(const ViscConsts &c, float2 e, floa
     }
     const float r = r2 * r_recip;
     const float2 w = __fadd2_rn(v0, make_float2(-dvel.x, -dvel.y));
-    const float u0 = (w.x * e.x + w.y * e.y) * r_recip;
+    const float u0 = __fmaf_rn(w.x, e.x, __fmul_rn(w.y, e.y)) * r_recip;
     // only approaching pairs (u > 0) push; the others run the same
     // instructions with u = 0, whose impulse is +-0 and leaves dv's bits
     // as they are (no divergent branch: about half the pairs of every
@@ -979,29 +979,6 @@ __device__ __noinline__ bool is_nudge(int i, int j, const Scene *S, const float4
     return owns_pair(cell_key(me.x, me.y, g), ids[i], make_float2(q.x, q.y), ids[j], g);
 }
 
-// The nudges of particle i, searched for again once its walk has met a pair
-// that may be one -- out of line, so that neither the ids nor the scene are
-// live across the walks.
-__device__ __noinline__ int count_nudges(int i, const Scene *S, const float4 *__restrict__ xr,
-                                         const int *__restrict__ ids, const int *__restrict__ start,
-                                         bool capped, int max_bucket, int n)
-{
-    const SG g = load_grid(S);
-    const float hh = __ldg(&S->P.smoothing_radius), h2 = __fmul_rn(hh, hh);
-    const float4 me = __ldg(xr + i);
-    const float2 mp = make_float2(-me.x, -me.y);
-    const unsigned key = cell_key(me.x, me.y, g);
-    int nudges = 0;
-    if (!searchable(key, i, start, g, capped, max_bucket)) return 0;
-    for_each_candidate(key, start, g, capped, max_bucket, n, [&](int j) {
-        const float4 q = __ldg(xr + j);
-        float2 e;
-        const float r2 = dist2_packed(mp, make_float2(q.x, q.y), e);
-        if (r2 <= 2e-12f && r2 <= h2 && is_nudge(i, j, S, xr, ids)) ++nudges;
-    });
-    return nudges;
-}
-
 // The pair term of one neighbour (r2 <= h2 known, not the particle itself):
 // returns whether it displaces the particle, by s (p - q) with d = q - p (the
 // caller adds -s d with one packed FMA); `rare` is set by a pair that may be
@@ -1018,11 +995,13 @@ __device__ __forceinline__ bool relax_pair_term(const WalkConsts &c, float2 p, f
         r_recip = rsqrtf(r2);
     }
     const float r = r2 * r_recip;
-    const float ratio = r * c.h_recip;
+    const float ratio = __fmul_rn(r, c.h_recip);
     if (!(ratio < 1.0f)) return false;
-    const float omr = 1.0f - ratio;
-    const float D = (c.Pd + c.kd * q.z) * omr + (c.Pnd + c.knd * q.w) * omr * omr +
-                    (c.hshd - c.hsd * r);
+    // rounded step by step: the same bits wherever this is compiled into
+    const float omr = __fsub_rn(1.0f, ratio);
+    const float near = __fmul_rn(__fmaf_rn(c.knd, q.w, c.Pnd), omr);
+    const float X = __fmaf_rn(__fmaf_rn(c.kd, q.z, c.Pd), omr, __fmul_rn(near, omr));
+    const float D = __fadd_rn(X, __fmaf_rn(-c.hsd, r, c.hshd));
     s = D * r_recip;
     return true;
 }
@@ -1034,58 +1013,6 @@ __device__ __forceinline__ void relax_pair_walk(const WalkConsts &c, float2 p, f
     float2 d;
     if (relax_pair_term(c, p, q, s, d, rare))
         a = __ffma2_rn(make_float2(-s, -s), d, a);  // += s (p - q), per component
-}
-
-// The displacement of a particle whose rows have no hit masks (a row too long
-// for them, or an overflowing bucket), in slot order, 32 candidates marked
-// and walked at a time.  Out of line: compiled into the relaxation it cost
-// the masked walk its registers.
-struct ColdSum {
-    float x, y;
-    int rare;
-};
-__device__ __noinline__ ColdSum relax_unmasked(int i, const Scene *S, const float4 *__restrict__ xr,
-                                               const int *__restrict__ start, bool capped,
-                                               int max_bucket, int n)
-{
-    const SG g = load_grid(S);
-    const RelaxConsts c = relax_consts(S);
-    const float4 me = __ldg(xr + i);
-    const WalkConsts wc = walk_consts(c, me);
-    const float2 p = make_float2(me.x, me.y), mp = make_float2(-me.x, -me.y);
-    float2 acc = make_float2(0.0f, 0.0f);
-    bool rare = false;
-    auto visit = [&](int, const float4 &q) { relax_pair_walk(wc, p, q, acc, rare); };
-    const unsigned key = cell_key(p.x, p.y, g);
-    if (searchable(key, i, start, g, capped, max_bucket)) {
-        if (!capped) {
-            int ra[3], rl[3];
-            stencil_rows(p, key, start, g, ra, rl, n);
-#pragma unroll 1
-            for (int r = 0; r < 3; ++r)
-#pragma unroll 1
-                for (int c0 = 0; c0 < rl[r]; c0 += 32) {
-                    const int a = ra[r] + c0, m = min(rl[r] - c0, 32);
-                    unsigned b = 0u;
-#pragma unroll 4
-                    for (int t = 0; t < m; ++t) {
-                        const float4 q = __ldg(xr + a + t);
-                        float2 e;
-                        if (dist2_packed(mp, make_float2(q.x, q.y), e) <= c.h2) b |= 1u << t;
-                    }
-                    if (r == 1 && (unsigned)(i - a) < 32u) b &= ~(1u << (i - a));
-                    walk_mask32<float4>(b, a, n, [&](int j) { return __ldg(xr + j); }, visit);
-                }
-        } else {
-            for_each_candidate(key, start, g, true, max_bucket, n, [&](int j) {
-                if (j == i) return;
-                const float4 q = __ldg(xr + j);
-                if (dist2(p.x - q.x, p.y - q.y) > c.h2) return;
-                visit(j, q);
-            });
-        }
-    }
-    return {acc.x, acc.y, rare ? 1 : 0};
 }
 
 // double_density_relaxation (fluid.c:541-611) in gather form:
@@ -1111,50 +1038,169 @@ struct LearnedIn {
     bool defer = false;  // leave the fallback particles to a second pass
 };
 
+// What a relaxation reads and writes.
+struct RelaxArrays {
+    Ctx c;
+    const float4 *xr;
+    const ulonglong2 *mask01;
+    const unsigned long long *mask2;
+    const int4 *rows;
+    const float2 *prev;
+    const int *ids, *start;
+    const unsigned *occ_in;  // the build's largest cell population
+    float2 *pos_out, *vel_out;
+    uint2 *kr_out;
+    unsigned *cnt;
+    float2 *probe_out;
+};
+
 // The end of a particle's relaxation: x += the displacement and the owner's
 // nudges, boundaryConditions, then updateVelocity (fluid.c:627-653):
 // v = (x - x_prev)/dt clamped to +-5, and the new position's cell key
 // counted into the build of the relaxed positions.
-__device__ __forceinline__ void relax_finish(int i, const Ctx &cx, const Scene *S, float2 p,
-                                             float2 acc, int nudges,
-                                             const float2 *__restrict__ prev,
-                                             float2 *__restrict__ pos_out,
-                                             float2 *__restrict__ vel_out,
-                                             uint2 *__restrict__ kr_out,
-                                             unsigned *__restrict__ cnt, int *tile_made)
+__device__ __forceinline__ void relax_finish(int i, const RelaxArrays &A, const Scene *S, float2 p,
+                                             float2 acc, int nudges, int *tile_made)
 {
     const float nd = (float)nudges * 0.000001f;
     float nx = __fadd_rn(__fadd_rn(p.x, acc.x), nd);
     float ny = __fadd_rn(__fadd_rn(p.y, acc.y), nd);
     boundary_of(nx, ny, S);
-    const float2 pv = prev[i];
+    const float2 pv = A.prev[i];
     const float dt_end = __ldg(&S->P.time_step);
     const float vx = clamp5(__fdiv_rn(__fsub_rn(nx, pv.x), dt_end));
     const float vy = clamp5(__fdiv_rn(__fsub_rn(ny, pv.y), dt_end));
     const unsigned k2 = cell_key(nx, ny, load_grid(S));
     unsigned rank = 0u;
-    if (in_bounds(k2, cx.M, kBadKey)) {
-        rank = atomicAdd(cnt + k2, 1u);
+    if (in_bounds(k2, A.c.M, kBadKey)) {
+        rank = atomicAdd(A.cnt + k2, 1u);
         if (tile_made)
             *tile_made = (int)(k2 / (unsigned)kBuildTile);
         else
-            add_tile_count(cx.tile_cnt, k2);
+            add_tile_count(A.c.tile_cnt, k2);
     }
-    pos_out[i] = make_float2(nx, ny);
-    vel_out[i] = make_float2(vx, vy);
-    kr_out[i] = make_uint2(k2, rank);
+    A.pos_out[i] = make_float2(nx, ny);
+    A.vel_out[i] = make_float2(vx, vy);
+    A.kr_out[i] = make_uint2(k2, rank);
 }
 
-template <bool PROBE, bool LEARNED = false, bool LM = false>
-__device__ __forceinline__ void relax_update_one(
-    int i, const Ctx &cx, const float4 *__restrict__ xr, const ulonglong2 *__restrict__ mask01,
-    const unsigned long long *__restrict__ mask2, const int4 *__restrict__ rows,
-    const float2 *__restrict__ prev, const int *__restrict__ ids, const int *__restrict__ start,
-    bool capped, float2 *__restrict__ pos_out, float2 *__restrict__ vel_out,
-    uint2 *__restrict__ kr_out, unsigned *__restrict__ cnt, float2 *__restrict__ probe_out,
-    const LearnedIn &L = LearnedIn(), bool *used_net = nullptr, int *tile_made = nullptr)
+// What the masked walk does not take itself is out of line and runs to the end
+// of the particle's relaxation, so that nothing of the caller lives across the
+// call: compiled into the pass, or called for a part of the work, these paths
+// cost the masked walk its registers.
+template <bool PROBE>
+__device__ __forceinline__ void relax_end_cold(int i, const RelaxArrays &A, const Scene *S, float2 p,
+                                               float2 acc, int nudges)
 {
+    if (PROBE) {
+        const float nd = (float)nudges * 0.000001f;
+        A.probe_out[i] = make_float2(acc.x + nd, acc.y + nd);
+        return;
+    }
+    relax_finish(i, A, S, p, acc, nudges, nullptr);
+}
+
+// A particle whose walk (to the displacement acc) has met a pair that may be a
+// nudge: they are searched for again.
+template <bool PROBE>
+__device__ __noinline__ void relax_nudged(int i, const RelaxArrays &A, float2 acc)
+{
+    const Scene *S = A.c.scenes + scene_of(A.c, i);
+    const SG g = load_grid(S);
+    const float hh = __ldg(&S->P.smoothing_radius), h2 = __fmul_rn(hh, hh);
+    const float4 me = __ldg(A.xr + i);
+    const float2 p = make_float2(me.x, me.y), mp = make_float2(-me.x, -me.y);
+    const unsigned key = cell_key(p.x, p.y, g);
+    const bool capped = *A.occ_in > (unsigned)A.c.max_bucket;
+    int nudges = 0;
+    if (searchable(key, i, A.start, g, capped, A.c.max_bucket))
+        for_each_candidate(key, A.start, g, capped, A.c.max_bucket, A.c.n, [&](int j) {
+            const float4 q = __ldg(A.xr + j);
+            float2 e;
+            const float r2 = dist2_packed(mp, make_float2(q.x, q.y), e);
+            if (r2 <= 2e-12f && r2 <= h2 && is_nudge(i, j, S, A.xr, A.ids)) ++nudges;
+        });
+    relax_end_cold<PROBE>(i, A, S, p, acc, nudges);
+}
+
+// A particle whose rows have no hit masks (a row too long for them, or an
+// overflowing bucket), in slot order as everywhere.  MARK: 32 candidates
+// marked and their hits walked at a time, where the lanes of a warp are of
+// different cells (the fallback list: 117 us for 219,000 particles, in one
+// loop over the candidates 129); one loop where they are mostly of one
+// (4,194,304 particles, compressed further: 475 -> 355 us; 64 compressed
+// scenes 206 -> 174 us).  No calls inside the loops, which would cost them
+// registers.
+template <bool PROBE, bool MARK>
+__device__ __noinline__ void relax_cold(int i, const RelaxArrays &A)
+{
+    const Ctx &cx = A.c;
     const Scene *S = cx.scenes + scene_of(cx, i);
+    const SG g = load_grid(S);
+    const RelaxConsts c = relax_consts(S);
+    const float4 *xr = A.xr;
+    const float4 me = __ldg(xr + i);
+    const WalkConsts wc = walk_consts(c, me);
+    const float2 p = make_float2(me.x, me.y), mp = make_float2(-me.x, -me.y);
+    const bool capped = *A.occ_in > (unsigned)cx.max_bucket;
+    const int n = cx.n;
+    float2 acc = make_float2(0.0f, 0.0f);
+    bool rare = false;
+    auto visit = [&](int, const float4 &q) { relax_pair_walk(wc, p, q, acc, rare); };
+    const unsigned key = cell_key(p.x, p.y, g);
+    if (searchable(key, i, A.start, g, capped, cx.max_bucket)) {
+        if (!capped) {
+            int ra[3], rl[3];
+            stencil_rows(p, key, A.start, g, ra, rl, n);
+#pragma unroll 1
+            for (int r = 0; r < 3; ++r) {
+                const int a = ra[r], l = rl[r];
+                if (MARK) {
+#pragma unroll 1
+                    for (int c0 = 0; c0 < l; c0 += 32) {
+                        const int m = min(l - c0, 32);
+                        unsigned b = 0u;
+#pragma unroll 4
+                        for (int t = 0; t < m; ++t) {
+                            const float4 q = __ldg(xr + a + c0 + t);
+                            float2 e;
+                            if (dist2_packed(mp, make_float2(q.x, q.y), e) <= c.h2) b |= 1u << t;
+                        }
+                        if (r == 1 && (unsigned)(i - a - c0) < 32u) b &= ~(1u << (i - a - c0));
+                        walk_mask32<float4>(b, a + c0, n, [&](int j) { return __ldg(xr + j); }, visit);
+                    }
+                } else {
+#pragma unroll 4
+                    for (int j = a; j < a + l; ++j) {
+                        const float4 q = __ldg(xr + j);
+                        float2 e;
+                        if (dist2_packed(mp, make_float2(q.x, q.y), e) <= c.h2 && j != i) visit(j, q);
+                    }
+                }
+            }
+        } else {
+            for_each_candidate(key, A.start, g, true, cx.max_bucket, n, [&](int j) {
+                if (j == i) return;
+                const float4 q = __ldg(xr + j);
+                if (dist2(p.x - q.x, p.y - q.y) > c.h2) return;
+                visit(j, q);
+            });
+        }
+    }
+    if (rare)
+        relax_nudged<PROBE>(i, A, acc);
+    else
+        relax_end_cold<PROBE>(i, A, S, p, acc, 0);
+}
+
+// MARK: as in relax_cold.
+template <bool PROBE, bool LEARNED = false, bool LM = false, bool MARK = false>
+__device__ __forceinline__ void relax_update_one(int i, const RelaxArrays &A,
+                                                 const LearnedIn &L = LearnedIn(),
+                                                 bool *used_net = nullptr, int *tile_made = nullptr)
+{
+    const Ctx &cx = A.c;
+    const Scene *S = cx.scenes + scene_of(cx, i);
+    const float4 *xr = A.xr;
     const float4 me = xr[i];
     // the plain pass requests the hit masks with the record and prefetches
     // the previous position, so that their DRAM latencies overlap instead of
@@ -1165,19 +1211,19 @@ __device__ __forceinline__ void relax_update_one(
     ulonglong2 m01 = make_ulonglong2(0ull, 0ull);
     unsigned long long m2 = 0ull;
     if (kHoist) {
-        m01 = __ldg(mask01 + i);
-        m2 = __ldg(mask2 + i);
-        if (!PROBE) asm volatile("prefetch.global.L1 [%0];" ::"l"(prev + i));
+        m01 = __ldg(A.mask01 + i);
+        m2 = __ldg(A.mask2 + i);
+        if (!PROBE) asm volatile("prefetch.global.L1 [%0];" ::"l"(A.prev + i));
     }
     const float2 p = make_float2(me.x, me.y);
     float2 acc = make_float2(0.0f, 0.0f);  // the displacement
-    bool rare = false, net = false;
+    bool net = false;
     if (LEARNED) {
         // the network's output requested with the count (not after it), and
         // the previous position prefetched for relax_finish: one DRAM latency
         // for a network particle instead of three in a row
         const float4 y = __ldg(L.net + i);
-        if (!PROBE) asm volatile("prefetch.global.L1 [%0];" ::"l"(prev + i));
+        if (!PROBE) asm volatile("prefetch.global.L1 [%0];" ::"l"(A.prev + i));
         if ((int)__ldg(L.nbc + i) <= L.max_nb && y.z <= L.thr_pct) {
             const RelaxConsts c = relax_consts(S);
             const float s = c.hh * c.dt2 * (c.k + c.k_near + 2.0f * c.half_spring);
@@ -1190,13 +1236,14 @@ __device__ __forceinline__ void relax_update_one(
     if (!net) {
         // the density pass's row record: the stencil rows' first slots, so
         // the walk needs neither the cell key nor the cell starts
-        const int4 rw = __ldg(rows + i);
+        const int4 rw = __ldg(A.rows + i);
         const int ra[3] = {rw.x, rw.y, rw.z};
+        bool rare = false;
         if (rw.w == kRowsMasked || (LM && rw.w == kRowsMasked2)) {
             const WalkConsts wc = walk_consts(relax_consts(S), me);
             if (!kHoist) {
-                m01 = __ldg(mask01 + i);
-                m2 = __ldg(mask2 + i);
+                m01 = __ldg(A.mask01 + i);
+                m2 = __ldg(A.mask2 + i);
             }
             const unsigned long long mm[3] = {m01.x, m01.y, m2};
             auto load = [&](int j) { return __ldg(xr + j); };
@@ -1214,51 +1261,38 @@ __device__ __forceinline__ void relax_update_one(
                     walk_mask<float4>(mh[r], ra[r] + kMaskRow, cx.n, load, visit);
                 }
             }
-        } else if (rw.w != kRowsNone) {
-            const ColdSum r = relax_unmasked(i, S, xr, start, capped, cx.max_bucket, cx.n);
-            acc = make_float2(r.x, r.y);
-            rare = r.rare != 0;
+        } else {
+            relax_cold<PROBE, MARK>(i, A);
+            return;
+        }
+        if (rare) {
+            relax_nudged<PROBE>(i, A, acc);
+            return;
         }
     }
-    const int nudges = rare ? count_nudges(i, S, xr, ids, start, capped, cx.max_bucket, cx.n) : 0;
     if (PROBE) {
-        const float nd = (float)nudges * 0.000001f;
-        probe_out[i] = make_float2(acc.x + nd, acc.y + nd);
+        A.probe_out[i] = acc;
         return;
     }
-    relax_finish(i, cx, S, p, acc, nudges, prev, pos_out, vel_out, kr_out, cnt, tile_made);
+    relax_finish(i, A, S, p, acc, 0, tile_made);
 }
 
-// 48 registers: 40 resident warps per SM instead of 32 (64 registers) for
+// 40 registers: 48 resident warps per SM instead of 32 (64 registers) for
 // this latency-bound pass; what the rare paths would need is out of line
-// (4,194,304 particles: 178 -> 160 us early in the dam break, 227 -> 209 us
-// compressed).
+// (4,194,304 particles: 64 registers 178 us early in the dam break and 227 us
+// compressed, 48 with the long rows' sum alone out of line 152 and 199, this
+// 138 and 172).
 template <bool PROBE, bool PERSIST = false, bool LM = false>
-__global__ void __maxnreg__(48)
-k_relax_update(Ctx c, const float4 *__restrict__ xr, const ulonglong2 *__restrict__ mask01,
-               const unsigned long long *__restrict__ mask2, const int4 *__restrict__ rows,
-               const float2 *__restrict__ prev,
-               const int *__restrict__ ids, const int *__restrict__ start,
-               const unsigned *__restrict__ occ_in, unsigned *occ_reset,
-               float2 *__restrict__ pos_out, float2 *__restrict__ vel_out,
-               uint2 *__restrict__ kr_out, unsigned *__restrict__ cnt,
-               float2 *__restrict__ probe_out)
+__global__ void __maxnreg__(40)
+k_relax_update(const __grid_constant__ RelaxArrays A, unsigned *occ_reset)
 {
     pdl_enter();
     const int i0 = blockIdx.x * blockDim.x + threadIdx.x;
     if (!PROBE && i0 == 0) *occ_reset = 0u;
-    const bool capped = *occ_in > (unsigned)c.max_bucket;
-    if (!PERSIST) {
-        if (i0 < c.n)
-            relax_update_one<PROBE, false, LM>(i0, c, xr, mask01, mask2, rows, prev, ids,
-                                                      start, capped, pos_out, vel_out, kr_out,
-                                                      cnt, probe_out);
-        return;
+    for (int i = i0; i < A.c.n; i += gridDim.x * blockDim.x) {
+        relax_update_one<PROBE, false, LM>(i, A);
+        if (!PERSIST) break;
     }
-    for (int i = i0; i < c.n; i += gridDim.x * blockDim.x)
-        relax_update_one<PROBE, false, LM>(i, c, xr, mask01, mask2, rows, prev, ids, start,
-                                                  capped, pos_out, vel_out, kr_out, cnt,
-                                                  probe_out);
 }
 
 // The relaxation pass of a learned step (one particle per thread).  PROBE:
@@ -1268,33 +1302,24 @@ k_relax_update(Ctx c, const float4 *__restrict__ xr, const ulonglong2 *__restric
 // the rare plain gathers do not hold up whole warps.  Block 0 counts the step.
 template <bool PROBE, bool LM = false>
 __global__ void __launch_bounds__(kBlock, 4)
-k_relax_learned(Ctx c, const float4 *__restrict__ xr, const ulonglong2 *__restrict__ mask01,
-                const unsigned long long *__restrict__ mask2, const int4 *__restrict__ rows,
-                const float2 *__restrict__ prev,
-                const int *__restrict__ ids, const int *__restrict__ start,
-                const unsigned *__restrict__ occ_in, unsigned *occ_reset,
-                float2 *__restrict__ pos_out, float2 *__restrict__ vel_out,
-                uint2 *__restrict__ kr_out, unsigned *__restrict__ cnt,
-                float2 *__restrict__ probe_out, LearnedIn L, DevState *st, int *__restrict__ fb_list)
+k_relax_learned(const __grid_constant__ RelaxArrays A, unsigned *occ_reset, LearnedIn L,
+                DevState *st, int *__restrict__ fb_list)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (!PROBE && i == 0) {
         *occ_reset = 0u;
         atomicAdd(&st->learned_steps, 1ull);
     }
-    const bool capped = *occ_in > (unsigned)c.max_bucket;
     bool used = true;
     L.defer = !PROBE;
     int t = -1;
-    if (i < c.n)
-        relax_update_one<PROBE, true, LM>(i, c, xr, mask01, mask2, rows, prev, ids, start, capped, pos_out,
-                                      vel_out, kr_out, cnt, probe_out, L, &used, &t);
+    if (i < A.c.n) relax_update_one<PROBE, true, LM>(i, A, L, &used, &t);
     if (PROBE) return;
-    if (c.tile_cnt) cta_tile_count(c.tile_cnt, t);
+    if (A.c.tile_cnt) cta_tile_count(A.c.tile_cnt, t);
     // fallback particles: those whose stencil rows fit the hit masks go to
     // the front of fb_list (one thread each in k_relax_fallback), those with
     // a row too long for a mask to the back (one warp each)
-    const bool longrow = !used && __ldg(rows + i).w == kRowsFull;
+    const bool longrow = !used && __ldg(A.rows + i).w == kRowsFull;
     const unsigned lane = threadIdx.x & 31u;
     const unsigned fbs = __ballot_sync(0xffffffffu, !used && !longrow);
     const unsigned fbl = __ballot_sync(0xffffffffu, longrow);
@@ -1310,7 +1335,7 @@ k_relax_learned(Ctx c, const float4 *__restrict__ xr, const ulonglong2 *__restri
         unsigned base = 0;
         if (lane == (unsigned)leader) base = atomicAdd(&st->fb_long, (unsigned)__popc(fbl));
         base = __shfl_sync(0xffffffffu, base, leader);
-        if (longrow) fb_list[c.n - 1 - (int)(base + __popc(fbl & ((1u << lane) - 1u)))] = i;
+        if (longrow) fb_list[A.c.n - 1 - (int)(base + __popc(fbl & ((1u << lane) - 1u)))] = i;
     }
 }
 
@@ -1418,7 +1443,7 @@ __device__ __forceinline__ void viscosity_group_one(
                 const float r_recip = rsqrtf(r2);
                 const float rr = r2 * r_recip;
                 const float2 dw = __fadd2_rn(v0, make_float2(-w.x, -w.y));
-                const float u = (dw.x * e.x + dw.y * e.y) * r_recip;
+                const float u = __fmaf_rn(dw.x, e.x, __fmul_rn(dw.y, e.y)) * r_recip;
                 push = u > 0.0f;
                 const float imp = fmaf(-dt_h, rr, dt) * u * fmaf(beta, u, sigma);
                 const float2 m = __fmul2_rn(__fmul2_rn(make_float2(imp, imp), e),
@@ -1552,19 +1577,17 @@ k_density_group(Ctx c, const float2 *__restrict__ pos, const int *__restrict__ s
 }
 
 template <int G, bool LM>
-__device__ __forceinline__ void relax_group_one(
-    const Group<G> &g, int i, bool valid, const Ctx &c, const float4 *__restrict__ xr,
-    const ulonglong2 *__restrict__ mask01, const unsigned long long *__restrict__ mask2,
-    const int4 *__restrict__ rows, const float2 *__restrict__ prev, const int *__restrict__ ids,
-    const int *__restrict__ start, float2 *__restrict__ pos_out, float2 *__restrict__ vel_out,
-    uint2 *__restrict__ kr_out, unsigned *__restrict__ cnt)
+__device__ __forceinline__ void relax_group_one(const Group<G> &g, int i, bool valid,
+                                                const RelaxArrays &A)
 {
+    const Ctx &c = A.c;
+    const float4 *xr = A.xr;
     // the particle's record, masks and rows, requested together
     const float4 me = __ldg(xr + i);
-    const int4 rw = __ldg(rows + i);
-    const ulonglong2 m01 = __ldg(mask01 + i);
-    const unsigned long long m2 = __ldg(mask2 + i);
-    asm volatile("prefetch.global.L1 [%0];" ::"l"(prev + i));
+    const int4 rw = __ldg(A.rows + i);
+    const ulonglong2 m01 = __ldg(A.mask01 + i);
+    const unsigned long long m2 = __ldg(A.mask2 + i);
+    asm volatile("prefetch.global.L1 [%0];" ::"l"(A.prev + i));
     const Scene *S = c.scenes + scene_of(c, i);
     const RelaxConsts rc = relax_consts(S);
     const float2 p = make_float2(me.x, me.y);
@@ -1588,8 +1611,8 @@ __device__ __forceinline__ void relax_group_one(
         const SG sg = load_grid(S);
         const unsigned key = cell_key(p.x, p.y, sg);
         ra[0] = ra[1] = ra[2] = 0;
-        if (searchable(key, i, start, sg, false, c.max_bucket))
-            stencil_rows(p, key, start, sg, ra, rl, c.n);
+        if (searchable(key, i, A.start, sg, false, c.max_bucket))
+            stencil_rows(p, key, A.start, sg, ra, rl, c.n);
     }
     const bool masked = mode != kRowsFull;
     auto wanted = [&](int r, int t) {
@@ -1620,7 +1643,7 @@ __device__ __forceinline__ void relax_group_one(
                 if (dist2_packed(mp, make_float2(q.x, q.y), e) <= rc.h2) {
                     bool rare = false;
                     apply = relax_pair_term(wc, p, q, s, d, rare);
-                    if (rare && is_nudge(i, j, S, xr, ids)) ++nudges;
+                    if (rare && is_nudge(i, j, S, xr, A.ids)) ++nudges;
                 }
             }
             g.ordered(g.ballot(apply), [&](int src, bool on) {
@@ -1634,33 +1657,24 @@ __device__ __forceinline__ void relax_group_one(
 #pragma unroll
     for (int o = G / 2; o > 0; o >>= 1) nudges += __shfl_xor_sync(Group<G>::kFull, nudges, o);
     if (valid && g.gl == 0)
-        relax_finish(i, c, S, p, acc, nudges, prev, pos_out, vel_out, kr_out, cnt, nullptr);
+        relax_finish(i, A, S, p, acc, nudges, nullptr);
 }
 
 template <int G, bool LM>
 __global__ void __launch_bounds__(kBlock)
-k_relax_group(Ctx c, const float4 *__restrict__ xr, const ulonglong2 *__restrict__ mask01,
-              const unsigned long long *__restrict__ mask2, const int4 *__restrict__ rows,
-              const float2 *__restrict__ prev, const int *__restrict__ ids,
-              const int *__restrict__ start, const unsigned *__restrict__ occ_in,
-              unsigned *occ_reset, float2 *__restrict__ pos_out, float2 *__restrict__ vel_out,
-              uint2 *__restrict__ kr_out, unsigned *__restrict__ cnt)
+k_relax_group(const __grid_constant__ RelaxArrays A, unsigned *occ_reset)
 {
     pdl_enter();
     const int th = blockIdx.x * blockDim.x + threadIdx.x;
     if (th == 0) *occ_reset = 0u;
-    const bool capped = *occ_in > (unsigned)c.max_bucket;
     const Group<G> g;
-    const bool valid = th / G < c.n;
-    const int i = valid ? th / G : c.n - 1;
-    if (capped) {
-        if (valid && g.gl == 0)
-            relax_update_one<false>(i, c, xr, mask01, mask2, rows, prev, ids, start, true, pos_out,
-                                    vel_out, kr_out, cnt, nullptr);
+    const bool valid = th / G < A.c.n;
+    const int i = valid ? th / G : A.c.n - 1;
+    if (*A.occ_in > (unsigned)A.c.max_bucket) {
+        if (valid && g.gl == 0) relax_update_one<false>(i, A);
         return;
     }
-    relax_group_one<G, LM>(g, i, valid, c, xr, mask01, mask2, rows, prev, ids, start, pos_out,
-                           vel_out, kr_out, cnt);
+    relax_group_one<G, LM>(g, i, valid, A);
 }
 
 // The fallback particles of a learned step: the plain relaxation + update for
@@ -1674,37 +1688,29 @@ k_relax_group(Ctx c, const float4 *__restrict__ xr, const ulonglong2 *__restrict
 // known on the device only.  Block 0 adds them to the fallback statistics.
 template <bool LM>
 __global__ void __launch_bounds__(kBlock, kFallbackCtas)
-k_relax_fallback(Ctx c, const float4 *__restrict__ xr, const ulonglong2 *__restrict__ mask01,
-                 const unsigned long long *__restrict__ mask2, const int4 *__restrict__ rows,
-                 const float2 *__restrict__ prev,
-                 const int *__restrict__ ids, const int *__restrict__ start,
-                 const unsigned *__restrict__ occ_in, float2 *__restrict__ pos_out,
-                 float2 *__restrict__ vel_out, uint2 *__restrict__ kr_out,
-                 unsigned *__restrict__ cnt, DevState *st, const int *__restrict__ fb_list)
+k_relax_fallback(const __grid_constant__ RelaxArrays A, DevState *st,
+                 const int *__restrict__ fb_list)
 {
     const unsigned front = st->fb_count, total = front + st->fb_long;
     if (blockIdx.x == 0 && threadIdx.x == 0)
         atomicAdd(&st->learned_fallback, (unsigned long long)total);
-    const bool capped = *occ_in > (unsigned)c.max_bucket;
+    const bool capped = *A.occ_in > (unsigned)A.c.max_bucket;
     const unsigned t0 = blockIdx.x * blockDim.x + threadIdx.x;
     const unsigned nt = gridDim.x * blockDim.x, resident = nt / kFallbackWaves;
-    auto slot_of = [&](unsigned k) { return fb_list[k < front ? (int)k : c.n - 1 - (int)(k - front)]; };
+    auto slot_of = [&](unsigned k) { return fb_list[k < front ? (int)k : A.c.n - 1 - (int)(k - front)]; };
     auto by_groups = [&](auto G) {
         const Group<G.value> g;
         const unsigned k = t0 / G.value, k0 = (t0 & ~31u) / G.value;
         if (k0 >= total) return;  // the whole warp
         const bool valid = k < total;
-        relax_group_one<G.value, LM>(g, slot_of(valid ? k : k0), valid, c, xr, mask01, mask2, rows, prev,
-                                     ids, start, pos_out, vel_out, kr_out, cnt);
+        relax_group_one<G.value, LM>(g, slot_of(valid ? k : k0), valid, A);
     };
     if (!capped && total <= resident / 32) {
         by_groups(std::integral_constant<int, 32>());
     } else if (!capped && total <= resident / 4) {
         by_groups(std::integral_constant<int, 4>());
     } else {
-        for (unsigned k = t0; k < total; k += nt)
-            relax_update_one<false, false, LM>(slot_of(k), c, xr, mask01, mask2, rows, prev, ids, start,
-                                               capped, pos_out, vel_out, kr_out, cnt, nullptr);
+        for (unsigned k = t0; k < total; k += nt) relax_update_one<false, false, LM, true>(slot_of(k), A);
     }
 }
 
@@ -2111,6 +2117,14 @@ int enqueue_predicted_state(sph_cuda *h)
     return cuda_fail(cudaGetLastError(), "predicted state");
 }
 
+// The relaxation of a step: the C order's density records to the B arrays.
+static RelaxArrays relax_arrays(const sph_cuda *h, float2 *probe_out = nullptr)
+{
+    return RelaxArrays{make_ctx(h), h->xr_c, h->mask01_c, h->mask2_c, h->rows_c, h->prev_c,
+                       h->id_c, h->start_c, &h->d_state->build_max_occ[SLOT_PREDICTED], h->pos_b,
+                       h->vel_b, h->kr_b, h->cnt, probe_out};
+}
+
 // The relaxation passes of a learned step (network particles, then the
 // fallback list); with probe_out, one pass writes every particle's
 // displacement (C order) instead of advancing.  `events` (two) are recorded
@@ -2126,25 +2140,19 @@ int launch_learned_relax(sph_cuda *h, float2 *probe_out, cudaEvent_t *events)
     // a negative threshold sends every particle to the plain relaxation
     L.max_nb = h->learned_thr < 0.0f ? -1 : SPH_LEARNED_MAX_NEIGHBORS;
     const int nb = blocks_for(h->n);
-    const unsigned *occ = &st->build_max_occ[SLOT_PREDICTED];
     const bool lm = h->long_masks;
+    const RelaxArrays arrays = relax_arrays(h, probe_out);
     if (probe_out) {
-        (lm ? k_relax_learned<true, true> : k_relax_learned<true, false>)<<<nb, kBlock, 0,
-                                                                          h->stream>>>(
-            c, h->xr_c, h->mask01_c, h->mask2_c, h->rows_c, h->prev_c, h->id_c, h->start_c, occ,
-            nullptr, nullptr, nullptr, nullptr, nullptr, probe_out, L, st, nullptr);
+        (lm ? k_relax_learned<true, true>
+            : k_relax_learned<true, false>)<<<nb, kBlock, 0, h->stream>>>(arrays, nullptr, L, st, nullptr);
         return cuda_fail(cudaGetLastError(), "learned relaxation probe");
     }
-    (lm ? k_relax_learned<false, true> : k_relax_learned<false, false>)<<<nb, kBlock, 0,
-                                                                        h->stream>>>(
-        c, h->xr_c, h->mask01_c, h->mask2_c, h->rows_c, h->prev_c, h->id_c, h->start_c, occ,
-        &st->build_max_occ[SLOT_RELAXED], h->pos_b, h->vel_b, h->kr_b, h->cnt, nullptr, L, st,
-        h->fb_list);
+    (lm ? k_relax_learned<false, true> : k_relax_learned<false, false>)<<<nb, kBlock, 0, h->stream>>>(
+        arrays, &st->build_max_occ[SLOT_RELAXED], L, st, h->fb_list);
     if (events) cudaEventRecord(events[0], h->stream);
     const int fb_blocks = kFallbackWaves * kFallbackCtas * h->num_sms;
     (lm ? k_relax_fallback<true> : k_relax_fallback<false>)<<<fb_blocks, kBlock, 0, h->stream>>>(
-        c, h->xr_c, h->mask01_c, h->mask2_c, h->rows_c, h->prev_c, h->id_c, h->start_c, occ,
-        h->pos_b, h->vel_b, h->kr_b, h->cnt, st, h->fb_list);
+        arrays, st, h->fb_list);
     if (events) cudaEventRecord(events[1], h->stream);
     return cuda_fail(cudaGetLastError(), "learned relaxation");
 }
@@ -2187,13 +2195,8 @@ int enqueue_step(sph_cuda *h, cudaEvent_t *events, int *nkernels, const tunable_
         if (lanes > 1) {
             with_lanes(lanes, [&](auto G) {
                 launch_step(h->long_masks ? k_relax_group<G.value, true> : k_relax_group<G.value, false>,
-                            blocks_for(n * G.value), kBlock, 0, h->stream, c,
-                            (const float4 *)h->xr_c, (const ulonglong2 *)h->mask01_c,
-                            (const unsigned long long *)h->mask2_c, (const int4 *)h->rows_c,
-                            (const float2 *)h->prev_c, (const int *)h->id_c,
-                            (const int *)h->start_c,
-                            (const unsigned *)&st->build_max_occ[SLOT_PREDICTED],
-                            &st->build_max_occ[SLOT_RELAXED], h->pos_b, h->vel_b, h->kr_b, h->cnt);
+                            blocks_for(n * G.value), kBlock, 0, h->stream, relax_arrays(h),
+                            &st->build_max_occ[SLOT_RELAXED]);
             });
         } else {
             auto kr = h->shape[2].persistent
@@ -2201,14 +2204,8 @@ int enqueue_step(sph_cuda *h, cudaEvent_t *events, int *nkernels, const tunable_
                                            : k_relax_update<false, true, false>)
                           : (h->long_masks ? k_relax_update<false, false, true>
                                            : k_relax_update<false, false, false>);
-            const size_t smem = 0;
-            launch_step(kr, gather_grid(h, h->shape[2]), h->shape[2].block, smem, h->stream, c,
-                        (const float4 *)h->xr_c, (const ulonglong2 *)h->mask01_c,
-                        (const unsigned long long *)h->mask2_c, (const int4 *)h->rows_c,
-                        (const float2 *)h->prev_c, (const int *)h->id_c, (const int *)h->start_c,
-                        (const unsigned *)&st->build_max_occ[SLOT_PREDICTED],
-                        &st->build_max_occ[SLOT_RELAXED], h->pos_b, h->vel_b, h->kr_b, h->cnt,
-                        (float2 *)nullptr);
+            launch_step(kr, gather_grid(h, h->shape[2]), h->shape[2].block, 0, h->stream, relax_arrays(h),
+                        &st->build_max_occ[SLOT_RELAXED]);
         }
         mark();
     }
@@ -2403,8 +2400,9 @@ int launch_probe(sph_cuda *h, int which, void *scratch, float2 *out)
         k_density<<<nb, kBlock, 0, h->stream>>>(c, h->pos_a, h->start_a, occ, xr, m01, m2, rw);
         if (which == 1)
             k_relax_update<true><<<nb, kBlock, 0, h->stream>>>(
-                c, xr, m01, m2, rw, nullptr, h->id_a, h->start_a, occ, nullptr, nullptr, nullptr,
-                nullptr, nullptr, sorted);
+                RelaxArrays{c, xr, m01, m2, rw, nullptr, h->id_a, h->start_a, occ, nullptr, nullptr,
+                            nullptr, nullptr, sorted},
+                nullptr);
         else
             k_xr_density<<<nb, kBlock, 0, h->stream>>>(n, xr, sorted);
     } else {
