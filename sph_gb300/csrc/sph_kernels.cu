@@ -32,7 +32,7 @@
 namespace sph {
 // Particles whose stencil rows have up to kShortRow candidates have their hits
 // marked first and then walked, the others are gathered in one loop over the
-// candidates (density_filter and viscosity_long_rows say why; with the line at 20 to 28
+// candidates (density_filter and viscosity_cold say why; with the line at 20 to 28
 // the dam break's 1,048,576 particles lost 2-8% of the viscosity pass and the
 // other states stayed within 1%).
 constexpr int kShortRow = 32;
@@ -519,16 +519,30 @@ k_permute_x(int n, const uint2 *__restrict__ kr, const int *__restrict__ start,
 // pass 1: gravity + viscosity (gather) + predict + boundary + cell key
 // ---------------------------------------------------------------------------
 
+// What the viscosity pass reads and writes.
+struct ViscArrays {
+    Ctx c;
+    const DevState *st;
+    const float2 *pos, *vel;
+    const int *start;
+    const unsigned *occ_in;  // the build's largest cell population
+    float2 *pos_out, *prev_out;
+    uint2 *kr_out;
+    unsigned *cnt;
+    float2 *probe_out;
+};
+
 // The end of a particle's viscosity pass: gravity and the impulses' sum dv on
 // its velocity v0, predict_positions with boundaryConditions, and the
 // predicted position's cell key counted into its build.
-__device__ __forceinline__ void viscosity_finish(int i, const Ctx &c, const Scene *S, const SG &g,
-                                                 float2 p, float2 v0, float2 dv,
-                                                 float2 *__restrict__ pos_out,
-                                                 float2 *__restrict__ prev_out,
-                                                 uint2 *__restrict__ kr_out,
-                                                 unsigned *__restrict__ cnt, int *tile_made)
+template <bool PROBE>
+__device__ __forceinline__ void viscosity_finish(int i, const ViscArrays &A, const Scene *S,
+                                                 const SG &g, float2 p, float2 v0, float2 dv)
 {
+    if (PROBE) {
+        A.probe_out[i] = dv;
+        return;
+    }
     const float dt = __ldg(&S->P.time_step);
     const float gdt = __fmul_rn(-__ldg(&S->P.g), dt);
     const float vx = __fadd_rn(v0.x, dv.x);
@@ -538,16 +552,13 @@ __device__ __forceinline__ void viscosity_finish(int i, const Ctx &c, const Scen
     boundary_of(nx, ny, S);
     const unsigned k2 = cell_key(nx, ny, g);
     unsigned rank = 0u;
-    if (in_bounds(k2, c.M, kBadKey)) {
-        rank = atomicAdd(cnt + k2, 1u);
-        if (tile_made)
-            *tile_made = (int)(k2 / (unsigned)kBuildTile);
-        else
-            add_tile_count(c.tile_cnt, k2);
+    if (in_bounds(k2, A.c.M, kBadKey)) {
+        rank = atomicAdd(A.cnt + k2, 1u);
+        add_tile_count(A.c.tile_cnt, k2);
     }
-    pos_out[i] = make_float2(nx, ny);
-    prev_out[i] = p;
-    kr_out[i] = make_uint2(k2, rank);
+    A.pos_out[i] = make_float2(nx, ny);
+    A.prev_out[i] = p;
+    A.kr_out[i] = make_uint2(k2, rank);
 }
 
 // The scene constants of a pair's viscosity impulse, and the impulse itself.
@@ -602,14 +613,15 @@ __device__ __forceinline__ void visc_impulse(const ViscConsts &c, float2 e, floa
 // the lanes of a warp are then mostly of one cell and read the same candidate
 // at a time, which a walk over each lane's own hits does not (the dam break's
 // 1,048,576 particles, compressed: all rows marked and walked 218 us, this 187
-// us; 64 compressed scenes 231 and 217 us).  Out of line: compiled into the
-// pass it cost the short rows' walk its registers.
-__device__ __noinline__ float2 viscosity_long_rows(int i, const Scene *S,
-                                                   const float2 *__restrict__ pos,
-                                                   const float2 *__restrict__ vel,
-                                                   const int *__restrict__ start, bool capped,
-                                                   int max_bucket, int n)
+// us; 64 compressed scenes 231 and 217 us).  Out of line and to the end of
+// the particle's pass: nothing of the short rows' walk lives across the call.
+template <bool PROBE>
+__device__ __noinline__ void viscosity_cold(int i, const ViscArrays &A)
 {
+    const Scene *S = A.c.scenes + scene_of(A.c, i);
+    const float2 *pos = A.pos, *vel = A.vel;
+    const bool capped = *A.occ_in > (unsigned)A.c.max_bucket;
+    const int n = A.c.n;
     const SG g = load_grid(S);
     const ViscConsts vc = visc_consts(S);
     const float2 p = __ldg(pos + i), v0 = __ldg(vel + i);
@@ -617,13 +629,14 @@ __device__ __noinline__ float2 viscosity_long_rows(int i, const Scene *S,
     const unsigned key = cell_key(p.x, p.y, g);
     float2 dv = make_float2(0.0f, 0.0f);
     if (capped) {
-        for_each_candidate(key, start, g, true, max_bucket, n, [&](int j) {
+        for_each_candidate(key, A.start, g, true, A.c.max_bucket, n, [&](int j) {
             const float2 q = __ldg(pos + j);
             float2 e;
             const float r2 = dist2_packed(mp, q, e);
             if (!(r2 > vc.h2)) visc_impulse(vc, e, r2, v0, __ldg(vel + j), dv);
         });
-        return dv;
+        viscosity_finish<PROBE>(i, A, S, g, p, v0, dv);
+        return;
     }
     auto one = [&](int j) {
         const float2 q = __ldg(pos + j), w = __ldg(vel + j);
@@ -632,14 +645,14 @@ __device__ __noinline__ float2 viscosity_long_rows(int i, const Scene *S,
         if (r2 <= vc.h2) visc_impulse(vc, e, r2, v0, w, dv);
     };
     int ra[3], rl[3];
-    stencil_rows(p, key, start, g, ra, rl, n);
+    stencil_rows(p, key, A.start, g, ra, rl, n);
 #pragma unroll 1
     for (int r = 0; r < 3; ++r) {
         const int a = ra[r], l = rl[r];
 #pragma unroll kViscLongUnroll
         for (int j = a; j < a + l; ++j) one(j);
     }
-    return dv;
+    viscosity_finish<PROBE>(i, A, S, g, p, v0, dv);
 }
 
 // apply_gravity (fluid.c:398-413), viscosity_impluses (fluid.c:416-478) in
@@ -649,21 +662,19 @@ __device__ __noinline__ float2 viscosity_long_rows(int i, const Scene *S,
 // u = ((v_i - v_j).(x_j - x_i))/r, all from the velocities after gravity.
 // PROBE writes dv instead of advancing.
 template <bool PROBE>
-__device__ __forceinline__ void viscosity_predict_one(
-    int i, const Ctx &c, const DevState *__restrict__ st, const float2 *__restrict__ pos,
-    const float2 *__restrict__ vel, const int *__restrict__ start, bool capped,
-    float2 *__restrict__ pos_out, float2 *__restrict__ prev_out, uint2 *__restrict__ kr_out,
-    unsigned *__restrict__ cnt, float2 *__restrict__ probe_out, int *tile_made = nullptr)
+__device__ __forceinline__ void viscosity_predict_one(int i, const ViscArrays &A)
 {
-    const Scene *S = c.scenes + scene_of(c, i);
+    const Scene *S = A.c.scenes + scene_of(A.c, i);
     const SG g = load_grid(S);
+    const float2 *pos = A.pos, *vel = A.vel;
+    const bool capped = *A.occ_in > (unsigned)A.c.max_bucket;
     const float2 p = pos[i];
     const float2 v0 = vel[i];  // before gravity
     float2 dv = make_float2(0.0f, 0.0f);
     const unsigned key = cell_key(p.x, p.y, g);
-    if ((PROBE || st->lists_valid) && searchable(key, i, start, g, capped, c.max_bucket)) {
+    if ((PROBE || A.st->lists_valid) && searchable(key, i, A.start, g, capped, A.c.max_bucket)) {
         int ra[3] = {0, 0, 0}, rl[3] = {0, 0, 0};
-        if (!capped) stencil_rows(p, key, start, g, ra, rl, c.n);
+        if (!capped) stencil_rows(p, key, A.start, g, ra, rl, A.c.n);
         if (!capped && max(rl[0], max(rl[1], rl[2])) <= kShortRow) {
             // two phases: a cheap scan marks the neighbours of the stencil
             // rows, then only they pay for the impulse (less SIMT waste)
@@ -674,7 +685,7 @@ __device__ __forceinline__ void viscosity_predict_one(
                                 ~(1u << (i - ra[1]));  // not the particle itself
             const unsigned b2 = hit_mask32<kMarkUnroll>(pos + ra[2], rl[2], mp, vc.h2);
             walk_three<float4>(
-                b0, ra[0], b1, ra[1], b2, ra[2], c.n,
+                b0, ra[0], b1, ra[1], b2, ra[2], A.c.n,
                 [&](int j) {
                     const float2 q = __ldg(pos + j), w = __ldg(vel + j);
                     return make_float4(q.x, q.y, w.x, w.y);
@@ -685,40 +696,27 @@ __device__ __forceinline__ void viscosity_predict_one(
                     visc_impulse(vc, e, r2, v0, make_float2(d.z, d.w), dv);
                 });
         } else {
-            dv = viscosity_long_rows(i, S, pos, vel, start, capped, c.max_bucket, c.n);
+            viscosity_cold<PROBE>(i, A);
+            return;
         }
     }
-    if (PROBE) {
-        probe_out[i] = dv;
-        return;
-    }
-    viscosity_finish(i, c, S, g, p, v0, dv, pos_out, prev_out, kr_out, cnt, tile_made);
+    viscosity_finish<PROBE>(i, A, S, g, p, v0, dv);
 }
 
-// 48 registers: more resident warps than the compiler's free choice (55),
-// without spills.
+// 40 registers (48 resident warps per SM): 4,194,304 particles 189 -> 184 us
+// early in the dam break and 237 -> 230 us compressed against 48 registers,
+// 200 and 253 with 56.
 template <bool PROBE, bool PERSIST = false>
-__global__ void __maxnreg__(48)
-k_viscosity_predict(Ctx c, const DevState *__restrict__ st, const float2 *__restrict__ pos,
-                    const float2 *__restrict__ vel, const int *__restrict__ start,
-                    const unsigned *__restrict__ occ_in, unsigned *occ_reset,
-                    float2 *__restrict__ pos_out, float2 *__restrict__ prev_out,
-                    uint2 *__restrict__ kr_out, unsigned *__restrict__ cnt,
-                    float2 *__restrict__ probe_out)
+__global__ void __maxnreg__(40)
+k_viscosity_predict(const __grid_constant__ ViscArrays A, unsigned *occ_reset)
 {
     pdl_enter();
     const int i0 = blockIdx.x * blockDim.x + threadIdx.x;
     if (!PROBE && i0 == 0) *occ_reset = 0u;
-    const bool capped = *occ_in > (unsigned)c.max_bucket;
-    if (!PERSIST) {
-        if (i0 < c.n)
-            viscosity_predict_one<PROBE>(i0, c, st, pos, vel, start, capped, pos_out, prev_out,
-                                         kr_out, cnt, probe_out);
-        return;
+    for (int i = i0; i < A.c.n; i += gridDim.x * blockDim.x) {
+        viscosity_predict_one<PROBE>(i, A);
+        if (!PERSIST) break;
     }
-    for (int i = i0; i < c.n; i += gridDim.x * blockDim.x)
-        viscosity_predict_one<PROBE>(i, c, st, pos, vel, start, capped, pos_out, prev_out, kr_out,
-                                     cnt, probe_out);
 }
 
 // ---------------------------------------------------------------------------
@@ -1393,12 +1391,11 @@ struct Group {
 // Particle i's viscosity pass by the group (every lane of the warp calls it;
 // `valid` per group; no overflowing buckets).
 template <int G>
-__device__ __forceinline__ void viscosity_group_one(
-    const Group<G> &g, int i, bool valid, const Ctx &c, const DevState *__restrict__ st,
-    const float2 *__restrict__ pos, const float2 *__restrict__ vel, const int *__restrict__ start,
-    float2 *__restrict__ pos_out, float2 *__restrict__ prev_out, uint2 *__restrict__ kr_out,
-    unsigned *__restrict__ cnt)
+__device__ __forceinline__ void viscosity_group_one(const Group<G> &g, int i, bool valid,
+                                                    const ViscArrays &A)
 {
+    const Ctx &c = A.c;
+    const float2 *pos = A.pos, *vel = A.vel;
     const Scene *S = c.scenes + scene_of(c, i);
     const SG sg = load_grid(S);
     const float2 p = __ldg(pos + i), v0 = __ldg(vel + i);
@@ -1409,8 +1406,8 @@ __device__ __forceinline__ void viscosity_group_one(
     const float sigma = __ldg(&S->P.sigma), beta = __ldg(&S->P.beta);
     const unsigned key = cell_key(p.x, p.y, sg);
     int ra[3] = {0, 0, 0}, rl[3] = {0, 0, 0};
-    if (valid && st->lists_valid && searchable(key, i, start, sg, false, c.max_bucket))
-        stencil_rows(p, key, start, sg, ra, rl, c.n);
+    if (valid && A.st->lists_valid && searchable(key, i, A.start, sg, false, c.max_bucket))
+        stencil_rows(p, key, A.start, sg, ra, rl, c.n);
     const float2 mp = make_float2(-p.x, -p.y);
     float2 dv = make_float2(0.0f, 0.0f);
     // the rows' first candidates, requested together
@@ -1459,31 +1456,24 @@ __device__ __forceinline__ void viscosity_group_one(
         }
     }
     if (valid && g.gl == 0)
-        viscosity_finish(i, c, S, sg, p, v0, dv, pos_out, prev_out, kr_out, cnt, nullptr);
+        viscosity_finish<false>(i, A, S, sg, p, v0, dv);
 }
 
 template <int G>
 __global__ void __launch_bounds__(kBlock)
-k_viscosity_group(Ctx c, const DevState *__restrict__ st, const float2 *__restrict__ pos,
-                  const float2 *__restrict__ vel, const int *__restrict__ start,
-                  const unsigned *__restrict__ occ_in, unsigned *occ_reset,
-                  float2 *__restrict__ pos_out, float2 *__restrict__ prev_out,
-                  uint2 *__restrict__ kr_out, unsigned *__restrict__ cnt)
+k_viscosity_group(const __grid_constant__ ViscArrays A, unsigned *occ_reset)
 {
     pdl_enter();
     const int th = blockIdx.x * blockDim.x + threadIdx.x;
     if (th == 0) *occ_reset = 0u;
-    const bool capped = *occ_in > (unsigned)c.max_bucket;
     const Group<G> g;
-    const bool valid = th / G < c.n;
-    const int i = valid ? th / G : c.n - 1;
-    if (capped) {  // overflowing buckets (pathological): the one-thread form
-        if (valid && g.gl == 0)
-            viscosity_predict_one<false>(i, c, st, pos, vel, start, true, pos_out, prev_out, kr_out,
-                                         cnt, nullptr);
+    const bool valid = th / G < A.c.n;
+    const int i = valid ? th / G : A.c.n - 1;
+    if (*A.occ_in > (unsigned)A.c.max_bucket) {  // overflowing buckets: the one-thread form
+        if (valid && g.gl == 0) viscosity_predict_one<false>(i, A);
         return;
     }
-    viscosity_group_one<G>(g, i, valid, c, st, pos, vel, start, pos_out, prev_out, kr_out, cnt);
+    viscosity_group_one<G>(g, i, valid, A);
 }
 
 template <int G, bool LM, bool BY_ID = false>
@@ -2039,23 +2029,19 @@ static void enqueue_predict_sort(sph_cuda *h, Mark &mark)
     const int nb = blocks_for(n);
     const Ctx c = make_ctx(h);
     DevState *st = h->d_state;
+    const ViscArrays arrays{c, st, h->pos_a, h->vel_a, h->start_a, &st->build_max_occ[SLOT_RELAXED],
+                            h->pos_b, h->prev_b, h->kr_b, h->cnt, nullptr};
     const int lanes = gather_lanes(h, 0);
     if (lanes > 1) {
         with_lanes(lanes, [&](auto G) {
-            launch_step(k_viscosity_group<G.value>, blocks_for(n * G.value), kBlock, 0, h->stream, c,
-                        (const DevState *)st, (const float2 *)h->pos_a, (const float2 *)h->vel_a,
-                        (const int *)h->start_a,
-                        (const unsigned *)&st->build_max_occ[SLOT_RELAXED],
-                        &st->build_max_occ[SLOT_PREDICTED], h->pos_b, h->prev_b, h->kr_b, h->cnt);
+            launch_step(k_viscosity_group<G.value>, blocks_for(n * G.value), kBlock, 0, h->stream, arrays,
+                        &st->build_max_occ[SLOT_PREDICTED]);
         });
     } else {
         auto kv = h->shape[0].persistent ? k_viscosity_predict<false, true>
                                          : k_viscosity_predict<false, false>;
-        launch_step(kv, gather_grid(h, h->shape[0]), h->shape[0].block, 0, h->stream, c,
-                    (const DevState *)st, (const float2 *)h->pos_a, (const float2 *)h->vel_a,
-                    (const int *)h->start_a, (const unsigned *)&st->build_max_occ[SLOT_RELAXED],
-                    &st->build_max_occ[SLOT_PREDICTED], h->pos_b, h->prev_b, h->kr_b, h->cnt,
-                    (float2 *)nullptr);
+        launch_step(kv, gather_grid(h, h->shape[0]), h->shape[0].block, 0, h->stream, arrays,
+                    &st->build_max_occ[SLOT_PREDICTED]);
     }
     mark();
     enqueue_cell_starts(h, h->start_c, &st->build_max_occ[SLOT_PREDICTED]);
@@ -2407,8 +2393,8 @@ int launch_probe(sph_cuda *h, int which, void *scratch, float2 *out)
             k_xr_density<<<nb, kBlock, 0, h->stream>>>(n, xr, sorted);
     } else {
         k_viscosity_predict<true><<<nb, kBlock, 0, h->stream>>>(
-            c, st, h->pos_a, h->vel_a, h->start_a, occ, nullptr, nullptr, nullptr, nullptr,
-            nullptr, sorted);
+            ViscArrays{c, st, h->pos_a, h->vel_a, h->start_a, occ, nullptr, nullptr, nullptr, nullptr, sorted},
+            nullptr);
     }
     k_by_id<<<nb, kBlock, 0, h->stream>>>(n, h->id_a, sorted, out);
     return cuda_fail(cudaGetLastError(), "probe");
