@@ -32,7 +32,7 @@
 namespace sph {
 // Particles whose stencil rows have up to kShortRow candidates have their hits
 // marked first and then walked, the others are gathered in one loop over the
-// candidates (density_filter and viscosity_cold say why; with the line at 20 to 28
+// candidates (density_one and viscosity_cold say why; with the line at 20 to 28
 // the dam break's 1,048,576 particles lost 2-8% of the viscosity pass and the
 // other states stayed within 1%).
 constexpr int kShortRow = 32;
@@ -729,75 +729,10 @@ k_viscosity_predict(const __grid_constant__ ViscArrays A, unsigned *occ_reset)
 // Writes xr = (x, y, rho, rho_near) and, per stencil row, the bit mask of the
 // candidates that are neighbours (r2 <= h2, self excluded), which the
 // relaxation pass of the same positions walks instead of the whole stencil.
-// The candidate filter of one particle over its three stencil rows (slots
-// [ra[r], ra[r] + rl[r])).  Rows of up to kShortRow candidates are marked
-// first and the marked ones walked: the terms are run for the hits alone,
-// where one loop over the candidates runs them for nearly every candidate of a
-// warp (some lane hits).  Particles with a longer row keep the one loop: there the lanes of a
-// warp are mostly of one cell and read the same candidate at a time, which a
-// walk over each lane's own hits does not.  4,194,304 particles: one loop for
-// every row 182 us early in the dam break and 201 us compressed, this 143 and
-// 176 us; two phases for rows of any length 162 and 197 us.
-// mx (long-row masks): where the hit bits of candidates kMaskRow..
-// 2 kMaskRow - 1 of each row go (3 words; null: nowhere).
-__device__ __forceinline__ void density_filter(int i, float2 mp, float h2, float h_recip,
-                                               const int (&ra)[3], const int (&rl)[3],
-                                               const float2 *__restrict__ pos, int n, float2 &ab,
-                                               unsigned long long (&m)[3],
-                                               unsigned long long *mx = nullptr)
-{
-    if (max(rl[0], max(rl[1], rl[2])) <= kShortRow) {
-        unsigned b0 = hit_mask32<kMarkUnroll>(pos + ra[0], rl[0], mp, h2);
-        unsigned b1 = hit_mask32<kMarkUnroll>(pos + ra[1], rl[1], mp, h2) &
-                      ~(1u << (i - ra[1]));  // not the particle itself
-        unsigned b2 = hit_mask32<kMarkUnroll>(pos + ra[2], rl[2], mp, h2);
-        m[0] = b0;
-        m[1] = b1;
-        m[2] = b2;
-        // walk_three without the record in flight, for which this pass has
-        // no registers
-        int a0 = ra[0], a1 = ra[1], a2 = ra[2];
-        if (!b1) { b1 = b2; a1 = a2; b2 = 0u; }
-        if (!b0) { b0 = b1; a0 = a1; b1 = b2; a1 = a2; b2 = 0u; }
-        while (b0) {
-            const int j = a0 + __ffs(b0) - 1;
-            b0 &= b0 - 1u;
-            if (!b0) { b0 = b1; a0 = a1; b1 = b2; a1 = a2; b2 = 0u; }
-            if (!in_bounds(j, n, kBadSlot)) continue;
-            float2 e;
-            add_density(ab, dist2_packed(mp, __ldg(pos + j), e), h_recip);
-        }
-        return;
-    }
-#pragma unroll
-    for (int r = 0; r < 3; ++r) {
-        const int len = rl[r];
-        unsigned long long w0 = 0ull, w1 = 0ull;
-        for (int c0 = 0; c0 < len; c0 += 32) {
-            const int a = ra[r] + c0, n = min(len - c0, 32);
-            const float2 *row = pos + a;
-            unsigned b = 0u;
-#pragma unroll kDensLongUnroll
-            for (int t = 0; t < n; ++t) {
-                float2 e;
-                const float r2 = dist2_packed(mp, __ldg(row + t), e);
-                if (r2 <= h2 && (r != 1 || a + t != i)) {
-                    b |= 1u << t;
-                    add_density(ab, r2, h_recip);
-                }
-            }
-            if (c0 < kMaskRow) w0 |= (unsigned long long)b << c0;
-            else if (c0 < 2 * kMaskRow) w1 |= (unsigned long long)b << (c0 - kMaskRow);
-        }
-        m[r] = w0;
-        if (mx != nullptr && len > kMaskRow) mx[r] = w1;
-    }
-}
-
 // Where a density pass by itself puts its results: by particle id.
 struct DensityById {
-    const int *ids;
-    float *rho, *rho_near;
+    const int *ids = nullptr;
+    float *rho = nullptr, *rho_near = nullptr;
     __device__ __forceinline__ void put(int i, float2 ab) const
     {
         const int id = __ldg(ids + i);
@@ -806,34 +741,66 @@ struct DensityById {
     }
 };
 
-// LM: long-row masks (rows of up to 2 kMaskRow candidates recorded as
-// kRowsMasked2, their second masks in c.maskx).  BY_ID: the densities alone,
-// to `by_id` (no record, masks or rows).
-template <bool LM = false, bool BY_ID = false>
-__device__ __forceinline__ void density_one(int i, const Ctx &c, const float2 *__restrict__ pos,
-                                            const int *__restrict__ start, bool capped,
-                                            float4 *__restrict__ xr_out,
-                                            ulonglong2 *__restrict__ mask01,
-                                            unsigned long long *__restrict__ mask2,
-                                            int4 *__restrict__ rows_out,
-                                            const DensityById &by_id = DensityById())
+// What a density pass reads and writes: the densities alone to by_id, or the
+// records, masks and rows.
+struct DensArrays {
+    Ctx c;
+    const float2 *pos;
+    const int *start;
+    const unsigned *occ_in;  // the build's largest cell population
+    float4 *xr_out;
+    ulonglong2 *mask01;
+    unsigned long long *mask2;
+    int4 *rows_out;
+    DensityById by_id;
+};
+
+template <bool BY_ID>
+__device__ __forceinline__ void density_finish(int i, const DensArrays &A, float2 p, float2 ab,
+                                               unsigned long long m0, unsigned long long m1,
+                                               unsigned long long m2, int4 rec)
 {
+    if (BY_ID) {
+        A.by_id.put(i, ab);
+        return;
+    }
+    A.xr_out[i] = make_float4(p.x, p.y, ab.x, ab.y);
+    A.mask01[i] = make_ulonglong2(m0, m1);
+    A.mask2[i] = m2;
+    A.rows_out[i] = rec;
+}
+
+// A particle with a stencil row of more than kShortRow candidates, or with an
+// overflowing bucket somewhere, in one loop over the candidates: the lanes of
+// a warp are then mostly of one cell and read the same candidate at a time,
+// which a walk over each lane's own hits does not.  The candidates come in
+// blocks without a remainder (as hit_mask32; four at a time 135 us early in the
+// dam break of 4,194,304 particles, with a remainder loop 141).  To the end of
+// the particle's pass, so that the short rows' walk shares no values with it;
+// out of line it was 5-10% slower in compressed states.
+// LM: long-row masks (rows of up to 2 kMaskRow candidates recorded as
+// kRowsMasked2, the hit bits of their candidates kMaskRow.. in c.maskx).
+template <bool LM, bool BY_ID>
+__device__ __forceinline__ void density_long_rows(int i, const DensArrays &A)
+{
+    const Ctx &c = A.c;
     const Scene *S = c.scenes + scene_of(c, i);
     const SG g = load_grid(S);
     const float hh = __ldg(&S->P.smoothing_radius);
     const float h2 = __fmul_rn(hh, hh);
     const float h_recip = __fdiv_rn(1.0f, hh);
-    const float2 p = pos[i];
-    const float2 mp = make_float2(-p.x, -p.y);
+    const float2 *pos = A.pos;
+    const float2 p = __ldg(pos + i), mp = make_float2(-p.x, -p.y);
     const unsigned key = cell_key(p.x, p.y, g);
+    const bool capped = *A.occ_in > (unsigned)c.max_bucket;
     float2 ab = make_float2(0.0f, 0.0f);  // (rho, rho_near)
     unsigned long long m[3] = {0ull, 0ull, 0ull};
     int4 rec = make_int4(0, 0, 0, kRowsNone);
-    if (searchable(key, i, start, g, capped, c.max_bucket)) {
+    if (searchable(key, i, A.start, g, capped, c.max_bucket)) {
         rec.w = kRowsFull;
         if (!capped) {
             int ra[3], rl[3];
-            stencil_rows(p, key, start, g, ra, rl, c.n);
+            stencil_rows(p, key, A.start, g, ra, rl, c.n);
             unsigned long long *mx = nullptr;
             if (rl[0] <= kMaskRow && rl[1] <= kMaskRow && rl[2] <= kMaskRow) {
                 rec = make_int4(ra[0], ra[1], ra[2], kRowsMasked);
@@ -843,9 +810,35 @@ __device__ __forceinline__ void density_one(int i, const Ctx &c, const float2 *_
                 mx = c.maskx + 3 * (size_t)i;
                 mx[0] = mx[1] = mx[2] = 0ull;  // rows of kMaskRow or fewer leave theirs
             }
-            density_filter(i, mp, h2, h_recip, ra, rl, pos, c.n, ab, m, LM ? mx : nullptr);
+#pragma unroll
+            for (int r = 0; r < 3; ++r) {
+                const int len = rl[r];
+                const float2 *row = pos + ra[r];
+                const int self = r == 1 ? i - ra[1] : -1;
+                unsigned long long w0 = 0ull, w1 = 0ull;
+#pragma unroll 1
+                for (int c0 = 0; c0 < len; c0 += kDensLongUnroll) {
+                    float2 q[kDensLongUnroll];
+#pragma unroll
+                    for (int k = 0; k < kDensLongUnroll; ++k) q[k] = __ldg(row + c0 + k);
+                    unsigned b = 0u;
+#pragma unroll
+                    for (int k = 0; k < kDensLongUnroll; ++k) {
+                        float2 e;
+                        const float r2 = dist2_packed(mp, q[k], e);
+                        if (r2 <= h2 && c0 + k < len && c0 + k != self) {
+                            b |= 1u << k;
+                            add_density(ab, r2, h_recip);
+                        }
+                    }
+                    if (c0 < kMaskRow) w0 |= (unsigned long long)b << c0;
+                    else if (c0 < 2 * kMaskRow) w1 |= (unsigned long long)b << (c0 - kMaskRow);
+                }
+                m[r] = w0;
+                if (LM && mx != nullptr && len > kMaskRow) mx[r] = w1;
+            }
         } else {
-            for_each_candidate(key, start, g, true, c.max_bucket, c.n, [&](int j) {
+            for_each_candidate(key, A.start, g, true, c.max_bucket, c.n, [&](int j) {
                 if (j == i) return;
                 const float2 q = __ldg(pos + j);
                 const float r2 = dist2(p.x - q.x, p.y - q.y);
@@ -854,47 +847,80 @@ __device__ __forceinline__ void density_one(int i, const Ctx &c, const float2 *_
             });
         }
     }
-    if (BY_ID) {
-        by_id.put(i, ab);
+    density_finish<BY_ID>(i, A, p, ab, m[0], m[1], m[2], rec);
+}
+
+// Particles whose rows have up to kShortRow candidates have their hits marked
+// first and the marked ones walked: the terms are run for the hits alone,
+// where one loop over the candidates runs them for nearly every candidate of a
+// warp (some lane hits).  4,194,304 particles: one loop for every row 182 us
+// early in the dam break and 201 us compressed, this 135 and 172 us; two
+// phases for rows of any length 162 and 197 us.
+template <bool LM = false, bool BY_ID = false>
+__device__ __forceinline__ void density_one(int i, const DensArrays &A)
+{
+    const Scene *S = A.c.scenes + scene_of(A.c, i);
+    const SG g = load_grid(S);
+    const float2 *pos = A.pos;
+    const float2 p = pos[i];
+    const unsigned key = cell_key(p.x, p.y, g);
+    const bool capped = *A.occ_in > (unsigned)A.c.max_bucket;
+    int ra[3] = {0, 0, 0}, rl[3] = {0, 0, 0};
+    int4 rec = make_int4(0, 0, 0, kRowsNone);
+    if (!capped && searchable(key, i, A.start, g, false, A.c.max_bucket)) {
+        stencil_rows(p, key, A.start, g, ra, rl, A.c.n);
+        rec = make_int4(ra[0], ra[1], ra[2], kRowsMasked);
+    }
+    if (capped || max(rl[0], max(rl[1], rl[2])) > kShortRow) {
+        density_long_rows<LM, BY_ID>(i, A);
         return;
     }
-    xr_out[i] = make_float4(p.x, p.y, ab.x, ab.y);
-    mask01[i] = make_ulonglong2(m[0], m[1]);
-    mask2[i] = m[2];
-    if (rows_out) rows_out[i] = rec;
+    const float hh = __ldg(&S->P.smoothing_radius);
+    const float h2 = __fmul_rn(hh, hh);
+    const float h_recip = __fdiv_rn(1.0f, hh);
+    const float2 mp = make_float2(-p.x, -p.y);
+    float2 ab = make_float2(0.0f, 0.0f);  // (rho, rho_near)
+    const unsigned m0 = hit_mask32<kMarkUnroll>(pos + ra[0], rl[0], mp, h2);
+    const unsigned m1 = hit_mask32<kMarkUnroll>(pos + ra[1], rl[1], mp, h2) &
+                        ~(1u << ((i - ra[1]) & 31));  // not the particle itself
+    const unsigned m2 = hit_mask32<kMarkUnroll>(pos + ra[2], rl[2], mp, h2);
+    // walk_three without the record in flight, for which this pass has no
+    // registers
+    unsigned b0 = m0, b1 = m1, b2 = m2;
+    int a0 = ra[0], a1 = ra[1], a2 = ra[2];
+    if (!b1) { b1 = b2; a1 = a2; b2 = 0u; }
+    if (!b0) { b0 = b1; a0 = a1; b1 = b2; a1 = a2; b2 = 0u; }
+    while (b0) {
+        const int j = a0 + __ffs(b0) - 1;
+        b0 &= b0 - 1u;
+        if (!b0) { b0 = b1; a0 = a1; b1 = b2; a1 = a2; b2 = 0u; }
+        if (!in_bounds(j, A.c.n, kBadSlot)) continue;
+        float2 e;
+        add_density(ab, dist2_packed(mp, __ldg(pos + j), e), h_recip);
+    }
+    density_finish<BY_ID>(i, A, p, ab, m0, m1, m2, rec);
 }
 
 // 32 registers (four 512-thread CTAs' worth per SM): full occupancy for this
 // issue-bound pass outweighs the few spilled values of its rare paths.
 template <bool PERSIST, bool LM = false>
 __global__ void __launch_bounds__(kMaxBlock, 4)
-k_density_t(Ctx c, const float2 *__restrict__ pos, const int *__restrict__ start,
-            const unsigned *__restrict__ occ_in, float4 *__restrict__ xr_out,
-            ulonglong2 *__restrict__ mask01, unsigned long long *__restrict__ mask2,
-            int4 *__restrict__ rows_out)
+k_density_t(const __grid_constant__ DensArrays A)
 {
     pdl_enter();
-    const bool capped = *occ_in > (unsigned)c.max_bucket;
     const int i0 = blockIdx.x * blockDim.x + threadIdx.x;
-    if (!PERSIST) {
-        if (i0 < c.n)
-            density_one<LM>(i0, c, pos, start, capped, xr_out, mask01, mask2, rows_out);
-        return;
+    for (int i = i0; i < A.c.n; i += gridDim.x * blockDim.x) {
+        density_one<LM>(i, A);
+        if (!PERSIST) break;
     }
-    for (int i = i0; i < c.n; i += gridDim.x * blockDim.x)
-        density_one<LM>(i, c, pos, start, capped, xr_out, mask01, mask2, rows_out);
 }
 
 // One density launch per block (the form other translation units call).
 __global__ void __launch_bounds__(kMaxBlock)
-k_density(Ctx c, const float2 *__restrict__ pos, const int *__restrict__ start,
-          const unsigned *__restrict__ occ_in, float4 *__restrict__ xr_out,
-          ulonglong2 *__restrict__ mask01, unsigned long long *__restrict__ mask2,
-          int4 *__restrict__ rows_out)
+k_density(const __grid_constant__ DensArrays A)
 {
-    const bool capped = *occ_in > (unsigned)c.max_bucket;
-    const int i0 = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i0 < c.n) density_one(i0, c, pos, start, capped, xr_out, mask01, mask2, rows_out);
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < A.c.n) density_one(i, A);
 }
 
 // ---------------------------------------------------------------------------
@@ -1477,12 +1503,11 @@ k_viscosity_group(const __grid_constant__ ViscArrays A, unsigned *occ_reset)
 }
 
 template <int G, bool LM, bool BY_ID = false>
-__device__ __forceinline__ void density_group_one(
-    const Group<G> &g, int i, bool valid, const Ctx &c, const float2 *__restrict__ pos,
-    const int *__restrict__ start, float4 *__restrict__ xr_out, ulonglong2 *__restrict__ mask01,
-    unsigned long long *__restrict__ mask2, int4 *__restrict__ rows_out,
-    const DensityById &by_id = DensityById())
+__device__ __forceinline__ void density_group_one(const Group<G> &g, int i, bool valid,
+                                                  const DensArrays &A)
 {
+    const Ctx &c = A.c;
+    const float2 *pos = A.pos;
     const Scene *S = c.scenes + scene_of(c, i);
     const SG sg = load_grid(S);
     const float2 p = __ldg(pos + i);
@@ -1491,9 +1516,9 @@ __device__ __forceinline__ void density_group_one(
     const float h_recip = __fdiv_rn(1.0f, hh);
     const float2 mp = make_float2(-p.x, -p.y);
     const unsigned key = cell_key(p.x, p.y, sg);
-    const bool search = valid && searchable(key, i, start, sg, false, c.max_bucket);
+    const bool search = valid && searchable(key, i, A.start, sg, false, c.max_bucket);
     int ra[3] = {0, 0, 0}, rl[3] = {0, 0, 0};
-    if (search) stencil_rows(p, key, start, sg, ra, rl, c.n);
+    if (search) stencil_rows(p, key, A.start, sg, ra, rl, c.n);
     float2 ab = make_float2(0.0f, 0.0f);
     unsigned long long m[3] = {0ull, 0ull, 0ull}, mx[3] = {0ull, 0ull, 0ull};
     float2 q0[3];
@@ -1523,12 +1548,8 @@ __device__ __forceinline__ void density_group_one(
         }
     }
     if (!valid || g.gl != 0) return;
-    if (BY_ID) {
-        by_id.put(i, ab);
-        return;
-    }
     int4 rec = make_int4(0, 0, 0, kRowsNone);
-    if (search) {
+    if (search && !BY_ID) {
         rec.w = kRowsFull;
         if (rl[0] <= kMaskRow && rl[1] <= kMaskRow && rl[2] <= kMaskRow) {
             rec = make_int4(ra[0], ra[1], ra[2], kRowsMasked);
@@ -1539,31 +1560,23 @@ __device__ __forceinline__ void density_group_one(
             x[0] = mx[0]; x[1] = mx[1]; x[2] = mx[2];
         }
     }
-    xr_out[i] = make_float4(p.x, p.y, ab.x, ab.y);
-    mask01[i] = make_ulonglong2(m[0], m[1]);
-    mask2[i] = m[2];
-    rows_out[i] = rec;
+    density_finish<BY_ID>(i, A, p, ab, m[0], m[1], m[2], rec);
 }
 
 template <int G, bool LM>
 __global__ void __launch_bounds__(kBlock)
-k_density_group(Ctx c, const float2 *__restrict__ pos, const int *__restrict__ start,
-                const unsigned *__restrict__ occ_in, float4 *__restrict__ xr_out,
-                ulonglong2 *__restrict__ mask01, unsigned long long *__restrict__ mask2,
-                int4 *__restrict__ rows_out)
+k_density_group(const __grid_constant__ DensArrays A)
 {
     pdl_enter();
-    const bool capped = *occ_in > (unsigned)c.max_bucket;
     const int th = blockIdx.x * blockDim.x + threadIdx.x;
     const Group<G> g;
-    const bool valid = th / G < c.n;
-    const int i = valid ? th / G : c.n - 1;
-    if (capped) {
-        if (valid && g.gl == 0)
-            density_one(i, c, pos, start, true, xr_out, mask01, mask2, rows_out);
+    const bool valid = th / G < A.c.n;
+    const int i = valid ? th / G : A.c.n - 1;
+    if (*A.occ_in > (unsigned)A.c.max_bucket) {
+        if (valid && g.gl == 0) density_one(i, A);
         return;
     }
-    density_group_one<G, LM>(g, i, valid, c, pos, start, xr_out, mask01, mask2, rows_out);
+    density_group_one<G, LM>(g, i, valid, A);
 }
 
 template <int G, bool LM>
@@ -2060,26 +2073,21 @@ static void enqueue_predict_sort(sph_cuda *h, Mark &mark)
 
 static void enqueue_density(sph_cuda *h)
 {
-    DevState *st = h->d_state;
+    const DensArrays arrays{make_ctx(h), h->pos_c, h->start_c,
+                            &h->d_state->build_max_occ[SLOT_PREDICTED], h->xr_c, h->mask01_c,
+                            h->mask2_c, h->rows_c, DensityById()};
     const int lanes = gather_lanes(h, 1);
     if (lanes > 1) {
         with_lanes(lanes, [&](auto G) {
             launch_step(h->long_masks ? k_density_group<G.value, true> : k_density_group<G.value, false>,
-                        blocks_for(h->n * G.value), kBlock, 0, h->stream, make_ctx(h),
-                        (const float2 *)h->pos_c, (const int *)h->start_c,
-                        (const unsigned *)&st->build_max_occ[SLOT_PREDICTED], h->xr_c, h->mask01_c,
-                        h->mask2_c, h->rows_c);
+                        blocks_for(h->n * G.value), kBlock, 0, h->stream, arrays);
         });
         return;
     }
     auto kd = h->shape[1].persistent
                   ? (h->long_masks ? k_density_t<true, true> : k_density_t<true, false>)
                   : (h->long_masks ? k_density_t<false, true> : k_density_t<false, false>);
-    const size_t smem = 0;
-    launch_step(kd, gather_grid(h, h->shape[1]), h->shape[1].block, smem, h->stream, make_ctx(h),
-                (const float2 *)h->pos_c, (const int *)h->start_c,
-                (const unsigned *)&st->build_max_occ[SLOT_PREDICTED], h->xr_c, h->mask01_c,
-                h->mask2_c, h->rows_c);
+    launch_step(kd, gather_grid(h, h->shape[1]), h->shape[1].block, 0, h->stream, arrays);
 }
 
 // The density pass of a step (the learned step's features start with it).
@@ -2383,7 +2391,8 @@ int launch_probe(sph_cuda *h, int which, void *scratch, float2 *out)
     int4 *rw = (int4 *)(base + 3 * a);
     float2 *sorted = (float2 *)(base + 4 * a);
     if (which == 0 || which == 1) {
-        k_density<<<nb, kBlock, 0, h->stream>>>(c, h->pos_a, h->start_a, occ, xr, m01, m2, rw);
+        k_density<<<nb, kBlock, 0, h->stream>>>(
+            DensArrays{c, h->pos_a, h->start_a, occ, xr, m01, m2, rw, DensityById()});
         if (which == 1)
             k_relax_update<true><<<nb, kBlock, 0, h->stream>>>(
                 RelaxArrays{c, xr, m01, m2, rw, nullptr, h->id_a, h->start_a, occ, nullptr, nullptr,
@@ -2472,24 +2481,20 @@ k_static_keys(Ctx c, SG g, const float *__restrict__ x, const float *__restrict_
 
 template <int G>
 __global__ void __launch_bounds__(kBlock)
-k_density_static(Ctx c, const float2 *__restrict__ pos, const int *__restrict__ start,
-                 const unsigned *__restrict__ occ_in, DensityById by_id)
+k_density_static(const __grid_constant__ DensArrays A)
 {
     pdl_enter();
-    const bool capped = *occ_in > (unsigned)c.max_bucket;
     const int th = blockIdx.x * blockDim.x + threadIdx.x;
     if constexpr (G > 1) {
         const Group<G> g;
-        const bool valid = th / G < c.n;
-        const int i = valid ? th / G : c.n - 1;
-        if (!capped) {
-            density_group_one<G, false, true>(g, i, valid, c, pos, start, nullptr, nullptr, nullptr,
-                                              nullptr, by_id);
-        } else if (valid && g.gl == 0) {
-            density_one<false, true>(i, c, pos, start, true, nullptr, nullptr, nullptr, nullptr, by_id);
-        }
-    } else if (th < c.n) {
-        density_one<false, true>(th, c, pos, start, capped, nullptr, nullptr, nullptr, nullptr, by_id);
+        const bool valid = th / G < A.c.n;
+        const int i = valid ? th / G : A.c.n - 1;
+        if (*A.occ_in <= (unsigned)A.c.max_bucket)
+            density_group_one<G, false, true>(g, i, valid, A);
+        else if (valid && g.gl == 0)
+            density_one<false, true>(i, A);
+    } else if (th < A.c.n) {
+        density_one<false, true>(th, A);
     }
 }
 
@@ -2528,16 +2533,15 @@ int launch_static_density(const Scene &sc, const StaticArrays &a, const float *x
                 (const int *)a.start, (const int *)a.tmp, (const int *)nullptr,
                 (const float2 *)a.pos_in, (const float2 *)nullptr, a.id_s, a.pos_s,
                 (float2 *)nullptr, (DevState *)nullptr);
-    const DensityById by_id{a.id_s, rho, rho_near};
+    const DensArrays arrays{c, a.pos_s, a.start, occ, nullptr, nullptr, nullptr, nullptr,
+                            DensityById{a.id_s, rho, rho_near}};
     const int lanes = lanes_for(n, 1);
     if (lanes > 1) {
         with_lanes(lanes, [&](auto G) {
-            launch_step(k_density_static<G.value>, blocks_for(n * G.value), kBlock, 0, st, c,
-                        (const float2 *)a.pos_s, (const int *)a.start, (const unsigned *)occ, by_id);
+            launch_step(k_density_static<G.value>, blocks_for(n * G.value), kBlock, 0, st, arrays);
         });
     } else {
-        launch_step(k_density_static<1>, nb, kBlock, 0, st, c, (const float2 *)a.pos_s,
-                    (const int *)a.start, (const unsigned *)occ, by_id);
+        launch_step(k_density_static<1>, nb, kBlock, 0, st, arrays);
     }
     return cuda_fail(cudaGetLastError(), "sph_cuda_density_static launch");
 }
