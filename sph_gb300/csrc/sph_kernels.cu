@@ -2008,10 +2008,12 @@ static const int kLearnedStepKernels = 11;
 // thread per particle fills it, and the shared form's votes and shuffles
 // cost more than they save (the relaxation, whose one-thread walk has the
 // least to do per neighbour, first).  Microseconds a step early / compressed,
-// one thread against this: 3,000 particles 98 / 89 against 37 / 37, 10,000
-// 87 / 125 against 47 / 59, 30,000 88 / 143 against 61 / 90; at 65,536, 8
-// lanes take 89 / 132 against 89 / 139.  A launch shape other than the
-// default asks for the one-thread kernels.
+// one thread against this: 3,000 particles 90 / 89 against 36 / 37, 12,000 77
+// / 130 against 44 / 66, 30,000 79 / 139 against 55 / 88.  In a uniform fluid
+// of 4 neighbours a particle the lines would lie lower (30,000: 52 against 58,
+// 14,000: 49 against 46); 4 lanes up to 100,000 gain 10-15% in compressed dam
+// breaks and lose 25-30% there.  A launch shape other than the default asks
+// for the one-thread kernels.
 static int lanes_for(int n, int k)
 {
     return n <= 5000 ? 32 : n <= 14000 ? 16 : n <= (k == 2 ? 30000 : 40000) ? 8 : 1;
