@@ -1,14 +1,14 @@
 // sph_kernels.cu -- the step kernels of libsph_cuda (sm_103a).
 //
-// One step (fluid.c:273-348) is eleven kernels on one stream, captured as a
+// One step (fluid.c:273-348) is nine kernels on one stream, captured as a
 // CUDA graph:
 //
 //   viscosity_predict   gravity + viscosity gather + predict + BCs + cell key   (A -> B)
-//   scan_reduce/apply   exclusive scan of the cell histogram -> cell starts      (C cells)
+//   cell_starts         exclusive scan of the cell histogram -> cell starts      (C cells)
 //   scatter, permute    counting-sort scatter, then in-cell order by id          (B -> C)
 //   density             density / near-density gather                           (C)
 //   relax_update        relaxation gather + BCs + velocity update + cell key     (C -> B)
-//   scan_reduce/apply   cell starts of the relaxed positions                     (A cells)
+//   cell_starts         cell starts of the relaxed positions                     (A cells)
 //   scatter, permute    back into (cell, id) order                              (B -> A)
 //
 // A handle holds one scene or many (an ensemble): every kernel runs over the
