@@ -1147,10 +1147,10 @@ __device__ __noinline__ void relax_nudged(int i, const RelaxArrays &A, float2 ac
 }
 
 // A particle whose rows have no hit masks (a row too long for them, or an
-// overflowing bucket), in slot order as everywhere.  MARK: 32 candidates
+// overflowing bucket), in slot order as everywhere.  MARK: 96 candidates
 // marked and their hits walked at a time, where the lanes of a warp are of
-// different cells (the fallback list: 117 us for 219,000 particles, in one
-// loop over the candidates 129); one loop where they are mostly of one
+// different cells (the fallback list: 106 us for 219,000 particles, 32 at a
+// time 117, in one loop over the candidates 129); one loop where they are mostly of one
 // (4,194,304 particles, compressed further: 475 -> 355 us; 64 compressed
 // scenes 206 -> 174 us).  No calls inside the loops, which would cost them
 // registers.
@@ -1180,17 +1180,22 @@ __device__ __noinline__ void relax_cold(int i, const RelaxArrays &A)
                 const int a = ra[r], l = rl[r];
                 if (MARK) {
 #pragma unroll 1
-                    for (int c0 = 0; c0 < l; c0 += 32) {
-                        const int m = min(l - c0, 32);
-                        unsigned b = 0u;
+                    for (int c0 = 0; c0 < l; c0 += 96) {
+                        unsigned b[3];
+#pragma unroll
+                        for (int k = 0; k < 3; ++k) {
+                            const int o = c0 + 32 * k, m = min(l - o, 32);
+                            b[k] = 0u;
 #pragma unroll 4
-                        for (int t = 0; t < m; ++t) {
-                            const float4 q = __ldg(xr + a + c0 + t);
-                            float2 e;
-                            if (dist2_packed(mp, make_float2(q.x, q.y), e) <= c.h2) b |= 1u << t;
+                            for (int t = 0; t < m; ++t) {
+                                const float4 q = __ldg(xr + a + o + t);
+                                float2 e;
+                                if (dist2_packed(mp, make_float2(q.x, q.y), e) <= c.h2) b[k] |= 1u << t;
+                            }
+                            if (r == 1 && (unsigned)(i - a - o) < 32u) b[k] &= ~(1u << (i - a - o));
                         }
-                        if (r == 1 && (unsigned)(i - a - c0) < 32u) b &= ~(1u << (i - a - c0));
-                        walk_mask32<float4>(b, a + c0, n, [&](int j) { return __ldg(xr + j); }, visit);
+                        walk_three<float4>(b[0], a + c0, b[1], a + c0 + 32, b[2], a + c0 + 64, n,
+                                           [&](int j) { return __ldg(xr + j); }, visit);
                     }
                 } else {
 #pragma unroll 4
