@@ -488,24 +488,4 @@ __device__ __forceinline__ unsigned hit_mask32(const float2 *__restrict__ row, i
     return n < 32 ? m & ((1u << n) - 1u) : m;
 }
 
-// Visits the set bits of a 32-bit mask as walk_mask does.
-template <class T, class Load, class Visit>
-__device__ __forceinline__ void walk_mask32(unsigned b, int base, int n, Load load, Visit visit)
-{
-    bool have = false;
-    int jp = 0;
-    T dp{};
-    while (b) {
-        const int j = base + __ffs(b) - 1;
-        b &= b - 1u;
-        if (!in_bounds(j, n, kBadSlot)) continue;
-        const T d = load(j);
-        if (have) visit(jp, dp);
-        jp = j;
-        dp = d;
-        have = true;
-    }
-    if (have) visit(jp, dp);
-}
-
 }  // namespace sph
