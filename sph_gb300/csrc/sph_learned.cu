@@ -12,7 +12,7 @@
 //
 // Training: k_train, the forward and backward pass of a batch on the tensor
 // cores (a tile of 128 samples at a time, weight gradients accumulated in
-// tensor memory), k_adam on FP32 master weights; sample collection and the
+// tensor memory), k_grad, k_adam on FP32 master weights; sample collection and the
 // calibration of the error output.
 #include <algorithm>
 #include <cstddef>
@@ -671,23 +671,22 @@ k_gemm(int M, int N, int K, const __nv_bfloat16 *__restrict__ A, long long sam, 
 }
 
 // ---------------------------------------------------------------------------
-// training: one batch is two kernels
+// training: one batch is three kernels
 // ---------------------------------------------------------------------------
 
 // Forward and backward pass of one batch, 128 samples at a time: a CTA
 // gathers a tile of samples, runs the three layers, the loss gradient and
 // the backward products with everything that passes between them in shared
-// memory, tensor memory or registers, and adds the tile's weight gradients
-// to accumulators that stay in tensor memory; at its end it writes its
-// partial gradients, which k_adam sums over the CTAs in their order.
+// memory, tensor memory or registers, and leaves the tiles that the weight
+// gradients are made of (k_grad).
 //
 // Why one kernel: a batch of 4,096 is 2.4e8 multiply-adds, about 1 us of one
 // SM's tensor core per tile, but as separate products its operands make
-// eight round trips through memory, and the weight gradients -- 4,096 deep
-// and at most 128 x 128 wide -- leave all but one SM idle.  What bounds a
-// tile here is the chain of its seven dependent products and their
-// epilogues.  A whole training step of 4,096 samples: 2.66 ms as separate
-// GEMMs and elementwise kernels, 20 us here (GB300).
+// eight round trips through memory.  What bounds a tile here is the chain of
+// its five dependent products and their epilogues.  A whole training step of
+// 4,096 samples: 2.66 ms as separate GEMMs and elementwise kernels, 67 us here
+// (GB300): 11 for this pass, 52 for k_grad (the bias sums; its products 25), 4
+// for k_adam.
 //
 // The transposed operands of the backward products (W2, W3 by rows; the
 // activations, gradients and features as M x K with K over the samples) are
@@ -695,13 +694,12 @@ k_gemm(int M, int N, int K, const __nv_bfloat16 *__restrict__ A, long long sam, 
 // arithmetic as the inference kernel in the same K order: the activations
 // are bit for bit its own.
 constexpr int kTrainThreads = 512;
-constexpr uint32_t kTrainTmem = 512;
-// tensor memory columns
-constexpr uint32_t kColAcc = 0;     // the running product
-constexpr uint32_t kColW2 = 128;    // dW2 [h2][h1]
-constexpr uint32_t kColW1 = 256;    // dW1 [h1][in]
-constexpr uint32_t kColW3 = 288;    // dW3^T [h2][out]
-constexpr uint32_t kColB2 = 304;    // db2 [h2] in the first of 16 columns
+constexpr uint32_t kTrainTmem = 128;
+constexpr uint32_t kColAcc = 0;  // tensor memory: the running product
+// What k_train leaves of a tile for k_grad: its operand tiles, as they lie in
+// shared memory (byte offsets).
+constexpr size_t kImgH1 = 0, kImgH2 = 128 * HID * 2, kImgZ1 = 2 * kImgH2, kImgZ2 = 3 * kImgH2,
+                 kImgX = 4 * kImgH2, kImgDy = kImgX + 128 * IN * 2, kTileImage = kImgDy + 128 * OUT * 2;
 
 struct alignas(128) TrainSmem {
     unsigned char w1[HID * IN * 2];
@@ -711,10 +709,8 @@ struct alignas(128) TrainSmem {
     unsigned char h1[128 * HID * 2];   // activations, then dZ1
     unsigned char h2[128 * HID * 2];   // activations, then dZ2
     unsigned char dy[128 * OUT * 2];
-    unsigned char ones[128 * 16 * 2];  // column 0 = 1: column sums as a product
     float b1[HID], b2[HID], b3[OUT];   // biases as the forward pass adds them
     double loss[4];
-    float db3[4][4];
     uint64_t mbar;
     uint32_t taddr;
 };
@@ -731,12 +727,12 @@ __device__ __forceinline__ bool join_for_mma(bool ok)
 }
 
 // cmask: outputs in the loss (bit 0, 1 displacement, bit 2 error); trunk =
-// false: the output layer's gradients alone.  part: gridDim.x x NPARAM
-// gradients, ploss: gridDim.x squared-error sums.
+// false: the output layer's gradients alone.  img: the tiles' images for
+// k_grad, ploss: gridDim.x squared-error sums.
 __global__ void __launch_bounds__(kTrainThreads, 1)
 k_train(int tiles, const int *__restrict__ order, const __nv_bfloat16 *__restrict__ X,
         const float4 *__restrict__ T, const __nv_bfloat16 *__restrict__ wbf,
-        const float *__restrict__ wf, int cmask, bool trunk, float *__restrict__ part,
+        const float *__restrict__ wf, int cmask, bool trunk, unsigned char *__restrict__ img,
         double *__restrict__ ploss, unsigned *__restrict__ err)
 {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
@@ -752,9 +748,6 @@ k_train(int tiles, const int *__restrict__ order, const __nv_bfloat16 *__restric
         tc::mbar_init(&s.mbar, 1);
         tc::mbar_fence_init();
     }
-    for (int e = t; e < 128 * 16; e += kTrainThreads)
-        *reinterpret_cast<__nv_bfloat16 *>(s.ones + tc::kmajor_offset(e >> 4, e & 15, 16)) =
-            __float2bfloat16((e & 15) == 0 ? 1.0f : 0.0f);
     // samples do not depend on the previous step; the weights do
     const int first = blockIdx.x;
     const int xr = t >> 2, xk = t & 3;  // the thread's 16-byte piece of a feature row
@@ -778,18 +771,17 @@ k_train(int tiles, const int *__restrict__ order, const __nv_bfloat16 *__restric
     const float rows_f = (float)(tiles * 128);
     const uint32_t lane_base = (uint32_t)(32 * (w & 3)) << 16;
     uint32_t tm = 0, phase = 0;
-    bool ok = true, any = false;
+    bool ok = true;
     double loss = 0.0;
-    float db3[3] = {0.0f, 0.0f, 0.0f};
     auto wait = [&]() {
         const bool done = tc::mbar_wait(&s.mbar, phase);
         phase ^= 1u;
         tc::fence_after_sync();
         return done;
     };
-    // z = product + bias; the activations go to tile h, act'(z) to g
+    // z = product + bias; the activations go to tile h and its image, act'(z) to g
     float g1[32], g2[32];
-    auto hidden = [&](unsigned char *h, const float *b, float (&g)[32]) {
+    auto hidden = [&](unsigned char *h, unsigned char *image, const float *b, float (&g)[32]) {
         float v[32];
         tc::tmem_ld32(tm + kColAcc + lane_base + (uint32_t)c0, v);
 #pragma unroll
@@ -803,12 +795,14 @@ k_train(int tiles, const int *__restrict__ order, const __nv_bfloat16 *__restric
                 g[c] = act_grad(z0);
                 g[c + 1] = act_grad(z1);
             }
-            *reinterpret_cast<uint4 *>(h + tc::kmajor_offset(row, c0 + 8 * q, HID)) =
-                make_uint4(o[0], o[1], o[2], o[3]);
+            const uint32_t at = tc::kmajor_offset(row, c0 + 8 * q, HID);
+            const uint4 v4 = make_uint4(o[0], o[1], o[2], o[3]);
+            *reinterpret_cast<uint4 *>(h + at) = v4;
+            *reinterpret_cast<uint4 *>(image + at) = v4;
         }
     };
-    // dZ = dH act'(z) into tile h
-    auto back = [&](unsigned char *h, const float (&g)[32]) {
+    // dZ = dH act'(z) into the image, and into tile h (if any)
+    auto back = [&](unsigned char *h, unsigned char *image, const float (&g)[32]) {
         float v[32];
         tc::tmem_ld32(tm + kColAcc + lane_base + (uint32_t)c0, v);
 #pragma unroll
@@ -819,15 +813,19 @@ k_train(int tiles, const int *__restrict__ order, const __nv_bfloat16 *__restric
                 const int c = 8 * q + 2 * e;
                 o[e] = tc::pack_bf16x2(v[c] * g[c], v[c + 1] * g[c + 1]);
             }
-            *reinterpret_cast<uint4 *>(h + tc::kmajor_offset(row, c0 + 8 * q, HID)) =
-                make_uint4(o[0], o[1], o[2], o[3]);
+            const uint32_t at = tc::kmajor_offset(row, c0 + 8 * q, HID);
+            const uint4 v4 = make_uint4(o[0], o[1], o[2], o[3]);
+            if (h) *reinterpret_cast<uint4 *>(h + at) = v4;
+            *reinterpret_cast<uint4 *>(image + at) = v4;
         }
     };
     const uint32_t aw1 = tc::smem_u32(s.w1), aw2 = tc::smem_u32(s.w2), aw3 = tc::smem_u32(s.w3),
                    ax = tc::smem_u32(s.x), ah1 = tc::smem_u32(s.h1), ah2 = tc::smem_u32(s.h2),
-                   ady = tc::smem_u32(s.dy), aones = tc::smem_u32(s.ones);
+                   ady = tc::smem_u32(s.dy);
     for (int tile = first; tile < tiles; tile += gridDim.x) {
+        unsigned char *gi = img + (size_t)tile * kTileImage;
         *reinterpret_cast<uint4 *>(s.x + tc::kmajor_offset(xr, 8 * xk, IN)) = xv;
+        *reinterpret_cast<uint4 *>(gi + kImgX + tc::kmajor_offset(xr, 8 * xk, IN)) = xv;
         const float4 target = tv;
         if (!join_for_mma(ok)) { ok = false; break; }
         tm = s.taddr;
@@ -838,7 +836,7 @@ k_train(int tiles, const int *__restrict__ order, const __nv_bfloat16 *__restric
         }
         if (tile + (int)gridDim.x < tiles) load_tile(tile + gridDim.x);
         ok = wait();
-        hidden(s.h1, s.b1, g1);
+        hidden(s.h1, gi + kImgH1, s.b1, g1);
         if (!join_for_mma(ok)) { ok = false; break; }
         // layer 2
         if (t == 0) {
@@ -846,7 +844,7 @@ k_train(int tiles, const int *__restrict__ order, const __nv_bfloat16 *__restric
             tc::mma_commit(&s.mbar);
         }
         ok = wait();
-        hidden(s.h2, s.b2, g2);
+        hidden(s.h2, gi + kImgH2, s.b2, g2);
         if (!join_for_mma(ok)) { ok = false; break; }
         // layer 3
         if (t == 0) {
@@ -868,106 +866,176 @@ k_train(int tiles, const int *__restrict__ order, const __nv_bfloat16 *__restric
                     loss += (double)d * d;
                     g = 2.0f * d / rows_f;
                 }
-                const __nv_bfloat16 gb = __float2bfloat16(g);
-                db3[c] += __bfloat162float(gb);
-                d16[c] = (uint32_t)__bfloat16_as_ushort(gb);
+                d16[c] = (uint32_t)__bfloat16_as_ushort(__float2bfloat16(g));
             }
-            *reinterpret_cast<uint4 *>(s.dy + tc::kmajor_offset(row, 0, OUT)) =
-                make_uint4(d16[0] | (d16[1] << 16), d16[2], 0u, 0u);
-            *reinterpret_cast<uint4 *>(s.dy + tc::kmajor_offset(row, 8, OUT)) = make_uint4(0u, 0u, 0u, 0u);
+            const uint4 d0 = make_uint4(d16[0] | (d16[1] << 16), d16[2], 0u, 0u), d1 = make_uint4(0u, 0u, 0u, 0u);
+            *reinterpret_cast<uint4 *>(s.dy + tc::kmajor_offset(row, 0, OUT)) = d0;
+            *reinterpret_cast<uint4 *>(s.dy + tc::kmajor_offset(row, 8, OUT)) = d1;
+            *reinterpret_cast<uint4 *>(gi + kImgDy + tc::kmajor_offset(row, 0, OUT)) = d0;
+            *reinterpret_cast<uint4 *>(gi + kImgDy + tc::kmajor_offset(row, 8, OUT)) = d1;
         }
         if (!join_for_mma(ok)) { ok = false; break; }
-        // dW3^T = H2^T dY, dH2 = dY W3
-        if (t == 0) {
-            tc::mma_operands(tm + kColW3, tc::mn_major(ah2, HID), tc::mn_major(ady, OUT), OUT, 128, any);
-            if (trunk)
-                tc::mma_operands(tm + kColAcc, tc::k_major(ady, OUT), tc::mn_major(aw3, HID), HID, OUT, false);
-            tc::mma_commit(&s.mbar);
-        }
-        ok = wait();
         if (trunk) {
-            back(s.h2, g2);
+            // dH2 = dY W3
+            if (t == 0) {
+                tc::mma_operands(tm + kColAcc, tc::k_major(ady, OUT), tc::mn_major(aw3, HID), HID, OUT, false);
+                tc::mma_commit(&s.mbar);
+            }
+            ok = wait();
+            back(s.h2, gi + kImgZ2, g2);
             if (!join_for_mma(ok)) { ok = false; break; }
-            // dH1 = dZ2 W2, dW2 = dZ2^T H1, db2 = dZ2^T 1
+            // dH1 = dZ2 W2
             if (t == 0) {
                 tc::mma_operands(tm + kColAcc, tc::k_major(ah2, HID), tc::mn_major(aw2, HID), HID, HID, false);
-                tc::mma_operands(tm + kColW2, tc::mn_major(ah2, HID), tc::mn_major(ah1, HID), HID, 128, any);
-                tc::mma_operands(tm + kColB2, tc::mn_major(ah2, HID), tc::mn_major(aones, 16), 16, 128, any);
                 tc::mma_commit(&s.mbar);
             }
             ok = wait();
-            back(s.h1, g1);
-            if (!join_for_mma(ok)) { ok = false; break; }
-            // dW1 = dZ1^T X
-            if (t == 0) {
-                tc::mma_operands(tm + kColW1, tc::mn_major(ah1, HID), tc::mn_major(ax, IN), IN, 128, any);
-                tc::mma_commit(&s.mbar);
-            }
-            ok = wait();
+            back(nullptr, gi + kImgZ1, g1);
         }
-        any = true;
         // the tile's buffers are free again once every thread is past its
         // wait: the next tile's join follows its feature store, so the store
         // itself must wait here
         if (!join_for_mma(ok)) { ok = false; break; }
     }
     if (ok) {
-        float *p = part + (size_t)blockIdx.x * NPARAM;
-        if (trunk) {
-            float v[32];
-            tc::tmem_ld32(tm + kColW2 + lane_base + (uint32_t)c0, v);
-            float4 *d = reinterpret_cast<float4 *>(p + OFF_W2 + row * HID + c0);
-#pragma unroll
-            for (int q = 0; q < 8; ++q) d[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
-            if (w < 4) {
-                tc::tmem_ld32(tm + kColW1 + lane_base, v);
-                float4 *d1 = reinterpret_cast<float4 *>(p + OFF_W1 + row * IN);
-#pragma unroll
-                for (int q = 0; q < 8; ++q)
-                    d1[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
-            } else if (w < 8) {
-                float u[16];
-                tc::tmem_ld16(tm + kColB2 + lane_base, u);
-                p[OFF_B2 + row] = u[0];
-            }
-        }
-        if (w >= 8 && w < 12) {
-            float u[16];
-            tc::tmem_ld16(tm + kColW3 + lane_base, u);
-#pragma unroll
-            for (int o = 0; o < OUT; ++o) p[OFF_W3 + o * HID + row] = u[o];
-        }
         if (w < 4) {
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                loss += __shfl_xor_sync(0xffffffffu, loss, o);
-#pragma unroll
-                for (int c = 0; c < 3; ++c) db3[c] += __shfl_xor_sync(0xffffffffu, db3[c], o);
-            }
-            if (lane == 0) {
-                s.loss[w] = loss;
-                for (int c = 0; c < 3; ++c) s.db3[w][c] = db3[c];
-            }
+            for (int o = 16; o > 0; o >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, o);
+            if (lane == 0) s.loss[w] = loss;
         }
     } else if (t == 0) {
         atomicAdd(err, 1u);
     }
     tc::fence_before_sync();
     __syncthreads();
-    if (ok && t < OUT)
-        part[(size_t)blockIdx.x * NPARAM + OFF_B3 + t] =
-            t < 3 ? s.db3[0][t] + s.db3[1][t] + s.db3[2][t] + s.db3[3][t] : 0.0f;
     if (ok && t == 0) ploss[blockIdx.x] = s.loss[0] + s.loss[1] + s.loss[2] + s.loss[3];
     if (w == 0) tc::tmem_dealloc(s.taddr, kTrainTmem);
 }
 
-// Sums the CTAs' partial gradients in their order, then Adam on the FP32
-// master weights and their BF16 copies; the batch's squared error is added
+// The weight gradients of a batch: sums over its samples, taken in the samples'
+// order by one accumulator each (the tiles' products one after another in
+// tensor memory, the biases' sums one row after another), so that they do not
+// depend on how many CTAs ran the batch (added up from the CTAs' partial sums
+// they were 1e-7 away, which BF16 copies of the weights and Adam made up to
+// 2e-5 of an epoch's loss).  A CTA per 16 columns of a product -- dW2 = dZ2^T H1
+// (0..7), dW1 = dZ1^T X (8, 9), dW3^T = H2^T dY (10) -- and one for each bias
+// (11: b2, 12: b3).  What bounds it is one SM reading a whole operand, 1 MB at
+// a batch of 4,096: 25 us, four tiles in flight.
+constexpr int kGradThreads = 256, kGradStages = 4, kGradRoles = 13, kGradSlice = 16;
+
+struct alignas(128) GradSmem {
+    unsigned char a[kGradStages][128 * HID * 2];
+    unsigned char b[kGradStages][128 * kGradSlice * 2];
+    uint64_t mbar[2];
+    uint32_t taddr;
+};
+
+__device__ __forceinline__ void copy16_async(unsigned char *smem, const unsigned char *src)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(tc::smem_u32(smem)), "l"(src) : "memory");
+}
+
+__global__ void __launch_bounds__(kGradThreads, 1)
+k_grad(int tiles, const unsigned char *__restrict__ img, bool trunk, float *__restrict__ grad,
+       unsigned *__restrict__ err)
+{
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    GradSmem &s = *reinterpret_cast<GradSmem *>(smem_raw);
+    const int t = threadIdx.x, w = t >> 5;
+    const int role = trunk ? (int)blockIdx.x : 10 + 2 * (int)blockIdx.x;
+    const bool product = role <= 10, has_a = role != 12, has_b = role != 11;
+    const size_t a_at = role == 10 ? kImgH2 : role == 8 || role == 9 ? kImgZ1 : kImgZ2;
+    const size_t b_at = role < 8 ? kImgH1 : role < 10 ? kImgX : kImgDy;
+    const int b_cols = role < 8 ? HID : role < 10 ? IN : OUT;
+    const int c0 = role < 8 ? kGradSlice * role : role < 10 ? kGradSlice * (role - 8) : 0;
+    if (w == 0) {
+        tc::tmem_alloc(&s.taddr, 32);
+        tc::tmem_relinquish();
+    }
+    if (t == 0) {
+        tc::mbar_init(&s.mbar[0], 1);
+        tc::mbar_init(&s.mbar[1], 1);
+        tc::mbar_fence_init();
+    }
+    pdl_enter();
+    auto load = [&](int k) {
+        if (k < tiles) {
+            const unsigned char *gi = img + (size_t)k * kTileImage;
+            const int st = k % kGradStages;
+            if (has_a)
+                for (int e = t; e < 128 * HID * 2 / 16; e += kGradThreads)
+                    // for the sums by rows: a warp's 32 columns side by side
+                    copy16_async(s.a[st] + 16 * e,
+                                 gi + a_at + (product ? 16 * e : (int)tc::kmajor_offset(e >> 4, 8 * (e & 15), HID)));
+            if (has_b)
+                copy16_async(s.b[st] + tc::kmajor_offset(t >> 1, 8 * (t & 1), kGradSlice),
+                             gi + b_at + tc::kmajor_offset(t >> 1, c0 + 8 * (t & 1), b_cols));
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    for (int k = 0; k < kGradStages - 1; ++k) load(k);
+    bool ok = true;
+    float sum = 0.0f;
+    uint32_t tm = 0;
+    for (int k = 0; k < tiles; ++k) {
+        const int st = k % kGradStages;
+        asm volatile("cp.async.wait_group %0;" ::"n"(kGradStages - 2) : "memory");
+        ok = join_for_mma(ok);  // the tile is there for every thread (and for the tensor core)
+        tm = s.taddr;
+        if (product) {
+            if (t == 0 && ok) {
+                tc::mma_operands(tm, tc::mn_major(tc::smem_u32(s.a[st]), HID),
+                                 tc::mn_major(tc::smem_u32(s.b[st]), kGradSlice), kGradSlice, 128, k > 0);
+                tc::mma_commit(&s.mbar[k & 1]);
+            }
+            // the stage loaded next was the last tile's
+            if (ok && k > 0) ok = tc::mbar_wait(&s.mbar[(k - 1) & 1], (uint32_t)((k - 1) >> 1) & 1u);
+        } else if (t < (role == 11 ? HID : OUT)) {
+            const unsigned char *tile = role == 11 ? s.a[st] : s.b[st];
+            // the rows' values requested together, then added one after another
+#pragma unroll 1
+            for (int r0 = 0; r0 < 128; r0 += 32) {
+                float v[32];
+#pragma unroll
+                for (int r = 0; r < 32; ++r)
+                    v[r] = __bfloat162float(*reinterpret_cast<const __nv_bfloat16 *>(
+                        tile + (role == 11 ? (uint32_t)((r0 + r) * HID * 2 + 2 * t)
+                                           : tc::kmajor_offset(r0 + r, t, OUT))));
+#pragma unroll
+                for (int r = 0; r < 32; ++r) sum = __fadd_rn(sum, v[r]);
+            }
+        }
+        load(k + kGradStages - 1);
+    }
+    if (product && ok) ok = tc::mbar_wait(&s.mbar[(tiles - 1) & 1], (uint32_t)((tiles - 1) >> 1) & 1u);
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    ok = join_for_mma(ok);
+    if (!ok) {
+        if (t == 0) atomicAdd(err, 1u);
+    } else if (!product) {
+        if (t < (role == 11 ? HID : OUT)) grad[(role == 11 ? OFF_B2 : OFF_B3) + t] = sum;
+    } else if (w < 4) {
+        float u[16];
+        tc::tmem_ld16(tm + ((uint32_t)(32 * w) << 16), u);
+        const int row = t;
+#pragma unroll
+        for (int e = 0; e < 16; ++e)
+            grad[role < 8    ? OFF_W2 + row * HID + c0 + e
+                 : role < 10 ? OFF_W1 + row * IN + c0 + e
+                             : OFF_W3 + e * HID + row] = u[e];
+    }
+    tc::fence_before_sync();
+    __syncthreads();
+    if (w == 0) tc::tmem_dealloc(s.taddr, 32);
+}
+
+// Adam on the FP32 master weights and their BF16 copies; the batch's squared
+// error (of `parts` CTAs) is added
 // to *loss.  trunk = false: the output layer's rows of cmask alone.  The
 // first layer's bias has no gradient: it acts through the weight of the
 // constant feature 31.
 __global__ void __launch_bounds__(128)
-k_adam(int parts, const float *__restrict__ part, const double *__restrict__ ploss,
+k_adam(int parts, const float *__restrict__ grad, const double *__restrict__ ploss,
        float *__restrict__ w, float *__restrict__ m, float *__restrict__ v, int cmask, bool trunk,
        float lr, float b1t, float b2t, __nv_bfloat16 *__restrict__ wbf, double *__restrict__ loss)
 {
@@ -984,10 +1052,7 @@ k_adam(int parts, const float *__restrict__ part, const double *__restrict__ plo
         train = (cmask >> (e >= OFF_B3 ? e - OFF_B3 : (e - OFF_W3) / HID)) & 1;
     if (train) {
         float g = 0.0f;
-        if (e < OFF_B1 || e >= OFF_W2) {
-#pragma unroll 8
-            for (int c = 0; c < parts; ++c) g += __ldcg(part + (size_t)c * NPARAM + e);
-        }
+        if (e < OFF_B1 || e >= OFF_W2) g = __ldcg(grad + e);
         const float mm = 0.9f * m[e] + 0.1f * g;
         const float vv = 0.999f * v[e] + 0.001f * g * g;
         m[e] = mm;
@@ -1170,10 +1235,11 @@ struct LearnedModel {
     // training workspace, kept between calls: partial gradients and squared
     // errors of a step's CTAs, the epoch's running sum (the last of `loss`),
     // the epoch's sample order
-    float *part = nullptr;
+    float *grad = nullptr;
+    unsigned char *img = nullptr;
     double *loss = nullptr;
     int *order = nullptr;
-    int parts_cap = 0, order_cap = 0;
+    int parts_cap = 0, order_cap = 0, img_cap = 0;
     // sph_learned_forward's workspace, kept between calls: two buffers of
     // at most kForwardRows float rows and their outputs, the second stream,
     // and a page-locked word that a wait that gave up sets
@@ -1204,6 +1270,7 @@ inline int nblk(long long n, int bs = 256) { return (int)((n + bs - 1) / bs); }
 
 size_t mlp_smem() { return sizeof(ml::MlpSmem) + 1024; }
 size_t train_smem() { return sizeof(ml::TrainSmem) + 1024; }
+size_t grad_smem() { return sizeof(ml::GradSmem) + 1024; }
 // At least 60 KB, so that at most three GEMM CTAs (3 x 128 TMEM columns)
 // share an SM.
 size_t gemm_smem() { return std::max(sizeof(ml::GemmSmem) + 1024, (size_t)60 * 1024); }
@@ -1215,6 +1282,7 @@ int configure_kernels()
     LCUDA(cudaFuncSetAttribute(ml::k_mlp<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mlp_smem()));
     LCUDA(cudaFuncSetAttribute(ml::k_mlp<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mlp_smem()));
     LCUDA(cudaFuncSetAttribute(ml::k_train, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)train_smem()));
+    LCUDA(cudaFuncSetAttribute(ml::k_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)grad_smem()));
     LCUDA(cudaFuncSetAttribute(ml::k_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gemm_smem()));
     done = true;
     return SPH_OK;
@@ -1278,15 +1346,20 @@ int ensure_forward(LearnedModel *l, int b, int rows)
 }
 
 // The training workspace for steps of `parts` CTAs and `rows` samples an epoch.
-int ensure_training(LearnedModel *l, int parts, int rows)
+int ensure_training(LearnedModel *l, int parts, int tiles, int rows)
 {
+    if (!l->grad) LCUDA(cudaMalloc(&l->grad, ml::NPARAM * sizeof(float)));
+    if (tiles > l->img_cap) {
+        cudaFree(l->img);
+        l->img = nullptr;
+        l->img_cap = 0;
+        LCUDA(cudaMalloc(&l->img, (size_t)tiles * ml::kTileImage));
+        l->img_cap = tiles;
+    }
     if (parts > l->parts_cap) {
-        cudaFree(l->part);
         cudaFree(l->loss);
-        l->part = nullptr;
         l->loss = nullptr;
         l->parts_cap = 0;
-        LCUDA(cudaMalloc(&l->part, (size_t)parts * ml::NPARAM * sizeof(float)));
         LCUDA(cudaMalloc(&l->loss, ((size_t)parts + 1) * sizeof(double)));
         l->parts_cap = parts;
     }
@@ -1309,10 +1382,12 @@ int train_batch(LearnedModel *l, const int *order, int batch, int parts, int cma
     using namespace ml;
     launch_step(k_train, parts, kTrainThreads, train_smem(), l->stream, batch / 128, order,
                (const __nv_bfloat16 *)l->X, (const float4 *)l->T, (const __nv_bfloat16 *)l->wbf,
-               (const float *)l->w, cmask, trunk, l->part, l->loss, l->d_err);
+               (const float *)l->w, cmask, trunk, l->img, l->loss, l->d_err);
+    launch_step(k_grad, trunk ? kGradRoles : 2, kGradThreads, grad_smem(), l->stream, batch / 128,
+               (const unsigned char *)l->img, trunk, l->grad, l->d_err);
     ++l->adam_t;
     const float b1t = powf(0.9f, (float)l->adam_t), b2t = powf(0.999f, (float)l->adam_t);
-    launch_step(k_adam, nblk(NPARAM, 128), 128, 0, l->stream, parts, (const float *)l->part,
+    launch_step(k_adam, nblk(NPARAM, 128), 128, 0, l->stream, parts, (const float *)l->grad,
                (const double *)l->loss, l->w, l->m, l->v, cmask, trunk, lr, b1t, b2t, l->wbf,
                l->loss + l->parts_cap);
     return cuda_fail(cudaGetLastError(), "training step");
@@ -1332,7 +1407,7 @@ int train_loop(LearnedModel *l, int first, int nsamples, int epochs, int batch, 
     const int per_epoch = nsamples / batch;
     // a CTA per tile of 128 samples, at most one per SM
     const int parts = std::min(batch / 128, num_sms());
-    LTRY(ensure_training(l, parts, per_epoch * batch));
+    LTRY(ensure_training(l, parts, batch / 128, per_epoch * batch));
     double *d_loss = l->loss + l->parts_cap;
     std::vector<int> order(nsamples);
     for (int i = 0; i < nsamples; ++i) order[i] = first + i;
@@ -1532,7 +1607,7 @@ int sph_learned_destroy(sph_learned_t *l)
     if (!l) return SPH_OK;
     if (l->stream) cudaStreamSynchronize(l->stream);
     if (l->stream2) cudaStreamSynchronize(l->stream2);
-    void *ptrs[] = {l->w, l->m, l->v, l->wbf, l->d_err, l->X, l->T, l->slot, l->part,
+    void *ptrs[] = {l->w, l->m, l->v, l->wbf, l->d_err, l->X, l->T, l->slot, l->grad, l->img,
                     l->loss, l->order, l->fwd_in[0], l->fwd_in[1], l->fwd_out[0], l->fwd_out[1]};
     for (void *p : ptrs)
         if (p) cudaFree(p);

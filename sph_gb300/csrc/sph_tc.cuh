@@ -128,18 +128,24 @@ __device__ __forceinline__ uint64_t globaltimer_ns()
 // kWaitNs nanoseconds of the GPU's global timer (or kSpinLimit polls) and
 // returns false (the caller records an error).
 constexpr uint64_t kWaitNs = 1000000000ull;  // 1 s: any tensor-core step takes microseconds
+__device__ __forceinline__ bool mbar_try(uint32_t a, uint32_t parity)
+{
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done) : "r"(a), "r"(parity) : "memory");
+    return done != 0;
+}
+
 __device__ __forceinline__ bool mbar_wait(uint64_t *mbar, uint32_t parity)
 {
     const uint32_t a = smem_u32(mbar);
+    if (mbar_try(a, parity)) return true;  // without a look at the clock
     const uint64_t t0 = globaltimer_ns();
     for (uint32_t it = 0; it < kSpinLimit; ++it) {
-        uint32_t done;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(done) : "r"(a), "r"(parity) : "memory");
-        if (done) return true;
+        if (mbar_try(a, parity)) return true;
         if (globaltimer_ns() - t0 > kWaitNs) return false;
     }
     return false;
