@@ -11,8 +11,8 @@
 //    particles that take the plain relaxation for k_relax_fallback)
 //
 // Training: k_train, the forward and backward pass of a batch on the tensor
-// cores (a tile of 128 samples at a time, weight gradients accumulated in
-// tensor memory), k_grad, k_adam on FP32 master weights; sample collection and the
+// cores (a tile of 128 samples at a time), k_grad, the weight gradients in the
+// samples' order, k_adam on FP32 master weights; sample collection and the
 // calibration of the error output.
 #include <algorithm>
 #include <cstddef>
@@ -684,9 +684,8 @@ k_gemm(int M, int N, int K, const __nv_bfloat16 *__restrict__ A, long long sam, 
 // SM's tensor core per tile, but as separate products its operands make
 // eight round trips through memory.  What bounds a tile here is the chain of
 // its five dependent products and their epilogues.  A whole training step of
-// 4,096 samples: 2.66 ms as separate GEMMs and elementwise kernels, 67 us here
-// (GB300): 11 for this pass, 52 for k_grad (the bias sums; its products 25), 4
-// for k_adam.
+// 4,096 samples: 2.66 ms as separate GEMMs and elementwise kernels, 46 us here
+// (GB300): 11 for this pass, 31 for k_grad, 4 for k_adam.
 //
 // The transposed operands of the backward products (W2, W3 by rows; the
 // activations, gradients and features as M x K with K over the samples) are
@@ -918,10 +917,11 @@ k_train(int tiles, const int *__restrict__ order, const __nv_bfloat16 *__restric
 // depend on how many CTAs ran the batch (added up from the CTAs' partial sums
 // they were 1e-7 away, which BF16 copies of the weights and Adam made up to
 // 2e-5 of an epoch's loss).  A CTA per 16 columns of a product -- dW2 = dZ2^T H1
-// (0..7), dW1 = dZ1^T X (8, 9), dW3^T = H2^T dY (10) -- and one for each bias
-// (11: b2, 12: b3).  What bounds it is one SM reading a whole operand, 1 MB at
-// a batch of 4,096: 25 us, four tiles in flight.
-constexpr int kGradThreads = 256, kGradStages = 4, kGradRoles = 13, kGradSlice = 16;
+// (0..7), dW1 = dZ1^T X (8, 9), dW3^T = H2^T dY (10) -- four for the second
+// bias (11..14) and one for the third.  What bounds it is one SM reading a whole operand, 1 MB at
+// a batch of 4,096, four tiles in flight, and the biases' chains of additions: 31
+// us (one CTA for all of b2: 50).
+constexpr int kGradThreads = 256, kGradStages = 4, kGradRoles = 16, kGradSlice = 16;
 
 struct alignas(128) GradSmem {
     unsigned char a[kGradStages][128 * HID * 2];
@@ -942,8 +942,8 @@ k_grad(int tiles, const unsigned char *__restrict__ img, bool trunk, float *__re
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     GradSmem &s = *reinterpret_cast<GradSmem *>(smem_raw);
     const int t = threadIdx.x, w = t >> 5;
-    const int role = trunk ? (int)blockIdx.x : 10 + 2 * (int)blockIdx.x;
-    const bool product = role <= 10, has_a = role != 12, has_b = role != 11;
+    const int role = trunk ? (int)blockIdx.x : 10 + 5 * (int)blockIdx.x;
+    const bool product = role <= 10, rows_b2 = role > 10 && role < 15, has_b = !rows_b2;
     const size_t a_at = role == 10 ? kImgH2 : role == 8 || role == 9 ? kImgZ1 : kImgZ2;
     const size_t b_at = role < 8 ? kImgH1 : role < 10 ? kImgX : kImgDy;
     const int b_cols = role < 8 ? HID : role < 10 ? IN : OUT;
@@ -962,11 +962,13 @@ k_grad(int tiles, const unsigned char *__restrict__ img, bool trunk, float *__re
         if (k < tiles) {
             const unsigned char *gi = img + (size_t)k * kTileImage;
             const int st = k % kGradStages;
-            if (has_a)
+            if (product)
                 for (int e = t; e < 128 * HID * 2 / 16; e += kGradThreads)
-                    // for the sums by rows: a warp's 32 columns side by side
+                    copy16_async(s.a[st] + 16 * e, gi + a_at + 16 * e);
+            if (rows_b2)  // 32 columns, row by row
+                for (int e = t; e < 128 * 4; e += kGradThreads)
                     copy16_async(s.a[st] + 16 * e,
-                                 gi + a_at + (product ? 16 * e : (int)tc::kmajor_offset(e >> 4, 8 * (e & 15), HID)));
+                                 gi + a_at + tc::kmajor_offset(e >> 2, 32 * (role - 11) + 8 * (e & 3), HID));
             if (has_b)
                 copy16_async(s.b[st] + tc::kmajor_offset(t >> 1, 8 * (t & 1), kGradSlice),
                              gi + b_at + tc::kmajor_offset(t >> 1, c0 + 8 * (t & 1), b_cols));
@@ -990,8 +992,8 @@ k_grad(int tiles, const unsigned char *__restrict__ img, bool trunk, float *__re
             }
             // the stage loaded next was the last tile's
             if (ok && k > 0) ok = tc::mbar_wait(&s.mbar[(k - 1) & 1], (uint32_t)((k - 1) >> 1) & 1u);
-        } else if (t < (role == 11 ? HID : OUT)) {
-            const unsigned char *tile = role == 11 ? s.a[st] : s.b[st];
+        } else if (t < (rows_b2 ? 32 : OUT)) {
+            const unsigned char *tile = rows_b2 ? s.a[st] : s.b[st];
             // the rows' values requested together, then added one after another
 #pragma unroll 1
             for (int r0 = 0; r0 < 128; r0 += 32) {
@@ -999,8 +1001,7 @@ k_grad(int tiles, const unsigned char *__restrict__ img, bool trunk, float *__re
 #pragma unroll
                 for (int r = 0; r < 32; ++r)
                     v[r] = __bfloat162float(*reinterpret_cast<const __nv_bfloat16 *>(
-                        tile + (role == 11 ? (uint32_t)((r0 + r) * HID * 2 + 2 * t)
-                                           : tc::kmajor_offset(r0 + r, t, OUT))));
+                        tile + (rows_b2 ? (uint32_t)((r0 + r) * 64 + 2 * t) : tc::kmajor_offset(r0 + r, t, OUT))));
 #pragma unroll
                 for (int r = 0; r < 32; ++r) sum = __fadd_rn(sum, v[r]);
             }
@@ -1013,7 +1014,7 @@ k_grad(int tiles, const unsigned char *__restrict__ img, bool trunk, float *__re
     if (!ok) {
         if (t == 0) atomicAdd(err, 1u);
     } else if (!product) {
-        if (t < (role == 11 ? HID : OUT)) grad[(role == 11 ? OFF_B2 : OFF_B3) + t] = sum;
+        if (t < (rows_b2 ? 32 : OUT)) grad[(rows_b2 ? OFF_B2 + 32 * (role - 11) : OFF_B3) + t] = sum;
     } else if (w < 4) {
         float u[16];
         tc::tmem_ld16(tm + ((uint32_t)(32 * w) << 16), u);
