@@ -19,6 +19,7 @@
 #include <climits>
 #include <cmath>
 #include <cstring>
+#include <mutex>
 #include <vector>
 
 #include <cuda_bf16.h>
@@ -1251,6 +1252,12 @@ struct LearnedModel {
     unsigned *h_err = nullptr;
     cudaStream_t stream = nullptr;
     unsigned long long seed = 0;
+    // Host threads may share a model.  busy: held by a call while it has work
+    // on the model's streams (a call of sph_learned_forward, an epoch), so
+    // that the forward workspace is one call's at a time and a call's pieces
+    // all see the same weights; train_busy: held by a whole training call,
+    // whose workspace outlives its epochs.  train_busy is taken first.
+    std::mutex busy, train_busy;
 };
 
 }  // namespace sph
@@ -1404,6 +1411,7 @@ int train_loop(LearnedModel *l, int first, int nsamples, int epochs, int batch, 
         return SPH_ERR_STATE;
     }
     LTRY(configure_kernels());
+    std::lock_guard<std::mutex> one_training(l->train_busy);
     batch = std::max(128, std::min(batch, nsamples) / 128 * 128);
     const int per_epoch = nsamples / batch;
     // a CTA per tile of 128 samples, at most one per SM
@@ -1423,6 +1431,7 @@ int train_loop(LearnedModel *l, int first, int nsamples, int epochs, int batch, 
     double last = 0.0;
     for (int ep = 0; ep < epochs; ++ep) {
         for (int i = nsamples - 1; i > 0; --i) std::swap(order[i], order[(int)(next() % (i + 1))]);
+        std::lock_guard<std::mutex> one_epoch(l->busy);
         LCUDA(cudaMemcpyAsync(l->order, order.data(), (size_t)per_epoch * batch * sizeof(int),
                               cudaMemcpyHostToDevice, l->stream));
         LCUDA(cudaMemsetAsync(d_loss, 0, sizeof(double), l->stream));
@@ -1635,6 +1644,7 @@ int sph_learned_set_params(sph_learned_t *l, const float *in)
         set_error("null argument");
         return SPH_ERR_INVALID;
     }
+    std::lock_guard<std::mutex> one_call(l->busy);
     LCUDA(cudaMemcpyAsync(l->w, in, ml::NPARAM * sizeof(float), cudaMemcpyHostToDevice, l->stream));
     LCUDA(cudaMemsetAsync(l->m, 0, ml::NPARAM * sizeof(float), l->stream));
     LCUDA(cudaMemsetAsync(l->v, 0, ml::NPARAM * sizeof(float), l->stream));
@@ -1697,6 +1707,7 @@ int sph_learned_forward(sph_learned_t *l, const float *features, int n, float *o
     }
     if (n == 0) return SPH_OK;
     LTRY(configure_kernels());
+    std::lock_guard<std::mutex> one_call(l->busy);
     // the caller's rows go to the device as they are, kForwardRows at a time
     // on two streams, so that the copies of one piece can overlap the
     // kernel and the copies of another

@@ -1,0 +1,53 @@
+"""The order of the host code's copies, waits and launches, on stand-ins for
+the CUDA runtime that run a stream's work as late as a GPU may."""
+import threading
+
+import numpy as np
+import pytest
+
+import host_runtime
+from sph_gb300 import LearnedModel, _lib
+
+
+@pytest.fixture(scope="module")
+def host_lib(tmp_path_factory):
+    return host_runtime.load(tmp_path_factory.mktemp("host"))
+
+
+@pytest.fixture
+def host(host_lib, monkeypatch):
+    monkeypatch.setattr(_lib, "_lib", host_lib)
+    host_lib.host_log()
+    return host_lib
+
+
+def copies_in(log):
+    """(destination, bytes) of the log's host-to-device copies."""
+    return [tuple(map(int, line.split()[1:])) for line in log.decode().splitlines()
+            if line.startswith("h2d ")]
+
+
+@pytest.mark.parametrize("first,second", [(1, 1), (20000, 300), (300, 20000), (200000, 131073)])
+def test_forward_calls_of_two_threads_keep_apart(host, first, second):
+    """While one call of the network is on its way, another thread's call on
+    the same model neither writes its rows over the first one's nor takes
+    its buffers away."""
+    with LearnedModel(0, seed=1) as m:
+        m.forward(np.ones((10, LearnedModel.IN), np.float32))
+        host.host_log()
+        threads = [threading.Thread(target=m.forward, args=(np.ones((n, LearnedModel.IN), np.float32),))
+                   for n in (first, second)]
+        host.host_hold()
+        threads[0].start()
+        assert host.host_wait_held()
+        mine = copies_in(host.host_log())
+        threads[1].start()
+        threads[1].join(1.0)
+        log = host.host_log()
+        host.host_release()
+        for t in threads:
+            t.join()
+    assert len(mine) == 1
+    assert not any(line.startswith(b"free ") for line in log.splitlines()), log
+    a, size = mine[0]
+    assert not any(b < a + size and a < b + k for b, k in copies_in(log)), (mine, log)
