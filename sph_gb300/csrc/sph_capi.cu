@@ -1046,11 +1046,14 @@ int sph_cuda_load_state(sph_cuda_t *h, const char *path)
         return SPH_ERR_INVALID;
     }
     SPH_TRY(sph_cuda_upload_particles(h, ps.data(), hd.n));
-    // the upload starts counters afresh: restore the step count and whether
-    // the next step applies viscosity
-    SPH_CUDA(cudaMemcpy(&h->d_state->steps, &hd.steps, sizeof(hd.steps), cudaMemcpyHostToDevice));
-    SPH_CUDA(cudaMemcpy(&h->d_state->lists_valid, &hd.lists_valid, sizeof(hd.lists_valid),
-                        cudaMemcpyHostToDevice));
+    // the upload starts counters afresh, in stream order and without waiting
+    // for it (nothing to read: an empty upload): restore the step count and
+    // whether the next step applies viscosity behind it
+    SPH_CUDA(cudaMemcpyAsync(&h->d_state->steps, &hd.steps, sizeof(hd.steps), cudaMemcpyHostToDevice,
+                             h->stream));
+    SPH_CUDA(cudaMemcpyAsync(&h->d_state->lists_valid, &hd.lists_valid, sizeof(hd.lists_valid),
+                             cudaMemcpyHostToDevice, h->stream));
+    SPH_CUDA(cudaStreamSynchronize(h->stream));
     return SPH_OK;
 }
 

@@ -1,12 +1,14 @@
 """The order of the host code's copies, waits and launches, on stand-ins for
 the CUDA runtime that run a stream's work as late as a GPU may."""
+import ctypes
+import struct
 import threading
 
 import numpy as np
 import pytest
 
 import host_runtime
-from sph_gb300 import LearnedModel, _lib
+from sph_gb300 import LearnedModel, Simulation, _lib, scenes
 
 
 @pytest.fixture(scope="module")
@@ -51,3 +53,19 @@ def test_forward_calls_of_two_threads_keep_apart(host, first, second):
     assert not any(line.startswith(b"free ") for line in log.splitlines()), log
     a, size = mine[0]
     assert not any(b < a + size and a < b + k for b, k in copies_in(log)), (mine, log)
+
+
+def simulation(n=1000):
+    sc = scenes.config2(n)
+    return Simulation(sc.params.as_dict(), sc.config(), sc.n)
+
+
+def test_empty_checkpoint_restores_its_counters(host, tmp_path):
+    """The step count of a checkpoint without particles is written after the
+    upload's clearing of the counters."""
+    path = tmp_path / "empty.ckpt"
+    path.write_bytes(struct.pack("<8sIiiIQI12x", b"SPHCKPT1", 1, 0, 1, 1, 77,
+                                 ctypes.sizeof(_lib.FluidParticle)))
+    with simulation() as sim:
+        sim.load_state(path)
+        assert sim.counters()["steps"] == 77
