@@ -1060,6 +1060,11 @@ int sph_cuda_load_state(sph_cuda_t *h, const char *path)
 int sph_cuda_rebuild_neighbors(sph_cuda_t *h)
 {
     SPH_TRY(check_handle(h));
+    // refused in a stream capture, like the other calls that are not a step
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    SPH_CUDA(cudaStreamIsCapturing(h->stream, &cap));
+    if (cap != cudaStreamCaptureStatusNone)
+        return cuda_fail(cudaErrorStreamCaptureUnsupported, "sph_cuda_rebuild_neighbors");
     // The sorted state always carries the cell lists of its current
     // positions, so the relation exists already: enable it.
     return launch_enable_lists(h);

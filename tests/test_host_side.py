@@ -8,7 +8,7 @@ import numpy as np
 import pytest
 
 import host_runtime
-from sph_gb300 import LearnedModel, Simulation, _lib, scenes
+from sph_gb300 import LearnedModel, Simulation, SphError, _lib, scenes
 
 
 @pytest.fixture(scope="module")
@@ -69,3 +69,12 @@ def test_empty_checkpoint_restores_its_counters(host, tmp_path):
     with simulation() as sim:
         sim.load_state(path)
         assert sim.counters()["steps"] == 77
+
+
+def test_rebuild_is_refused_in_a_capture(host):
+    with simulation() as sim:
+        _lib.check(host.sph_cuda_set_stream(sim.handle, host.host_stream(1)))
+        host.host_log()
+        with pytest.raises(SphError, match="(?i)captur"):
+            sim.rebuild_neighbors()
+        assert b"launch" not in host.host_log()
