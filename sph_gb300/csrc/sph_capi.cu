@@ -269,12 +269,15 @@ int run_steps(sph_cuda *h, int nsteps)
     int t = 0;
     if (nsteps >= kManySteps) {
         if (!h->exec_many && ++h->many_calls == kManyCalls) {
+            // without it (memory) the steps run one graph at a time
             cudaGraph_t g = nullptr;
             int nk = 0;
-            SPH_TRY(capture_steps(h, kManySteps, &g, &nk));
-            const cudaError_t ie = cudaGraphInstantiate(&h->exec_many, g, 0);
-            cudaGraphDestroy(g);
-            SPH_CUDA(ie);
+            if (capture_steps(h, kManySteps, &g, &nk) != SPH_OK ||
+                cudaGraphInstantiate(&h->exec_many, g, 0) != cudaSuccess) {
+                h->exec_many = nullptr;
+                (void)cudaGetLastError();
+            }
+            if (g) cudaGraphDestroy(g);
         }
         if (h->exec_many)
             for (; t + kManySteps <= nsteps; t += kManySteps)

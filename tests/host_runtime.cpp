@@ -91,6 +91,13 @@ void host_fail(const char *call, int after, int error)
     std::lock_guard<std::recursive_mutex> l(g_mu);
     g_fail[call] = {after, (cudaError_t)error};
 }
+void host_reset(void)
+{
+    std::lock_guard<std::recursive_mutex> l(g_mu);
+    g_fail.clear();
+    g_log.clear();
+    g_last = cudaSuccess;
+}
 const char *host_log(void)  // and starts a new one
 {
     static std::string out;
@@ -242,8 +249,9 @@ cudaError_t W(cudaEventElapsedTime)(float *ms, cudaEvent_t, cudaEvent_t) { *ms =
 
 cudaError_t W(cudaStreamBeginCapture)(cudaStream_t st, cudaStreamCaptureMode)
 {
-    reinterpret_cast<Stream *>(st)->capturing = true;
-    return failing("cudaStreamBeginCapture");
+    const cudaError_t e = failing("cudaStreamBeginCapture");
+    reinterpret_cast<Stream *>(st)->capturing = e == cudaSuccess;
+    return e;
 }
 cudaError_t W(cudaStreamEndCapture)(cudaStream_t st, cudaGraph_t *g)
 {

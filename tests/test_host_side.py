@@ -19,7 +19,7 @@ def host_lib(tmp_path_factory):
 @pytest.fixture
 def host(host_lib, monkeypatch):
     monkeypatch.setattr(_lib, "_lib", host_lib)
-    host_lib.host_log()
+    host_lib.host_reset()
     return host_lib
 
 
@@ -78,3 +78,22 @@ def test_rebuild_is_refused_in_a_capture(host):
         with pytest.raises(SphError, match="(?i)captur"):
             sim.rebuild_neighbors()
         assert b"launch" not in host.host_log()
+
+
+@pytest.mark.parametrize("call", ["cudaGraphInstantiate", "cudaStreamBeginCapture"])
+def test_steps_go_on_without_the_multi_step_graph(host, call):
+    with simulation() as sim:
+        x = np.linspace(1.0, 2.0, 100, dtype=np.float32)
+        sim.upload(x, x)
+        sim.step(None, 4)
+        host.host_log()
+        host.host_fail(call.encode(), 0, 2)  # cudaErrorMemoryAllocation
+        for _ in range(9):
+            sim.step(None, 4)
+        log = host.host_log().splitlines()
+        assert sum(line.startswith(b"graph ") for line in log) == 9 * 4
+        # the graph of a single step is not optional
+        host.host_fail(call.encode(), 0, 2)
+        sim.upload(x[:50], x[:50])
+        with pytest.raises(SphError):
+            sim.step(None, 4)
