@@ -191,6 +191,9 @@ struct sph_cuda {
     // tunables (made at the kManyCalls-th such call; null: not yet)
     cudaGraphExec_t exec_many = nullptr;
     int many_calls = 0;
+    // a call that queues cell builds failed: counters of a key producer without
+    // its build may be left, which the next upload clears
+    bool cells_dirty = false;
     cudaEvent_t timer[2] = {nullptr, nullptr};
     int launches_per_step = 0;
 

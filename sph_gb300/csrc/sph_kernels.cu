@@ -2115,7 +2115,9 @@ int enqueue_predicted_state(sph_cuda *h)
     auto none = []() {};
     enqueue_predict_sort(h, none);
     enqueue_density(h);
-    return cuda_fail(cudaGetLastError(), "predicted state");
+    const int rc = cuda_fail(cudaGetLastError(), "predicted state");
+    h->cells_dirty |= rc != SPH_OK;
+    return rc;
 }
 
 // The relaxation of a step: the C order's density records to the B arrays.
@@ -2165,7 +2167,8 @@ int launch_learned_relax(sph_cuda *h, float2 *probe_out, cudaEvent_t *events)
 // relaxation and the velocity update -- where the reference's compute rank
 // receives new tunables inside a step (fluid.c:293-294, between
 // predict_positions at :279 and hash_fluid at :315).  Single-scene handles.
-int enqueue_step(sph_cuda *h, cudaEvent_t *events, int *nkernels, const tunable_parameters *mid_tp)
+static int enqueue_step_kernels(sph_cuda *h, cudaEvent_t *events, int *nkernels,
+                                const tunable_parameters *mid_tp)
 {
     const int n = h->n;
     const int nb = blocks_for(n);
@@ -2216,6 +2219,13 @@ int enqueue_step(sph_cuda *h, cudaEvent_t *events, int *nkernels, const tunable_
     mark();
     if (nkernels) *nkernels = e - 1;
     return cuda_fail(cudaGetLastError(), "step launch");
+}
+
+int enqueue_step(sph_cuda *h, cudaEvent_t *events, int *nkernels, const tunable_parameters *mid_tp)
+{
+    const int rc = enqueue_step_kernels(h, events, nkernels, mid_tp);
+    h->cells_dirty |= rc != SPH_OK;
+    return rc;
 }
 
 unsigned bounds_flags_kernels() { return read_bounds_flag(); }
@@ -2317,15 +2327,19 @@ int upload_device(sph_cuda *h, int n, const UploadSource &src)
 {
     if (n == 0) return SPH_OK;
     DevState *st = h->d_state;
-    // a fresh state starts every step's build from zero tile counts,
-    // whatever an interrupted step left
+    // a fresh state starts every build from zero tile counts and cell
+    // counters, whatever an interrupted step left: k_cell_starts looks at the
+    // counters of the counted tiles alone, and zeroes them itself
     cudaMemsetAsync(h->build_tiles, 0, (size_t)h->ntiles * sizeof(unsigned), h->stream);
+    if (h->cells_dirty) cudaMemsetAsync(h->cnt, 0, (size_t)h->M * sizeof(unsigned), h->stream);
     launch_step(k_upload, blocks_for(n), kBlock, 0, h->stream, make_ctx(h), src, h->pos_b, h->vel_b,
                 h->prev_c, h->xr_c, h->id_c, h->kr_b, h->cnt, &st->build_max_occ[SLOT_RELAXED]);
     cudaEventRecord(h->host_ev, h->stream);  // the source has been read
     enqueue_cell_starts(h, h->start_a, &st->build_max_occ[SLOT_RELAXED]);
     enqueue_a_order(h, nullptr, [] {});
-    return cuda_fail(cudaGetLastError(), "upload kernels");
+    const int rc = cuda_fail(cudaGetLastError(), "upload kernels");
+    h->cells_dirty = rc != SPH_OK;
+    return rc;
 }
 
 int launch_unpermute(sph_cuda *h, float2 *out)

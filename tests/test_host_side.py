@@ -97,3 +97,29 @@ def test_steps_go_on_without_the_multi_step_graph(host, call):
         sim.upload(x[:50], x[:50])
         with pytest.raises(SphError):
             sim.step(None, 4)
+
+
+@pytest.mark.parametrize("interrupted", ["step", "upload"])
+def test_upload_after_an_interrupted_build_clears_the_counters(host, interrupted):
+    """A key producer that ran without its cell starts leaves counters that a
+    later build would add its own to."""
+    sc = scenes.config2(1000)
+    size = 4 * (sc.size_x * sc.size_y + 1)
+    x = np.linspace(1.0, 2.0, 100, dtype=np.float32)
+
+    def cleared(sim):
+        host.host_log()
+        sim.upload(x, x)
+        return any(line.startswith(b"memset ") and int(line.split()[2]) == size
+                   for line in host.host_log().splitlines())
+
+    with Simulation(sc.params.as_dict(), sc.config(), 200) as sim:
+        assert not cleared(sim)
+        host.host_fail(b"launch", 1, 701)  # the cell starts: cudaErrorLaunchOutOfResources
+        with pytest.raises(SphError):
+            if interrupted == "step":
+                sim.step_split(None, sc.params.as_dict())
+            else:
+                sim.upload(x, x)
+        assert cleared(sim)
+        assert not cleared(sim)
