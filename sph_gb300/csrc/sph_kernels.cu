@@ -988,19 +988,17 @@ __device__ __forceinline__ WalkConsts walk_consts(const RelaxConsts &c, float4 m
     return wc;
 }
 
-// Whether the pair of particle i (cell `key`) with slot j, r2 <= 2e-12, is one
-// whose owner i is nudged (fluid.c:583-586): r <= 1e-6 and i holds it.
-__device__ __noinline__ bool is_nudge(int i, int j, const Scene *S, const float4 *__restrict__ xr,
-                                      const int *__restrict__ ids)
+// The largest float whose correctly rounded root is at most 1e-6.
+constexpr float kNudgeR2 = 0x1.19799ap-40f;
+
+// Whether particle i at `p` (cell `key`) is nudged by its pair with slot j at
+// `q` (fluid.c:583-586): r <= 1e-6 and i holds the pair.
+__device__ __forceinline__ bool is_nudge(int i, int j, float2 p, unsigned key, float2 q, const SG &g,
+                                         const int *__restrict__ ids)
 {
-    if (j == i) return false;
-    const float4 me = __ldg(xr + i), q = __ldg(xr + j);
     float2 e;
-    const float r2 = dist2_packed(make_float2(-me.x, -me.y), make_float2(q.x, q.y), e);
-    const float r = r2 > 0.0f ? __fsqrt_rn(r2) : 0.0f;
-    if (!(r <= 0.000001f)) return false;
-    const SG g = load_grid(S);
-    return owns_pair(cell_key(me.x, me.y, g), ids[i], make_float2(q.x, q.y), ids[j], g);
+    return dist2_packed(make_float2(-p.x, -p.y), q, e) <= kNudgeR2 && j != i &&
+           owns_pair(key, __ldg(ids + i), q, __ldg(ids + j), g);
 }
 
 // The pair term of one neighbour (r2 <= h2 known, not the particle itself):
@@ -1107,10 +1105,7 @@ __device__ __forceinline__ void relax_finish(int i, const RelaxArrays &A, const 
     A.kr_out[i] = make_uint2(k2, rank);
 }
 
-// What the masked walk does not take itself is out of line and runs to the end
-// of the particle's relaxation, so that nothing of the caller lives across the
-// call: compiled into the pass, or called for a part of the work, these paths
-// cost the masked walk its registers.
+// The end of a relaxation in a function of its own (relax_cold).
 template <bool PROBE>
 __device__ __forceinline__ void relax_end_cold(int i, const RelaxArrays &A, const Scene *S, float2 p,
                                                float2 acc, int nudges)
@@ -1123,10 +1118,38 @@ __device__ __forceinline__ void relax_end_cold(int i, const RelaxArrays &A, cons
     relax_finish(i, A, S, p, acc, nudges, nullptr);
 }
 
-// A particle whose walk (to the displacement acc) has met a pair that may be a
-// nudge: they are searched for again.
-template <bool PROBE>
-__device__ __noinline__ void relax_nudged(int i, const RelaxArrays &A, float2 acc)
+// The nudges of a particle whose walk has met a pair that may be one (r2 <=
+// 2e-12): such pairs are searched for again.  Hardly any particle has one,
+// but early in the dam break of 41,000 to 200,000 particles a step waits for
+// the warp of the one that does, and most of that wait is the fetch of code
+// that nothing else runs: so there is little of it (relax_update 20.5 us
+// with the search and the rest of the relaxation out of line, 14.3 so).
+template <bool LM>
+__device__ __forceinline__ int masked_nudges(int i, const RelaxArrays &A, const Scene *S, float2 p,
+                                             const int4 &rw)
+{
+    const SG g = load_grid(S);
+    const unsigned key = cell_key(p.x, p.y, g);
+    int nudges = 0;
+    // the rows' masks, then (LM) those of their candidates beyond kMaskRow
+#pragma unroll 1
+    for (int w = 0; w < (LM && rw.w == kRowsMasked2 ? 6 : 3); ++w) {
+        const int r = w < 3 ? w : w - 3;
+        const int base = (r == 0 ? rw.x : r == 1 ? rw.y : rw.z) + (w < 3 ? 0 : kMaskRow);
+        const unsigned long long *at = w >= 3 ? A.c.maskx + 3 * (size_t)i + r
+                                       : r < 2 ? &A.mask01[i].x + r : A.mask2 + i;
+#pragma unroll 1
+        for (unsigned long long m = __ldg(at); m; m &= m - 1ull) {
+            const int j = base + __ffsll(m) - 1;
+            const float4 q = __ldg(A.xr + j);
+            nudges += is_nudge(i, j, p, key, make_float2(q.x, q.y), g, A.ids);
+        }
+    }
+    return nudges;
+}
+
+// The same over the whole stencil, for particles without hit masks.
+__device__ __noinline__ int nudges_of(int i, const RelaxArrays &A)
 {
     const Scene *S = A.c.scenes + scene_of(A.c, i);
     const SG g = load_grid(S);
@@ -1140,10 +1163,10 @@ __device__ __noinline__ void relax_nudged(int i, const RelaxArrays &A, float2 ac
         for_each_candidate(key, A.start, g, capped, A.c.max_bucket, A.c.n, [&](int j) {
             const float4 q = __ldg(A.xr + j);
             float2 e;
-            const float r2 = dist2_packed(mp, make_float2(q.x, q.y), e);
-            if (r2 <= 2e-12f && r2 <= h2 && is_nudge(i, j, S, A.xr, A.ids)) ++nudges;
+            if (dist2_packed(mp, make_float2(q.x, q.y), e) <= h2)
+                nudges += is_nudge(i, j, p, key, make_float2(q.x, q.y), g, A.ids);
         });
-    relax_end_cold<PROBE>(i, A, S, p, acc, nudges);
+    return nudges;
 }
 
 // A particle whose rows have no hit masks (a row too long for them, or an
@@ -1215,10 +1238,7 @@ __device__ __noinline__ void relax_cold(int i, const RelaxArrays &A)
             });
         }
     }
-    if (rare)
-        relax_nudged<PROBE>(i, A, acc);
-    else
-        relax_end_cold<PROBE>(i, A, S, p, acc, 0);
+    relax_end_cold<PROBE>(i, A, S, p, acc, rare ? nudges_of(i, A) : 0);
 }
 
 // MARK: as in relax_cold.
@@ -1246,6 +1266,7 @@ __device__ __forceinline__ void relax_update_one(int i, const RelaxArrays &A,
     }
     const float2 p = make_float2(me.x, me.y);
     float2 acc = make_float2(0.0f, 0.0f);  // the displacement
+    int nudges = 0;
     bool net = false;
     if (LEARNED) {
         // the network's output requested with the count (not after it), and
@@ -1294,16 +1315,14 @@ __device__ __forceinline__ void relax_update_one(int i, const RelaxArrays &A,
             relax_cold<PROBE, MARK>(i, A);
             return;
         }
-        if (rare) {
-            relax_nudged<PROBE>(i, A, acc);
-            return;
-        }
+        if (rare) nudges = masked_nudges<LM>(i, A, S, p, rw);
     }
     if (PROBE) {
-        A.probe_out[i] = acc;
+        const float nd = (float)nudges * 0.000001f;
+        A.probe_out[i] = make_float2(acc.x + nd, acc.y + nd);
         return;
     }
-    relax_finish(i, A, S, p, acc, 0, tile_made);
+    relax_finish(i, A, S, p, acc, nudges, tile_made);
 }
 
 // 40 registers: 48 resident warps per SM instead of 32 (64 registers) for
@@ -1651,7 +1670,10 @@ __device__ __forceinline__ void relax_group_one(const Group<G> &g, int i, bool v
                 if (dist2_packed(mp, make_float2(q.x, q.y), e) <= rc.h2) {
                     bool rare = false;
                     apply = relax_pair_term(wc, p, q, s, d, rare);
-                    if (rare && is_nudge(i, j, S, xr, A.ids)) ++nudges;
+                    if (rare) {
+                        const SG sg = load_grid(S);
+                        nudges += is_nudge(i, j, p, cell_key(p.x, p.y, sg), make_float2(q.x, q.y), sg, A.ids);
+                    }
                 }
             }
             g.ordered(g.ballot(apply), [&](int src, bool on) {
