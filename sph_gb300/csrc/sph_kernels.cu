@@ -36,6 +36,16 @@ namespace sph {
 // the dam break's 1,048,576 particles lost 2-8% of the viscosity pass and the
 // other states stayed within 1%).
 constexpr int kShortRow = 32;
+// Handles of up to this many particles run the viscosity pass in the form that
+// marks and walks rows of up to kMaskRow candidates: with so few warps a pass
+// takes as long as its longest warp, and one of both short and long rows runs
+// the walk and then the loop over the long ones.  Steps of a dam break (early)
+// / a fluid at rest with rows of about 28, some above kShortRow / the same of
+// 18, one form and the other: 100,000 particles 67.7 and 59.1 us / 71.1 and
+// 60.0 / 43.7 and 45.4, 300,000 84.7 and 76.4 / 112 and 101 / 73.0 and 72.8,
+// 500,000 95.5 and 93.8 / 150 and 141 / 102.6 and 102.5, where larger handles
+// keep what compressed states of 4,194,304 particles gain by the loop.
+constexpr int kFewParticles = 300000;
 // Unroll factors of the candidate loops (tuned on GB300): the blocks of a
 // mark-then-walk scan (hit_mask32), and the single-phase loops of the density
 // and viscosity passes' long rows.
@@ -661,7 +671,9 @@ __device__ __noinline__ void viscosity_cold(int i, const ViscArrays &A)
 // I_ij = dt (1 - r/h)(sigma u + beta u^2) (x_j - x_i)/r for u > 0,
 // u = ((v_i - v_j).(x_j - x_i))/r, all from the velocities after gravity.
 // PROBE writes dv instead of advancing.
-template <bool PROBE>
+// FEW (kFewParticles): rows of up to kMaskRow candidates are marked and walked,
+// except in a warp that has a longer one and takes the loop for it anyway.
+template <bool PROBE, bool FEW>
 __device__ __forceinline__ void viscosity_predict_one(int i, const ViscArrays &A)
 {
     const Scene *S = A.c.scenes + scene_of(A.c, i);
@@ -675,26 +687,41 @@ __device__ __forceinline__ void viscosity_predict_one(int i, const ViscArrays &A
     if ((PROBE || A.st->lists_valid) && searchable(key, i, A.start, g, capped, A.c.max_bucket)) {
         int ra[3] = {0, 0, 0}, rl[3] = {0, 0, 0};
         if (!capped) stencil_rows(p, key, A.start, g, ra, rl, A.c.n);
-        if (!capped && max(rl[0], max(rl[1], rl[2])) <= kShortRow) {
+        const int longest = max(rl[0], max(rl[1], rl[2]));
+        int marked = kShortRow;
+        if (FEW && !__any_sync(__activemask(), longest > kMaskRow)) marked = kMaskRow;
+        if (!capped && longest <= marked) {
             // two phases: a cheap scan marks the neighbours of the stencil
             // rows, then only they pay for the impulse (less SIMT waste)
             const ViscConsts vc = visc_consts(S);
             const float2 mp = make_float2(-p.x, -p.y);
-            const unsigned b0 = hit_mask32<kMarkUnroll>(pos + ra[0], rl[0], mp, vc.h2);
-            const unsigned b1 = hit_mask32<kMarkUnroll>(pos + ra[1], rl[1], mp, vc.h2) &
-                                ~(1u << (i - ra[1]));  // not the particle itself
-            const unsigned b2 = hit_mask32<kMarkUnroll>(pos + ra[2], rl[2], mp, vc.h2);
-            walk_three<float4>(
-                b0, ra[0], b1, ra[1], b2, ra[2], A.c.n,
-                [&](int j) {
-                    const float2 q = __ldg(pos + j), w = __ldg(vel + j);
-                    return make_float4(q.x, q.y, w.x, w.y);
-                },
-                [&](int, const float4 &d) {
-                    float2 e;
-                    const float r2 = dist2_packed(mp, make_float2(d.x, d.y), e);
-                    visc_impulse(vc, e, r2, v0, make_float2(d.z, d.w), dv);
-                });
+            auto load = [&](int j) {
+                const float2 q = __ldg(pos + j), w = __ldg(vel + j);
+                return make_float4(q.x, q.y, w.x, w.y);
+            };
+            auto visit = [&](int, const float4 &d) {
+                float2 e;
+                const float r2 = dist2_packed(mp, make_float2(d.x, d.y), e);
+                visc_impulse(vc, e, r2, v0, make_float2(d.z, d.w), dv);
+            };
+            if (FEW) {
+                unsigned long long m[3];
+#pragma unroll
+                for (int r = 0; r < 3; ++r) {
+                    const float2 *row = pos + ra[r];
+                    const unsigned lo = hit_mask32<kMarkUnroll>(row, min(rl[r], 32), mp, vc.h2);
+                    const unsigned hi = hit_mask32<kMarkUnroll>(row + 32, max(rl[r] - 32, 0), mp, vc.h2);
+                    m[r] = (unsigned long long)hi << 32 | lo;
+                }
+                m[1] &= ~(1ull << (i - ra[1]));  // not the particle itself
+                walk_rows<float4>(m, ra, A.c.n, load, visit);
+            } else {
+                const unsigned b0 = hit_mask32<kMarkUnroll>(pos + ra[0], rl[0], mp, vc.h2);
+                const unsigned b1 = hit_mask32<kMarkUnroll>(pos + ra[1], rl[1], mp, vc.h2) &
+                                    ~(1u << (i - ra[1]));  // not the particle itself
+                const unsigned b2 = hit_mask32<kMarkUnroll>(pos + ra[2], rl[2], mp, vc.h2);
+                walk_three<float4>(b0, ra[0], b1, ra[1], b2, ra[2], A.c.n, load, visit);
+            }
         } else {
             viscosity_cold<PROBE>(i, A);
             return;
@@ -706,17 +733,31 @@ __device__ __forceinline__ void viscosity_predict_one(int i, const ViscArrays &A
 // 40 registers (48 resident warps per SM): 4,194,304 particles 189 -> 184 us
 // early in the dam break and 237 -> 230 us compressed against 48 registers,
 // 200 and 253 with 56.
-template <bool PROBE, bool PERSIST = false>
-__global__ void __maxnreg__(40)
-k_viscosity_predict(const __grid_constant__ ViscArrays A, unsigned *occ_reset)
+template <bool PROBE, bool PERSIST, bool FEW>
+__device__ __forceinline__ void viscosity_predict(const ViscArrays &A, unsigned *occ_reset)
 {
     pdl_enter();
     const int i0 = blockIdx.x * blockDim.x + threadIdx.x;
     if (!PROBE && i0 == 0) *occ_reset = 0u;
     for (int i = i0; i < A.c.n; i += gridDim.x * blockDim.x) {
-        viscosity_predict_one<PROBE>(i, A);
+        viscosity_predict_one<PROBE, FEW>(i, A);
         if (!PERSIST) break;
     }
+}
+
+template <bool PROBE, bool PERSIST = false>
+__global__ void __maxnreg__(40)
+k_viscosity_predict(const __grid_constant__ ViscArrays A, unsigned *occ_reset)
+{
+    viscosity_predict<PROBE, PERSIST, false>(A, occ_reset);
+}
+
+// 48 registers: no spills (40 and 64 take the same time, within 2%).
+template <bool PROBE, bool PERSIST = false>
+__global__ void __maxnreg__(48)
+k_viscosity_predict_few(const __grid_constant__ ViscArrays A, unsigned *occ_reset)
+{
+    viscosity_predict<PROBE, PERSIST, true>(A, occ_reset);
 }
 
 // ---------------------------------------------------------------------------
@@ -1520,7 +1561,7 @@ k_viscosity_group(const __grid_constant__ ViscArrays A, unsigned *occ_reset)
     const bool valid = th / G < A.c.n;
     const int i = valid ? th / G : A.c.n - 1;
     if (*A.occ_in > (unsigned)A.c.max_bucket) {  // overflowing buckets: the one-thread form
-        if (valid && g.gl == 0) viscosity_predict_one<false>(i, A);
+        if (valid && g.gl == 0) viscosity_predict_one<false, true>(i, A);
         return;
     }
     viscosity_group_one<G>(g, i, valid, A);
@@ -2080,8 +2121,10 @@ static void enqueue_predict_sort(sph_cuda *h, Mark &mark)
                         &st->build_max_occ[SLOT_PREDICTED]);
         });
     } else {
-        auto kv = h->shape[0].persistent ? k_viscosity_predict<false, true>
-                                         : k_viscosity_predict<false, false>;
+        auto kv = n <= kFewParticles ? (h->shape[0].persistent ? k_viscosity_predict_few<false, true>
+                                                               : k_viscosity_predict_few<false, false>)
+                                     : (h->shape[0].persistent ? k_viscosity_predict<false, true>
+                                                               : k_viscosity_predict<false, false>);
         launch_step(kv, gather_grid(h, h->shape[0]), h->shape[0].block, 0, h->stream, arrays,
                     &st->build_max_occ[SLOT_PREDICTED]);
     }
@@ -2444,7 +2487,7 @@ int launch_probe(sph_cuda *h, int which, void *scratch, float2 *out)
         else
             k_xr_density<<<nb, kBlock, 0, h->stream>>>(n, xr, sorted);
     } else {
-        k_viscosity_predict<true><<<nb, kBlock, 0, h->stream>>>(
+        (n <= kFewParticles ? k_viscosity_predict_few<true> : k_viscosity_predict<true>)<<<nb, kBlock, 0, h->stream>>>(
             ViscArrays{c, st, h->pos_a, h->vel_a, h->start_a, occ, nullptr, nullptr, nullptr, nullptr, sorted},
             nullptr);
     }
