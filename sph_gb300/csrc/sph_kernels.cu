@@ -1479,6 +1479,17 @@ struct Group {
     }
 };
 
+// Whether a group kernel shares its particles among lanes: where a cell is
+// populated enough for it (min_occ, from lanes_min_occ) and no bucket
+// overflows.  Else its first n threads take a particle each and the other
+// warps leave.
+template <class Arrays>
+__device__ __forceinline__ bool shared_by_lanes(const Arrays &A, unsigned min_occ)
+{
+    const unsigned occ = *A.occ_in;
+    return occ >= min_occ && occ <= (unsigned)A.c.max_bucket;
+}
+
 // Particle i's viscosity pass by the group (every lane of the warp calls it;
 // `valid` per group; no overflowing buckets).
 template <int G>
@@ -1552,18 +1563,18 @@ __device__ __forceinline__ void viscosity_group_one(const Group<G> &g, int i, bo
 
 template <int G>
 __global__ void __launch_bounds__(kBlock)
-k_viscosity_group(const __grid_constant__ ViscArrays A, unsigned *occ_reset)
+k_viscosity_group(const __grid_constant__ ViscArrays A, unsigned *occ_reset, unsigned min_occ)
 {
     pdl_enter();
     const int th = blockIdx.x * blockDim.x + threadIdx.x;
     if (th == 0) *occ_reset = 0u;
+    if (!shared_by_lanes(A, min_occ)) {
+        if (th < A.c.n) viscosity_predict_one<false, true>(th, A);
+        return;
+    }
     const Group<G> g;
     const bool valid = th / G < A.c.n;
     const int i = valid ? th / G : A.c.n - 1;
-    if (*A.occ_in > (unsigned)A.c.max_bucket) {  // overflowing buckets: the one-thread form
-        if (valid && g.gl == 0) viscosity_predict_one<false, true>(i, A);
-        return;
-    }
     viscosity_group_one<G>(g, i, valid, A);
 }
 
@@ -1630,17 +1641,17 @@ __device__ __forceinline__ void density_group_one(const Group<G> &g, int i, bool
 
 template <int G, bool LM>
 __global__ void __launch_bounds__(kBlock)
-k_density_group(const __grid_constant__ DensArrays A)
+k_density_group(const __grid_constant__ DensArrays A, unsigned min_occ)
 {
     pdl_enter();
     const int th = blockIdx.x * blockDim.x + threadIdx.x;
+    if (!shared_by_lanes(A, min_occ)) {
+        if (th < A.c.n) density_one<LM>(th, A);
+        return;
+    }
     const Group<G> g;
     const bool valid = th / G < A.c.n;
     const int i = valid ? th / G : A.c.n - 1;
-    if (*A.occ_in > (unsigned)A.c.max_bucket) {
-        if (valid && g.gl == 0) density_one(i, A);
-        return;
-    }
     density_group_one<G, LM>(g, i, valid, A);
 }
 
@@ -1733,18 +1744,18 @@ __device__ __forceinline__ void relax_group_one(const Group<G> &g, int i, bool v
 
 template <int G, bool LM>
 __global__ void __launch_bounds__(kBlock)
-k_relax_group(const __grid_constant__ RelaxArrays A, unsigned *occ_reset)
+k_relax_group(const __grid_constant__ RelaxArrays A, unsigned *occ_reset, unsigned min_occ)
 {
     pdl_enter();
     const int th = blockIdx.x * blockDim.x + threadIdx.x;
     if (th == 0) *occ_reset = 0u;
+    if (!shared_by_lanes(A, min_occ)) {
+        if (th < A.c.n) relax_update_one<false, false, LM>(th, A);
+        return;
+    }
     const Group<G> g;
     const bool valid = th / G < A.c.n;
     const int i = valid ? th / G : A.c.n - 1;
-    if (*A.occ_in > (unsigned)A.c.max_bucket) {
-        if (valid && g.gl == 0) relax_update_one<false>(i, A);
-        return;
-    }
     relax_group_one<G, LM>(g, i, valid, A);
 }
 
@@ -2070,27 +2081,38 @@ static const char *const kLearnedKernelNames[] = {
     "cell_starts_2",     "cell_scatter_2", "cell_permute_2"};
 static const int kLearnedStepKernels = 11;
 
-// Lanes per particle of gather k.  The lines lie where the times of the two
-// neighbouring choices cross (dam breaks, early and compressed): the fewer
-// the particles, the more lanes it takes to fill the GPU; beyond ~40,000 one
-// thread per particle fills it, and the shared form's votes and shuffles
-// cost more than they save (the relaxation, whose one-thread walk has the
-// least to do per neighbour, first).  Microseconds a step early / compressed,
-// one thread against this: 3,000 particles 90 / 89 against 36 / 37, 12,000 77
-// / 130 against 44 / 66, 30,000 79 / 139 against 55 / 88.  In a uniform fluid
-// of 4 neighbours a particle the lines would lie lower (30,000: 52 against 58,
-// 14,000: 49 against 46); 4 lanes up to 100,000 gain 10-15% in compressed dam
-// breaks and lose 25-30% there.  A launch shape other than the default asks
-// for the one-thread kernels.
-static int lanes_for(int n, int k)
+// Lanes per particle of a handle's gathers, for states dense enough
+// (lanes_min_occ): the fewer the particles, the more lanes it takes to fill
+// the GPU.  The lines lie where two neighbouring choices cross, in
+// microseconds a step of a dam break early / compressed: 32 and 16 lanes at
+// 5,000 particles 38.2 / 43.3 and 35.0 / 43.8, 16 and 8 at 10,000 40.7 / 58.4
+// and 39.5 / 65.2, 8 and one thread at 30,000 53.8 / 84.6 and 56 / 135, at
+// 55,000 73 / 117 and 54 / 136.
+static int lanes_for(int n)
 {
-    return n <= 5000 ? 32 : n <= 14000 ? 16 : n <= (k == 2 ? 30000 : 40000) ? 8 : 1;
+    return n <= 5000 ? 32 : n <= 11000 ? 16 : n <= 40000 ? 8 : 1;
 }
 
+// The largest cell population from which gather k shares a particle among
+// lanes: with one thread a particle a pass takes as long as its longest rows,
+// with lanes as long as there are particles.  Below it the lanes' votes and
+// shuffles cost more than the walk that they share, in the relaxation, which
+// does the least per neighbour, first.  Microseconds a step with 8 lanes
+// and with one thread a particle, 14,000 / 30,000 particles at rest with
+// a largest cell of 1 29.2 and 27.0 / 39.2 and 27.0, of 9 37.7 and 38.2 / 56.9
+// and 39.2, of 16 51.5 and 76 / 82.8 and 76; dam break, early (18) 41.5 and
+// 56 / 53.5 and 56, compressed (44) 70.4 and 132 / 84.8 and 135.
+static unsigned lanes_min_occ(int n, int k)
+{
+    constexpr int per[kGathers] = {1400, 2200, 800};
+    return (unsigned)((n + per[k] - 1) / per[k]);
+}
+
+// A launch shape other than the default asks for the one-thread kernels.
 static int gather_lanes(const sph_cuda *h, int k)
 {
     if (h->shape[k].block != kBlock || h->shape[k].persistent != 0) return 1;
-    return lanes_for(h->n, k);
+    return lanes_for(h->n);
 }
 
 // f(std::integral_constant<int, G>) for the G lanes of a group kernel.
@@ -2118,7 +2140,7 @@ static void enqueue_predict_sort(sph_cuda *h, Mark &mark)
     if (lanes > 1) {
         with_lanes(lanes, [&](auto G) {
             launch_step(k_viscosity_group<G.value>, blocks_for(n * G.value), kBlock, 0, h->stream, arrays,
-                        &st->build_max_occ[SLOT_PREDICTED]);
+                        &st->build_max_occ[SLOT_PREDICTED], lanes_min_occ(n, 0));
         });
     } else {
         auto kv = n <= kFewParticles ? (h->shape[0].persistent ? k_viscosity_predict_few<false, true>
@@ -2152,7 +2174,7 @@ static void enqueue_density(sph_cuda *h)
     if (lanes > 1) {
         with_lanes(lanes, [&](auto G) {
             launch_step(h->long_masks ? k_density_group<G.value, true> : k_density_group<G.value, false>,
-                        blocks_for(h->n * G.value), kBlock, 0, h->stream, arrays);
+                        blocks_for(h->n * G.value), kBlock, 0, h->stream, arrays, lanes_min_occ(h->n, 1));
         });
         return;
     }
@@ -2265,7 +2287,7 @@ static int enqueue_step_kernels(sph_cuda *h, cudaEvent_t *events, int *nkernels,
             with_lanes(lanes, [&](auto G) {
                 launch_step(h->long_masks ? k_relax_group<G.value, true> : k_relax_group<G.value, false>,
                             blocks_for(n * G.value), kBlock, 0, h->stream, relax_arrays(h),
-                            &st->build_max_occ[SLOT_RELAXED]);
+                            &st->build_max_occ[SLOT_RELAXED], lanes_min_occ(n, 2));
             });
         } else {
             auto kr = h->shape[2].persistent
@@ -2567,18 +2589,19 @@ k_static_keys(Ctx c, SG g, const float *__restrict__ x, const float *__restrict_
 
 template <int G>
 __global__ void __launch_bounds__(kBlock)
-k_density_static(const __grid_constant__ DensArrays A)
+k_density_static(const __grid_constant__ DensArrays A, unsigned min_occ)
 {
     pdl_enter();
     const int th = blockIdx.x * blockDim.x + threadIdx.x;
     if constexpr (G > 1) {
+        if (!shared_by_lanes(A, min_occ)) {
+            if (th < A.c.n) density_one<false, true>(th, A);
+            return;
+        }
         const Group<G> g;
         const bool valid = th / G < A.c.n;
         const int i = valid ? th / G : A.c.n - 1;
-        if (*A.occ_in <= (unsigned)A.c.max_bucket)
-            density_group_one<G, false, true>(g, i, valid, A);
-        else if (valid && g.gl == 0)
-            density_one<false, true>(i, A);
+        density_group_one<G, false, true>(g, i, valid, A);
     } else if (th < A.c.n) {
         density_one<false, true>(th, A);
     }
@@ -2621,13 +2644,14 @@ int launch_static_density(const Scene &sc, const StaticArrays &a, const float *x
                 (float2 *)nullptr, (DevState *)nullptr);
     const DensArrays arrays{c, a.pos_s, a.start, occ, nullptr, nullptr, nullptr, nullptr,
                             DensityById{a.id_s, rho, rho_near}};
-    const int lanes = lanes_for(n, 1);
+    const int lanes = lanes_for(n);
     if (lanes > 1) {
         with_lanes(lanes, [&](auto G) {
-            launch_step(k_density_static<G.value>, blocks_for(n * G.value), kBlock, 0, st, arrays);
+            launch_step(k_density_static<G.value>, blocks_for(n * G.value), kBlock, 0, st, arrays,
+                        lanes_min_occ(n, 1));
         });
     } else {
-        launch_step(k_density_static<1>, nb, kBlock, 0, st, arrays);
+        launch_step(k_density_static<1>, nb, kBlock, 0, st, arrays, 0u);
     }
     return cuda_fail(cudaGetLastError(), "sph_cuda_density_static launch");
 }
