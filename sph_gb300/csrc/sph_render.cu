@@ -22,6 +22,7 @@
 // The blur passes' texture-coordinate flips (liquid_gl.c:146-160 and
 // render_liquid_texture.vert) cancel in pairs and the kernel is symmetric,
 // so images are kept bottom row first until the final file order.
+#include <algorithm>
 #include <cmath>
 
 #include "sph_device.cuh"
@@ -67,8 +68,9 @@ __device__ __forceinline__ void splat_row(const Sprite &s, int y, int pitch, flo
 {
     const float inv = 1.0f / radius;
     const float dy = ((float)y + 0.5f - s.cy) * inv;
+    if (dy * dy > 0.34f) return;  // beside the disc: most rows of a sprite of a few texels
     // the row's span, a texel wider than the disc on either side
-    const float half = sqrtf(fmaxf(0.34f - dy * dy, 0.0f)) * radius + 1.0f;
+    const float half = sqrtf(0.34f - dy * dy) * radius + 1.0f;
     const int xa = max(s.x0, (int)floorf(s.cx - 0.5f - half));
     const int xb = min(s.x1, (int)ceilf(s.cx - 0.5f + half));
     unsigned *row = acc + (size_t)y * pitch;
@@ -106,7 +108,7 @@ __device__ __forceinline__ void splat_row(const Sprite &s, int y, int pitch, flo
 // two passes -- a sample of the particles, then the rest against the sample's
 // full blocks -- the interior of a fluid costs a few bit tests a particle.
 // 1,048,576 particles on 960 x 540 texels: 322 us in one pass with an atomic
-// per fragment, 54 us so.  More lanes in the second pass only send more
+// per fragment, 54 us so.  In a large second pass more lanes only send more
 // atomics to texels that are about to be full.
 constexpr int kBlk = 4;
 
@@ -285,8 +287,21 @@ k_composite(int W, int H, int w, int h, const unsigned char *__restrict__ a,
 
 int launch_pack(sph_cuda *h, short2 *out);
 
-// Particles from which the splat runs in two passes.
+// Particles from which the splat runs in two passes.  Microseconds an image
+// of a dam break (1,280 x 720 / 1,920 x 1,080 / 3,840 x 2,160) in one pass and
+// in two: 32,000 particles 68 and 65 / 92 and 95 / 240 and 260, 65,536 88 and
+// 62 / 120 and 95 / 265 and 262, 300,000 219 and 73 / 265 and 106 / 424 and
+// 272.  Spread evenly over the image, which leaves few blocks full, one pass is
+// up to a fifth faster below 1,000,000.
 constexpr int kSplatTwoPass = 65536;
+// Every how manieth particle the first pass takes: a sixteenth of them, down to
+// a sixty-fourth, about 16,384 in between, which fill what the fluid covers
+// (300,000 particles, 1,280 x 720: 73 us, a thirty-second 130).
+constexpr int kSampleMin = 16, kSampleMax = 64, kSampleSize = 16384;
+// Particles up to which the second pass takes them with four lanes, to have the
+// GPU filled (200,000, 1,920 x 1,080: 112 us with one, 101 with four; 500,000
+// 112 and 119).
+constexpr int kSplatFew = 400000;
 
 // The whole image from device coordinates; scratch (render_scratch bytes,
 // 256-byte aligned) holds the reduced textures.  *alpha is set to the blurred
@@ -335,15 +350,15 @@ static int render_alpha(cudaStream_t st, const short2 *coords, int n, int W, int
     auto blocks = [](long long k) { return (int)((k + 255) / 256); };
     // two passes where the particles are many enough for full blocks to be
     // likely and to pay for the two launches more
-    constexpr int kSample = 64;
     if (n >= kSplatTwoPass) {
-        const int first = (n + kSample - 1) / kSample;
-        launch_step(k_splat<8>, blocks((long long)first * 8), 256, 0, st, n, kSample, coords, w, h, radius,
+        const int step = std::max(kSampleMin, std::min(kSampleMax, n / kSampleSize));
+        const int first = (n + step - 1) / step, lanes = n <= kSplatFew ? 4 : 1;
+        launch_step(k_splat<8>, blocks((long long)first * 8), 256, 0, st, n, step, coords, w, h, radius,
                     lay.pitch, acc, (const unsigned *)nullptr, 0);
         launch_step(k_full_blocks, dim3((lay.words_x * 32 + 255) / 256, lay.blocks_y), 256, 0, st, w, h,
                     lay.pitch, (const unsigned *)acc, full, lay.words_x);
-        launch_step(k_splat<1>, blocks((long long)(n - first) * 1), 256, 0, st, n, kSample, coords, w, h, radius,
-                    lay.pitch, acc, (const unsigned *)full, lay.words_x);
+        launch_step(lanes > 1 ? k_splat<4> : k_splat<1>, blocks((long long)(n - first) * lanes), 256, 0, st, n,
+                    step, coords, w, h, radius, lay.pitch, acc, (const unsigned *)full, lay.words_x);
     } else if (n > 0) {
         launch_step(k_splat<8>, blocks((long long)n * 8), 256, 0, st, n, 1, coords, w, h, radius, lay.pitch, acc,
                     (const unsigned *)nullptr, 0);
