@@ -1903,21 +1903,26 @@ constexpr int kDiagPiece = 2048;
 // Per-scene FP64 sums, each scene cut into gridDim.y pieces (fixed order: the
 // pieces' sums are added in theirs by k_diag_scenes_final).  One block a
 // scene left the whole pass to the largest scene's block (64 scenes of 1,024
-// to 65,536 particles: 200 us, so 45 us).  The density records are in C order
-// and the velocities in A order; both keep every scene in its own slot range.
+// to 65,536 particles: 200 us, so 45 us).  Where no scene is large enough to
+// be cut its block writes the means itself (a call for two scenes of 2,048: 28
+// us, 30 with the second kernel).  The density records are in C order and the
+// velocities in A order; both keep every scene in its own slot range.
 __global__ void __launch_bounds__(kBlock)
 k_diag_scenes(Ctx c, const float4 *__restrict__ xr_c, const float2 *__restrict__ vel_a,
-              double *__restrict__ partials)
+              double *__restrict__ partials, double *__restrict__ out)
 {
+    pdl_enter();
     __shared__ double sh[3][kBlock / 32];
     const int s = blockIdx.x;
     const int s0 = __ldg(c.p_off + s), s1 = __ldg(c.p_off + s + 1);
     // at least kDiagPiece particles a block: the block's own reduction is FP64
     // arithmetic too, which is what this pass is made of
     const int piece = max(kDiagPiece, (s1 - s0 + (int)gridDim.y - 1) / (int)gridDim.y);
-    const int b0 = (int)min((long long)s1, s0 + (long long)blockIdx.y * piece), b1 = min(s1, b0 + piece);
+    const bool whole = gridDim.y == 1;
+    const int b0 = (int)min((long long)s1, s0 + (long long)blockIdx.y * piece), b1 = whole ? s1 : min(s1, b0 + piece);
+    double *const at = whole ? out + 3 * s : partials + 3 * ((size_t)s * gridDim.y + blockIdx.y);
     if (b0 >= s1) {
-        if (threadIdx.x < 3) partials[3 * ((size_t)s * gridDim.y + blockIdx.y) + threadIdx.x] = 0.0;
+        if (threadIdx.x < 3) at[threadIdx.x] = 0.0;
         return;
     }
     double a = 0.0, b = 0.0, k = 0.0;
@@ -1935,13 +1940,14 @@ k_diag_scenes(Ctx c, const float4 *__restrict__ xr_c, const float2 *__restrict__
     if (threadIdx.x < 3) {
         double t = 0;
         for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += sh[threadIdx.x][w];
-        partials[3 * ((size_t)s * gridDim.y + blockIdx.y) + threadIdx.x] = t;
+        at[threadIdx.x] = whole ? t / (s1 - s0) : t;
     }
 }
 
 __global__ void __launch_bounds__(kBlock)
 k_diag_scenes_final(Ctx c, int pieces, const double *__restrict__ partials, double *__restrict__ out)
 {
+    pdl_enter();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= 3 * c.nscenes) return;
     const int s = t / 3, q = t - 3 * s;
@@ -2469,8 +2475,11 @@ int launch_scene_diagnostics(sph_cuda *h, double *d_out, double *partials)
     if (h->nscenes == 0) return SPH_OK;
     const Ctx c = make_ctx(h);
     const int pieces = scene_diagnostic_pieces(h);
-    k_diag_scenes<<<dim3(h->nscenes, pieces), kBlock, 0, h->stream>>>(c, h->xr_c, h->vel_a, partials);
-    k_diag_scenes_final<<<blocks_for(3 * h->nscenes), kBlock, 0, h->stream>>>(c, pieces, partials, d_out);
+    launch_step(k_diag_scenes, dim3(h->nscenes, pieces), kBlock, 0, h->stream, c, (const float4 *)h->xr_c,
+                (const float2 *)h->vel_a, partials, d_out);
+    if (pieces > 1)
+        launch_step(k_diag_scenes_final, blocks_for(3 * h->nscenes), kBlock, 0, h->stream, c, pieces,
+                    (const double *)partials, d_out);
     return cuda_fail(cudaGetLastError(), "scene diagnostics");
 }
 
