@@ -64,7 +64,9 @@ int sph_learned_clear_samples(sph_learned_t *l);
  * (mean squared error, Adam, FP32 master weights).  Stage 2 (calibrate):
  * on the handle's current state, measures the density error each particle
  * gets from the network's displacement instead of the plain one and trains
- * the error output on it.  losses receive the last epoch's mean loss. */
+ * the error output on it.  losses receive the last epoch's mean loss.  The
+ * model keeps what a batch of up to 59,904 samples needs (64 MB at most) for
+ * its next training call; a larger batch's is freed when the call ends. */
 int sph_learned_train(sph_learned_t *l, int epochs, int batch, float lr, float *loss);
 int sph_learned_calibrate(sph_learned_t *l, sph_cuda_t *h, int epochs, float lr, float *loss);
 
@@ -75,7 +77,10 @@ int sph_learned_get_params(sph_learned_t *l, float *out);
 int sph_learned_set_params(sph_learned_t *l, const float *in);
 
 /* Network outputs for host feature rows (n x 32, FP32, converted to BF16):
- * out (n x 16, FP32).  For tests of the tensor-core kernels. */
+ * out (n x 16, FP32).  For tests of the tensor-core kernels.  Several
+ * host threads may call it on one model: the calls wait for one another, for an
+ * epoch of a training call and for set_params.  The model keeps staging buffers
+ * for its largest call so far, 50 MB at most. */
 int sph_learned_forward(sph_learned_t *l, const float *features, int n, float *out);
 
 /* Feature rows of the state handle h's next step relaxes (n x 32 FP32, by

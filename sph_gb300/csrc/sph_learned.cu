@@ -1353,6 +1353,10 @@ int ensure_forward(LearnedModel *l, int b, int rows)
     return SPH_OK;
 }
 
+// Tile images that a model keeps between training calls: 64 MB, a batch of
+// 59,904.
+constexpr int kKeptTiles = 468;
+
 // The training workspace for steps of `parts` CTAs and `rows` samples an epoch.
 int ensure_training(LearnedModel *l, int parts, int tiles, int rows)
 {
@@ -1416,6 +1420,18 @@ int train_loop(LearnedModel *l, int first, int nsamples, int epochs, int batch, 
     const int per_epoch = nsamples / batch;
     // a CTA per tile of 128 samples, at most one per SM
     const int parts = std::min(batch / 128, num_sms());
+    // tile images of large batches (143 KB for every 128 samples) are given
+    // back when the call ends, on every way out
+    struct Trim {
+        LearnedModel *l;
+        ~Trim()
+        {
+            if (l->img_cap <= kKeptTiles) return;
+            cudaFree(l->img);
+            l->img = nullptr;
+            l->img_cap = 0;
+        }
+    } trim{l};
     LTRY(ensure_training(l, parts, batch / 128, per_epoch * batch));
     double *d_loss = l->loss + l->parts_cap;
     std::vector<int> order(nsamples);
