@@ -266,11 +266,13 @@ int ensure_stage(sph_cuda *h, size_t bytes);
 // 65,536 particles 18.5 / 16 us, 262,144 23 / 27.  Feature rows up to
 // kInPlaceRows: 1,024 rows 43 / 26 us, 8,192 59 / 49, 16,384 78 / 86.  Images
 // up to kInPlaceImage: 1,280 x 720 of 262,144 particles 96 / 81 us, 1,920 x
-// 1,080 140 / 127, 3,840 x 2,160 (25 MB) 344 / 312.
+// 1,080 140 / 127, 3,840 x 2,160 (24 MB) 344 / 312, 3,840 x 2,720 (30 MB) 395 /
+// 356; arrays from 32 MB on are commonly new memory at every call, where the
+// copy is the faster: 725 / 800 (used again: 412 / 371).
 constexpr size_t kInPlaceBytes = (size_t)4 << 20;
 constexpr size_t kInPlacePack = (size_t)256 << 10;
 constexpr size_t kInPlaceRows = (size_t)1 << 20;
-constexpr size_t kInPlaceImage = (size_t)32 << 20;
+constexpr size_t kInPlaceImage = (size_t)30 << 20;
 void *host_in_place(const void *p, size_t bytes, size_t align, bool write);
 
 // Particles to upload, where a kernel reads them: arrays (vx, vy may be null:
