@@ -141,8 +141,8 @@ int sph_cuda_scene_diagnostics(sph_cuda_t *h, double *out);
  * per tile of particles or the number of resident blocks per SM for a
  * persistent grid-stride launch.  Any shape gives the same results.  At the
  * default shape {256, 0} a handle of at most 40,000 particles runs its
- * gathers with several lanes per particle; any other shape asks for one
- * thread per particle. */
+ * gathers with several lanes per particle while its cells are populated enough
+ * for it; any other shape asks for one thread per particle. */
 int sph_cuda_set_launch_shapes(sph_cuda_t *h, const int *shapes);
 int sph_cuda_get_launch_shapes(sph_cuda_t *h, int *shapes);
 
@@ -177,7 +177,9 @@ int sph_cuda_set_stream(sph_cuda_t *h, void *stream);
  * from the caller's pointer array and sorts them into cells.  Neighbour
  * lists start empty, as after fluid.c:202's calloc: the first step after an
  * upload has no viscosity impulses, exactly like the reference's first step.
- * Replaces initParticles' hand-off (fluid.c:238). */
+ * Replaces initParticles' hand-off (fluid.c:238).  This and the uploads below
+ * return once the caller's arrays have been read; the sort goes on in stream
+ * order, and an error in it is reported by a later call. */
 int sph_cuda_upload(sph_cuda_t *h, fluid_particle *const *particle_pointers, int n);
 
 /* Same, from a contiguous array (particles[i] has id i). */
@@ -192,7 +194,8 @@ int sph_cuda_upload_soa(sph_cuda_t *h, const float *x, const float *y, const flo
  * sequence fluid.c:273-348: apply_gravity, viscosity_impluses,
  * predict_positions, hash_fluid(.., true), double_density_relaxation,
  * updateVelocities, hash_fluid(.., false) -- with viscosity and relaxation as
- * deterministic gathers (Jacobi form).  Captured as one CUDA graph per step. */
+ * deterministic gathers (Jacobi form).  Captured as one CUDA graph per step;
+ * from the eighth call of four steps or more, four of them are one graph. */
 int sph_cuda_step(sph_cuda_t *h, const tunable_parameters *tp, int nsteps);
 
 /* Runs nsteps steps, step t using tps[t] (e.g. a moving mover); single scene. */
@@ -257,7 +260,8 @@ int sph_cuda_load_state(sph_cuda_t *h, const char *path);
 
 /* Rebuilds the neighbour relation on the current positions, like
  * hash_fluid(.., false) (fluid.c:341): after it, the next step applies
- * viscosity impulses even if it is the first step after an upload. */
+ * viscosity impulses even if it is the first step after an upload.  Returns
+ * once it is queued.  Refused while the handle's stream is being captured. */
 int sph_cuda_rebuild_neighbors(sph_cuda_t *h);
 
 /* Waits for all queued work of the handle. */
@@ -281,7 +285,9 @@ int sph_cuda_diagnostics(sph_cuda_t *h, double out[3]);
  * later particles of its own cell then the forward cells (0,+1), (+1,-1),
  * (+1,0), (+1,+1), each cell in id order, cut at max_neighbors.
  * counts[id] entries each, concatenated by id into ids (capacity max_total);
- * *total receives the number of entries. */
+ * *total receives the number of entries.  The handle keeps 8 bytes a particle
+ * and up to 64 MB for the entries (4 max_total, where that is less) as
+ * scratch. */
 int sph_cuda_neighbor_lists(sph_cuda_t *h, int *counts, int *ids, long long max_total,
                             long long *total);
 

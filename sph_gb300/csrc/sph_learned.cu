@@ -690,9 +690,10 @@ k_gemm(int M, int N, int K, const __nv_bfloat16 *__restrict__ A, long long sam, 
 //
 // The transposed operands of the backward products (W2, W3 by rows; the
 // activations, gradients and features as M x K with K over the samples) are
-// MN-major views of the very tiles the forward pass staged.  The same
-// arithmetic as the inference kernel in the same K order: the activations
-// are bit for bit its own.
+// MN-major views of the very tiles the forward pass staged.  The products are
+// those of the inference kernel in the same K order; the biases, which are
+// weights of its products, are added in FP32 here, so an activation may differ
+// from inference by a BF16 unit.
 constexpr int kTrainThreads = 512;
 constexpr uint32_t kTrainTmem = 128;
 constexpr uint32_t kColAcc = 0;  // tensor memory: the running product
