@@ -1537,18 +1537,19 @@ __device__ __forceinline__ void viscosity_group_one(const Group<G> &g, int i, bo
             float cx = 0.0f, cy = 0.0f;
             bool push = false;
             if (t < rl[r] && r2 <= h2 && r2 != 0.0f) {
-                // as viscosity_predict_one; a pair that does not approach
-                // (u <= 0) adds +-0 there and nothing here
+                // as visc_impulse: a pair that does not approach has u = 0 and
+                // adds +-0 there and nothing here (or a NaN in both, with
+                // tunables without bounds)
                 const float r_recip = rsqrtf(r2);
                 const float rr = r2 * r_recip;
                 const float2 dw = __fadd2_rn(v0, make_float2(-w.x, -w.y));
-                const float u = __fmaf_rn(dw.x, e.x, __fmul_rn(dw.y, e.y)) * r_recip;
-                push = u > 0.0f;
+                const float u = fmaxf(__fmaf_rn(dw.x, e.x, __fmul_rn(dw.y, e.y)) * r_recip, 0.0f);
                 const float imp = fmaf(-dt_h, rr, dt) * u * fmaf(beta, u, sigma);
                 const float2 m = __fmul2_rn(__fmul2_rn(make_float2(imp, imp), e),
                                             make_float2(r_recip, r_recip));
                 cx = clamp5(m.x);
                 cy = clamp5(m.y);
+                push = cx != 0.0f || cy != 0.0f;
             }
             g.ordered(g.ballot(push), [&](int src, bool on) {
                 const float sx = __shfl_sync(Group<G>::kFull, cx, src);

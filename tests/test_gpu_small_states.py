@@ -9,7 +9,7 @@ import pytest
 
 from conftest import bits_equal
 from sph_gb300 import Ensemble, Simulation, scenes
-from test_gpu_lanes import block
+from test_gpu_lanes import ONE_THREAD, block
 
 pytestmark = pytest.mark.gpu
 
@@ -58,3 +58,25 @@ def test_small_handles_equal_large_ones(cuda_lib, case, long_masks, max_bucket):
         pytest.skip("no overflowing bucket here; in the ensemble there is")
     for f in FIELDS:
         assert bits_equal(got[f], ref[f]), f
+
+
+@pytest.mark.parametrize("name", ["sigma", "beta", "k", "k_near", "k_spring", "g", "rest_density"])
+@pytest.mark.parametrize("value", [float("inf"), float("nan"), -1e38])
+def test_tunables_without_bounds(cuda_lib, name, value):
+    """An infinity or a NaN among the tunables reaches the same particles,
+    whether lanes share them or not."""
+    sc = block(3000, 0.4, 0.7)
+    rng = np.random.default_rng(4)
+    v = rng.uniform(-1.0, 1.0, (2, sc.n)).astype(np.float32)
+    P = dict(sc.params.as_dict(), **{name: value})
+    out = []
+    for shapes in (None, ONE_THREAD):
+        with Simulation.from_scene(sc) as s:
+            if shapes:
+                s.set_launch_shapes(shapes)
+            s.upload(sc.x, sc.y, *v)
+            s.rebuild_neighbors()
+            s.step(P, 1)
+            out.append(s.download())
+    for f in FIELDS:
+        assert np.array_equal(out[0][f], out[1][f], equal_nan=True), f
