@@ -1743,8 +1743,11 @@ __device__ __forceinline__ void relax_group_one(const Group<G> &g, int i, bool v
         relax_finish(i, A, S, p, acc, nudges, nullptr);
 }
 
+// Left to itself the compiler takes 64 registers and spills; 75 to 80 without
+// spills (frames of the dam break of 3,000 / 7,000 / 15,000 particles 134 ->
+// 132, 192 -> 188 and 261 -> 257 us; 86 with the long-row masks: 5% slower).
 template <int G, bool LM>
-__global__ void __launch_bounds__(kBlock)
+__global__ void __launch_bounds__(kBlock, G == 8 || LM ? 3 : 1)
 k_relax_group(const __grid_constant__ RelaxArrays A, unsigned *occ_reset, unsigned min_occ)
 {
     pdl_enter();
@@ -2090,29 +2093,32 @@ static const int kLearnedStepKernels = 11;
 
 // Lanes per particle of a handle's gathers, for states dense enough
 // (lanes_min_occ): the fewer the particles, the more lanes it takes to fill
-// the GPU.  The lines lie where two neighbouring choices cross, in
-// microseconds a step of a dam break early / compressed: 32 and 16 lanes at
-// 5,000 particles 38.2 / 43.3 and 35.0 / 43.8, 16 and 8 at 10,000 40.7 / 58.4
-// and 39.5 / 65.2, 8 and one thread at 30,000 53.8 / 84.6 and 56 / 135, at
-// 55,000 73 / 117 and 54 / 136.
+// the GPU.  The lines lie where two neighbouring choices cross over a dam
+// break, in microseconds a step early / compressed: 32 and 16 lanes at 5,000
+// particles 38.2 / 43.3 and 35.0 / 43.8, 16 and 8 at 12,500 45.2 / 66.5 and 41.5
+// / 70.7 (at step 200 50.7 and 59.7), 8 and one thread at 40,000 59.8 / 95.1
+// and 54.0 / 135, at 55,000 73 / 117 and 54 / 136.
 static int lanes_for(int n)
 {
-    return n <= 5000 ? 32 : n <= 11000 ? 16 : n <= 40000 ? 8 : 1;
+    return n <= 5000 ? 32 : n <= 14000 ? 16 : n <= 40000 ? 8 : 1;
 }
 
 // The largest cell population from which gather k shares a particle among
 // lanes: with one thread a particle a pass takes as long as its longest rows,
 // with lanes as long as there are particles.  Below it the lanes' votes and
 // shuffles cost more than the walk that they share, in the relaxation, which
-// does the least per neighbour, first.  Microseconds a step with 8 lanes
-// and with one thread a particle, 14,000 / 30,000 particles at rest with
-// a largest cell of 1 29.2 and 27.0 / 39.2 and 27.0, of 9 37.7 and 38.2 / 56.9
-// and 39.2, of 16 51.5 and 76 / 82.8 and 76; dam break, early (18) 41.5 and
-// 56 / 53.5 and 56, compressed (44) 70.4 and 132 / 84.8 and 135.
+// does the least per neighbour, first.  From a population whose rows may be
+// too long for a hit mask on the rows are longest by far, and lanes pay in
+// every handle that has them.  Microseconds a step with lanes and with one
+// thread a particle, 14,000 / 28,000 / 40,000 particles at rest with a largest
+// cell of 9 39.6 and 37.2 / 55.6 and 38.1 / 64.1 and 39.3, of 16 53.8 and 74.0 /
+// 78.7 and 74.0 / 97.5 and 78.2; dam break at step 40 (18) 41.8 and 53.0 / 50.6
+// and 52.7 / 59.8 and 54.0, at step 100 (28) 52.4 and 87.6 / 55.6 and 87.5 /
+// 63.7 and 89.2.
 static unsigned lanes_min_occ(int n, int k)
 {
     constexpr int per[kGathers] = {1400, 2200, 800};
-    return (unsigned)((n + per[k] - 1) / per[k]);
+    return (unsigned)std::min(kMaskRow / 3 + 1, (n + per[k] - 1) / per[k]);
 }
 
 // A launch shape other than the default asks for the one-thread kernels.

@@ -16,7 +16,7 @@ pytestmark = pytest.mark.gpu
 FIELDS = ("x", "y", "v_x", "v_y", "density", "density_near")
 # particles and lattice spacing: the fullest cell below and above the line of
 # each gather, rows of 32, 33 to 64 and more candidates, in one warp too
-CASES = [(700, 0.95), (5000, 0.5), (5001, 0.3), (11000, 0.34), (11001, 0.25), (20000, 0.3),
+CASES = [(700, 0.95), (5000, 0.5), (5001, 0.3), (11000, 0.34), (14000, 0.25), (14001, 0.25), (20000, 0.3),
          (40000, 0.22), (40000, 0.5), (40001, 0.24), (60001, 0.16)]
 
 
